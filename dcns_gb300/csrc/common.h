@@ -65,6 +65,32 @@ struct RecDesc {
   int32_t nduo, chunk, warm, pad;  // chunk = INT32_MAX: one tile per duo
 };
 
+// The seed-scan filter (scanfilter.cu).  A task is one warp: column tile rel / nch and row chunk rel % nch of a pair,
+// rel = task - task_begin; it leaves wpc words of 32 marks (16 rows each) per lane and half at
+// words[word_begin + (rel * wpc + word) * 64 + 32 * half + lane].  Pairs lie in the order of the level-0 table.
+constexpr int kFiltCols = 16;    // query columns per lane and half (a strip)
+constexpr int kFiltOverlap = 3;  // strips a system repeats of the one before: at least kScanW - 1 columns
+static_assert(kFiltOverlap * kFiltCols >= kScanW - 1, "a window's path must fit behind a system's first strips");
+struct FiltPair {
+  int64_t ref_base, qry_base, word_begin, duo_begin;
+  int32_t n1, n2, task_begin, nch, wpc, pad;
+};
+struct FiltDesc {
+  const FiltPair *pairs;
+  const int32_t *slot;  // pair -> place in `pairs`
+  uint32_t *words;
+  int32_t npairs, ntasks, chunk, warm;  // chunk: rows per row chunk; warm: the exact scan's warm-up rows
+};
+// Rows [rb, re) of level-0 duo b of pair slot a, or of task a: what the exact scan runs after the filter.
+struct FiltTile {
+  int32_t a, b, rb, re;
+};
+struct FiltTiles {
+  FiltTile *list;
+  int *count;  // tiles wanted (more than cap: the list is incomplete)
+  int32_t cap, rows;  // rows: the most a tile counts
+};
+
 // A level-0 window whose maximum reached min_score, compacted in task order.
 struct L0Rec {
   int32_t task, score, end1, end2, start1, start2;
@@ -172,6 +198,14 @@ void launch_scan(RecDesc d, int64_t ntiles, Arena ar, Params p, unsigned long lo
                  cudaStream_t st);
 void launch_scan_l0(L0Desc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter,
                     int64_t grid, cudaStream_t st);
+// The filter, its tile lists, and the exact scan over a tile list (level 0; a round's tasks).
+void launch_filter(const FiltDesc &D, Arena ar, Params p, int thr, cudaStream_t st);
+void launch_filter_plan_l0(const FiltDesc &D, L0Desc L, int64_t nduo, FiltTiles T, cudaStream_t st);
+void launch_filter_plan_rec(const FiltDesc &D, const ScanTask *tasks, int first, int n, FiltTiles T, cudaStream_t st);
+void launch_scan_tiles_l0(L0Desc d, FiltTiles T, Arena ar, Params p, unsigned long long *keys, int *work_counter,
+                          int grid, cudaStream_t st);
+void launch_scan_tiles_rec(RecDesc d, FiltTiles T, Arena ar, Params p, unsigned long long *keys, int *work_counter,
+                           int grid, cudaStream_t st);
 // Compacts the level-0 tasks whose maximum reached min_score (in task order) and runs their reverse scans.
 // scratch: >= (n0 / 256 + 2) ints.  Returns nothing; the count is written to *count (device).
 void launch_l0_select(const unsigned long long *keys, int64_t n0, const int64_t *wstart, const int2 *plen, int np,

@@ -37,12 +37,22 @@
 namespace dcns {
 
 // ------------------------------------------------------------------ buffers
+// Gives the seed-scan filter's buffers back (a call can do without them); true when there were any.
+static bool drop_filter(Context &C) {
+  if (C.d_fpairs.cap + C.d_fwords.cap + C.d_ftiles.cap == 0) return false;
+  if (C.st) cudaStreamSynchronize(C.st);  // what reads them is ordered before this stream's work
+  C.filt_on = false;
+  for (DevBuf *b : {&C.d_fpairs, &C.d_fwords, &C.d_ftiles}) b->release(C);
+  return true;
+}
+
 void DevBuf::ensure(Context &C, size_t bytes) {
   if (bytes <= cap) return;
   size_t want = std::max(bytes, cap + cap / 2);
   want = (want + 255) & ~size_t(255);
   if (C.used - cap + want > C.budget) {
     want = bytes;
+    if (C.used - cap + want > C.budget) drop_filter(C);
     if (C.used - cap + want > C.budget)
       throw Error(DCNS_ERR_NOMEM, "device memory budget exhausted (" + std::to_string(C.used - cap + want) +
                                       " > " + std::to_string(C.budget) + " bytes)");
@@ -54,6 +64,10 @@ void DevBuf::ensure(Context &C, size_t bytes) {
     cap = 0;
   }
   cudaError_t e = cudaMalloc(&p, want);
+  if (e == cudaErrorMemoryAllocation && drop_filter(C)) {
+    (void)cudaGetLastError();
+    e = cudaMalloc(&p, want);
+  }
   if (e != cudaSuccess) {
     p = nullptr;
     (void)cudaGetLastError();
@@ -92,7 +106,9 @@ void release_device_buffers(Context &C) {
   if (C.st) cudaStreamSynchronize(C.st);  // nothing of the context still reads them
   DevBuf *bufs[] = {&C.d_codes, &C.d_srcoff, &C.d_dstbase, &C.d_len, &C.d_pk, &C.d_nm, &C.d_seqbase, &C.d_flag,
                     &C.d_tasks, &C.d_keys, &C.d_tiles, &C.d_counter, &C.d_idx, &C.d_scratch, &C.d_x, &C.d_tb,
-                    &C.d_cig, &C.d_sg, &C.d_sgtb, &C.d_bnd, &C.d_wts, &C.d_cats};
+                    &C.d_cig, &C.d_sg, &C.d_sgtb, &C.d_bnd, &C.d_wts, &C.d_cats, &C.d_spill, &C.d_flow,
+                    &C.d_fpairs, &C.d_fwords, &C.d_ftiles};
+  C.filt_on = false;
   for (DevBuf *b : bufs) b->release(C);
 }
 
@@ -154,6 +170,7 @@ void init_context(Context &C, int device, size_t budget) {
   }
   if (const char *e = std::getenv("DCNS_XDROP_GROUP_FROM")) C.xdrop_group_from = std::max(0, std::atoi(e));
   if (const char *e = std::getenv("DCNS_SCAN_TILES")) C.scan_tiles_per_thread = std::max(1, std::min(64, std::atoi(e)));
+  if (const char *e = std::getenv("DCNS_SCAN_FILTER")) C.scan_filter = std::atoi(e) != 0;
   if (const char *e = std::getenv("DCNS_SG_WARPS")) {
     const int v = std::atoi(e);
     C.sg_warps = (v == 2 || v == 4 || v == kSgNW) ? v : 0;
@@ -467,6 +484,122 @@ int warmup_rows(const Params &P, int tw) {
   return tw + (P.match * tw + g - 1) / g + 4;
 }
 
+// The lowest value the filter's bound still has at the checked row at or after a cell of min_score.
+int filter_threshold(const Params &P) { return P.min_score + P.open1 + 2 * P.ext1; }
+
+// Whether the seed-scan filter pays.  It needs windows that overlap (step), scores that random sequence keeps low
+// (mismatches and gaps that cost what a match gains or more; a threshold of at least 12 matches: under the default
+// scoring, a threshold of 24 marks one 16 x 16 block in 5,000 by chance, the actual 32 one in 100,000), 16-bit room
+// for a row chunk's highest score, and a warm-up for the exact scan's tiles.
+bool filter_ok(const Params &P) {
+  const int K = warmup_rows(P, kScanW);
+  return fast_scan_ok(P) && P.step <= kScanW && P.mismatch <= -P.match && P.open1 <= -P.match &&
+         2 * P.ext1 <= -P.match && filter_threshold(P) >= 12 * P.match && P.min_score <= 16000 && K != INT_MAX &&
+         30000 / P.match >= 4 * K + 512;
+}
+
+// Filter tasks of pairs in level-0 order (order, nduo per pair): the table, the marks' words, and the buffers.
+// False: not now (the buffers do not fit the budget), scan every window instead.
+bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vector<int64_t> &order,
+                  const std::vector<int32_t> &nfast, const Params &P) {
+  const int64_t np = (int64_t)pairs.size();
+  const int K = warmup_rows(P, kScanW), fnew = 32 - kFiltOverlap;
+  auto ntile = [&](int64_t p) -> int64_t {
+    if (nfast[p] <= 0) return 0;
+    const int strips = (pairs[p].n2 + kFiltCols - 1) / kFiltCols;
+    const int sys = std::max(1, (strips - kFiltOverlap + fnew - 1) / fnew);
+    return (sys + 1) / 2;
+  };
+  int64_t rows = 0, tasks = 0;
+  for (int64_t p = 0; p < np; ++p) {
+    const int64_t t = ntile(p);
+    tasks += t;
+    rows += t * pairs[p].n1;
+  }
+  if (tasks == 0) return false;
+  // row chunks: none longer than 16-bit scores allow; shorter ones where there are too few tasks for the GPU
+  const int64_t limit = 30000 / P.match - K - 256, want = (int64_t)C.nsm * 20 * 8;
+  int64_t chunk = limit;
+  if (tasks < want) chunk = std::min(limit, std::max<int64_t>(2 * K, (rows + want - 1) / want));
+  std::vector<FiltPair> tab(np);
+  std::vector<int32_t> slot(np);
+  int64_t words = 0, duos = 0, task = 0;
+  for (int64_t q = 0; q < np; ++q) {
+    const int64_t p = order[q];
+    FiltPair &e = tab[q];
+    e.ref_base = C.seq_base[2 * p];
+    e.qry_base = C.seq_base[2 * p + 1];
+    e.word_begin = words;
+    e.duo_begin = duos;
+    e.n1 = pairs[p].n1;
+    e.n2 = pairs[p].n2;
+    e.task_begin = (int32_t)task;
+    const int64_t t = ntile(p);
+    e.nch = (int32_t)std::max<int64_t>(1, (e.n1 + chunk - 1) / chunk);
+    const int64_t steps = std::min<int64_t>(e.n1, chunk) + K + 49;
+    e.wpc = (int32_t)((steps + 511) / 512);
+    e.pad = 0;
+    slot[p] = (int32_t)q;
+    words += t * e.nch * e.wpc * 64;
+    duos += (nfast[p] + 1) / 2;
+    task += t * e.nch;
+  }
+  if (task >= INT32_MAX / 2) return false;
+  const int64_t cap = std::min<int64_t>(1 << 26, std::max<int64_t>(1 << 16, 4 * duos));
+  const size_t tb = sizeof(FiltPair) * np + sizeof(int32_t) * np + 256;
+  const size_t need = tb + sizeof(uint32_t) * words + sizeof(FiltTile) * cap;
+  const size_t have = C.d_fpairs.cap + C.d_fwords.cap + C.d_ftiles.cap;
+  if (need > have && C.used - have + 2 * need > C.budget) return false;
+  C.d_fpairs.ensure(C, tb);
+  C.d_fwords.ensure(C, sizeof(uint32_t) * words);
+  C.d_ftiles.ensure(C, sizeof(FiltTile) * cap);
+  if (!C.d_fpairs.cap || !C.d_fwords.cap || !C.d_ftiles.cap) return false;  // one made room for another
+  int32_t *d_slot = reinterpret_cast<int32_t *>(C.d_fpairs.as<FiltPair>() + np);
+  h2d(C, C.d_fpairs, tab.data(), (size_t)np);
+  DCNS_CK(cudaMemcpyAsync(d_slot, slot.data(), sizeof(int32_t) * np, cudaMemcpyHostToDevice, C.st));
+  C.filt = FiltDesc{C.d_fpairs.as<FiltPair>(), d_slot, C.d_fwords.as<uint32_t>(), (int32_t)np, (int32_t)task,
+                    (int32_t)chunk, K};
+  C.filt_on = true;
+  return true;
+}
+
+// The tile list for `items` duos or tasks; short tiles where there are few, so that they spread over the GPU.
+FiltTiles filter_tiles(Context &C, int64_t items, int *count) {
+  const int64_t cap = std::min<int64_t>(INT32_MAX, (int64_t)(C.d_ftiles.cap / sizeof(FiltTile)));
+  return FiltTiles{C.d_ftiles.as<FiltTile>(), count, (int32_t)cap,
+                   items >= (int64_t)C.nsm * C.scan_blocks_per_sm * kScanThreads ? 256 : 64};
+}
+
+// A round's scan through the filter's marks (tasks [first, first + n) are on the device), then the reverse scans and
+// the download.  False: the tile list was too short, and the keys hold only part of the maxima.
+bool run_filtered_round(Context &C, ScanState &S, const Params &P, int64_t first, int64_t n, int warm) {
+  auto tx = Clock::now();
+  const int64_t d0 = first - S.ns;
+  int *cnt = C.d_counter.as<int>();  // [0]: the scan's queue, [1]: tiles
+  const FiltTiles T = filter_tiles(C, n, cnt + 1);
+  DCNS_CK(cudaMemsetAsync(C.d_keys.as<unsigned long long>() + d0, 0, sizeof(unsigned long long) * n, C.st));
+  DCNS_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * 2, C.st));
+  const RecDesc D{nullptr, C.d_tasks.as<ScanTask>(), C.seqbase_dev, 0, INT32_MAX, warm, 0};
+  DCNS_CK(cudaEventRecord(C.ev0, C.st));
+  launch_filter_plan_rec(C.filt, C.d_tasks.as<ScanTask>(), (int)d0, (int)n, T, C.st);
+  launch_scan_tiles_rec(D, T, C.arena, P, C.d_keys.as<unsigned long long>(), cnt, C.nsm * C.scan_blocks_per_sm, C.st);
+  DCNS_CK(cudaEventRecord(C.ev1, C.st));
+  launch_reverse(C.d_tasks.as<ScanTask>(), (int)d0, (int)n, C.d_keys.as<unsigned long long>(), C.seqbase_dev,
+                 nullptr, C.arena, P, C.st);
+  C.stats.scan_launches += 1;
+  C.stats.kernel_launches += 3;
+  int tiles = 0;
+  DCNS_CK(cudaMemcpyAsync(&tiles, cnt + 1, sizeof(int), cudaMemcpyDeviceToHost, C.st));
+  d2h(C, S.tasks.data() + first, C.d_tasks, (size_t)n, (size_t)d0);
+  sync(C);
+  C.stats.scan_rounds += 1;
+  C.stats.ms_scan_xfer += ms_since(tx);
+  float ms = 0;
+  DCNS_CK(cudaEventElapsedTime(&ms, C.ev0, C.ev1));
+  C.stats.ms_scan_kernel += ms;
+  return tiles <= T.cap;
+}
+
 // Launches the scan over `tiles` plus the generic kernel over `generic` (device slots), then the reverse scans for
 // recursion tasks [first, first+n) (device slots first - ns ...); downloads those tasks.
 void run_scan_round(Context &C, ScanState &S, const Params &P, int64_t first, int64_t n, const RecDuo *duos,
@@ -542,6 +675,28 @@ void compute_scan_tasks(Context &C, ScanState &S, const Params &P) {
   auto t0 = Clock::now();
   auto tp = t0;
   const bool fast_ok = fast_scan_ok(P);
+  if (C.filt_on) {  // a round of windows under the filter (all of them short reads: the fast kernel's)
+    bool fast = true;
+    for (int64_t k = first; k < first + n; ++k) {
+      ScanTask &T = S.task(k);
+      T.striped = striped_for_host(T.hi - T.lo, T.tw, P.open1, P.ext1, P.match) ? 1 : 0;
+      fast &= T.striped && T.tw <= kScanW;
+    }
+    C.d_keys.ensure(C, sizeof(unsigned long long) * (S.size() - S.ns));
+    C.d_tasks.ensure(C, sizeof(ScanTask) * (S.size() - S.ns));
+    if (fast && C.filt_on) {  // still: the buffers above may have needed its room
+      C.stats.ms_scan_prep += ms_since(t0);
+      h2d(C, C.d_tasks, S.tasks.data() + first, (size_t)n, (size_t)(first - S.ns));
+      const bool done = run_filtered_round(C, S, P, first, n, warmup_rows(P, kScanW));
+      tp = phase(C, "sc_filtered", tp);
+      if (done) {
+        C.stats.ms_scan += ms_since(t0);
+        S.left.resize(S.size(), -1);
+        S.right.resize(S.size(), -1);
+        return;
+      }
+    }
+  }
   std::vector<int32_t> fast, generic;  // device slots
   for (int64_t k = first; k < first + n; ++k) {
     ScanTask &T = S.task(k);
@@ -659,6 +814,7 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
     cells += (int64_t)n1 * tws;
   }
   const int64_t n0 = wstart[np];
+  C.filt_on = false;
   S.tasks.clear();
   S.pbeg.assign(np + 1, 0);
   if (!fast_scan_ok(P)) {
@@ -741,11 +897,13 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   int2 *d_plen = reinterpret_cast<int2 *>(d_wst + np + 1);
   int *d_blk = reinterpret_cast<int *>(d_plen + np);
   int *d_count = C.d_counter.as<int>() + 1;
+  const bool filtered = C.scan_filter && filter_ok(P) && filter_setup(C, pairs, order, nfast, P);
+  const FiltTiles ft = filtered ? filter_tiles(C, nduo, C.d_counter.as<int>() + 2) : FiltTiles{};
   h2d(C, C.d_tiles, tab, (size_t)np);
   DCNS_CK(cudaMemcpyAsync(d_wst, wst, sizeof(int64_t) * (np + 1), cudaMemcpyHostToDevice, C.st));
   DCNS_CK(cudaMemcpyAsync(d_plen, plen, sizeof(int2) * np, cudaMemcpyHostToDevice, C.st));
   DCNS_CK(cudaMemsetAsync(C.d_keys.p, 0, sizeof(unsigned long long) * n0, C.st));
-  DCNS_CK(cudaMemsetAsync(C.d_counter.p, 0, sizeof(int) * 2, C.st));
+  DCNS_CK(cudaMemsetAsync(C.d_counter.p, 0, sizeof(int) * 3, C.st));
   L0Desc D{C.d_tiles.as<L0Pair>(), (int32_t)np, P.step, P.window, (int32_t)chunk, K, 0};
   // One thread per tile (not a persistent grid): blocks retire as they finish, so the short kernels of other lanes,
   // on higher-priority streams, are scheduled in between instead of waiting for the whole level-0 scan.
@@ -760,7 +918,18 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   DCNS_CK(cudaEventRecord(C.ev_bulk, C.st));
   DCNS_CK(cudaStreamWaitEvent(bulk, C.ev_bulk, 0));
   DCNS_CK(cudaEventRecord(C.ev0, bulk));
-  launch_scan_l0(D, ntiles, C.arena, P, C.d_keys.as<unsigned long long>(), C.d_counter.as<int>(), grid, bulk);
+  auto scan_all = [&](cudaStream_t on) {
+    launch_scan_l0(D, ntiles, C.arena, P, C.d_keys.as<unsigned long long>(), C.d_counter.as<int>(), grid, on);
+  };
+  if (filtered) {
+    launch_filter(C.filt, C.arena, P, filter_threshold(P), bulk);
+    launch_filter_plan_l0(C.filt, D, nduo, ft, bulk);
+    launch_scan_tiles_l0(D, ft, C.arena, P, C.d_keys.as<unsigned long long>(), C.d_counter.as<int>(),
+                         C.nsm * C.scan_blocks_per_sm, bulk);
+    C.stats.kernel_launches += 2;
+  } else {
+    scan_all(bulk);
+  }
   DCNS_CK(cudaEventRecord(C.ev1, bulk));
   DCNS_CK(cudaStreamWaitEvent(C.st, C.ev1, 0));
   if (C.l0_turn) {
@@ -771,13 +940,27 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   C.stats.scan_launches += 1;
   C.stats.scan_rounds += 1;
   C.stats.kernel_launches += 1;
-  launch_l0_select(C.d_keys.as<unsigned long long>(), n0, d_wst, d_plen, (int)np, C.seqbase_dev, C.arena, P, d_blk,
-                   d_count, C.d_tasks.as<L0Rec>(), C.nsm, C.st);
-  C.stats.kernel_launches += 4;
-  int nsel = 0;
-  DCNS_CK(cudaMemcpyAsync(&nsel, d_count, sizeof(int), cudaMemcpyDeviceToHost, C.st));
+  auto select = [&] {
+    launch_l0_select(C.d_keys.as<unsigned long long>(), n0, d_wst, d_plen, (int)np, C.seqbase_dev, C.arena, P, d_blk,
+                     d_count, C.d_tasks.as<L0Rec>(), C.nsm, C.st);
+    C.stats.kernel_launches += 4;
+  };
+  select();
+  int got[2] = {0, 0};  // windows selected, tiles the filter wanted
+  DCNS_CK(cudaMemcpyAsync(got, d_count, sizeof(got), cudaMemcpyDeviceToHost, C.st));
   tp = phase(C, "l0_launch", tp);
   sync(C);
+  if (filtered && got[1] > ft.cap) {  // marked nearly everywhere: every window against its whole reference after all
+    C.filt_on = false;
+    DCNS_CK(cudaMemsetAsync(C.d_counter.p, 0, sizeof(int) * 3, C.st));
+    scan_all(C.st);
+    select();
+    C.stats.scan_launches += 1;
+    C.stats.kernel_launches += 1;
+    DCNS_CK(cudaMemcpyAsync(got, d_count, sizeof(got), cudaMemcpyDeviceToHost, C.st));
+    sync(C);
+  }
+  const int nsel = got[0];
   tp = phase(C, "l0_sync", tp);
   C.h_tasks.ensure(sizeof(L0Rec) * std::max(nsel, 1));
   L0Rec *rec = C.h_tasks.as<L0Rec>();
@@ -1005,6 +1188,7 @@ void scan_and_link(Context &C, const std::vector<PairIn> &pairs, const Params &P
     if (nreq == 0) break;
     if (round > 100000) throw Error(DCNS_ERR_DEVICE, "seed recursion did not converge");
   }
+  C.filt_on = false;  // the marks are this call's sequences'
   C.stats.cells_scan += cells;
   C.stats.cells_scan_reverse += cells_rev;
   C.stats.tasks_scan += level0_tasks + visited_final;
@@ -2359,6 +2543,7 @@ void align_core(Context &C, const std::vector<PairIn> &pairs, const Params &P, i
         L.sg_flow = C.sg_flow;
         L.sg_flow_blocks = C.sg_flow_blocks;
         L.scan_tiles_per_thread = bt.scan_tiles;
+        L.scan_filter = C.scan_filter;
         L.call_t0 = C.call_t0;
         L.lane_id = l;
         L.trace = C.trace;
@@ -2456,6 +2641,7 @@ void smith_waterman_batch(Context &C, const std::vector<PairIn> &tasks, const Pa
   validate(P);
   const int64_t n = (int64_t)tasks.size();
   C.stats = dcns_stats{};
+  C.filt_on = false;
   if (n == 0) return;
   upload(C, tasks);
   ScanState S;
@@ -2572,6 +2758,7 @@ void sliding_window(Context &C, const int8_t *const *seqs, const int32_t *lens, 
                     double *score, int32_t *max_out) {
   validate(P);
   C.stats = dcns_stats{};
+  C.filt_on = false;
   if (n < 2) return;
   // pair k-1 = (other sequence k as the scanned "reference", sequence 0 as the windowed "read"),
   // as slidingWindowAlignment calls SmithWaterman(seq_i, refwindow, ...) (impl/slidingWindowAlignment.cpp:36)

@@ -106,6 +106,11 @@ struct Context {
   DevBuf d_codes, d_srcoff, d_dstbase, d_len, d_pk, d_nm, d_seqbase, d_flag;
   DevBuf d_tasks, d_keys, d_tiles, d_counter, d_idx, d_scratch;
   DevBuf d_x, d_tb, d_cig, d_sg, d_sgtb, d_bnd, d_wts, d_cats, d_spill, d_flow;
+  // the seed-scan filter's tables, marks and tile list (scanfilter.cu); `filt` describes the marks of the call's
+  // sequences while `filt_on`.  Buffers that later work needs the room of are given back (drop_filter).
+  DevBuf d_fpairs, d_fwords, d_ftiles;
+  FiltDesc filt{};
+  bool filt_on = false;
   const WeightSet *weights = nullptr;  // set during a weighted call
   // pinned staging
   HostBuf h_codes, h_misc, h_out, h_tasks, h_tiles;
@@ -145,6 +150,7 @@ struct Context {
   // seed-scan tiling target: reference rows are split into chunks while a launch has fewer tiles than this many per
   // resident thread (DCNS_SCAN_TILES)
   int scan_tiles_per_thread = 8;
+  bool scan_filter = true;  // DCNS_SCAN_FILTER=0: every window against its whole reference, as without the filter
   // per-bin x-drop pass forms and seed-scan tiling target chosen by the autotuner (empty: the values above for every
   // bin)
   struct BinTune {

@@ -1,0 +1,275 @@
+// Seed-scan filter: which rows of the reference can give a window of the query a Smith-Waterman maximum of at least
+// min_score.  The windows of the drivers overlap (38 columns every 8), so scanning each window by itself computes
+// every (reference, query) cell 4.75 times, and nine windows in ten never reach min_score.  The filter computes every
+// cell once, as an upper bound of the value any window's own DP can have there, and marks the places where the bound
+// reaches the threshold; the exact window scan (seedscan.cu) then runs only there.  Windows that stay below
+// min_score everywhere are never looked at again by the host, so what the filter leaves out cannot change a result.
+//
+// The bound.  a(i,j) = max(a(i-1,j-1) + s, q, 0), q = max(R(i-1,j), R(i,j-1)), R(i,j) = max(q + ext, a + open): a
+// local alignment over the whole query in which a gap may turn between the two directions without opening anew.  By
+// induction a is at least the H of any window's DP at (i,j), and R at least its E and F behind the cell.  A gap state
+// in common costs one operation a cell less than E and F apart (three add-max operations per two cells where the
+// exact scan takes four and a half), and lets through hardly more: a gap that turns once already costs open + ext.
+//
+// The check.  A cell with H >= T raises a(r,j) at every later row r by the vertical gap from it, so it is enough to
+// look at every fourth row for a >= T + open + 2 ext: a third of a maximum per four cells instead of per cell.
+//
+// The tile.  One warp computes two column systems (the int16x2 halves) of 32 strips of 16 columns over a run of
+// reference rows: lane l owns strip l of both systems and computes row t - l at step t, with the row's value to the
+// left (a + open and R of lane l - 1's last column) by __shfl_up_sync.  A window's path spans 38 columns, so a system
+// repeats the last three strips (48 columns) of the one before it and starts from zero there.  Reference rows before
+// and after the tile's own are computed as they come (they only raise the bound), so no step is guarded.  State and
+// scores take 48 registers and one 128-bit load from the warp's query profile per four columns; at 16 columns a lane
+// the two shuffles of a step cost 2 of its 70 instructions.
+//
+// Measured on the 10,000-pair batch (534 G cells over all windows, 112 G over the pairs; serialised launch times):
+// level 0 87 ms before, now 17.3 ms in the filter, 0.5 ms in its lists and 4.8 ms in the exact scan of the marked
+// rows; the recursion rounds, which reuse the marks, 12 ms before and 3.4 ms now.  The whole call: 143 to 71 ms; two
+// 200 kb pairs: 166 to 83 ms.  Bound: integer issue, as the exact scan.  References that are marked nearly everywhere
+// (tandem repeats against themselves) overflow the tile list and pay for the filter on top of the whole scan.
+#include <type_traits>
+
+#include "device_common.cuh"
+
+namespace dcns {
+
+namespace {
+
+constexpr int kFC = kFiltCols;               // columns per lane and half
+constexpr int kFNew = 32 - kFiltOverlap;     // strips of a system that no earlier system covers
+constexpr int kFWarps = 4;
+
+__device__ __forceinline__ uint32_t fpack2(int v) { return (uint32_t)(uint16_t)(int16_t)v * 0x00010001u; }
+
+// The pair with task_begin <= t.
+__device__ __forceinline__ int filt_pair_of(const FiltDesc &D, int t) {
+  int lo = 0, hi = D.npairs - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (D.pairs[mid].task_begin <= t)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  return lo;
+}
+
+struct Stream {  // a lane's reference symbols, sixteen at a time
+  const uint32_t *pk, *nm;
+  int64_t k;  // arena index of the next sixteen
+  __device__ __forceinline__ void load(uint32_t &w, uint32_t &n) {
+    if (k < 0) {  // the arena's first sequence: A's in the places before its first base
+      const int before = (int)-k;
+      w = before < 16 ? __ldg(pk) << (2 * before) : 0u;
+      n = before < 16 ? (__ldg(nm) << before) & 0xFFFFu : 0u;
+    } else {
+      const uint32_t a = __ldg(pk + (k >> 4)), b = __ldg(pk + (k >> 4) + 1);
+      w = __funnelshift_r(a, b, 2u * (uint32_t)(k & 15));
+      const uint32_t c = __ldg(nm + (k >> 5)), d = __ldg(nm + (k >> 5) + 1);
+      n = __funnelshift_r(c, d, (uint32_t)(k & 31)) & 0xFFFFu;
+    }
+    k += 16;
+  }
+};
+
+__global__ void __launch_bounds__(32 * kFWarps, 5)
+    filter_kernel(FiltDesc D, Arena ar, int open, int ext, int match, int mismatch, int thr) {
+  __shared__ uint4 prof_all[kFWarps][4 * (kFC / 4) * 32];
+  const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
+  const int t = blockIdx.x * kFWarps + wb;
+  if (t >= D.ntasks) return;  // whole warp
+  const FiltPair P = D.pairs[filt_pair_of(D, t)];
+  const int rel = t - P.task_begin, ct = rel / P.nch, ch = rel % P.nch;
+  uint4 *const prof = prof_all[wb];
+  const uint32_t open2 = fpack2(open), ext2 = fpack2(ext), nopen2 = fpack2(-open);
+  {
+    // profile: score - open of both halves' columns against A, C, G, T; columns past the query hold -16384
+    const int c0 = kFC * (2 * ct * kFNew + lane), c1 = c0 + kFC * kFNew;
+    uint32_t *const w32 = reinterpret_cast<uint32_t *>(prof);
+    for (int p = 0; p < kFC; ++p) {
+      const int a = c0 + p < P.n2 ? base_code(ar, P.qry_base + c0 + p) : -1;
+      const int b = c1 + p < P.n2 ? base_code(ar, P.qry_base + c1 + p) : -1;
+#pragma unroll
+      for (int sym = 0; sym < 4; ++sym) {
+        const int c = sym + (sym >> 1);
+        const int sa = a < 0 ? -16384 : score_of(c, a, match, mismatch) - open;
+        const int sb = b < 0 ? -16384 : score_of(c, b, match, mismatch) - open;
+        w32[((sym * (kFC / 4) + (p >> 2)) * 32 + lane) * 4 + (p & 3)] = (uint32_t)(uint16_t)sa | ((uint32_t)sb << 16);
+      }
+    }
+    __syncwarp();
+  }
+  const int rows0 = ch * D.chunk, rows1 = min(P.n1, rows0 + D.chunk);
+  const int rbeg = ch == 0 ? 0 : rows0 - D.warm;  // lane 0's row at step 0
+  const int nblk = (rows1 - rbeg + 31 + 3 + 15) / 16;
+  uint32_t *out = D.words + P.word_begin + (int64_t)rel * P.wpc * 64 + lane;
+  Stream str{ar.pk, ar.nm, P.ref_base + rbeg - lane};
+  uint32_t wcur, ncur, wnext, nnext;
+  str.load(wcur, ncur);
+
+  uint32_t Ga[kFC], Gb[kFC], R[kFC];  // a + open of the last row (two banks, as in the exact scan), R
+#pragma unroll
+  for (int p = 0; p < kFC; ++p) Ga[p] = open2, R[p] = open2;
+  uint32_t lastT = open2, dg = open2, mrun;
+  uint32_t acc0 = 0, acc1 = 0;
+  const uint32_t thr2 = fpack2(thr + open - 1);
+
+  // One step: Gi holds the lane's previous row, Go receives this one.
+  auto row = [&](uint32_t(&Gi)[kFC], uint32_t(&Go)[kFC], auto check, auto with_n) {
+    uint32_t upT = __shfl_up_sync(0xFFFFFFFFu, lastT, 1);
+    uint32_t left = __shfl_up_sync(0xFFFFFFFFu, R[kFC - 1], 1);
+    upT = lane == 0 ? open2 : upT;
+    left = lane == 0 ? open2 : left;
+    const uint4 *pr = prof + (wcur & 3u) * (kFC / 4 * 32) + lane;
+    const bool isn = decltype(with_n)::value && (ncur & 1u);
+    wcur >>= 2;
+    if (decltype(with_n)::value) ncur >>= 1;
+    uint32_t gd = dg;
+    uint4 q4 = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int p = 0; p < kFC; ++p) {
+      if ((p & 3) == 0) q4 = pr[(p >> 2) * 32];
+      uint32_t s = (p & 3) == 0 ? q4.x : (p & 3) == 1 ? q4.y : (p & 3) == 2 ? q4.z : q4.w;
+      if (decltype(with_n)::value) s = isn ? nopen2 : s;  // N scores 0 against everything
+      const uint32_t q = __vmaxs2(R[p], left);
+      const uint32_t a = __viaddmax_s16x2_relu(gd, s, q);
+      gd = Gi[p];
+      const uint32_t tv = __vadd2(a, open2);
+      left = __viaddmax_s16x2(q, ext2, tv);
+      R[p] = left;
+      Go[p] = tv;
+      if (decltype(check)::value && (p & 1)) mrun = __vimax3_s16x2(mrun, Go[p - 1], tv);
+    }
+    dg = upT;
+    lastT = Go[kFC - 1];
+  };
+  using Yes = std::true_type;
+  using No = std::false_type;
+  for (int blk = 0; blk < nblk; ++blk) {
+    str.load(wnext, nnext);
+    mrun = 0x80008000u;
+    if (!__any_sync(0xFFFFFFFFu, ncur != 0)) {
+#pragma unroll 1
+      for (int k = 0; k < 4; ++k) {
+        row(Ga, Gb, No{}, No{});
+        row(Gb, Ga, No{}, No{});
+        row(Ga, Gb, No{}, No{});
+        row(Gb, Ga, Yes{}, No{});
+      }
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < 8; ++k) {
+        row(Ga, Gb, No{}, Yes{});
+        row(Gb, Ga, Yes{}, Yes{});
+      }
+    }
+    wcur = wnext, ncur = nnext;
+    const uint32_t gt = __vcmpgts2(mrun, thr2);
+    const uint32_t bit = 1u << (blk & 31);
+    acc0 |= (gt & 0xFFFFu) ? bit : 0u;
+    acc1 |= (gt >> 16) ? bit : 0u;
+    if ((blk & 31) == 31 || blk == nblk - 1) {
+      out[0] = acc0;
+      out[32] = acc1;
+      out += 64;
+      acc0 = acc1 = 0;
+    }
+  }
+}
+
+// Calls emit(row_begin, row_end) for the runs of marked rows of columns [c_lo, c_hi) within rows [lo, hi), in row
+// order; runs closer than the exact scan's warm-up are one (the rows between them would be computed twice).
+template <class Emit>
+__device__ __forceinline__ void filt_runs(const FiltDesc &D, const FiltPair &P, int c_lo, int c_hi, int lo, int hi,
+                                          Emit emit) {
+  const int k0 = c_lo / kFC, k1 = (c_hi - 1) / kFC;
+  int cs = -1, ce = -1;
+  for (int ch = lo / D.chunk; ch <= (hi - 1) / D.chunk; ++ch) {
+    const int rbeg = ch == 0 ? 0 : ch * D.chunk - D.warm;
+    const int rlo = max(lo, ch * D.chunk), rhi = (int)min((int64_t)hi, (int64_t)(ch + 1) * D.chunk);
+    const int w0 = (rlo - rbeg) >> 9, w1 = min(P.wpc - 1, (rhi - 1 - rbeg + 31) >> 9);
+    for (int wi = w0; wi <= w1; ++wi) {
+      uint32_t v = 0;
+      int lmin = 31, lmax = 0;
+      for (int k = k0; k <= k1; ++k) {
+        const int sys = k >= kFiltOverlap ? (k - kFiltOverlap) / kFNew : 0, l = k - sys * kFNew;
+        const int64_t task = (int64_t)(sys >> 1) * P.nch + ch;
+        v |= __ldg(D.words + P.word_begin + (task * P.wpc + wi) * 64 + 32 * (sys & 1) + l);
+        lmin = min(lmin, l), lmax = max(lmax, l);
+      }
+      while (v) {
+        const int b = __ffs(v) - 1;
+        const int len = __ffs(~(v >> b)) - 1;  // ones from bit b on (-1: all 32)
+        const int nb = len < 0 ? 32 : len;
+        v = nb + b >= 32 ? 0u : v & (0xFFFFFFFFu << (b + nb));
+        const int a = max(rlo, rbeg + 512 * wi + 16 * b - lmax);
+        const int e = min(rhi, rbeg + 512 * wi + 16 * (b + nb) - lmin);
+        if (a >= e) continue;
+        if (cs >= 0 && a - D.warm <= ce) {
+          ce = max(ce, e);
+        } else {
+          if (cs >= 0) emit(cs, ce);
+          cs = a, ce = e;
+        }
+      }
+    }
+  }
+  if (cs >= 0) emit(cs, ce);
+}
+
+__device__ __forceinline__ void filt_emit(const FiltTiles &T, int a, int b, int rb, int re) {
+  const int n = (re - rb + T.rows - 1) / T.rows, per = (re - rb + n - 1) / n;
+  const int at = atomicAdd(T.count, n);
+  for (int k = 0; k < n; ++k)
+    if (at + k < T.cap) T.list[at + k] = FiltTile{a, b, rb + k * per, min(re, rb + (k + 1) * per)};
+}
+
+// Level-0 tiles: one thread per two windows of a pair (slot of the level-0 table, duo).
+__global__ void __launch_bounds__(256) filter_plan_l0_kernel(FiltDesc D, L0Desc L, int64_t nduo, FiltTiles T) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nduo) return;
+  int lo = 0, hi = D.npairs - 1;
+  while (lo < hi) {  // the pair whose duos hold t
+    const int mid = (lo + hi + 1) >> 1;
+    if (D.pairs[mid].duo_begin <= t)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  const FiltPair P = D.pairs[lo];
+  const int duo = (int)(t - P.duo_begin), last = min(2 * duo + 1, L.pairs[lo].nfast - 1);
+  const int c_lo = 2 * duo * L.step, c_hi = min(P.n2, last * L.step + L.window);
+  filt_runs(D, P, c_lo, c_hi, 0, P.n1, [&](int a, int b) { filt_emit(T, lo, duo, a, b); });
+}
+
+// Tiles of a round's tasks: one thread per task.
+__global__ void __launch_bounds__(256) filter_plan_rec_kernel(FiltDesc D, const ScanTask *__restrict__ tasks,
+                                                              int first, int n, FiltTiles T) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const ScanTask x = tasks[first + k];
+  if (x.tw <= 0 || x.hi <= x.lo) return;
+  const FiltPair P = D.pairs[D.slot[x.pair]];
+  filt_runs(D, P, x.s2, x.s2 + x.tw, x.lo, x.hi, [&](int a, int b) { filt_emit(T, first + k, 0, a, b); });
+}
+
+}  // namespace
+
+void launch_filter(const FiltDesc &D, Arena ar, Params p, int thr, cudaStream_t st) {
+  if (D.ntasks <= 0) return;
+  filter_kernel<<<(D.ntasks + kFWarps - 1) / kFWarps, 32 * kFWarps, 0, st>>>(D, ar, p.open1, p.ext1, p.match,
+                                                                            p.mismatch, thr);
+}
+
+void launch_filter_plan_l0(const FiltDesc &D, L0Desc L, int64_t nduo, FiltTiles T, cudaStream_t st) {
+  if (nduo <= 0) return;
+  filter_plan_l0_kernel<<<(unsigned)((nduo + 255) / 256), 256, 0, st>>>(D, L, nduo, T);
+}
+
+void launch_filter_plan_rec(const FiltDesc &D, const ScanTask *tasks, int first, int n, FiltTiles T,
+                            cudaStream_t st) {
+  if (n <= 0) return;
+  filter_plan_rec_kernel<<<(n + 255) / 256, 256, 0, st>>>(D, tasks, first, n, T);
+}
+
+}  // namespace dcns

@@ -9,7 +9,7 @@
 //                       thread's query profile in shared memory (a 128-bit load per four columns), fused add-max DPX
 //                       instructions for H, E, the merged H and the next F, and a three-way row maximum every second
 //                       column.  M = 1: level-0 tiles derived from the per-pair table; M = 2: recursion rounds from
-//                       the duo table
+//                       the duo table; M = 3, 4: level 0 and rounds over the rows the filter marked (scanfilter.cu)
 //   scan_generic_kernel int32 lanes, any window width, both reference semantics (striped / scalar); used where the
 //                       fast kernel's static int16 bound or width does not hold
 //   scan_generic_wave_kernel  the same semantics for one large task per warp (long reads: kernel-level calls)
@@ -132,6 +132,42 @@ __device__ __forceinline__ ScanTile l0_tile(const L0Desc &D, int64_t t) {
   return tl;
 }
 
+// Level-0 tile of the filter's list: rows [f.rb, f.re) of duo f.b of table slot f.a.
+__device__ __forceinline__ ScanTile l0_filtered_tile(const L0Desc &D, const FiltTile &f) {
+  const L0Pair P = D.pairs[f.a];
+  ScanTile tl;
+  tl.ref_base = P.ref_base;
+  tl.qry_base = P.qry_base;
+  for (int h = 0; h < 2; ++h) {
+    const int w = 2 * f.b + h;
+    const bool on = w < P.nfast;
+    const int s2 = w * D.step;
+    tl.s2[h] = on ? s2 : 0;
+    tl.tw[h] = on ? min(D.window, P.n2 - s2) : 0;
+    tl.lo[h] = 0;
+    tl.hi[h] = P.n1;
+    tl.task[h] = on ? (int32_t)(P.wstart + w) : -1;
+  }
+  tl.cnt_begin = f.rb;
+  tl.row_end = f.re;
+  tl.row_begin = max(0, f.rb - D.warm);
+  return tl;
+}
+
+// Tile of the filter's list for a round: rows [f.rb, f.re) of task f.a, alone in its tile.
+__device__ __forceinline__ ScanTile rec_filtered_tile(const RecDesc &D, const FiltTile &f) {
+  const ScanTask A = D.tasks[f.a];
+  ScanTile tl;
+  tl.ref_base = D.seqbase[2 * A.pair];
+  tl.qry_base = D.seqbase[2 * A.pair + 1];
+  tl.s2[0] = A.s2, tl.tw[0] = A.tw, tl.lo[0] = A.lo, tl.hi[0] = A.hi, tl.task[0] = f.a;
+  tl.s2[1] = 0, tl.tw[1] = 0, tl.lo[1] = A.lo, tl.hi[1] = A.hi, tl.task[1] = -1;
+  tl.cnt_begin = f.rb;
+  tl.row_end = f.re;
+  tl.row_begin = max(A.lo, f.rb - D.warm);
+  return tl;
+}
+
 // Tile t of a duo-described round (RecDesc).
 __device__ __forceinline__ ScanTile rec_tile(const RecDesc &D, int64_t t) {
   int lo = 0, hi = D.nduo - 1;
@@ -165,13 +201,14 @@ __device__ __forceinline__ ScanTile rec_tile(const RecDesc &D, int64_t t) {
   return tl;
 }
 
-// MODE 1: level-0 tiles from the per-pair table; MODE 2: round tiles from the duo table.
+// MODE 1: level-0 tiles from the per-pair table; MODE 2: round tiles from the duo table; MODE 3, 4: level-0 and round
+// tiles from the filter's list.
 constexpr int kProfGroups = (kScanW + 3) / 4;  // query columns in groups of four (one 128-bit shared load)
 constexpr int kProfSyms = 4;                   // reference symbols A, C, G, T (2-bit codes 0..3); N rows below
 constexpr size_t kProfBytes = sizeof(uint4) * kProfSyms * kProfGroups * kScanThreads;
 
 template <int W, int MODE>
-__global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc l0, int64_t ntiles,
+__global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc l0, FiltTiles ft, int64_t ntiles,
                                                    Arena ar, int open, int ext, int match, int mismatch,
                                                    unsigned long long *__restrict__ keys, int *__restrict__ counter) {
   // Score table per reference symbol (index = 2-bit code | N << 2): bytes 0..4 = s(ref, read code 0..4) - open,
@@ -202,10 +239,14 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc 
   const uint32_t open2 = pack2(open), ext2 = pack2(ext), fext2 = pack2(max(ext, open));
   const uint32_t open_lo = open2 & 0xFFFFu, open_hi = open2 & 0xFFFF0000u;
 
+  if (MODE >= 3) ntiles = *ft.count <= ft.cap ? *ft.count : 0;  // an incomplete list: the host scans everything
   for (;;) {
     const int t = atomicAdd(counter, 1);
     if (t >= ntiles) break;
-    const ScanTile tl = MODE == 1 ? l0_tile(l0, t) : rec_tile(rec, t);
+    const ScanTile tl = MODE == 1   ? l0_tile(l0, t)
+                        : MODE == 2 ? rec_tile(rec, t)
+                        : MODE == 3 ? l0_filtered_tile(l0, ft.list[t])
+                                    : rec_filtered_tile(rec, ft.list[t]);
 
     // Registers hold G = H + open (not H): then the diagonal term H + s is G + (s - open) from the table, the
     // horizontal candidate H + open is G itself, and H + open = max(F + open, Hpre + open) is one fused op.
@@ -363,14 +404,26 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc 
 void launch_scan(RecDesc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter, int grid,
                  cudaStream_t st) {
   if (ntiles <= 0) return;
-  scan_kernel<kScanW, 2><<<grid, kScanThreads, kProfBytes, st>>>(d, L0Desc{}, ntiles, ar, p.open1, p.ext1, p.match,
+  scan_kernel<kScanW, 2><<<grid, kScanThreads, kProfBytes, st>>>(d, L0Desc{}, FiltTiles{}, ntiles, ar, p.open1, p.ext1, p.match,
                                                                  p.mismatch, keys, work_counter);
 }
 
 void launch_scan_l0(L0Desc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter,
                     int64_t grid, cudaStream_t st) {
   if (ntiles <= 0) return;
-  scan_kernel<kScanW, 1><<<(unsigned)grid, kScanThreads, kProfBytes, st>>>(RecDesc{}, d, ntiles, ar, p.open1, p.ext1, p.match,
+  scan_kernel<kScanW, 1><<<(unsigned)grid, kScanThreads, kProfBytes, st>>>(RecDesc{}, d, FiltTiles{}, ntiles, ar, p.open1, p.ext1, p.match,
+                                                                 p.mismatch, keys, work_counter);
+}
+
+void launch_scan_tiles_l0(L0Desc d, FiltTiles T, Arena ar, Params p, unsigned long long *keys, int *work_counter,
+                          int grid, cudaStream_t st) {
+  scan_kernel<kScanW, 3><<<grid, kScanThreads, kProfBytes, st>>>(RecDesc{}, d, T, 0, ar, p.open1, p.ext1, p.match,
+                                                                 p.mismatch, keys, work_counter);
+}
+
+void launch_scan_tiles_rec(RecDesc d, FiltTiles T, Arena ar, Params p, unsigned long long *keys, int *work_counter,
+                           int grid, cudaStream_t st) {
+  scan_kernel<kScanW, 4><<<grid, kScanThreads, kProfBytes, st>>>(d, L0Desc{}, T, 0, ar, p.open1, p.ext1, p.match,
                                                                  p.mismatch, keys, work_counter);
 }
 
@@ -738,14 +791,15 @@ void launch_reverse(ScanTask *tasks, int first, int n, const unsigned long long 
 
 namespace dcns {
 // Resident blocks per SM of the fast scan kernel at 128 threads (sizes the persistent grid).
-// Opts both scan kernels in to their dynamic shared memory (above the 48 KB default) and returns the resident blocks
+// Opts the scan kernels in to their dynamic shared memory (above the 48 KB default) and returns the resident blocks
 // per SM.  Called once per context before any scan launch.
 int scan_occupancy_impl() {
   int nb = 0;
-  if (cudaFuncSetAttribute(scan_kernel<kScanW, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProfBytes) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(scan_kernel<kScanW, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProfBytes) !=
-          cudaSuccess) {
+  const auto opt_in = [](auto k) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProfBytes) == cudaSuccess;
+  };
+  if (!opt_in(scan_kernel<kScanW, 1>) || !opt_in(scan_kernel<kScanW, 2>) || !opt_in(scan_kernel<kScanW, 3>) ||
+      !opt_in(scan_kernel<kScanW, 4>)) {
     (void)cudaGetLastError();
     return 0;
   }
