@@ -140,8 +140,8 @@ struct SgTask {
   int64_t base1, base2;
   int32_t a1, a2, n1, n2;
   int32_t dir, want_codes;
-  int64_t tb_off;                      // byte offset of the direction-code store (want_codes)
-  int64_t tb_bytes;
+  int64_t tb_off;                      // byte offset of the direction codes (want_codes), or of the row checkpoints
+  int64_t ck_off;                      // the flow form: byte offset of the column checkpoints
   // outputs
   int32_t score, end1, end2, rows;     // end1/end2 1-based (-1 when none) ; rows evaluated
   int32_t status, ncig;
@@ -169,7 +169,12 @@ struct SgRec {
   int m, f1, f2;
 };
 
-// The stripe-flow form of the unweighted semi-global kernel (semiglobal.cu, sg_flow_kernel): per DP, its boundary
+// The same record as the stripe-flow form passes it between stripes, in one 128-bit store and load.
+struct __align__(16) SgCell {
+  int m, f1, f2, tag;  // tag: 1 + the stripe that wrote it (zero before the launch)
+};
+
+// The stripe-flow form of the semi-global kernel (semiglobal.cu, sg_flow_kernel): per DP, its boundary
 // row and the state of its in-order row evaluation; per launch, the DPs in queue order and their stripes as units.
 struct SgFlowDP {
   int64_t bnd_off;                  // the DP's boundary row: n2 + 2 records of SgFlow::bnd
@@ -180,11 +185,9 @@ struct SgFlowDP {
 struct SgFlow {
   SgTask *tasks;
   const int *idx;                   // queue order: DP q is tasks[idx[q]]
-  const int64_t *unit_begin;        // [n]: first unit (stripe) of DP q; DP q has max(1, stripes) units
   const int2 *order;                // [total_units]: (q, stripe) in hand-out order (each DP's stripes ascending)
   SgFlowDP *dps;                    // [n], queue order
-  SgRec *bnd;
-  int *prog;                        // [total_units]: columns of the unit's last row published (zero before launch)
+  SgCell *bnd;                      // boundary rows of the DPs without a path (tags zero before the launch)
   unsigned long long *unit_counter; // zero before launch
   int *err;                         // set to 1 when a wait ran out of iterations (zero before launch)
   int64_t total_units;
@@ -256,20 +259,21 @@ void launch_xdrop_cigar_pack(XTask *tasks, int n, const uint32_t *cig, uint32_t 
 void launch_semiglobal(SgTask *tasks, const int *idx, int n, Arena ar, Params p, uint8_t *tb, void *bnd,
                        int max_n2, int *work_counter, int grid, int nw, cudaStream_t st);
 int sg_ctas_per_sm(int nw);
-// codes: the DPs keep direction codes (every DP of a launch alike)
-// minb: 5 or 6 resident blocks per SM (the register budget of the kernel instantiation)
-void launch_semiglobal_flow(const SgFlow &f, Arena ar, Params p, uint8_t *tb, bool codes, int nsm, int minb,
-                            cudaStream_t st);
+// wt: the weighted DPs (null: the unweighted).  path: the DPs keep traceback checkpoints in tb (row checkpoints, zero
+// before the launch, and column checkpoints, at 16-byte offsets; every DP of a launch alike).  minb: 4, 5 or 6
+// resident blocks per SM (the register budget of the unweighted kernel's instantiation).
+void launch_semiglobal_flow(const SgFlow &f, Arena ar, Params p, const SgWeights *wt, uint8_t *tb, bool path, int nsm,
+                            int minb, cudaStream_t st);
 int64_t sg_flow_units(int n1, int n2, int w);  // stripe units of one DP in the flow form (at least 1)
 int64_t sg_flow_grid_warps(int nsm, int minb);  // warps of the flow kernel's persistent grid
+int64_t sg_ck_row_bytes(int n1, int n2, int w);  // checkpoints of one DP (multiples of 16): the rows between stripes,
+int64_t sg_ck_col_bytes(int n1, int n2, int w);  // and the columns between tiles
+void launch_sg_retrace(SgTask *tasks, const int *idx, int n, Arena ar, Params p, const SgWeights *wt, uint8_t *tb,
+                       uint32_t *cig, int nsm, cudaStream_t st);
 int64_t sg_bnd_bytes(int grid, int max_n2, int nw);
 // tb_bytes: size of the code store tb (the traceback reads nothing past it)
 void launch_sg_traceback(SgTask *tasks, const int *idx, int n, int bandwidth, const uint8_t *tb, int64_t tb_bytes,
-                         uint32_t *cig, cudaStream_t st, bool weighted_layout = false);
+                         uint32_t *cig, cudaStream_t st);
 int64_t sg_tb_bytes(int n1, int n2, int w);
-int64_t sgw_tb_bytes(int n1, int n2, int w);
-int64_t sgw_bnd_bytes(int warps, int max_n2);
-void launch_semiglobal_weighted(SgTask *tasks, const int *idx, int n, Arena ar, Params p, SgWeights wt, uint8_t *tb,
-                                void *bnd, int max_n2, int *work_counter, int warps, cudaStream_t st);
 
 }  // namespace dcns

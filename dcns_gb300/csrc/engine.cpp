@@ -178,7 +178,10 @@ void init_context(Context &C, int device, size_t budget) {
   if (const char *e = std::getenv("DCNS_SG_FLOW")) {
     C.sg_flow = std::atoi(e) != 0;
   }
-  if (const char *e = std::getenv("DCNS_SG_FLOW_BLOCKS")) C.sg_flow_blocks = std::atoi(e) == 6 ? 6 : 5;
+  if (const char *e = std::getenv("DCNS_SG_FLOW_BLOCKS")) {
+    const int v = std::atoi(e);
+    C.sg_flow_blocks = (v == 5 || v == 6) ? v : 4;
+  }
   if (const char *e = std::getenv("DCNS_BIN_RATIO")) C.bin_ratio = std::max(0.1, std::min(4.0, std::atof(e)));
   if (const char *e = std::getenv("DCNS_BINS_BY_SIZE")) C.bins_by_size = std::atoi(e) != 0;
 }
@@ -1667,34 +1670,40 @@ void run_semiglobal(Context &C, std::vector<SgTask> &G, const Params &P, bool wa
   const int64_t cap_bytes = std::max<int64_t>((int64_t)(free_budget / 2), (int64_t)64 << 20);
   int64_t k0 = 0;
   C.d_sg.ensure(C, sizeof(SgTask) * n);
-  // the stripe-flow form (unweighted DPs): per DP also its boundary row and flow state, per stripe a progress flag
-  const bool flow = W == nullptr && C.sg_flow;
+  // the stripe-flow form: per DP also its boundary row (DPs without a path) and flow state
+  const bool flow = W != nullptr || C.sg_flow;
+  auto ck_bytes = [&](const SgTask &g) {
+    return sg_ck_row_bytes(g.n1, g.n2, P.bandwidth) + sg_ck_col_bytes(g.n1, g.n2, P.bandwidth);
+  };
   auto flow_bytes = [&](const SgTask &g) -> int64_t {
-    return flow ? (int64_t)sizeof(SgRec) * (std::max(g.n2, 0) + 2) + (int64_t)sizeof(SgFlowDP) + 8 +
-                      12 * sg_flow_units(g.n1, g.n2, P.bandwidth)
+    return flow ? (want_codes ? 0 : (int64_t)sizeof(SgCell) * (std::max(g.n2, 0) + 2)) + (int64_t)sizeof(SgFlowDP) + 8 * sg_flow_units(g.n1, g.n2, P.bandwidth)
                 : 0;
   };
   while (k0 < n) {
-    int64_t bytes = 0, extra = 0, k1 = k0;
+    int64_t bytes = 0, rows = 0, extra = 0, k1 = k0;  // rows: of the bytes, the flow form's row checkpoints
     while (k1 < n) {
       const int64_t b =
-          !want_codes ? 0 : W ? sgw_tb_bytes(G[k1].n1, G[k1].n2, P.bandwidth) : sg_tb_bytes(G[k1].n1, G[k1].n2, P.bandwidth);
+          !want_codes ? 0 : flow ? ck_bytes(G[k1]) : sg_tb_bytes(G[k1].n1, G[k1].n2, P.bandwidth);
       const int64_t e = flow_bytes(G[k1]);
       if (k1 > k0 && bytes + extra + b + e > cap_bytes) break;
-      G[k1].tb_off = bytes;
-      G[k1].tb_bytes = b;
+      G[k1].tb_off = flow ? rows : bytes;
+      if (flow && want_codes) rows += sg_ck_row_bytes(G[k1].n1, G[k1].n2, P.bandwidth);
       G[k1].want_codes = want_codes ? 1 : 0;
       bytes += b;
       extra += e;
       ++k1;
     }
+    if (flow && want_codes)
+      for (int64_t q = k0, at = rows; q < k1; ++q) {
+        G[q].ck_off = at;
+        at += sg_ck_col_bytes(G[q].n1, G[q].n2, P.bandwidth);
+      }
     const int64_t m = k1 - k0;
     if (want_codes) C.d_sgtb.ensure(C, (size_t)std::max<int64_t>(bytes, 1));
-    // unweighted: the stripe flow (or, with sg_flow off, one CTA per DP); weighted: one warp per DP, 16 warps per SM.
-    // CTA shape of the unweighted CTA kernel: many DPs run two warps each (short DPs stop within a few stripes, and
+    // the stripe flow (or, with sg_flow off, one CTA per unweighted DP).  CTA shape of the CTA kernel: many DPs run two warps each (short DPs stop within a few stripes, and
     // more of them run at once); few DPs keep eight warps each for the stripes of long DPs
     const int nw = C.sg_warps > 0 ? C.sg_warps : (m >= (int64_t)C.nsm * 8 ? 2 : kSgNW);
-    const int grid = (int)std::min<int64_t>(m, W ? (int64_t)C.nsm * 16 : (int64_t)C.nsm * sg_ctas_per_sm(nw));
+    const int grid = (int)std::min<int64_t>(m, (int64_t)C.nsm * sg_ctas_per_sm(nw));
     int maxn2 = 1;
     for (int64_t q = k0; q < k1; ++q) maxn2 = std::max(maxn2, G[q].n2);
     C.d_counter.ensure(C, 64);
@@ -1713,18 +1722,16 @@ void run_semiglobal(Context &C, std::vector<SgTask> &G, const Params &P, bool wa
     SgFlow F{};
     if (flow) {
       // units (stripes) and boundary rows in queue order; flow state in one buffer:
-      // unit_begin | dps | order | prog | counters
-      std::vector<int64_t> ub((size_t)m);
+      // dps | order | counters
       std::vector<int32_t> nst((size_t)m);
       std::vector<SgFlowDP> dps((size_t)m);
       int64_t units = 0, brows = 0;
       for (int64_t q = 0; q < m; ++q) {
         const SgTask &g = G[idx[q]];
-        ub[q] = units;
         nst[q] = (int32_t)sg_flow_units(g.n1, g.n2, P.bandwidth);
         units += nst[q];
         dps[q] = SgFlowDP{brows, 0, 0, 0, -1, -1, 0, kOut, kOut};
-        brows += std::max(g.n2, 0) + 2;
+        if (!want_codes) brows += std::max(g.n2, 0) + 2;
       }
       // hand-out order: stripe-major within groups of consecutive DPs holding at least eight grid-fulls of units;
       // inside a group the DPs go by stripe count, most first, so the DPs that have a stripe s form a prefix
@@ -1748,35 +1755,33 @@ void run_semiglobal(Context &C, std::vector<SgTask> &G, const Params &P, bool wa
         if (u != units) throw Error(DCNS_ERR_DEVICE, "semi-global stripe order: unit count mismatch");
       }
       auto al = [](int64_t b) { return (b + 255) / 256 * 256; };
-      const int64_t o_dps = al(8 * m), o_ord = o_dps + al((int64_t)sizeof(SgFlowDP) * m);
-      const int64_t o_prog = o_ord + al(8 * units), o_cnt = o_prog + al(4 * units), total = o_cnt + 256;
+      const int64_t o_ord = al((int64_t)sizeof(SgFlowDP) * m), o_cnt = o_ord + al(8 * units), total = o_cnt + 256;
       C.d_flow.ensure(C, (size_t)total);
-      C.d_bnd.ensure(C, (size_t)(sizeof(SgRec) * brows));
+      C.d_bnd.ensure(C, (size_t)(sizeof(SgCell) * std::max<int64_t>(brows, 1)));
       char *base = static_cast<char *>(C.d_flow.p);
-      DCNS_CK(cudaMemcpyAsync(base, ub.data(), 8 * m, cudaMemcpyHostToDevice, C.st));
-      DCNS_CK(cudaMemcpyAsync(base + o_dps, dps.data(), sizeof(SgFlowDP) * m, cudaMemcpyHostToDevice, C.st));
+      DCNS_CK(cudaMemcpyAsync(base, dps.data(), sizeof(SgFlowDP) * m, cudaMemcpyHostToDevice, C.st));
       DCNS_CK(cudaMemcpyAsync(base + o_ord, order.data(), 8 * units, cudaMemcpyHostToDevice, C.st));
-      DCNS_CK(cudaMemsetAsync(base + o_prog, 0, (size_t)(total - o_prog), C.st));
+      DCNS_CK(cudaMemsetAsync(base + o_cnt, 0, 256, C.st));
+      // the stripes know each other's cells by their tags
+      if (want_codes)
+        DCNS_CK(cudaMemsetAsync(C.d_sgtb.p, 0, (size_t)rows, C.st));
+      else
+        DCNS_CK(cudaMemsetAsync(C.d_bnd.p, 0, (size_t)(sizeof(SgCell) * brows), C.st));
       F.tasks = C.d_sg.as<SgTask>();
       F.idx = C.d_idx.as<int>();
-      F.unit_begin = reinterpret_cast<const int64_t *>(base);
-      F.dps = reinterpret_cast<SgFlowDP *>(base + o_dps);
+      F.dps = reinterpret_cast<SgFlowDP *>(base);
       F.order = reinterpret_cast<const int2 *>(base + o_ord);
-      F.bnd = C.d_bnd.as<SgRec>();
-      F.prog = reinterpret_cast<int *>(base + o_prog);
+      F.bnd = C.d_bnd.as<SgCell>();
       F.unit_counter = reinterpret_cast<unsigned long long *>(base + o_cnt);
       F.err = reinterpret_cast<int *>(base + o_cnt + 8);
       F.total_units = units;
       F.n = (int)m;
     } else {
-      C.d_bnd.ensure(C, (size_t)(W ? sgw_bnd_bytes((grid + 3) / 4 * 4, maxn2) : sg_bnd_bytes(grid, maxn2, nw)));
+      C.d_bnd.ensure(C, (size_t)sg_bnd_bytes(grid, maxn2, nw));
     }
     DCNS_CK(cudaEventRecord(C.ev0, C.st));
-    if (W)
-      launch_semiglobal_weighted(C.d_sg.as<SgTask>(), C.d_idx.as<int>(), (int)m, C.arena, P, *W,
-                                 C.d_sgtb.as<uint8_t>(), C.d_bnd.p, maxn2, C.d_counter.as<int>(), grid, C.st);
-    else if (flow)
-      launch_semiglobal_flow(F, C.arena, P, C.d_sgtb.as<uint8_t>(), want_codes, C.nsm, C.sg_flow_blocks, C.st);
+    if (flow)
+      launch_semiglobal_flow(F, C.arena, P, W, C.d_sgtb.as<uint8_t>(), want_codes, C.nsm, C.sg_flow_blocks, C.st);
     else
       launch_semiglobal(C.d_sg.as<SgTask>(), C.d_idx.as<int>(), (int)m, C.arena, P, C.d_sgtb.as<uint8_t>(),
                         C.d_bnd.p, maxn2, C.d_counter.as<int>(), grid, nw, C.st);
@@ -1807,8 +1812,12 @@ void run_semiglobal(Context &C, std::vector<SgTask> &G, const Params &P, bool wa
       C.d_cig.ensure(C, sizeof(uint32_t) * std::max<int64_t>(cw, 1));
       h2d(C, C.d_sg, G.data(), (size_t)n);
       DCNS_CK(cudaEventRecord(C.ev0, C.st));
-      launch_sg_traceback(C.d_sg.as<SgTask>(), C.d_idx.as<int>(), (int)m, P.bandwidth, C.d_sgtb.as<uint8_t>(), bytes,
-                          C.d_cig.as<uint32_t>(), C.st, W != nullptr);
+      if (flow)
+        launch_sg_retrace(C.d_sg.as<SgTask>(), C.d_idx.as<int>(), (int)m, C.arena, P, W, C.d_sgtb.as<uint8_t>(),
+                          C.d_cig.as<uint32_t>(), C.nsm, C.st);
+      else
+        launch_sg_traceback(C.d_sg.as<SgTask>(), C.d_idx.as<int>(), (int)m, P.bandwidth, C.d_sgtb.as<uint8_t>(), bytes,
+                            C.d_cig.as<uint32_t>(), C.st);
       DCNS_CK(cudaEventRecord(C.ev1, C.st));
       C.stats.kernel_launches += 1;
       C.h_out.ensure(sizeof(uint32_t) * std::max<int64_t>(cw, 1));
@@ -1832,7 +1841,7 @@ void run_semiglobal(Context &C, std::vector<SgTask> &G, const Params &P, bool wa
   for (auto &g : G) {
     const int64_t cells = sg_band_cells(g.rows, P.bandwidth, g.n2);
     C.stats.cells_semiglobal += cells;
-    if (want_codes) C.stats.bytes_codes_sg += cells;
+    if (want_codes) C.stats.bytes_codes_sg += flow ? ck_bytes(g) : cells;
   }
   C.stats.ms_semiglobal += ms_since(t0);
 }
@@ -2402,19 +2411,19 @@ void autotune(Context &C, Batch &B, const Params &P, int mode) {
     for (int b = 0; b < nb; ++b) C.bin_tune[b].scan_tiles = bin_t[b];
   }
   if (mode == DCNS_MODE_TWO_GAP) {
-    // the stripe flow with 5 or 6 blocks per SM (-5, -6 below), or one CTA per DP with 2, 4 or 8 warps (0: by the
-    // number of DPs)
-    int best_w = -5;
+    // the stripe flow with 4, 5 or 6 blocks per SM (-4, -5, -6 below), or one CTA per DP with 2, 4 or 8 warps (0: by
+    // the number of DPs)
+    int best_w = -4;
     double best_w_ms = 1e300;
-    for (int nw : {-5, -6, 0, 2, 4, kSgNW}) {
+    for (int nw : {-4, -5, -6, 0, 2, 4, kSgNW}) {
       C.sg_flow = nw < 0;
-      C.sg_flow_blocks = nw == -6 ? 6 : 5;
+      C.sg_flow_blocks = nw < 0 ? -nw : 4;
       C.sg_warps = std::max(nw, 0);
       const double ms = std::min(run(best), run(best));
       if (best_w_ms == 1e300 || better(ms, best_w_ms)) best_w_ms = ms, best_w = nw;
     }
     C.sg_flow = best_w < 0;
-    C.sg_flow_blocks = best_w == -6 ? 6 : 5;
+    C.sg_flow_blocks = best_w < 0 ? -best_w : 4;
     C.sg_warps = std::max(best_w, 0);
   }
 }

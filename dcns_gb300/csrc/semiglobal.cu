@@ -11,12 +11,14 @@
 // the maximum and the reference's comparison bit at once.
 //
 // Two schedules of the stripes.  The batched path runs every stripe of every DP as an independent unit of one
-// persistent grid (sg_flow_kernel: a long DP spreads over as many warps as it has stripes).  The one-pair entry point
-// without allocation keeps a whole DP on one CTA whose warps take its stripes in turn on a barrier schedule
-// (sg_kernel), which needs only one CTA's boundary rows.
+// persistent grid (sg_flow_kernel: a long DP spreads over as many warps as it has stripes; the weighted drivers' DPs
+// too).  The one-pair entry point without allocation keeps a whole DP on one CTA whose warps take its stripes in turn
+// on a barrier schedule (sg_kernel), which needs only one CTA's boundary rows.
 //
-// Direction codes are one byte per cell (state 0..4 in bits 0-2, gap-continuation flags in bits 3-6): the reference's
-// traceback needs all seven bits to stay bit-exact.  Layout: stripe-major, then step, then lane, one 32-bit word per
+// A direction code is one byte per cell (state 0..4 in bits 0-2, gap-continuation flags in bits 3-6): the reference's
+// traceback needs all seven bits to stay bit-exact.  sg_kernel stores them for every cell; the flow's DPs store
+// checkpoints, and the traceback computes the codes again in the tiles its path goes through.  Layout of the stored
+// codes: stripe-major, then step, then lane, one 32-bit word per
 // lane and step holding its four rows, so the 32 lanes of a step write 128 consecutive bytes.  Cells the reference
 // never writes (outside the band and the band's last column) are never read: the traceback's bounds test returns 255
 // for them.
@@ -27,6 +29,7 @@
 // from the two values the DP left there.
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 
 #include "device_common.cuh"
 
@@ -324,26 +327,26 @@ void launch_semiglobal(SgTask *tasks, const int *idx, int n, Arena ar, Params p,
 
 // ------------------------------------------------------------------ stripes as a flow of independent warp units
 // The DPs of a launch are cut into their 128-row stripes (units), handed out by one atomic counter in the order of
-// SgFlow::order; every warp of a persistent grid takes the next unit, computes it with the per-cell code of sg_kernel
-// (same wavefront, same code layout), and takes the next.  The host orders the units stripe-major within groups of
-// consecutive DPs (queue order: largest DPs first): stripe 0 of every DP of the group, then stripe 1, ... so that
-// when a warp takes stripe s its stripe s - 1 has been running for a while, even when a few DPs of 200,000 rows make
-// up the whole launch (in DP order the late stripes of one long DP would wait for its wavefront to reach them).
-// Stripe s of a DP depends only
-// on stripe s - 1: the last row of s - 1 reaches s through the DP's boundary row in global memory (one row per DP:
-// stripe s reads a column before it overwrites it with its own last row, and s + 1 reads it only after s published
-// it), and s - 1 publishes how many columns of that row it has written (release / acquire per 32-column chunk).  So
-// a long DP runs on as many warps as it has stripes, each one chunk pair behind the stripe above it, instead of on
-// one CTA.  Each DP's stripes are handed out in increasing order and a stripe waits only on lower stripes of its own
-// DP, which are held by running warps, so the waits always end; each still has an iteration limit, after which the
-// warp flags a device error (SgFlow::err) and abandons the DP.
+// SgFlow::order; every warp of a persistent grid takes the next unit, computes it and takes the next.  The host orders
+// the units stripe-major within groups of consecutive DPs (queue order: largest DPs first): stripe 0 of every DP of
+// the group, then stripe 1, ... so that when a warp takes stripe s its stripe s - 1 has been running for a while, even
+// when a few DPs of 200,000 rows make up the whole launch (in DP order the late stripes of one long DP would wait for
+// its wavefront to reach them).  Stripe s of a DP depends only on stripe s - 1, whose last row reaches it through
+// global memory: one boundary row per DP (stripe s reads a column before it overwrites it with its own last row), or,
+// for DPs with a path, a row per stripe that stays as a checkpoint.  A boundary cell carries the number of the stripe
+// that wrote it, in the same 128-bit store, so the consumer sees by the cell itself that it is there: no fence, no
+// progress counter.  So a long DP runs on as many warps as it has stripes, each a few chunks behind the stripe above
+// it.  Each DP's stripes are handed out in increasing order and a stripe waits only on lower stripes of its own DP,
+// which are held by running warps, so the waits always end; each still has an iteration limit, after which the warp
+// flags a device error (SgFlow::err) and abandons the DP.
 //
 // Row-level decisions (running maximum, z-drop, non-positive row maximum) are taken in row order: after computing
 // stripe s, its warp waits until s - 1 is evaluated, evaluates its 128 rows from the DP's running state and
 // publishes it; the stripe whose rows stop the DP, or its last stripe, writes the DP's result.  Stripes computed past
-// the stop are abandoned at their next chunk (their codes lie past the DP's last row and are never read).
-// Iteration limit of every wait: each iteration is an L2 load and a ~200 ns sleep, so a wait gives up after about a
-// second or more; the longest legitimate wait (a stripe of 200,000 columns while its SM is shared) is some tens of ms.
+// the stop are abandoned at their next chunk (their checkpoints lie past the DP's last row and are never read).
+// Iteration limit of every wait: each iteration is an L2 load and a 100-200 ns sleep, so a wait gives up after about
+// a second or more; the longest legitimate wait (a stripe of 200,000 columns while its SM is shared) is some tens of
+// ms.
 constexpr int kSgSpin = 1 << 22;
 
 __device__ __forceinline__ int sg_ld_acquire(const int *p) {
@@ -358,6 +361,24 @@ __device__ __forceinline__ int sg_ld_relaxed(const int *p) {
   int v;
   asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
+}
+
+// A boundary cell and the tag that says which stripe wrote it, in one 128-bit access: the consumer of a column knows by
+// the tag that the values beside it are the ones it waits for, without a fence and a counter between the two.
+__device__ __forceinline__ void sg_st_cell(SgCell *p, int m, int f1, int f2, int tag) {
+  const uint64_t lo = (uint64_t)(uint32_t)m | (uint64_t)(uint32_t)f1 << 32;
+  const uint64_t hi = (uint64_t)(uint32_t)f2 | (uint64_t)(uint32_t)tag << 32;
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(lo),
+               "l"(hi)
+               : "memory");
+}
+__device__ __forceinline__ SgCell sg_ld_cell(const SgCell *p) {
+  uint64_t lo, hi;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+  return SgCell{(int)(uint32_t)lo, (int)(lo >> 32), (int)(uint32_t)hi, (int)(hi >> 32)};
 }
 
 // Waits until *flag >= need, or until *stop_flag != 0; every lane polls (one broadcast load).  Returns 1 when the
@@ -375,59 +396,192 @@ __device__ __forceinline__ int sg_wait_at_least(const int *flag, int need, const
 }
 
 constexpr int kSgFlowWarps = 4;  // warps per block of the flow kernel
+constexpr int kSgChunk = 16;      // steps between two looks at the stripe above
 
-// One cell of a flow stripe, branch-free: (aF1, aF2) = the vertical gap states of the cell above (kOut at the row's
-// last band column, which no row above has in its band or updates), dg = the diagonal cell.  Cells outside the band
-// leave kOut in M and both F, and reset the row's horizontal states to kOut (the reference starts a row with them
-// OUT); the band's last column takes the cell's maximum but leaves kOut in both F (its gap states are not updated,
-// and the row's horizontal states are not read again).  With CODES, *d gets the cell's direction code: the winning
-// state (priority order diag, F1, E1, F2, E2, a later state winning ties) and the four gap-continuation flags;
-// codes of cells outside the band or on its last column are never read by the traceback.
-template <bool CODES>
+// ---- traceback checkpoints
+// A DP whose path is wanted keeps no direction code per cell.  It keeps what is needed to compute any 128 x 128 tile
+// of itself again: the row above every stripe (M, F1, F2 by column, what the stripes pass to each other anyway) and,
+// for every stripe, each column that is a multiple of 128 (M and the two horizontal states behind it, by row): 28
+// bytes per 128 cells instead of one per cell, and a forward pass of 12 integer operations a cell instead of about
+// 26.  The traceback computes the tiles that its path goes through again, with codes, in shared memory.
+constexpr int kSgTile = 128;  // columns between two column checkpoints
+
+__host__ __device__ inline int64_t sg_ck_row_stride(int n2, int w) { return (n2 < 2 * (int64_t)w ? n2 : 2 * (int64_t)w) + 2; }
+__host__ __device__ inline int64_t sg_ck_cols(int n2, int w) {
+  const int64_t span = 2 * (int64_t)w + kSgRows;
+  return (n2 < span ? n2 : span) / kSgTile + 2;
+}
+__host__ __device__ inline int64_t sg_ck_stripes(int n1, int n2, int w) {
+  if (n1 <= 0 || n2 <= 0) return 0;
+  const int64_t n1_eff = n1 < (int64_t)n2 + w ? n1 : (int64_t)n2 + w;
+  return (n1_eff + kSgRows - 1) / kSgRows;
+}
+int64_t sg_ck_row_bytes(int n1, int n2, int w) {
+  return sg_ck_stripes(n1, n2, w) * sg_ck_row_stride(n2, w) * (int64_t)sizeof(SgCell);
+}
+int64_t sg_ck_col_bytes(int n1, int n2, int w) {
+  return sg_ck_stripes(n1, n2, w) * sg_ck_cols(n2, w) * 3 * kSgRows * (int64_t)sizeof(int);
+}
+
+// The row above stripe s as an array by column j (columns from jstart - 1 on exist).
+__device__ __forceinline__ SgCell *sg_ck_row(uint8_t *tb, const SgTask &T, int w, int s) {
+  const int jstart = max(kSgRows * s + 1 - w, 1);
+  return reinterpret_cast<SgCell *>(tb + T.tb_off) + (int64_t)s * sg_ck_row_stride(T.n2, w) - (jstart - 1);
+}
+// Column j (a multiple of kSgTile, at least jstart) of stripe s: M, then E1, then E2, each by row.
+__device__ __forceinline__ int *sg_ck_col(uint8_t *tb, const SgTask &T, int w, int s, int j) {
+  const int jstart = max(kSgRows * s + 1 - w, 1);
+  const int64_t q = (int64_t)s * sg_ck_cols(T.n2, w) + (j / kSgTile - jstart / kSgTile);
+  return reinterpret_cast<int *>(tb + T.ck_off) + q * 3 * kSgRows;
+}
+
+// ---- scoring of a lane's rows.  KIND 0: the same parameters everywhere; 1, 2: the weighted drivers with one or two
+// gap pieces (SemiGlobal_single_gap_penalty and SemiGlobal with weights, impl/sequenceAlignment3.cpp:1483-1890): row i
+// takes the category of its seq1 base for the substitution, the horizontal gap states and the z-drop, and the
+// category of the next base for the vertical gap states it leaves (a row at the end of seq1 keeps its own).
+__device__ __forceinline__ int sgw_cat(const SgTask &T, const int16_t *__restrict__ wt, int i) {
+  // category of DP row i (1-based): forward rows follow seq1 from a1, reverse rows go down from a1
+  const int64_t pos = T.dir == 0 ? (int64_t)T.a1 + i - 1 : (int64_t)T.a1 - (i - 1);
+  return wt[T.wbase + pos];
+}
+
+__device__ __forceinline__ int sgw_next_cat(const SgTask &T, const int16_t *__restrict__ wt, int i, int own) {
+  const int64_t pos = T.dir == 0 ? (int64_t)T.a1 + i : (int64_t)T.a1 - i;
+  return (pos < 0 || pos >= T.wlen) ? own : wt[T.wbase + pos];
+}
+
+template <int KIND>
+struct SgRowParams {  // one row's: horizontal and vertical gap pieces, substitution scores
+  int o1h, x1h, o2h, x2h, o1v, x1v, o2v, x2v, mt, mm;
+  __device__ __forceinline__ void load(const SgTask &T, const SgWeights &W, int i, bool live) {
+    const int rc = live ? sgw_cat(T, W.weights, i) : 0;
+    const int nc = live ? sgw_next_cat(T, W.weights, i, rc) : 0;
+    const int32_t *a = W.cats + 7 * rc, *b = W.cats + 7 * nc;
+    mt = __ldg(a), mm = __ldg(a + 1), o1h = __ldg(a + 2), x1h = __ldg(a + 3), o2h = __ldg(a + 4), x2h = __ldg(a + 5);
+    o1v = __ldg(b + 2), x1v = __ldg(b + 3), o2v = __ldg(b + 4), x2v = __ldg(b + 5);
+  }
+};
+template <>
+struct SgRowParams<0> {};
+
+// Scores of one row against a column, from the column's selector: byte 0..3 of `prof` is the score against the 2-bit
+// code 0..3, and a column N selects the zero bytes behind it; a row N has prof = 0 (Scorei: N scores 0).  A selector
+// repeats the byte's sign into the upper bytes.
+__device__ __forceinline__ uint32_t sg_selector(int code) {
+  const uint32_t k = code == 2 ? 4u : (uint32_t)(code - (code >> 1) + (code >> 2));  // 0 1 3 4 -> 0 1 2 3
+  return k == 4u ? 0x4444u : k | (k | 8u) * 0x1110u;
+}
+__device__ __forceinline__ uint32_t sg_profile(int ci, int match, int mismatch) {
+  if (ci == 2) return 0u;
+  uint32_t r = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) r |= (uint32_t)(uint8_t)(int8_t)(ci == k + (k >> 1) ? match : mismatch) << (8 * k);
+  return r;
+}
+__device__ __forceinline__ int sg_score(uint32_t prof, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(prof), "r"(0u), "r"(sel));
+  return (int)d;
+}
+template <int KIND>
+__device__ __forceinline__ int sg_row_score(uint32_t prof, const SgRowParams<KIND> &r, uint32_t sel) {
+  if constexpr (KIND == 0) {
+    return sg_score(prof, sel);
+  } else {  // prof: 1 in the byte of the row's own code, so the selected byte says match; categories score in 32 bits
+    const int same = sg_score(prof, sel);
+    return (prof == 0u || sel == 0x4444u) ? 0 : (same != 0 ? r.mt : r.mm);
+  }
+}
+
+// One cell: (aF1, aF2) = the vertical gap states of the cell above, dg = the diagonal cell, sc its score.  INSIDE:
+// the cell is in the band, off the band's last column.  Otherwise cells outside the band leave kOut in M and both F
+// and reset the row's horizontal states to kOut (the reference starts a row with them OUT).  The band's last column
+// takes no vertical gap from above; under KIND 0 it takes the cell's maximum but leaves kOut in both F (its gap
+// states are not updated, and the row's horizontal states are not read again), so that the row below reads kOut
+// there by itself; the weighted DPs update every column and drop the states on reading.  With CODES, *d gets the
+// cell's direction code: the winning state (priority order diag, F1, E1, F2, E2, a later state winning ties) and the
+// four gap-continuation flags; codes of cells outside the band are never read by the traceback, nor is the last
+// column's under KIND 0.
+template <bool CODES, int KIND, bool INSIDE>
 __device__ __forceinline__ int sg_cell(int sc, int dg, int aF1, int aF2, int &e1, int &e2, bool valid, bool last,
-                                       int o1, int x1, int o2, int x2, int &cF1, int &cF2, uint32_t *d) {
-  int v = sc + dg, nF1, nF2, nE1, nE2;
-  if (CODES) {
-    bool pr;
+                                       const SgRowParams<KIND> &r, const Params &P, int &cF1, int &cF2, uint32_t *d) {
+  int o1h, x1h, o2h, x2h, o1v, x1v, o2v, x2v;
+  if constexpr (KIND == 0) {
+    o1h = o1v = P.open1, x1h = x1v = P.ext1, o2h = o2v = P.open2, x2h = x2v = P.ext2;
+  } else {
+    o1h = r.o1h, x1h = r.x1h, o2h = r.o2h, x2h = r.x2h, o1v = r.o1v, x1v = r.x1v, o2v = r.o2v, x2v = r.x2v;
+    if (!INSIDE && last) aF1 = kOut, aF2 = kOut;
+  }
+  int v, nF1, nF2 = kOut, nE1, nE2 = kOut;
+  if constexpr (CODES) {
+    bool pr, p1, p2, p3 = false, p4 = false;
     uint32_t c = 0;
-    v = __vibmax_s32(aF1, v, &pr);  // pr: !(v > F1)
+    v = __vibmax_s32(aF1, sc + dg, &pr);  // pr: !(v > F1)
     c = pr ? 1u : c;
     v = __vibmax_s32(e1, v, &pr);
     c = pr ? 2u : c;
-    v = __vibmax_s32(aF2, v, &pr);
-    c = pr ? 3u : c;
-    v = __vibmax_s32(e2, v, &pr);
-    c = pr ? 4u : c;
-    const int h = v + o1, h2 = v + o2;
-    bool p1, p2, p3, p4;
-    nF1 = __vibmax_s32(aF1 + x1, h, &p1);
-    nE1 = __vibmax_s32(e1 + x1, h, &p2);
-    nF2 = __vibmax_s32(aF2 + x2, h2, &p3);
-    nE2 = __vibmax_s32(e2 + x2, h2, &p4);
+    if constexpr (KIND != 1) {
+      v = __vibmax_s32(aF2, v, &pr);
+      c = pr ? 3u : c;
+      v = __vibmax_s32(e2, v, &pr);
+      c = pr ? 4u : c;
+      nF2 = __vibmax_s32(aF2 + x2v, v + o2v, &p3);
+      nE2 = __vibmax_s32(e2 + x2h, v + o2h, &p4);
+    }
+    nF1 = __vibmax_s32(aF1 + x1v, v + o1v, &p1);
+    nE1 = __vibmax_s32(e1 + x1h, v + o1h, &p2);
     *d = c | (p1 ? 8u : 0u) | (p2 ? 16u : 0u) | (p3 ? 32u : 0u) | (p4 ? 64u : 0u);
   } else {
-    v = __vimax3_s32(__vimax3_s32(v, aF1, e1), aF2, e2);
-    nF1 = __viaddmax_s32(aF1, x1, v + o1);
-    nE1 = __viaddmax_s32(e1, x1, v + o1);
-    nF2 = __viaddmax_s32(aF2, x2, v + o2);
-    nE2 = __viaddmax_s32(e2, x2, v + o2);
+    v = __viaddmax_s32(dg, sc, aF1);
+    if constexpr (KIND != 1) {
+      v = max(__vimax3_s32(v, e1, aF2), e2);
+      nF2 = __viaddmax_s32(aF2, x2v, v + o2v);
+      nE2 = __viaddmax_s32(e2, x2h, v + o2h);
+    } else {
+      v = max(v, e1);
+    }
+    nF1 = __viaddmax_s32(aF1, x1v, v + o1v);
+    nE1 = __viaddmax_s32(e1, x1h, v + o1h);
   }
-  const bool upd = valid && !last;
-  cF1 = upd ? nF1 : kOut;
-  cF2 = upd ? nF2 : kOut;
-  e1 = valid ? nE1 : kOut;
-  e2 = valid ? nE2 : kOut;
-  return valid ? v : kOut;
+  if constexpr (INSIDE) {
+    cF1 = nF1, cF2 = nF2, e1 = nE1, e2 = nE2;
+    return v;
+  } else {
+    const bool upd = valid && (KIND != 0 || !last);
+    cF1 = upd ? nF1 : kOut;
+    cF2 = upd ? nF2 : kOut;
+    e1 = valid ? nE1 : kOut;
+    e2 = valid ? nE2 : kOut;
+    return valid ? v : kOut;
+  }
 }
 
-// MINB: resident blocks per SM the register allocation must allow (5: 96 registers; 6: 80, a few spilled words)
-template <bool CODES, int MINB>
-__global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow F, Arena ar, Params P,
+// A column of the row above, as a lane-0 cell reads it, with the column's selector in the place of the padding.
+struct __align__(16) SgFeed {
+  int m, f1, f2;
+  uint32_t sel;
+};
+
+// CK: the DPs keep traceback checkpoints.  MINB: resident blocks per SM the register allocation must allow.
+//
+// Steps run in chunks of 16.  A chunk whose columns lie inside the band of every row of the stripe, off the band's
+// last column and the stale column, takes the cell without any band test (9 of 22 operations): under the default band
+// of 20,000 all but the first two and the last of a stripe.
+//
+// Bound: integer issue (ALU pipe at 59 %, issue slots at 55 %) where there are many DPs, and the chain of stripes (a
+// stripe starts 31 + 3 chunks + the band's 128 columns of steps after the one above) where there are few long ones.
+// Measured on one GB300, against direction codes for every cell, band tests in every cell, progress counters with
+// release and acquire, and 5 blocks per SM: 2,715 DPs of the 500-pair batch 39.9 -> 16.8 ms, 400 DPs of 3 kb with a
+// path 14.3 -> 4.85 ms, 30 DPs of a 200 kb pair 497 -> 159 ms.  Chunks of 8, 16 and 32 steps: 162, 159 and 170 ms on
+// the long DPs, 18.3, 16.8 and 16.7 ms on the batch; 3, 4, 5 and 6 blocks per SM (before the tagged cells): 173, 183,
+// 215 and 250 ms and 19.5, 19.1, 20.5 and 22.8 ms.  The weighted DPs ran one warp each before, 32 rows at a time:
+// 1,072 DPs 128.5 -> 4.8 ms.
+template <bool CK, int KIND, int MINB>
+__global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow F, Arena ar, Params P, SgWeights W,
                                                                          uint8_t *__restrict__ tb) {
-  __shared__ SgRec stage[kSgFlowWarps][2][32];
-  __shared__ int stage_c[kSgFlowWarps][2][32];
+  __shared__ SgFeed stage[kSgFlowWarps][2][kSgChunk];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int o1 = P.open1, x1 = P.ext1, o2 = P.open2, x2 = P.ext2, w = P.bandwidth;
+  const int w = P.bandwidth;
   for (;;) {
     long long u = 0;
     if (lane == 0) u = (long long)atomicAdd(F.unit_counter, 1ull);
@@ -436,10 +590,8 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow
     if (__any_sync(0xFFFFFFFFu, sg_ld_relaxed(F.err) != 0)) break;  // a wait ran out: the launch fails as a whole
     const int2 qs = F.order[u];  // the u-th unit handed out: stripe qs.y of DP qs.x
     const int q = qs.x, s = qs.y;
-    const int64_t ui = F.unit_begin[q] + s;  // its progress counter
     SgTask &T = F.tasks[F.idx[q]];
     SgFlowDP &D = F.dps[q];
-    int *const prog_self = F.prog + ui;
     const int n1 = T.n1, n2 = T.n2;
     const int n1_eff = (n1 <= 0 || n2 <= 0) ? 0 : min(n1, n2 + w);
     const int nstripes = (n1_eff + kSgRows - 1) / kSgRows;
@@ -447,128 +599,158 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow
       if (lane == 0) T.score = 0, T.end1 = -1, T.end2 = -1, T.rows = 0, T.status = 0;
       continue;
     }
-    if (__any_sync(0xFFFFFFFFu, sg_ld_relaxed(&D.stop) != 0)) {
-      if (lane == 31) sg_st_release(prog_self, INT_MAX);
-      continue;
-    }
+    if (__any_sync(0xFFFFFFFFu, sg_ld_relaxed(&D.stop) != 0)) continue;
     const SeqView s1{T.base1, T.a1, T.dir}, s2{T.base2, T.a2, T.dir};
     const int r_last = n2 - 1 + w;
-    const int64_t stride = sg_stride_steps(n2, w);
-    SgRec *const brow = F.bnd + D.bnd_off;  // the DP's boundary row, by column
-    const int *const prog_up = s > 0 ? F.prog + (ui - 1) : nullptr;
+    const bool produce = s + 1 < nstripes;
+    // the row above and the row this stripe leaves, by column
+    const SgCell *const bin = CK ? sg_ck_row(tb, T, w, s) : F.bnd + D.bnd_off;
+    SgCell *const bout = CK ? sg_ck_row(tb, T, w, s + 1) : F.bnd + D.bnd_off;
     const int i0 = kSgRows * s + 1 + kSgR * lane;
-    const bool live = i0 <= n1_eff;
-    // per row of the lane: band [c0, c0 + span] (rows past the DP: an empty band), its base, the stale-column role,
-    // running states
-    int ci[kSgR], rmask[kSgR], c0[kSgR], span[kSgR], e1[kSgR], e2[kSgR], best[kSgR], bestj[kSgR], prevM[kSgR];
+    // per row of the lane: band [c0, c0 + span] (rows past the DP: an empty band), scores, running states
+    uint32_t prof[kSgR];
+    SgRowParams<KIND> rp[kSgR];
+    int e1[kSgR], e2[kSgR], best[kSgR], bestj[kSgR], prevM[kSgR];
     int stale_rows = 0;  // bit k: row k is row r_last (bit 4 + k: row r_last - 1)
 #pragma unroll
     for (int k = 0; k < kSgR; ++k) {
       const int i = i0 + k;
       const bool lv = i <= n1_eff;
-      c0[k] = lv ? max(i - w, 1) : INT_MAX / 2;
-      span[k] = lv ? min(i + w, n2) - c0[k] : 0;
-      ci[k] = lv ? s1.at(ar, i - 1) : 0;
-      rmask[k] = ci[k] == 2 ? 0 : -1;  // Scorei: an N row scores 0 against every base
-      if (lv && i == r_last) stale_rows |= 1 << k;
-      if (lv && i == r_last - 1) stale_rows |= 16 << k;
+      const int ci = lv ? s1.at(ar, i - 1) : 2;
+      prof[k] = KIND == 0 ? sg_profile(ci, P.match, P.mismatch) : sg_profile(ci, 1, 0);
+      if constexpr (KIND != 0) rp[k].load(T, W, i, lv);
+      if (KIND == 0 && lv && i == r_last) stale_rows |= 1 << k;
+      if (KIND == 0 && lv && i == r_last - 1) stale_rows |= 16 << k;
       e1[k] = kOut, e2[k] = kOut, best[k] = 0, bestj[k] = 0, prevM[k] = kOut;
     }
     const int r0 = kSgRows * s + 1, rl = min(kSgRows * s + kSgRows, n1_eff);
-    const int jstart = max(r0 - w, 1);
-    const int nsteps = min(rl + w, n2) - jstart + 1 + 31;
+    const int jstart = max(r0 - w, 1), jend = min(rl + w, n2);
+    const int nsteps = jend - jstart + 1 + 31;
     const int upB = min(kSgRows * s + w, n2);  // the row above (128s) holds columns [max(128s - w, 1), upB]
-    const bool produce = s + 1 < nstripes;
-    uint32_t *const trow = CODES ? reinterpret_cast<uint32_t *>(tb + T.tb_off) + (int64_t)s * stride * 32 : nullptr;
+    // steps [in_lo, in_hi) have every lane's column in [max(r0 + 127 - w, 1), min(r0 + w, n2 - 1)): inside the band of
+    // all rows, off the last and the stale column (rows past the DP compute what nobody reads)
+    const int in_lo = max(r0 + kSgRows - 1 - w, 1) - jstart + 31;
+    const int in_hi = min(r0 + w, n2 - 1) - jstart;
     int abandon = 0;  // 0 computing, 1 the DP stopped, -1 a wait ran out
-    // columns jstart + 32 * chunk + lane of the row above, into stage[warp][chunk & 1]; the producer must have
-    // published them first
-    auto stage_chunk = [&](int chunk) {
-      if (s > 0 && abandon == 0) {
-        const int need = min(jstart + 32 * chunk + 31, upB);
-        const int r = sg_wait_at_least(prog_up, need, &D.stop, F.err);
-        if (r <= 0) abandon = r == 0 ? 1 : -1;
-      }
-      const int j = jstart + 32 * chunk + lane;
-      SgRec rec{kOut, kOut, kOut};
-      if (s > 0 && abandon == 0 && j >= 1 && j <= upB) {
-        rec.m = __ldcg(&brow[j].m);
-        rec.f1 = __ldcg(&brow[j].f1);
-        rec.f2 = __ldcg(&brow[j].f2);
-      }
-      stage[warp][chunk & 1][lane] = rec;
-      stage_c[warp][chunk & 1][lane] = (j >= 1 && j <= n2) ? s2.at(ar, j - 1) : 0;
+    // column jstart + kSgChunk * chunk + lane of the row above, as it is now, and whether stripe s - 1 has written it
+    // (tag s; the columns past row 128s's band hold kOut)
+    auto look = [&](int chunk, SgCell &v) {
+      const int j = jstart + kSgChunk * chunk + lane;
+      v = SgCell{kOut, kOut, kOut, s};
+      if (s > 0 && lane < kSgChunk && j <= upB) v = sg_ld_cell(bin + j);
     };
-    stage_chunk(0);  // waits for columns up to jstart + 31, which include the diagonal column jstart - 1
-    // the diagonal of the stripe's first row at column jstart: cell (0, 0) = 0 for the DP's first row, else the
-    // row above at jstart - 1 (kOut at column 0)
-    int diag = kOut;
-    if (lane == 0) diag = s == 0 ? 0 : (jstart > 1 && abandon == 0) ? __ldcg(&brow[jstart - 1].m) : kOut;
-    stage_chunk(1);
-    __syncwarp();
-    int outM = kOut, outF1 = kOut, outF2 = kOut, outC = 0;
-    const bool lane0 = lane == 0, write_bnd = lane == 31 && produce;
-    for (int tc = 0; tc < nsteps && abandon == 0; tc += 32) {  // 32-step chunks
-      if (tc > 0) {
-        // chunk boundary: publish the columns of this stripe's last row written so far, stop early if the DP
-        // ended, stage the chunk two ahead of lane 0's reads
-        if (write_bnd) sg_st_release(prog_self, jstart + tc - 32);
+    auto stage_cells = [&](int chunk, const SgCell &v) {
+      const int j = jstart + kSgChunk * chunk + lane;
+      if (lane < kSgChunk)
+        stage[warp][chunk & 1][lane] = SgFeed{v.m, v.f1, v.f2, j <= n2 ? sg_selector(s2.at(ar, j - 1)) : 0x4444u};
+    };
+    // Looks until stripe s - 1 has written the chunk's columns (every wait ends or runs out of iterations, as
+    // sg_wait_at_least).
+    auto wait_cells = [&](int chunk, SgCell &v) {
+      for (int it = 0;; ++it) {
+        look(chunk, v);
+        if (__all_sync(0xFFFFFFFFu, v.tag == s)) return;
         if (__any_sync(0xFFFFFFFFu, sg_ld_relaxed(&D.stop) != 0)) {
           abandon = 1;
-          break;
+          return;
         }
-        __syncwarp();
-        stage_chunk((tc >> 5) + 1);
-        if (abandon != 0) break;
+        if (it >= kSgSpin || ((it & 63) == 63 && __any_sync(0xFFFFFFFFu, sg_ld_relaxed(F.err) != 0))) {
+          abandon = -1;
+          return;
+        }
+        __nanosleep(100);
       }
-      const SgRec *const srow = stage[warp][(tc >> 5) & 1];
-      const int *const scol = stage_c[warp][(tc >> 5) & 1];
-      const int tend = min(tc + 32, nsteps);
-      for (int t = tc; t < tend; ++t) {
-        int upM = __shfl_up_sync(0xFFFFFFFFu, outM, 1);
-        int upF1 = __shfl_up_sync(0xFFFFFFFFu, outF1, 1);
-        int upF2 = __shfl_up_sync(0xFFFFFFFFu, outF2, 1);
-        int cj = __shfl_up_sync(0xFFFFFFFFu, outC, 1);
-        const int j = jstart + t - lane;
-        if (lane0) {
-          const SgRec r = srow[t - tc];
-          upM = r.m, upF1 = r.f1, upF2 = r.f2;
-          cj = scol[t - tc];
-        }
-        int aF1 = upF1, aF2 = upF2, dg = diag;
-        uint32_t word = 0;
-        const int mt = cj == 2 ? 0 : P.match, mm = cj == 2 ? 0 : P.mismatch;  // Scorei: N scores 0
-        const bool stale_col = stale_rows != 0 && j == n2 - 1;
-#pragma unroll
-        for (int k = 0; k < kSgR; ++k) {
-          const int dj = j - c0[k];
-          const bool valid = (unsigned)dj <= (unsigned)span[k];
-          const bool last = dj == span[k];
-          const int sc = (ci[k] == cj ? mt : mm) & rmask[k];
-          int cF1, cF2;
-          uint32_t d = 0;
-          const int cM = sg_cell<CODES>(sc, dg, aF1, aF2, e1[k], e2[k], valid, last, o1, x1, o2, x2, cF1, cF2, &d);
-          if (CODES) word |= d << (8 * k);
-          bool keep;
-          best[k] = __vibmax_s32(best[k], cM, &keep);  // keep: !(cM > best), the first maximum of the row stays
-          bestj[k] = keep ? bestj[k] : j;
-          if (stale_col && valid) {
-            if ((stale_rows >> k) & 1) D.stale_last = cM;
-            if ((stale_rows >> (4 + k)) & 1) D.stale_prev = cM;
-          }
-          if (k == kSgR - 1 && write_bnd && valid) brow[j] = SgRec{cM, cF1, cF2};
-          dg = prevM[k];  // row k at column j - 1: the diagonal of row k + 1
-          prevM[k] = cM;
-          aF1 = cF1, aF2 = cF2;
-          if (k == kSgR - 1) outM = cM;
-        }
-        if (CODES && live) trow[(int64_t)t * 32 + lane] = word;
-        diag = upM;
-        outF1 = aF1, outF2 = aF2, outC = cj;
-      }
+    };
+    SgCell ahead;
+    wait_cells(0, ahead);
+    stage_cells(0, ahead);
+    // the diagonal of the stripe's first row at column jstart: cell (0, 0) = 0 for the DP's first row, else the
+    // row above at jstart - 1 (kOut at column 0), written before column jstart
+    int diag = kOut;
+    if (s == 0) diag = lane == 0 ? 0 : kOut;
+    if (s > 0 && jstart > 1 && abandon == 0) {
+      SgCell d{kOut, kOut, kOut, 0};
+      for (int it = 0; it < kSgSpin && d.tag != s; ++it) d = sg_ld_cell(bin + (jstart - 1));
+      if (lane == 0) diag = d.m;
+      if (__any_sync(0xFFFFFFFFu, d.tag != s)) abandon = -1;
     }
+    if (abandon == 0) wait_cells(1, ahead);
+    stage_cells(1, ahead);
     __syncwarp();
-    if (lane == 31) sg_st_release(prog_self, INT_MAX);  // every column written (or abandoned): release the consumer
+    int outM = kOut, outF1 = kOut, outF2 = kOut;
+    uint32_t outS = 0x4444u;
+    const bool lane0 = lane == 0, write_bnd = lane == 31 && produce;
+
+    auto step = [&](int t, const SgFeed *srow, auto inside) {
+      constexpr bool IN = decltype(inside)::value;
+      int upM = __shfl_up_sync(0xFFFFFFFFu, outM, 1);
+      int aF1 = __shfl_up_sync(0xFFFFFFFFu, outF1, 1);
+      int aF2 = KIND == 1 ? kOut : __shfl_up_sync(0xFFFFFFFFu, outF2, 1);
+      uint32_t sel = __shfl_up_sync(0xFFFFFFFFu, outS, 1);
+      const SgFeed rec = srow[t & (kSgChunk - 1)];  // every lane reads it, lane 0 uses it
+      upM = lane0 ? rec.m : upM;
+      aF1 = lane0 ? rec.f1 : aF1;
+      if (KIND != 1) aF2 = lane0 ? rec.f2 : aF2;
+      sel = lane0 ? rec.sel : sel;
+      const int j = jstart + t - lane;
+      int dg = diag;
+      const bool stale_col = !IN && KIND == 0 && stale_rows != 0 && j == n2 - 1;
+#pragma unroll
+      for (int k = 0; k < kSgR; ++k) {
+        bool valid = true, last = false;
+        if constexpr (!IN) {
+          const int i = i0 + k, c0 = max(i - w, 1), c1 = min(i + w, n2);
+          valid = i <= n1_eff && j >= c0 && j <= c1;
+          last = j == c1;
+        }
+        int cF1, cF2;
+        const int cM = sg_cell<false, KIND, IN>(sg_row_score<KIND>(prof[k], rp[k], sel), dg, aF1, aF2, e1[k], e2[k],
+                                                valid, last, rp[k], P, cF1, cF2, nullptr);
+        bool keep;
+        best[k] = __vibmax_s32(best[k], cM, &keep);  // keep: !(cM > best), the first maximum of the row stays
+        bestj[k] = keep ? bestj[k] : j;
+        if (stale_col && valid) {
+          if ((stale_rows >> k) & 1) D.stale_last = cM;
+          if ((stale_rows >> (4 + k)) & 1) D.stale_prev = cM;
+        }
+        if (k == kSgR - 1 && write_bnd && valid) sg_st_cell(bout + j, cM, cF1, cF2, s + 1);
+        dg = prevM[k];  // row k at column j - 1: the diagonal of row k + 1
+        prevM[k] = cM;
+        aF1 = cF1, aF2 = cF2;
+        if (k == kSgR - 1) outM = cM;
+      }
+      if constexpr (CK) {
+        if ((j & (kSgTile - 1)) == 0 && (IN || (j >= jstart && j <= jend))) {
+          int *const c = sg_ck_col(tb, T, w, s, j) + kSgR * lane;
+          *reinterpret_cast<int4 *>(c) = make_int4(prevM[0], prevM[1], prevM[2], prevM[3]);
+          *reinterpret_cast<int4 *>(c + kSgRows) = make_int4(e1[0], e1[1], e1[2], e1[3]);
+          if (KIND != 1) *reinterpret_cast<int4 *>(c + 2 * kSgRows) = make_int4(e2[0], e2[1], e2[2], e2[3]);
+        }
+      }
+      diag = upM;
+      outF1 = aF1, outF2 = aF2, outS = sel;
+    };
+
+    // Chunks of kSgChunk steps.  At a chunk's start the warp looks at the columns of the chunk two ahead (and at the
+    // DP's stop flag); at its end they are staged if they were all there, so the steps hide the round trip to L2, and
+    // a warp that runs too close behind its producer waits there.
+    for (int tc = 0; tc < nsteps && abandon == 0; tc += kSgChunk) {
+      const int chunk = tc / kSgChunk;
+      const SgFeed *const srow = stage[warp][chunk & 1];
+      const int stopped = sg_ld_relaxed(&D.stop);
+      look(chunk + 2, ahead);
+      if (tc >= in_lo && tc + kSgChunk <= in_hi) {
+        for (int t = tc; t < tc + kSgChunk; ++t) step(t, srow, std::true_type{});
+      } else {
+        const int tend = min(tc + kSgChunk, nsteps);
+        for (int t = tc; t < tend; ++t) step(t, srow, std::false_type{});
+      }
+      if (__any_sync(0xFFFFFFFFu, stopped != 0)) abandon = 1;  // the DP ended
+      if (abandon == 0 && !__all_sync(0xFFFFFFFFu, ahead.tag == s)) wait_cells(chunk + 2, ahead);
+      __syncwarp();
+      stage_cells(chunk + 2, ahead);
+      __syncwarp();
+    }
     if (abandon < 0 && lane == 0) {
       atomicExch(F.err, 1);
       atomicExch(&D.stop, 1);
@@ -591,18 +773,29 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow
     int mx = 0, e1r = -1, e2r = -1, rows = 0;  // ends are 1-based and stay -1 while no cell is positive
     if (s > 0) mx = sg_ld_relaxed(&D.mx), e1r = sg_ld_relaxed(&D.e1r), e2r = sg_ld_relaxed(&D.e2r),
                rows = sg_ld_relaxed(&D.rows);
+    int zd[kSgR];  // the rows' z-drop, per category
+    if constexpr (KIND != 0) {
+#pragma unroll
+      for (int k = 0; k < kSgR; ++k)
+        zd[k] = i0 + k <= n1_eff ? __ldg(W.cats + 7 * sgw_cat(T, W.weights, i0 + k) + 6) : 0;
+    }
     bool stop = false;
     for (int ol = 0; ol < 32; ++ol) {  // row 128s + 1 + 4 ol + k is lane ol's row k
 #pragma unroll
       for (int k = 0; k < kSgR; ++k) {
         const int tm = __shfl_sync(0xFFFFFFFFu, best[k], ol), tj = __shfl_sync(0xFFFFFFFFu, bestj[k], ol);
+        int z = P.zdrop, x = P.ext2;
+        if constexpr (KIND != 0) {
+          z = __shfl_sync(0xFFFFFFFFu, zd[k], ol);
+          x = KIND == 1 ? 0 : __shfl_sync(0xFFFFFFFFu, rp[k].x2h, ol);
+        }
         const int ii = r0 + kSgR * ol + k;
         if (!stop && ii <= n1_eff) {
           if (tm > mx) mx = tm, e1r = ii, e2r = tj;
           int l = (ii - e1r) - (tj - e2r);
           l = l > 0 ? l : -l;
           rows = ii;
-          if (mx - tm > P.zdrop + l * x2)
+          if (mx - tm > z + l * x)
             stop = true;
           else if (tj <= 0)
             stop = true;
@@ -610,7 +803,7 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow
       }
     }
     if (lane == 0) {
-      if (!stop && s == nstripes - 1 && n1 > n1_eff && n2 >= 1) {
+      if (KIND == 0 && !stop && s == nstripes - 1 && n1 > n1_eff && n2 >= 1) {
         // empty-band rows: only the last column, from the stale column n2-1 of the row with the same parity
         const int c2 = s2.at(ar, n2 - 1);
         const int st_last = sg_ld_relaxed(&D.stale_last), st_prev = sg_ld_relaxed(&D.stale_prev);
@@ -623,12 +816,14 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow
           int l = (ii - e1r) - (tj - e2r);
           l = l > 0 ? l : -l;
           rows = ii;
-          if (mx - tm > P.zdrop + l * x2)
+          if (mx - tm > P.zdrop + l * P.ext2)
             stop = true;
           else if (tj <= 0)
             stop = true;
         }
       }
+      // the weighted DPs end at their first row with an empty band
+      if (KIND != 0 && !stop && s == nstripes - 1 && n1 > n1_eff) rows = n1_eff + 1;
       if (stop || s == nstripes - 1) {
         T.score = mx;
         T.end1 = e1r;
@@ -651,49 +846,287 @@ int64_t sg_flow_units(int n1, int n2, int w) {
   return std::max<int64_t>(1, (n1_eff + kSgRows - 1) / kSgRows);
 }
 
-int sg_flow_blocks_per_sm(int minb) {
-  static int nb[2] = {0, 0};
-  int &r = nb[minb == 6 ? 1 : 0];
-  if (r == 0) {
-    int v = 0;
-    const cudaError_t e = minb == 6 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, sg_flow_kernel<true, 6>,
-                                                                                     32 * kSgFlowWarps, 0)
-                                    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, sg_flow_kernel<true, 5>,
-                                                                                     32 * kSgFlowWarps, 0);
-    if (e != cudaSuccess) {
-      (void)cudaGetLastError();
-      v = 1;
-    }
-    r = v > 0 ? v : 1;
-  }
-  return r;
-}
+int64_t sg_flow_grid_warps(int nsm, int minb) { return (int64_t)nsm * minb * kSgFlowWarps; }
 
-int64_t sg_flow_grid_warps(int nsm, int minb) { return (int64_t)nsm * sg_flow_blocks_per_sm(minb) * kSgFlowWarps; }
-
-void launch_semiglobal_flow(const SgFlow &f, Arena ar, Params p, uint8_t *tb, bool codes, int nsm, int minb,
-                            cudaStream_t st) {
+void launch_semiglobal_flow(const SgFlow &f, Arena ar, Params p, const SgWeights *wt, uint8_t *tb, bool path, int nsm,
+                            int minb, cudaStream_t st) {
   if (f.total_units <= 0) return;
   const int64_t warps = std::min<int64_t>(f.total_units, sg_flow_grid_warps(nsm, minb));
-  const int blocks = (int)((warps + kSgFlowWarps - 1) / kSgFlowWarps);
-  if (minb == 6) {
-    if (codes)
-      sg_flow_kernel<true, 6><<<blocks, 32 * kSgFlowWarps, 0, st>>>(f, ar, p, tb);
-    else
-      sg_flow_kernel<false, 6><<<blocks, 32 * kSgFlowWarps, 0, st>>>(f, ar, p, tb);
-  } else {
-    if (codes)
-      sg_flow_kernel<true, 5><<<blocks, 32 * kSgFlowWarps, 0, st>>>(f, ar, p, tb);
-    else
-      sg_flow_kernel<false, 5><<<blocks, 32 * kSgFlowWarps, 0, st>>>(f, ar, p, tb);
+  const int blocks = (int)((warps + kSgFlowWarps - 1) / kSgFlowWarps), threads = 32 * kSgFlowWarps;
+  auto run = [&](auto kernel) { kernel<<<blocks, threads, 0, st>>>(f, ar, p, wt ? *wt : SgWeights{}, tb); };
+  if (wt && wt->pieces == 1)
+    path ? run(sg_flow_kernel<true, 1, 4>) : run(sg_flow_kernel<false, 1, 4>);
+  else if (wt)
+    path ? run(sg_flow_kernel<true, 2, 4>) : run(sg_flow_kernel<false, 2, 4>);
+  else if (minb == 6)
+    path ? run(sg_flow_kernel<true, 0, 6>) : run(sg_flow_kernel<false, 0, 6>);
+  else if (minb == 5)
+    path ? run(sg_flow_kernel<true, 0, 5>) : run(sg_flow_kernel<false, 0, 5>);
+  else
+    path ? run(sg_flow_kernel<true, 0, 4>) : run(sg_flow_kernel<false, 0, 4>);
+}
+
+// ------------------------------------------------------------------ traceback of the flow's DPs: tiles computed again
+// The walk of sg_traceback_warp_kernel below (the same state machine, ends, padding and reversal), over the tiles of
+// 128 rows x 128 columns that the path goes through, computed again from the checkpoints around them with their
+// direction codes in shared memory.  One block of NT warps per DP: each warp computes one of the next NT tiles in the
+// direction of the walk's state (a diagonal; a row or a column inside a gap, since the second gap piece may run over
+// thousands of cells), because a tile takes one warp some 15 us whatever else the SM does; then the first warp walks
+// them until the path leaves them all.  The walk takes a run at a time: the lanes look at the next 32 cells in the
+// current direction, and a ballot says how far the state holds.  NT = 8 where the DPs leave SMs idle anyway (one
+// block per SM), else 4 (three blocks per SM).
+
+struct SgTile {
+  int s, ja, jb, tr;  // stripe, columns [ja, jb], rows up to tr
+};
+
+template <int KIND, bool INSIDE>
+__device__ __forceinline__ void sg_tile_codes(const SgTask &T, const Arena &ar, const Params &P, const SgWeights &W,
+                                              uint8_t *__restrict__ tb, const SgTile &X, uint32_t (*code)[32],
+                                              SgFeed *feed, int lane) {
+  const int w = P.bandwidth, n2 = T.n2, n1_eff = min(T.n1, n2 + w);
+  const SeqView s1{T.base1, T.a1, T.dir}, s2{T.base2, T.a2, T.dir};
+  const int ts = X.s, ja = X.ja, jb = X.jb;
+  const int jstart = max(kSgRows * ts + 1 - w, 1), upB = min(kSgRows * ts + w, n2);
+  const int left = (jb - 1) / kSgTile * kSgTile;  // the column checkpoint left of the tile
+  const SgCell *const bin = sg_ck_row(tb, T, w, ts);
+  for (int c = lane; c <= jb - ja; c += 32) {
+    const int j = ja + c;
+    SgFeed rec{kOut, kOut, kOut, sg_selector(s2.at(ar, j - 1))};
+    if (ts > 0 && j <= upB) rec.m = bin[j].m, rec.f1 = bin[j].f1, rec.f2 = bin[j].f2;
+    feed[c] = rec;
   }
+  const int i0 = kSgRows * ts + 1 + kSgR * lane;
+  uint32_t prof[kSgR];
+  SgRowParams<KIND> rp[kSgR];
+  int e1[kSgR], e2[kSgR], prevM[kSgR];
+  const bool from = left >= jstart;
+  const int *const col = from ? sg_ck_col(tb, T, w, ts, left) + kSgR * lane : nullptr;
+#pragma unroll
+  for (int k = 0; k < kSgR; ++k) {
+    const int i = i0 + k;
+    const bool lv = i <= n1_eff;
+    const int ci = lv ? s1.at(ar, i - 1) : 2;
+    prof[k] = KIND == 0 ? sg_profile(ci, P.match, P.mismatch) : sg_profile(ci, 1, 0);
+    if constexpr (KIND != 0) rp[k].load(T, W, i, lv);
+    prevM[k] = from ? col[k] : kOut;
+    e1[k] = from ? col[kSgRows + k] : kOut;
+    e2[k] = (from && KIND != 1) ? col[2 * kSgRows + k] : kOut;
+  }
+  // the diagonal of the lane's first row at column ja: lanes above 0 take the lane above's checkpoint by shuffle
+  int diag = kOut;
+  if (lane == 0) diag = ts == 0 ? (ja == 1 ? 0 : kOut) : (ja > 1 && ja - 1 <= upB) ? bin[ja - 1].m : kOut;
+  int outM = prevM[kSgR - 1], outF1 = kOut, outF2 = kOut;
+  __syncwarp();
+  const int nsteps = jb - ja + 1 + (X.tr - 1 - kSgRows * ts) / kSgR;
+  for (int t = 0; t < nsteps; ++t) {
+    int upM = __shfl_up_sync(0xFFFFFFFFu, outM, 1);
+    int aF1 = __shfl_up_sync(0xFFFFFFFFu, outF1, 1);
+    int aF2 = __shfl_up_sync(0xFFFFFFFFu, outF2, 1);
+    const int c = t - lane, j = ja + c;
+    const bool on = c >= 0 && j <= jb;
+    const SgFeed rec = feed[on ? c : 0];
+    if (lane == 0) upM = rec.m, aF1 = rec.f1, aF2 = rec.f2;
+    if (on) {
+      int dg = diag;
+      uint32_t word = 0;
+#pragma unroll
+      for (int k = 0; k < kSgR; ++k) {
+        bool valid = true, last = false;
+        if constexpr (!INSIDE) {
+          const int i = i0 + k, c0 = max(i - w, 1), c1 = min(i + w, n2);
+          valid = i <= n1_eff && j >= c0 && j <= c1;
+          last = j == c1;
+        }
+        int cF1, cF2;
+        uint32_t d = 0;
+        const int cM = sg_cell<true, KIND, INSIDE>(sg_row_score<KIND>(prof[k], rp[k], rec.sel), dg, aF1, aF2, e1[k],
+                                                   e2[k], valid, last, rp[k], P, cF1, cF2, &d);
+        word |= d << (8 * k);
+        dg = prevM[k];
+        prevM[k] = cM;
+        aF1 = cF1, aF2 = cF2;
+      }
+      outM = prevM[kSgR - 1];
+      code[c][lane] = word;
+      outF1 = aF1, outF2 = aF2;
+    }
+    diag = upM;
+  }
+  __syncwarp();
+}
+
+template <int KIND, int NT>
+__global__ void __launch_bounds__(32 * NT) sg_retrace_kernel(SgTask *__restrict__ tasks,
+                                                                   const int *__restrict__ idx, Arena ar, Params P,
+                                                                   SgWeights W, uint8_t *__restrict__ tb,
+                                                                   uint32_t *__restrict__ cig) {
+  extern __shared__ uint4 rt_smem[];  // per warp: codes [column][lane] (a lane's four rows a word), then the feed
+  __shared__ SgTile tile[NT];
+  __shared__ int more;
+  const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
+  auto codes_of = [&](int k) { return reinterpret_cast<uint32_t(*)[32]>(rt_smem) + k * kSgTile; };
+  SgFeed *const feed = reinterpret_cast<SgFeed *>(reinterpret_cast<uint32_t(*)[32]>(rt_smem) + NT * kSgTile) +
+                       wb * kSgTile;
+  const int w = P.bandwidth;
+  SgTask &T = tasks[idx[blockIdx.x]];
+  const int n1 = T.n1, n2 = T.n2, n1_eff = (n1 <= 0 || n2 <= 0) ? 0 : min(n1, n2 + w), rows = T.rows;
+  // the walk's state: the same in every lane of the first warp
+  int ii = T.end1, jj = T.end2, state = 0, nc = 0;
+  uint32_t *const out = cig + T.cig_off;
+  const int cap = T.cig_cap;
+  uint32_t last = 0xFFFFFFFFu;
+  bool full = false;
+  auto push = [&](uint32_t op, int n) {
+    if (nc > 0 && (last & 0xFu) == op) {
+      last += (uint32_t)n << 4;
+    } else {
+      if (nc >= cap) {
+        full = true;
+        return;
+      }
+      last = ((uint32_t)n << 4) | op;
+      ++nc;
+    }
+    if (lane == 0) out[nc - 1] = last;
+  };
+  auto in_band = [&](int i, int j) {
+    return i > 0 && j > 0 && i <= rows && j >= max(i - w, 1) && (j < min(i + w, n2) || (KIND != 0 && j == min(i + w, n2)));
+  };
+  if (threadIdx.x < NT) tile[threadIdx.x].s = -1;
+  for (;;) {
+    __syncthreads();
+    if (wb == 0) {
+      int need = 0;
+      int cur = 0;
+      while (ii > 0 && jj > 0) {
+        if (!in_band(ii, jj)) {  // reads 255: a gap state holds, anything else moves left
+          if (state >= 1 && state <= 4) {
+          } else {
+            state = 7;
+          }
+          if (state == 1 || state == 3) {
+            push(2, 1);
+            --ii;
+          } else {
+            push(1, 1);
+            --jj;
+          }
+          continue;
+        }
+        const int s = (ii - 1) / kSgRows;
+        int k = 0;
+        for (; k < NT; ++k) {
+          const SgTile &X = tile[(cur + k) % NT];
+          if (X.s == s && jj >= X.ja && jj <= X.jb && ii <= X.tr) break;
+        }
+        if (k == NT) {
+          need = 1;
+          break;
+        }
+        cur = (cur + k) % NT;
+        const SgTile X = tile[cur];
+        uint32_t(*const code)[32] = codes_of(cur);
+        const int rtop = kSgRows * s;  // rows above the tile end here
+        // the next 32 cells in the direction of the state
+        const int di = state == 2 || state >= 4 ? 0 : 1, dj = state == 1 || state == 3 ? 0 : 1;
+        const int ci = ii - di * lane, cj = jj - dj * lane;
+        const bool in = ci > rtop && cj >= X.ja && in_band(ci, cj);
+        int c = 255;
+        if (in) c = (int)((code[cj - X.ja][(ci - 1 - rtop) / kSgR] >> (8 * ((ci - 1 - rtop) % kSgR))) & 0xFFu);
+        const bool hold = in && (state == 0 ? (c & 7) == 0 : ((c >> (state + 2)) & 1) != 0);
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, hold);
+        const int run = m == 0xFFFFFFFFu ? 32 : __ffs(~m) - 1;
+        if (run > 0) {
+          push(state == 0 ? 0u : (state == 1 || state == 3) ? 2u : 1u, run);
+          ii -= di * run;
+          jj -= dj * run;
+        }
+        if (run < 32) {  // the cell the run ends at, if it lies in this tile, starts a new state
+          const int there = __shfl_sync(0xFFFFFFFFu, (int)in, run), fresh = __shfl_sync(0xFFFFFFFFu, c & 7, run);
+          if (there) {
+            state = fresh;
+            if (state == 1 || state == 3) {
+              push(2, 1);
+              --ii;
+            } else if (state != 0) {
+              push(1, 1);
+              --jj;
+            }
+          }
+        }
+      }
+      if (lane == 0) {
+        more = need;
+        if (need) {  // the next tiles in the direction of the state
+          int i = ii, j = jj;
+          const bool go_up = state != 2 && state != 4, go_left = state != 1 && state != 3;
+          for (int k = 0; k < NT; ++k) {
+            SgTile X{-1, 0, -1, 0};
+            if (i > 0 && j > 0) {
+              X.s = (i - 1) / kSgRows;
+              const int r0 = kSgRows * X.s + 1, jstart = max(r0 - w, 1);
+              const int c0 = max((j - 1) / kSgTile * kSgTile + 1, jstart);
+              X.ja = c0;
+              X.jb = k == 0 ? j : min((j - 1) / kSgTile * kSgTile + kSgTile, min(min(r0 + kSgRows - 1, n1_eff) + w, n2));
+              X.tr = k == 0 ? i : min(r0 + kSgRows - 1, rows);
+              if (X.jb < X.ja) X.s = -1;
+              const int up = i - r0 + 1, lf = j - c0 + 1;  // moves until the diagonal leaves at the top, at the left
+              const int d = !go_up ? lf : !go_left ? up : min(up, lf);
+              if (go_up) i -= d;
+              if (go_left) j -= d;
+            }
+            tile[k] = X;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (!more) break;
+    const SgTile X = tile[wb];
+    if (X.s >= 0) {
+      const int r0 = kSgRows * X.s + 1, r1 = r0 + kSgRows - 1;
+      if (r1 <= n1_eff && X.ja >= max(r1 - w, 1) && X.jb < min(r0 + w, n2))
+        sg_tile_codes<KIND, true>(T, ar, P, W, tb, X, codes_of(wb), feed, lane);
+      else
+        sg_tile_codes<KIND, false>(T, ar, P, W, tb, X, codes_of(wb), feed, lane);
+    }
+  }
+  if (threadIdx.x == 0) {
+    if (ii > 0) push(2, ii);
+    if (jj > 0) push(1, jj);
+    for (int a = 0, b = nc - 1; a < b; ++a, --b) {  // the reference reverses the walk (:915)
+      const uint32_t tmp = out[a];
+      out[a] = out[b];
+      out[b] = tmp;
+    }
+    T.ncig = nc;
+    if (full) T.status = 3;
+  }
+}
+
+void launch_sg_retrace(SgTask *tasks, const int *idx, int n, Arena ar, Params p, const SgWeights *wt, uint8_t *tb,
+                       uint32_t *cig, int nsm, cudaStream_t st) {
+  if (n <= 0) return;
+  auto run = [&](auto kernel, int nt) {
+    const int smem = nt * kSgTile * (32 * (int)sizeof(uint32_t) + (int)sizeof(SgFeed));
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    kernel<<<n, 32 * nt, smem, st>>>(tasks, idx, ar, p, wt ? *wt : SgWeights{}, tb, cig);
+  };
+  const bool few = n <= nsm;
+  if (!wt)
+    few ? run(sg_retrace_kernel<0, 8>, 8) : run(sg_retrace_kernel<0, 4>, 4);
+  else if (wt->pieces == 1)
+    few ? run(sg_retrace_kernel<1, 8>, 8) : run(sg_retrace_kernel<1, 4>, 4);
+  else
+    few ? run(sg_retrace_kernel<2, 8>, 8) : run(sg_retrace_kernel<2, 4>, 4);
 }
 
 // ------------------------------------------------------------------ traceback (:869-914)
 // State machine of impl/sequenceAlignment3.cpp:869-914: start in the state that produced the cell; a gap state persists
 // while the cell's continuation flag is set; unwritten cells (outside the band, and the unweighted DP's last band
-// column) read 255; the remaining rows and columns pad the walk as D and I, and the CIGAR is reversed.  R: rows per
-// lane of the layout that wrote the codes (kSgR for the unweighted kernels, 1 for the weighted kernel).
+// column) read 255; the remaining rows and columns pad the walk as D and I, and the CIGAR is reversed. 
+// (The codes of sg_kernel, one CTA per DP; the flow's DPs are walked by sg_retrace_kernel above.)
 //
 // One warp per DP walks through shared-memory windows of the code store.  In the stripe / step / lane
 // layout every move of the walk (diagonal, up, left) goes to a lower address, at most 2 x 32 x R + R bytes lower,
@@ -710,11 +1143,10 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-template <int R>
 __global__ void __launch_bounds__(128) sg_traceback_warp_kernel(SgTask *__restrict__ tasks, const int *__restrict__ idx,
                                                                 int n, int w, const uint8_t *__restrict__ tb,
                                                                 int64_t tb_bytes, uint32_t *__restrict__ cig) {
-  constexpr int kRows = 32 * R;
+  constexpr int R = kSgR, kRows = 32 * R;
   // two windows per warp: lane 0 walks one while the warp's asynchronous copies fill the other with the window just
   // below it, where the walk goes next unless it crosses into the stripe above (a jump: then a synchronous fill)
   __shared__ __align__(16) uint8_t win2[4][2][kSgTbWin];
@@ -763,7 +1195,7 @@ __global__ void __launch_bounds__(128) sg_traceback_warp_kernel(SgTask *__restri
       while (ii > 0 && jj > 0) {
         int code = 255;
         const int c0 = max(ii - w, 1), c1 = min(ii + w, n2);
-        if (ii <= T.rows && jj >= c0 && (jj < c1 || (R == 1 && jj == c1))) {
+        if (ii <= T.rows && jj >= c0 && jj < c1) {
           const int s = (ii - 1) / kRows, rr = (ii - 1) % kRows, l = rr / R, kk = rr % R;
           const int jstart = max(kRows * s + 1 - w, 1);
           const int64_t t = jj - jstart + l;
@@ -830,179 +1262,9 @@ __global__ void __launch_bounds__(128) sg_traceback_warp_kernel(SgTask *__restri
 }
 
 void launch_sg_traceback(SgTask *tasks, const int *idx, int n, int bandwidth, const uint8_t *tb, int64_t tb_bytes,
-                         uint32_t *cig, cudaStream_t st, bool weighted_layout) {
+                         uint32_t *cig, cudaStream_t st) {
   if (n <= 0) return;
-  const int blocks = (n + 3) / 4;
-  if (weighted_layout)
-    sg_traceback_warp_kernel<1><<<blocks, 128, 0, st>>>(tasks, idx, n, bandwidth, tb, tb_bytes, cig);
-  else
-    sg_traceback_warp_kernel<kSgR><<<blocks, 128, 0, st>>>(tasks, idx, n, bandwidth, tb, tb_bytes, cig);
-}
-
-// ------------------------------------------------------------------ weighted DPs (one warp per DP)
-// SemiGlobal with weights (impl/sequenceAlignment3.cpp:1483-1709, pieces = 2) and SemiGlobal_single_gap_penalty
-// (:1710-1890, pieces = 1).  Row i takes the category of its seq1 base for the substitution, the horizontal gap
-// states and the z-drop, and the category of the next base for the vertical gap states it leaves (a row at the end
-// of seq1 keeps its own).  Every band column, the last included, updates the gap states and writes its code; a row
-// with an empty band ends the DP (no stale column, unlike the unweighted DP).
-//
-// One warp runs one DP: 32-row stripes one after another, lane l owning row 32s+1+l as an anti-diagonal wavefront,
-// the stripe's last row kept for the next stripe in the warp's global scratch (each column is read by lane 0 at least
-// 31 steps before lane 31 overwrites it).  Rows are evaluated in order after each stripe; the DP ends at the stop row.
-// Codes: one byte per cell, stripe / step / lane, the traceback layout of 32-row stripes.
-__host__ __device__ inline int64_t sgw_stride_steps(int n2, int w) {
-  const int64_t span = 2 * (int64_t)w + 32;
-  return (n2 < span ? (int64_t)n2 : span) + 32;
-}
-
-int64_t sgw_tb_bytes(int n1, int n2, int w) {
-  if (n1 <= 0 || n2 <= 0) return 0;
-  return (int64_t)((n1 + 31) / 32) * sgw_stride_steps(n2, w) * 32;
-}
-
-int64_t sgw_bnd_bytes(int warps, int max_n2) { return (int64_t)warps * ((int64_t)max_n2 + 2) * sizeof(SgRec); }
-
-__device__ __forceinline__ int sgw_cat(const SgTask &T, const int16_t *__restrict__ wt, int i) {
-  // category of DP row i (1-based): forward rows follow seq1 from a1, reverse rows go down from a1
-  const int64_t pos = T.dir == 0 ? (int64_t)T.a1 + i - 1 : (int64_t)T.a1 - (i - 1);
-  return wt[T.wbase + pos];
-}
-
-__device__ __forceinline__ int sgw_next_cat(const SgTask &T, const int16_t *__restrict__ wt, int i, int own) {
-  const int64_t pos = T.dir == 0 ? (int64_t)T.a1 + i : (int64_t)T.a1 - i;
-  return (pos < 0 || pos >= T.wlen) ? own : wt[T.wbase + pos];
-}
-
-__global__ void __launch_bounds__(128) sgw_kernel(SgTask *__restrict__ tasks, const int *__restrict__ idx, int n,
-                                                  Arena ar, Params P, SgWeights W, uint8_t *__restrict__ tb,
-                                                  SgRec *__restrict__ bnd_all, int64_t bnd_stride,
-                                                  int *__restrict__ counter) {
-  __shared__ int cat[kSgwMaxCats][7];
-  for (int k = threadIdx.x; k < W.n_cats * 7; k += blockDim.x) cat[k / 7][k % 7] = W.cats[k];
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  SgRec *bnd = bnd_all + (int64_t)gw * bnd_stride;
-  const int w = P.bandwidth;
-  const bool two = W.pieces == 2;
-  for (;;) {
-    int q = 0;
-    if (lane == 0) q = atomicAdd(counter, 1);
-    q = __shfl_sync(0xFFFFFFFFu, q, 0);
-    if (q >= n) break;
-    SgTask &T = tasks[idx[q]];
-    const int n1 = T.n1, n2 = T.n2;
-    const SeqView s1{T.base1, T.a1, T.dir}, s2{T.base2, T.a2, T.dir};
-    const bool codes = T.want_codes != 0;
-    const int64_t stride = sgw_stride_steps(n2, w);
-    const int nstripes = (n1 > 0 && n2 > 0) ? (n1 + 31) / 32 : 0;
-    int mx = 0, e1r = -1, e2r = -1, rows = 0;  // lane 0's running evaluation
-    bool stop = false;
-    for (int s = 0; s < nstripes && !stop; ++s) {
-      const int i = 32 * s + 1 + lane;
-      const bool live = i <= n1;
-      const int c0 = max(i - w, 1), c1 = min(i + w, n2);
-      const int ci = live ? s1.at(ar, i - 1) : 0;
-      const int rc = live ? sgw_cat(T, W.weights, i) : 0;
-      const int nc = live ? sgw_next_cat(T, W.weights, i, rc) : 0;
-      const int mt = cat[rc][0], mm = cat[rc][1], o1h = cat[rc][2], x1h = cat[rc][3], o2h = cat[rc][4], x2h = cat[rc][5];
-      const int o1v = cat[nc][2], x1v = cat[nc][3], o2v = cat[nc][4], x2v = cat[nc][5];
-      const int r0 = 32 * s + 1, rl = min(32 * s + 32, n1);
-      const int jstart = max(r0 - w, 1), jend = min(rl + w, n2);
-      const int nsteps = jend >= jstart ? jend - jstart + 1 + 31 : 0;
-      uint8_t *trow = tb + T.tb_off + (int64_t)s * stride * 32;
-      int e1 = kOut, e2 = kOut, best = 0, bestj = two ? kOut : -1;
-      int diag = (lane == 0 && s > 0 && jstart > 1) ? bnd[jstart - 1].m : kOut;
-      int outM = kOut, outF1 = kOut, outF2 = kOut, outC = 0;
-      for (int t = 0; t < nsteps; ++t) {
-        int upM = __shfl_up_sync(0xFFFFFFFFu, outM, 1);
-        int upF1 = __shfl_up_sync(0xFFFFFFFFu, outF1, 1);
-        int upF2 = __shfl_up_sync(0xFFFFFFFFu, outF2, 1);
-        int cj = __shfl_up_sync(0xFFFFFFFFu, outC, 1);
-        const int j = jstart + t - lane;
-        if (lane == 0) {
-          upM = kOut, upF1 = kOut, upF2 = kOut;
-          if (s > 0 && j >= 1 && j <= n2) {
-            const SgRec r = bnd[j];
-            upM = r.m, upF1 = r.f1, upF2 = r.f2;
-          }
-          cj = (j >= 1 && j <= n2) ? s2.at(ar, j - 1) : 0;
-        }
-        int cM = kOut, cF1 = kOut, cF2 = kOut;
-        uint8_t code = 255;
-        if (live && j >= c0 && j <= c1) {
-          const int dg = (j == 1) ? (i == 1 ? 0 : kOut) : diag;
-          const bool last = (j == c1);
-          const int fin1 = last ? kOut : upF1, fin2 = last ? kOut : upF2;
-          int v = ((ci == 2 || cj == 2) ? 0 : (ci == cj ? mt : mm)) + dg;
-          int d = 0;
-          bool pr;
-          v = __vibmax_s32(fin1, v, &pr);
-          d = pr ? 1 : d;
-          v = __vibmax_s32(e1, v, &pr);
-          d = pr ? 2 : d;
-          if (two) {
-            v = __vibmax_s32(fin2, v, &pr);
-            d = pr ? 3 : d;
-            v = __vibmax_s32(e2, v, &pr);
-            d = pr ? 4 : d;
-          }
-          cM = v;
-          if (v > best) best = v, bestj = j;
-          cF1 = __vibmax_s32(fin1 + x1v, v + o1v, &pr);
-          d |= pr ? 8 : 0;
-          e1 = __vibmax_s32(e1 + x1h, v + o1h, &pr);
-          d |= pr ? 16 : 0;
-          if (two) {
-            cF2 = __vibmax_s32(fin2 + x2v, v + o2v, &pr);
-            d |= pr ? 32 : 0;
-            e2 = __vibmax_s32(e2 + x2h, v + o2h, &pr);
-            d |= pr ? 64 : 0;
-          }
-          code = (uint8_t)d;
-        }
-        if (codes && live) trow[(int64_t)t * 32 + lane] = code;
-        __syncwarp();
-        if (lane == 31 && live && j >= c0 && j <= c1) bnd[j] = SgRec{cM, cF1, cF2};
-        __syncwarp();
-        diag = upM;
-        outM = cM, outF1 = cF1, outF2 = cF2, outC = cj;
-      }
-      // the stripe's rows in order (lane 0 decides; every lane takes part in the shuffles)
-      for (int r = 0; r < 32; ++r) {
-        const int tm = __shfl_sync(0xFFFFFFFFu, best, r), tj = __shfl_sync(0xFFFFFFFFu, bestj, r);
-        const int zd = __shfl_sync(0xFFFFFFFFu, cat[rc][6], r), xr = __shfl_sync(0xFFFFFFFFu, x2h, r);
-        const int ii = 32 * s + 1 + r;
-        if (stop || ii > n1) continue;
-        if (tm > mx) mx = tm, e1r = ii, e2r = tj;
-        rows = ii;
-        if (two) {
-          int l = (ii - e1r) - (tj - e2r);
-          l = l > 0 ? l : -l;
-          if (mx - tm > zd + l * xr) stop = true;
-        } else if (mx - tm > zd) {
-          stop = true;
-        }
-        if (!stop && tj <= 0) stop = true;
-      }
-      __syncwarp();
-    }
-    if (lane == 0) {
-      T.score = mx;
-      T.end1 = e1r;
-      T.end2 = e2r;
-      T.rows = rows;
-      T.status = 0;
-    }
-    __syncwarp();
-  }
-}
-
-void launch_semiglobal_weighted(SgTask *tasks, const int *idx, int n, Arena ar, Params p, SgWeights wt, uint8_t *tb,
-                                void *bnd, int max_n2, int *work_counter, int warps, cudaStream_t st) {
-  if (n <= 0) return;
-  sgw_kernel<<<(warps + 3) / 4, 128, 0, st>>>(tasks, idx, n, ar, p, wt, tb, (SgRec *)bnd, (int64_t)max_n2 + 2,
-                                              work_counter);
+  sg_traceback_warp_kernel<<<(n + 3) / 4, 128, 0, st>>>(tasks, idx, n, bandwidth, tb, tb_bytes, cig);
 }
 
 }  // namespace dcns

@@ -92,7 +92,8 @@ typedef struct {
   double ms_sg_kernel;        /* device: semi-global DP kernels, CUDA events */
   double ms_sg_tb_kernel;     /* device: semi-global traceback kernels, CUDA events */
   int64_t bytes_codes_xdrop;  /* direction codes of the final-width x-drop passes that kept them: 4 bits per band cell */
-  int64_t bytes_codes_sg;     /* direction codes of the semi-global DPs that kept them: 1 byte per band cell */
+  int64_t bytes_codes_sg;     /* what the semi-global DPs with a path keep for it: checkpoints, or (one CTA per DP)
+                                 direction codes of 1 byte per band cell */
   int64_t bytes_device;       /* device memory the context's buffers hold after the call (they are kept for reuse) */
 } dcns_stats;
 
@@ -193,7 +194,7 @@ typedef struct {
   int32_t sg_warps;               /* warps per 2-piece DP when one CTA runs a DP (0: two for launches of many DPs,
                                      else eight) */
   int32_t sg_flow;                /* 1: 2-piece DPs run as a flow of 128-row stripe units over one persistent grid */
-  int32_t sg_flow_blocks;         /* resident blocks per SM of that grid: 5 or 6 */
+  int32_t sg_flow_blocks;         /* resident blocks per SM of that grid: 4, 5 or 6 */
   int32_t bins_by_size;           /* 1: bins are runs of pairs in increasing size (the largest last); 0: mixed */
   int32_t n_bins_tuned;           /* bins with their own x-drop forms below (0: every bin uses bin 0's values) */
   int32_t xdrop_warp_from[16], xdrop_wave_max_w[16], xdrop_flat[16], xdrop_handoff[16], xdrop_resume_lanes[16];
