@@ -489,12 +489,6 @@ int dcns_get_tuning(const dcns_ctx *ctx, dcns_tuning *out) {
   out->n_bins_tuned = (int32_t)std::min<size_t>(C.bin_tune.size(), 16);
   for (int b = 0; b < 16; ++b) {
     const bool own = b < (int)C.bin_tune.size();
-    out->xdrop_warp_from[b] = own ? C.bin_tune[b].xdrop_warp_from : C.xdrop_warp_from;
-    out->xdrop_wave_max_w[b] = own ? C.bin_tune[b].xdrop_wave_max_w : C.xdrop_wave_max_w;
-    out->xdrop_flat[b] = (own ? C.bin_tune[b].xdrop_flat : C.xdrop_flat) ? 1 : 0;
-    out->xdrop_handoff[b] = own ? C.bin_tune[b].xdrop_handoff : C.xdrop_handoff;
-    out->xdrop_resume_lanes[b] = own ? C.bin_tune[b].xdrop_resume_lanes : C.xdrop_resume_lanes;
-    out->xdrop_group_from[b] = own ? C.bin_tune[b].xdrop_group_from : C.xdrop_group_from;
     out->scan_tiles[b] = own ? C.bin_tune[b].scan_tiles : C.scan_tiles_per_thread;
   }
   return DCNS_OK;

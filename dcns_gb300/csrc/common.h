@@ -130,7 +130,7 @@ struct XTask {
   int32_t status;                      // 0 done, 1 band-edge restart needed (w doubled), 2 traceback slot too small
   int32_t iii, jjj, ncig;              // traceback results
   int64_t cig_off;                     // CIGAR slot (uint32 entries) and its capacity
-  int32_t cig_cap, pad;
+  int32_t cig_cap, tb_rows;            // tb_rows: rows to make room for in a slot taken from the arena
   int64_t cig_dense;                   // chained form: offset of the CIGAR in the batch's packed CIGAR array
 };
 
@@ -222,36 +222,25 @@ void launch_scan_generic_wave(const ScanTask *tasks, const int *idx, int n, cons
                               cudaStream_t st);
 void launch_reverse(ScanTask *tasks, int first, int n, const unsigned long long *keys, const int64_t *pair_base,
                     const int32_t *pair_len, Arena ar, Params p, cudaStream_t st);
-// wcap: 10 or 20 (one thread per pass, band in registers), 0 (one warp per pass, band in scratch), -1 (one warp per
-// pass as a wavefront, w <= 256: for long passes)
-void launch_xdrop(XTask *tasks, const int *idx, int n, Arena ar, Params p, uint32_t *tb, int wcap, int32_t *scratch,
-                  int64_t scratch_per_thread, cudaStream_t st);
-// tb_words: size of the band store tb (the traceback reads nothing past it)
-void launch_xdrop_traceback(XTask *tasks, const int *idx, int n, const uint32_t *tb, int64_t tb_words, uint32_t *cig,
-                            cudaStream_t st);
-// Chained x-drop levels (one launch per band width, work lists and counts in device memory).
-void launch_xdrop_iota(int *list, int n, int *count, cudaStream_t st);
-// Hand-off of long register-band passes to the wavefront form: a pass of a row-interleaved level still running after
-// `rows` rows moves its band state to one of `cap` spill slots (2 x (2 x 20 + 2) ints each) and its id to list;
-// *count (zero before the level) counts the slots taken; `lanes` lanes then run each such pass.  rows = 0 or
-// cap = 0: off.
-struct XHandoff {
-  int *list, *count;
-  int32_t *spill;
-  int cap, rows;
-  int lanes;  // lanes per handed-off pass: 4, 8 or 16 (G-lane groups, 32 / G passes per warp) or 32 (one warp)
+// Chained x-drop levels (one launch per band width, work lists and counts in device memory): a level runs the passes
+// of list_in, appends those that must restart to list_out (band doubled) and those whose traceback slot did not fit to
+// retry.  fetch: passes handed out, zero before the launch.  A host-driven round has no list_out (the host reads the
+// passes' status) and no tb_cursor (the passes have their slots).
+struct XLevel {
+  const int *list_in, *count_in;
+  int *list_out, *count_out, *retry, *retry_count, *fetch;
+  unsigned long long *tb_cursor;
+  int64_t tb_words;
 };
-constexpr int kXdropSpillInts = 2 * (2 * 20 + 2);
-// fetch: the level's pass counter, zero before the launch (the row-interleaved register-band kernel, flat = true).
-// Traceback slots hold min(n1, slot_rows) rows.  group_from > 0: register-band levels of band group_from and wider
-// run every pass on H.lanes-lane groups from row 1 (no one-thread form).  Returns the number of kernels launched.
-int launch_xdrop_level(XTask *tasks, const int *list_in, const int *count_in, int *list_out, int *count_out,
-                       int *retry, int *retry_count, unsigned long long *tb_cursor, int64_t tb_words, int slot_rows,
-                       int *fetch, const XHandoff &H, Arena ar, Params p, uint32_t *tb, int w, int n_bound, int nsm,
-                       int32_t *scratch, int64_t per_warp, int warps, int warp_from, int wave_max_w, bool flat,
-                       int group_from, bool codes, cudaStream_t st);
-void launch_xdrop_traceback_all(XTask *tasks, int n, const uint32_t *tb, int64_t tb_words, uint32_t *cig,
-                                unsigned long long *cig_cursor, cudaStream_t st);
+constexpr int kXdropBandMaxW = 325;  // wider bands run one warp per pass with the band in scratch
+int64_t xd_slot_words(int w, int64_t rows);  // 32-bit words of a traceback slot (a multiple of 4)
+void launch_xdrop_iota(int *list, int n, int *count, cudaStream_t st);
+// packed: match * min(n1, n2) < 2^20 for every pass.  scratch, per_warp, warps: bands above kXdropBandMaxW.
+void launch_xdrop_level(XTask *tasks, const XLevel &lv, Arena ar, Params p, uint32_t *tb, int w, int n_bound, int nsm,
+                        int32_t *scratch, int64_t per_warp, int warps, bool codes, bool packed, cudaStream_t st);
+void launch_xdrop_traceback(XTask *tasks, const int *idx, int n, const uint32_t *tb, uint32_t *cig, cudaStream_t st);
+void launch_xdrop_traceback_all(XTask *tasks, int n, const uint32_t *tb, uint32_t *cig, unsigned long long *cig_cursor,
+                                cudaStream_t st);
 // Packs the CIGARs of every finished task in task order into dense (cig_dense offsets); *total = their words.
 void launch_xdrop_cigar_pack(XTask *tasks, int n, const uint32_t *cig, uint32_t *dense, unsigned long long *total,
                              cudaStream_t st);

@@ -106,7 +106,7 @@ void release_device_buffers(Context &C) {
   if (C.st) cudaStreamSynchronize(C.st);  // nothing of the context still reads them
   DevBuf *bufs[] = {&C.d_codes, &C.d_srcoff, &C.d_dstbase, &C.d_len, &C.d_pk, &C.d_nm, &C.d_seqbase, &C.d_flag,
                     &C.d_tasks, &C.d_keys, &C.d_tiles, &C.d_counter, &C.d_idx, &C.d_scratch, &C.d_x, &C.d_tb,
-                    &C.d_cig, &C.d_sg, &C.d_sgtb, &C.d_bnd, &C.d_wts, &C.d_cats, &C.d_spill, &C.d_flow,
+                    &C.d_cig, &C.d_sg, &C.d_sgtb, &C.d_bnd, &C.d_wts, &C.d_cats, &C.d_flow,
                     &C.d_fpairs, &C.d_fwords, &C.d_ftiles};
   C.filt_on = false;
   for (DevBuf *b : bufs) b->release(C);
@@ -160,15 +160,6 @@ void init_context(Context &C, int device, size_t budget) {
   if (const char *e = std::getenv("DCNS_LANES")) C.max_lanes = std::max(1, std::min(8, std::atoi(e)));
   if (const char *e = std::getenv("DCNS_BINS")) C.bins = std::max(1, std::min(64, std::atoi(e)));
   if (const char *e = std::getenv("DCNS_TRACE")) C.trace = std::atoi(e);
-  if (const char *e = std::getenv("DCNS_XDROP_WARP_FROM")) C.xdrop_warp_from = std::max(0, std::atoi(e));
-  if (const char *e = std::getenv("DCNS_XDROP_WAVE")) C.xdrop_wave_max_w = std::max(0, std::atoi(e));
-  if (const char *e = std::getenv("DCNS_XDROP_FLAT")) C.xdrop_flat = std::atoi(e) != 0;
-  if (const char *e = std::getenv("DCNS_XDROP_HANDOFF")) C.xdrop_handoff = std::max(0, std::atoi(e));
-  if (const char *e = std::getenv("DCNS_XDROP_RESUME_LANES")) {
-    const int v = std::atoi(e);
-    C.xdrop_resume_lanes = (v == 4 || v == 8 || v == 16 || v == 32) ? v : 8;
-  }
-  if (const char *e = std::getenv("DCNS_XDROP_GROUP_FROM")) C.xdrop_group_from = std::max(0, std::atoi(e));
   if (const char *e = std::getenv("DCNS_SCAN_TILES")) C.scan_tiles_per_thread = std::max(1, std::min(64, std::atoi(e)));
   if (const char *e = std::getenv("DCNS_SCAN_FILTER")) C.scan_filter = std::atoi(e) != 0;
   if (const char *e = std::getenv("DCNS_SG_WARPS")) {
@@ -1229,8 +1220,6 @@ int64_t band_cells(int rows, int w, int n2) {
   return total;
 }
 
-int wpr_of(int w) { return (2 * w + 1 + 7) / 8; }
-
 // Device bytes the context's buffers hold, its lanes' included (buffers only grow, so after a call this is at least
 // what the call used).
 int64_t device_bytes(const Context &C) {
@@ -1240,14 +1229,36 @@ int64_t device_bytes(const Context &C) {
   return b;
 }
 
+// Scratch of the x-drop levels wider than the band form: warps and ints per warp of the kernel (512 MB at most).
+struct XScratch {
+  int warps = 0;
+  int64_t per_warp = 0;
+};
+XScratch xdrop_scratch(const Context &C, int64_t w, int64_t n) {
+  XScratch s;
+  if (w <= kXdropBandMaxW) return s;
+  s.per_warp = 2 * (2 * w + 2);
+  const int64_t cap = std::max<int64_t>(32, ((int64_t)512 << 20) / (4 * s.per_warp));
+  s.warps = (int)(std::min<int64_t>({n, cap, (int64_t)C.nsm * 64}) + 3) / 4 * 4;  // whole blocks of 4 warps
+  return s;
+}
+
+// The row maximum and its cell fit one word (launch_xdrop_level's packed form).
+bool xdrop_packed(const std::vector<XTask> &X, const Params &P) {
+  int64_t d = 0;
+  for (const XTask &T : X) d = std::max<int64_t>(d, std::min(T.n1, T.n2));
+  return d * P.match < (1 << 20);
+}
+
 // Runs the passes `subset` of X to completion in host-driven rounds (band restarts, traceback-slot growth), then
-// their tracebacks when want_codes; X lives on the host between launches.  Traceback slots start at the whole pass
-// (full_slots) or at min(n1, 1024) rows.  With want_codes, every finished pass's CIGAR is appended to *flat and
-// (*hoff)[k] is its offset there (X[k].ncig words).
+// their tracebacks when want_codes; X lives on the host between launches.  A round runs its passes by band width,
+// one launch each.  Traceback slots start at the whole pass (full_slots) or at min(n1, 1024) rows.  With want_codes,
+// every finished pass's CIGAR is appended to *flat and (*hoff)[k] is its offset there (X[k].ncig words).
 void run_xdrop_rounds(Context &C, std::vector<XTask> &X, const Params &P, bool want_codes, std::vector<uint32_t> *flat,
                       std::vector<int64_t> *hoff, const std::vector<int32_t> &subset, bool full_slots) {
   if (subset.empty()) return;
   const int64_t n = (int64_t)X.size();
+  const bool packed = xdrop_packed(X, P);
   std::vector<int64_t> rows_cap(n, 0);
   for (int32_t k : subset) {
     X[k].want_codes = want_codes ? 1 : 0;
@@ -1265,7 +1276,7 @@ void run_xdrop_rounds(Context &C, std::vector<XTask> &X, const Params &P, bool w
     if (want_codes)
       for (int32_t k : pend) {
         X[k].tb_off = words;
-        X[k].tb_cap = (int32_t)std::min<int64_t>(INT32_MAX, rows_cap[k] * wpr_of(X[k].w));
+        X[k].tb_cap = (int32_t)std::min<int64_t>(INT32_MAX / 4 * 4, xd_slot_words(X[k].w, rows_cap[k]));
         words += X[k].tb_cap;
       }
     if (want_codes) C.d_tb.ensure(C, sizeof(uint32_t) * std::max<int64_t>(words, 1));
@@ -1276,44 +1287,36 @@ void run_xdrop_rounds(Context &C, std::vector<XTask> &X, const Params &P, bool w
       for (int64_t q = b * 4096, e = std::min(m, q + 4096); q < e; ++q) Xc[q] = X[pend[q]];
     });
     h2d(C, C.d_x, Xc, (size_t)m);
-    // passes known to be long (they outgrew their slot in the levels: full_slots) run as wavefronts up to w = 256
-    std::vector<int32_t> g10, g20, gw, gwave;
-    int maxw = 0;
-    for (int64_t q = 0; q < m; ++q) {
-      const int w = Xc[q].w;
-      if (full_slots && w <= 256)
-        gwave.push_back((int32_t)q);
-      else if (w <= 10)
-        g10.push_back((int32_t)q);
-      else if (w <= 20)
-        g20.push_back((int32_t)q);
-      else
-        gw.push_back((int32_t)q), maxw = std::max(maxw, w);
+    std::map<int, std::vector<int32_t>> by_w;
+    for (int64_t q = 0; q < m; ++q) by_w[Xc[q].w].push_back((int32_t)q);
+    // one index list, then each width's count and its kernel's fetch counter
+    std::vector<int32_t> idx;
+    idx.reserve((size_t)m + 2 * by_w.size());
+    int64_t scratch_ints = 1;
+    for (const auto &e : by_w) {
+      idx.insert(idx.end(), e.second.begin(), e.second.end());
+      const XScratch sc = xdrop_scratch(C, e.first, (int64_t)e.second.size());
+      scratch_ints = std::max(scratch_ints, sc.warps * sc.per_warp);
     }
-    C.d_idx.ensure(C, sizeof(int32_t) * m);
-    size_t off = 0;
-    auto launch_group = [&](std::vector<int32_t> &g, int wcap) {
-      if (g.empty()) return;
-      h2d(C, C.d_idx, g.data(), g.size(), off);
-      int32_t *scratch = nullptr;
-      int64_t per = 0;
-      if (wcap == 0) {  // warp per pass: M and F of 2w+2 cells each
-        per = 2 * (2 * (int64_t)maxw + 2);
-        C.d_scratch.ensure(C, sizeof(int32_t) * per * g.size());
-        scratch = C.d_scratch.as<int32_t>();
-      }
-      launch_xdrop(C.d_x.as<XTask>(), C.d_idx.as<int>() + off, (int)g.size(), C.arena, P, C.d_tb.as<uint32_t>(),
-                   wcap, scratch, per, C.st);
-      C.stats.kernel_launches += 1;
-      C.stats.xdrop_passes += (int64_t)g.size();
-      off += g.size();
-    };
+    for (const auto &e : by_w) idx.push_back((int32_t)e.second.size()), idx.push_back(0);
+    C.d_idx.ensure(C, sizeof(int32_t) * idx.size());
+    if (scratch_ints > 1) C.d_scratch.ensure(C, sizeof(int32_t) * scratch_ints);
+    h2d(C, C.d_idx, idx.data(), idx.size());
     tp = phase(C, "xd_prep", tp);
     DCNS_CK(cudaEventRecord(C.ev0, C.st));
-    launch_group(gwave, -1);
-    launch_group(g10, 10);
-    launch_group(g20, 20);
-    launch_group(gw, 0);
+    int64_t off = 0, g = m;
+    for (const auto &e : by_w) {
+      int *const d = C.d_idx.as<int>();
+      const int64_t cnt = (int64_t)e.second.size();
+      const XScratch sc = xdrop_scratch(C, e.first, cnt);
+      const XLevel lv{d + off, d + g, nullptr, nullptr, nullptr, nullptr, d + g + 1, nullptr, 0};
+      launch_xdrop_level(C.d_x.as<XTask>(), lv, C.arena, P, C.d_tb.as<uint32_t>(), e.first, (int)cnt, C.nsm,
+                         C.d_scratch.as<int32_t>(), sc.per_warp, sc.warps, want_codes, packed, C.st);
+      C.stats.kernel_launches += 1;
+      C.stats.xdrop_passes += cnt;
+      off += cnt;
+      g += 2;
+    }
     DCNS_CK(cudaEventRecord(C.ev1, C.st));
     d2h(C, Xc, C.d_x, (size_t)m);
     sync(C);
@@ -1354,7 +1357,7 @@ void run_xdrop_rounds(Context &C, std::vector<XTask> &X, const Params &P, bool w
       h2d(C, C.d_x, Xc, (size_t)m);
       h2d(C, C.d_idx, fin_c.data(), fin_c.size());
       DCNS_CK(cudaEventRecord(C.ev1, C.st));
-      launch_xdrop_traceback(C.d_x.as<XTask>(), C.d_idx.as<int>(), (int)fin_c.size(), C.d_tb.as<uint32_t>(), words,
+      launch_xdrop_traceback(C.d_x.as<XTask>(), C.d_idx.as<int>(), (int)fin_c.size(), C.d_tb.as<uint32_t>(),
                              C.d_cig.as<uint32_t>(), C.st);
       DCNS_CK(cudaEventRecord(C.ev2, C.st));
       C.stats.kernel_launches += 1;
@@ -1397,6 +1400,7 @@ void run_xdrop_rounds(Context &C, std::vector<XTask> &X, const Params &P, bool w
 // are enqueued at once with their work lists in device memory, then one synchronisation.  Passes whose traceback
 // slot was too small (or the arena full) finish in host-driven rounds with whole-pass slots.  With want_codes,
 // every pass's CIGAR is in *flat at (*hoff)[k] (X[k].ncig words), in task order.
+// Passes with codes may say in tb_rows how many rows their slot should hold (0: unknown).
 void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_codes, std::vector<uint32_t> *flat,
                std::vector<int64_t> *hoff) {
   if (X.empty()) return;
@@ -1415,24 +1419,33 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
     T.score = T.end1 = T.end2 = T.rows = 0;
     T.iii = T.jjj = T.ncig = 0;
     maxdim = std::max<int64_t>(maxdim, std::max(T.n1, T.n2));
-    max_n1 = std::max<int64_t>(max_n1, T.n1);
+    if (T.tb_rows <= 0) max_n1 = std::max<int64_t>(max_n1, T.n1);
     if (want_codes) cig_words += (int64_t)std::max(T.n1, 0) + std::max(T.n2, 0) + 2;
   }
-  // Traceback slots of min(n1, slot_rows) rows, the arena sized for three slots per pass (a band restart takes a new
-  // slot of twice the width).  A slot is reserved for the pass's bound n1, not for the rows it will use, so slot_rows
-  // stays at 1,024-2,048: the longest pass up to 2,048 rows when that arena fits a quarter of the free device budget
-  // (passes longer than their slot are retried with whole-pass slots).
-  int slot_rows = 1024;
+  // Traceback slots: as many rows as the pass expects, or min(n1, slot_rows), the arena sized for eight or four slots
+  // at the first width (a band restart takes a new slot of twice the width).  Where nothing is known a slot is reserved for
+  // the pass's bound n1, not for the rows it will use, so slot_rows stays at 1,024-2,048: the longest pass up to
+  // 2,048 rows when that arena fits a quarter of the free device budget (passes longer than their slot are retried
+  // with whole-pass slots).
   if (want_codes) {
     auto words_for = [&](int64_t rows) {
       int64_t wsum = 1 << 20;
-      for (int64_t k = 0; k < n; ++k) wsum += 3 * std::min<int64_t>(X[k].n1, rows) * wpr_of(w0);
+      for (int64_t k = 0; k < n; ++k)
+        wsum += X[k].tb_rows > 0 ? 8 * xd_slot_words(w0, std::min<int64_t>(X[k].n1, X[k].tb_rows))
+                                 : 4 * xd_slot_words(w0, std::min<int64_t>(X[k].n1, rows));
       return wsum;
     };
     const int64_t room = (int64_t)((C.budget > C.used ? C.budget - C.used : 0) / 4);
     const int64_t want = std::min<int64_t>(max_n1, 2048);
+    int slot_rows = 1024;
     if (want > 1024 && (int64_t)sizeof(uint32_t) * words_for(want) <= room) slot_rows = (int)want;
     tb_words = words_for(slot_rows);
+    if ((int64_t)sizeof(uint32_t) * tb_words > room) {  // expected rows beyond the room: the long ones are retried
+      for (int64_t k = 0; k < n; ++k) X[k].tb_rows = std::min(X[k].tb_rows, 1024);
+      tb_words = words_for(slot_rows);
+    }
+    for (int64_t k = 0; k < n; ++k)
+      if (X[k].tb_rows <= 0) X[k].tb_rows = slot_rows;
   }
   auto tp = phase(C, "xc_setup", t0);
   if (!uniform || n >= INT32_MAX / 4) {
@@ -1440,27 +1453,17 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
     for (int64_t k = 0; k < n; ++k) all[k] = (int32_t)k;
     run_xdrop_rounds(C, X, P, want_codes, flat, hoff, all, false);
   } else {
+    const bool packed = xdrop_packed(X, P);
     int nlev = 1;
     while (((int64_t)w0 << (nlev - 1)) < maxdim) ++nlev;
-    // per level: warps of the wide-band kernel and their scratch (2 x (2w + 2) ints per warp, 512 MB at most)
-    std::vector<int> warps(nlev, 0);
-    std::vector<int64_t> per_warp(nlev, 0);
+    std::vector<XScratch> scr(nlev);
     int64_t scratch_ints = 1;
     for (int L = 0; L < nlev; ++L) {
-      const int64_t w = (int64_t)w0 << L;
-      if (w <= C.xdrop_warp_from || w <= std::min(C.xdrop_wave_max_w, 256)) continue;  // register band / wavefront
-      per_warp[L] = 2 * (2 * w + 2);
-      const int64_t cap = std::max<int64_t>(32, ((int64_t)512 << 20) / (4 * per_warp[L]));
-      warps[L] = (int)(std::min<int64_t>({n, cap, (int64_t)C.nsm * 64}) + 3) / 4 * 4;  // whole blocks of 4 warps
-      scratch_ints = std::max(scratch_ints, warps[L] * per_warp[L]);
+      scr[L] = xdrop_scratch(C, (int64_t)w0 << L, n);
+      scratch_ints = std::max(scratch_ints, scr[L].warps * scr[L].per_warp);
     }
-    // hand-off slots of the register-band levels (one level at a time: the resume kernel empties them before the
-    // next level starts)
-    const bool any_flat = C.xdrop_flat && C.xdrop_handoff > 0 && std::min(C.xdrop_warp_from, 20) >= w0;
-    const int spill_cap = any_flat ? (int)std::min<int64_t>(n, 1 << 16) : 0;
     C.d_x.ensure(C, sizeof(XTask) * n);
-    C.d_idx.ensure(C, sizeof(int32_t) * (3 * n + spill_cap + 4 + 2 * nlev + 64));
-    if (spill_cap > 0) C.d_spill.ensure(C, sizeof(int32_t) * (size_t)spill_cap * kXdropSpillInts);
+    C.d_idx.ensure(C, sizeof(int32_t) * (3 * n + 4 + nlev + 64));
     C.d_counter.ensure(C, 64);
     if (want_codes) {
       C.d_tb.ensure(C, sizeof(uint32_t) * tb_words);
@@ -1468,37 +1471,32 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
     }
     if (scratch_ints > 1) C.d_scratch.ensure(C, sizeof(int32_t) * scratch_ints);
     int *lists = C.d_idx.as<int>();
-    // [0], [1]: the two work-list counts, [2]: retry count, [4 + L]: level L's fetch, [4 + nlev + L]: its hand-offs
-    int *cnt = lists + 3 * n;
-    int *long_list = cnt + 4 + 2 * nlev + 64;
+    int *cnt = lists + 3 * n;  // [0], [1]: the two work-list counts, [2]: retry count, [4 + L]: level L's fetch
     unsigned long long *cur = C.d_counter.as<unsigned long long>();  // [0]: traceback arena, [1]: CIGAR arena
     h2d(C, C.d_x, X.data(), (size_t)n);
-    DCNS_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * (4 + 2 * nlev), C.st));
+    DCNS_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * (4 + nlev), C.st));
     DCNS_CK(cudaMemsetAsync(cur, 0, sizeof(unsigned long long) * 2, C.st));
     launch_xdrop_iota(lists, (int)n, cnt, C.st);
     DCNS_CK(cudaEventRecord(C.ev0, C.st));
-    int in = 0, launched = 0;
+    int in = 0;
     for (int L = 0; L < nlev; ++L) {
       const int out = 1 - in;
       DCNS_CK(cudaMemsetAsync(cnt + out, 0, sizeof(int), C.st));
-      const XHandoff H{long_list, cnt + 4 + nlev + L, C.d_spill.as<int32_t>(), spill_cap, C.xdrop_handoff,
-                       C.xdrop_resume_lanes};
-      launched += launch_xdrop_level(C.d_x.as<XTask>(), lists + in * n, cnt + in, lists + out * n, cnt + out,
-                                     lists + 2 * n, cnt + 2, cur, want_codes ? tb_words : 0, slot_rows, cnt + 4 + L, H,
-                                     C.arena, P, C.d_tb.as<uint32_t>(), w0 << L, (int)n, C.nsm,
-                                     C.d_scratch.as<int32_t>(), per_warp[L], warps[L], C.xdrop_warp_from,
-                                     C.xdrop_wave_max_w, C.xdrop_flat, C.xdrop_group_from, want_codes, C.st);
+      const XLevel lv{lists + in * n, cnt + in, lists + out * n, cnt + out, lists + 2 * n, cnt + 2, cnt + 4 + L, cur,
+                      want_codes ? tb_words : 0};
+      launch_xdrop_level(C.d_x.as<XTask>(), lv, C.arena, P, C.d_tb.as<uint32_t>(), w0 << L, (int)n, C.nsm,
+                         C.d_scratch.as<int32_t>(), scr[L].per_warp, scr[L].warps, want_codes, packed, C.st);
       in = out;
     }
     DCNS_CK(cudaEventRecord(C.ev1, C.st));
     if (want_codes) {
-      launch_xdrop_traceback_all(C.d_x.as<XTask>(), (int)n, C.d_tb.as<uint32_t>(), tb_words, C.d_cig.as<uint32_t>(),
-                                 cur + 1, C.st);
+      launch_xdrop_traceback_all(C.d_x.as<XTask>(), (int)n, C.d_tb.as<uint32_t>(), C.d_cig.as<uint32_t>(), cur + 1,
+                                 C.st);
       launch_xdrop_cigar_pack(C.d_x.as<XTask>(), (int)n, C.d_cig.as<uint32_t>(), C.d_cig.as<uint32_t>() + cig_words,
                               cur + 1, C.st);
       DCNS_CK(cudaEventRecord(C.ev2, C.st));
     }
-    C.stats.kernel_launches += launched + 1 + (want_codes ? 3 : 0);
+    C.stats.kernel_launches += nlev + 1 + (want_codes ? 3 : 0);
     C.stats.xdrop_rounds += 1;
     C.h_misc.ensure(sizeof(int32_t) * (n + 8) + 64);
     int32_t *hret = C.h_misc.as<int32_t>();  // [0]: leftover count, [1]: retry count, [8..]: retry list
@@ -1574,7 +1572,6 @@ void extend_seeds(Context &C, const std::vector<PairIn> &pairs, const Params &P,
   const int64_t np = (int64_t)pairs.size();
   res.assign(np, {});
   std::vector<XTask> F;
-  std::vector<std::pair<int32_t, int32_t>> owner;
   for (int64_t p = 0; p < np; ++p) {
     res[p].resize(linked[p].size());
     for (size_t s = 0; s < linked[p].size(); ++s) {
@@ -1589,7 +1586,6 @@ void extend_seeds(Context &C, const std::vector<PairIn> &pairs, const Params &P,
       x.dir = 0;
       x.w = P.w;
       F.push_back(x);
-      owner.push_back({(int32_t)p, (int32_t)s});
     }
   }
   C.stats.seeds += (int64_t)F.size();
@@ -1597,61 +1593,90 @@ void extend_seeds(Context &C, const std::vector<PairIn> &pairs, const Params &P,
   run_xdrop(C, F, P, false, nullptr, nullptr);
   tp = phase(C, "xs_run_fwd", tp);
   const int64_t nf = (int64_t)F.size();
-  std::vector<int32_t> rslot(nf + 1, 0);  // reverse task of forward pass k (exclusive prefix over kept passes)
-  parallel_for((nf + 4095) / 4096, [&](int64_t b) {
-    for (int64_t k = b * 4096, e = std::min(nf, k + 4096); k < e; ++k) {
+  // The reverse pass depends on the forward end alone, and the seeds of one alignment mostly extend to the same end:
+  // one reverse pass per distinct end of a pair serves them all.  rev[k]: forward pass k's reverse pass within its
+  // pair (-1: no forward end); rfirst[p]: the pair's first reverse pass.
+  std::vector<int64_t> fbeg(np + 1, 0), rfirst(np + 1, 0);
+  for (int64_t p = 0; p < np; ++p) fbeg[p + 1] = fbeg[p] + (int64_t)linked[p].size();
+  std::vector<int32_t> rev(nf);
+  std::vector<int32_t> rlead(nf);  // at fbeg[p] + q: the forward pass that reverse pass q of pair p was made from
+  parallel_for(np, [&](int64_t p) {
+    std::vector<std::pair<std::pair<int32_t, int32_t>, int32_t>> ends;
+    for (int64_t k = fbeg[p]; k < fbeg[p + 1]; ++k) {
       const XTask &f = F[k];
-      XSeedOut &o = res[owner[k].first][owner[k].second];
+      XSeedOut &o = res[p][k - fbeg[p]];
       o.ok = false;
       o.score = f.score;
       o.cig_off = 0;
       o.cig_len = 0;
-      rslot[k + 1] = (f.end1 - 1 < 0 || f.end2 - 1 < 0) ? 0 : 1;  // p = 100 otherwise
+      rev[k] = -1;
+      if (f.end1 - 1 < 0 || f.end2 - 1 < 0) continue;  // p = 100
+      ends.push_back({{f.a1 + f.end1 - 1, f.a2 + f.end2 - 1}, (int32_t)k});
     }
+    std::sort(ends.begin(), ends.end());
+    int32_t q = -1;
+    for (size_t i = 0; i < ends.size(); ++i) {
+      if (i == 0 || ends[i].first != ends[i - 1].first) rlead[fbeg[p] + ++q] = ends[i].second;
+      rev[ends[i].second] = q;
+    }
+    rfirst[p + 1] = q + 1;
   });
-  for (int64_t k = 0; k < nf; ++k) rslot[k + 1] += rslot[k];
-  std::vector<XTask> R(rslot[nf]);
-  std::vector<int32_t> rmap(rslot[nf]);
-  parallel_for((nf + 4095) / 4096, [&](int64_t b) {
-    for (int64_t k = b * 4096, e = std::min(nf, k + 4096); k < e; ++k) {
-      if (rslot[k + 1] == rslot[k]) continue;
-      const XTask &f = F[k];
-      const int32_t b1 = f.a1 + f.end1 - 1, b2 = f.a2 + f.end2 - 1;
+  for (int64_t p = 0; p < np; ++p) rfirst[p + 1] += rfirst[p];
+  std::vector<XTask> R((size_t)rfirst[np]);
+  const int64_t slack = 512 + std::min<int64_t>(16384, ((int64_t)16 << 20) / std::max<int64_t>(rfirst[np], 1));
+  parallel_for(np, [&](int64_t p) {
+    for (int64_t q = rfirst[p]; q < rfirst[p + 1]; ++q) {
+      const XTask &f = F[rlead[fbeg[p] + q - rfirst[p]]];
       XTask r{};
       r.base1 = f.base1;
       r.base2 = f.base2;
-      r.a1 = b1;
-      r.a2 = b2;
-      r.n1 = b1 + 1;
-      r.n2 = b2 + 1;
+      r.a1 = f.a1 + f.end1 - 1;
+      r.a2 = f.a2 + f.end2 - 1;
+      r.n1 = r.a1 + 1;
+      r.n2 = r.a2 + 1;
       r.dir = 1;
       r.w = P.w;
-      R[rslot[k]] = r;
-      rmap[rslot[k]] = (int32_t)k;
+      R[q] = r;
     }
+    // rows a reverse pass will need: about those of the longest forward pass that ends there, and what it adds
+    // beyond that pass's start (more of it where there are few passes)
+    for (int64_t k = fbeg[p]; k < fbeg[p + 1]; ++k)
+      if (rev[k] >= 0) {
+        XTask &r = R[rfirst[p] + rev[k]];
+        r.tb_rows = (int32_t)std::max<int64_t>(r.tb_rows, std::min<int64_t>(r.n1, slack + F[k].end1 + F[k].end1 / 2));
+      }
   });
   std::vector<int64_t> hoff;
   tp = phase(C, "xs_build_rev", tp);
+  const int64_t cells0 = C.stats.cells_xdrop, codes0 = C.stats.bytes_codes_xdrop, passes0 = C.stats.xdrop_passes;
   run_xdrop(C, R, P, want_cigar, want_cigar ? &cig_flat : nullptr, want_cigar ? &hoff : nullptr);
+  // the algorithm's cells and passes: one reverse pass per seed
+  C.stats.cells_xdrop = cells0, C.stats.bytes_codes_xdrop = codes0, C.stats.xdrop_passes = passes0;
   tp = phase(C, "xs_run_rev", tp);
-  for (size_t q = 0; q < R.size(); ++q) {
-    const XTask &r = R[q];
-    const XTask &f = F[rmap[q]];
-    XSeedOut &o = res[owner[rmap[q]].first][owner[rmap[q]].second];
-    o.score = r.score;
-    if (want_cigar) o.cig_off = hoff[q], o.cig_len = r.ncig;
-    if (r.end1 - 1 < 0 || r.end2 - 1 < 0) continue;
-    const int32_t b1 = f.a1 + f.end1 - 1, b2 = f.a2 + f.end2 - 1;
-    o.ok = true;
-    o.end1 = b1;
-    o.end2 = b2;
-    o.start1 = b1 - (r.end1 - 1);
-    o.start2 = b2 - (r.end2 - 1);
-    if (want_cigar) {
-      o.end1 -= r.iii;
-      o.end2 -= r.jjj;
+  for (int64_t p = 0; p < np; ++p)
+    for (int64_t k = fbeg[p]; k < fbeg[p + 1]; ++k) {
+      if (rev[k] < 0) continue;
+      const int64_t q = rfirst[p] + rev[k];
+      const XTask &r = R[q], &f = F[k];
+      XSeedOut &o = res[p][k - fbeg[p]];
+      const int64_t cells = band_cells(r.rows, r.w, r.n2);
+      C.stats.cells_xdrop += cells;
+      if (want_cigar) C.stats.bytes_codes_xdrop += (cells + 1) / 2;
+      for (int w = P.w; w <= r.w; w *= 2) C.stats.xdrop_passes += 1;
+      o.score = r.score;
+      if (want_cigar) o.cig_off = hoff[q], o.cig_len = r.ncig;
+      if (r.end1 - 1 < 0 || r.end2 - 1 < 0) continue;
+      const int32_t b1 = f.a1 + f.end1 - 1, b2 = f.a2 + f.end2 - 1;
+      o.ok = true;
+      o.end1 = b1;
+      o.end2 = b2;
+      o.start1 = b1 - (r.end1 - 1);
+      o.start2 = b2 - (r.end2 - 1);
+      if (want_cigar) {
+        o.end1 -= r.iii;
+        o.end2 -= r.jjj;
+      }
     }
-  }
 }
 
 // ------------------------------------------------------------------ 2-gap stage (:532-616)
@@ -2347,36 +2372,10 @@ void autotune(Context &C, Batch &B, const Params &P, int mode) {
   }
   C.max_lanes = best.lanes, C.bins = best.bins, C.bin_ratio = best.ratio, C.bins_by_size = best.by_size;
 
-  // Per bin: the x-drop pass forms (register-band levels row-interleaved or one pass per thread, the band where one
-  // warp per pass takes over, the widest band of the wavefront form, the rows after which a register-band pass moves
-  // to the wavefront form), chosen by that bin's x-drop kernel time with
-  // each candidate applied to every bin; the bins differ in how many long and wide-band passes they hold.
+  // every bin starts from the call's tiling target
   C.bin_tune.clear();
-  if (C.max_lanes > 1 && (int64_t)B.lens.size() >= 4096) {
-    const int h = C.xdrop_handoff, g = C.xdrop_resume_lanes, gf = C.xdrop_group_from, ts = C.scan_tiles_per_thread;
-    // the first candidate is the context's setting (the incumbent)
-    const Context::BinTune cands[] = {
-        {C.xdrop_warp_from, C.xdrop_wave_max_w, C.xdrop_flat, h, g, gf, ts},
-        {20, 256, false, 0, g, 0, ts},    {10, 256, true, h, g, gf, ts},   {20, 256, true, 0, g, 0, ts},
-        {20, 256, true, 48, g, gf, ts},   {20, 256, true, 192, g, gf, ts}, {20, 256, true, 48, 32, 0, ts},
-        {20, 256, true, 96, 32, 0, ts},   {20, 128, true, h, g, gf, ts},   {20, 256, true, h, 4, gf, ts},
-        {20, 256, true, 48, 4, gf, ts},   {20, 256, true, h, g, 20, ts},   {20, 256, true, 48, g, 20, ts},
-        {20, 256, true, h, 4, 20, ts},    {20, 256, true, h, g, 10, ts}};
-    const int nb = std::max(C.bins, C.max_lanes);
-    std::vector<double> best_ms(nb, 1e300);
-    std::vector<Context::BinTune> choice(nb, cands[0]);
-    for (const Context::BinTune &cd : cands) {
-      C.bin_tune.assign(nb, cd);
-      run(best);
-      std::vector<double> ms = C.last_bin_xdrop_ms;
-      run(best);
-      for (int b = 0; b < nb && b < (int)ms.size() && b < (int)C.last_bin_xdrop_ms.size(); ++b) {
-        const double m = std::min(ms[b], C.last_bin_xdrop_ms[b]);
-        if (best_ms[b] == 1e300 || better(m, best_ms[b])) best_ms[b] = m, choice[b] = cd;
-      }
-    }
-    C.bin_tune = choice;
-  }
+  if (C.max_lanes > 1 && (int64_t)B.lens.size() >= 4096)
+    C.bin_tune.assign(std::max(C.bins, C.max_lanes), Context::BinTune{C.scan_tiles_per_thread});
   // the scan's tiling target (tiles per resident thread before reference rows are split into chunks; it matters
   // for batches of few long pairs) and, on the 2-gap path, the 2-piece kernel's warps per DP: by whole-call time
   // (for the whole call, and per bin by that bin's seed-scan kernel time over the same runs)
@@ -2513,7 +2512,7 @@ void align_core(Context &C, const std::vector<PairIn> &pairs, const Params &P, i
   std::vector<std::string> errs(nl);
   std::vector<int> codes(nl, 0);
   std::vector<dcns_stats> st(nl, dcns_stats{});
-  std::vector<double> bin_xdrop_ms(kBins, 0.0), bin_scan_ms(kBins, 0.0);
+  std::vector<double> bin_scan_ms(kBins, 0.0);
   auto worker = [&](int l) {
     Context &L = *C.lanes[l];
     try {
@@ -2539,15 +2538,9 @@ void align_core(Context &C, const std::vector<PairIn> &pairs, const Params &P, i
                                 cudaMemcpyHostToDevice, L.st));
         L.seqbase_dev = L.d_seqbase.as<int64_t>();
         L.stats = dcns_stats{};
-        // the bin's kernel shapes: the autotuner's per-bin choice, else the parent context's
-        const Context::BinTune bt = b < (int)C.bin_tune.size()
-                                        ? C.bin_tune[b]
-                                        : Context::BinTune{C.xdrop_warp_from, C.xdrop_wave_max_w, C.xdrop_flat,
-                                                           C.xdrop_handoff, C.xdrop_resume_lanes, C.xdrop_group_from,
-                                                           C.scan_tiles_per_thread};
-        L.xdrop_warp_from = bt.xdrop_warp_from, L.xdrop_wave_max_w = bt.xdrop_wave_max_w, L.xdrop_flat = bt.xdrop_flat;
-        L.xdrop_handoff = bt.xdrop_handoff, L.xdrop_resume_lanes = bt.xdrop_resume_lanes;
-        L.xdrop_group_from = bt.xdrop_group_from;
+        // the bin's tiling target: the autotuner's per-bin choice, else the parent context's
+        const Context::BinTune bt =
+            b < (int)C.bin_tune.size() ? C.bin_tune[b] : Context::BinTune{C.scan_tiles_per_thread};
         L.sg_warps = C.sg_warps;
         L.sg_flow = C.sg_flow;
         L.sg_flow_blocks = C.sg_flow_blocks;
@@ -2564,7 +2557,6 @@ void align_core(Context &C, const std::vector<PairIn> &pairs, const Params &P, i
         align_single(L, sub, P, mode, so);
         pass.failed = false;
         for (size_t k = 0; k < ids.size(); ++k) out[ids[k]] = std::move(so[k]);
-        bin_xdrop_ms[b] = L.stats.ms_xdrop_kernel;
         bin_scan_ms[b] = L.stats.ms_scan_kernel;
         add_stats(st[l], L.stats);
       }
@@ -2584,7 +2576,6 @@ void align_core(Context &C, const std::vector<PairIn> &pairs, const Params &P, i
   for (int l = 0; l < nl; ++l)
     if (codes[l]) throw Error(codes[l], errs[l]);
   for (int l = 0; l < nl; ++l) add_stats(C.stats, st[l]);
-  C.last_bin_xdrop_ms = std::move(bin_xdrop_ms);
   C.last_bin_scan_ms = std::move(bin_scan_ms);
 }
 

@@ -105,7 +105,7 @@ struct Context {
   // device buffers
   DevBuf d_codes, d_srcoff, d_dstbase, d_len, d_pk, d_nm, d_seqbase, d_flag;
   DevBuf d_tasks, d_keys, d_tiles, d_counter, d_idx, d_scratch;
-  DevBuf d_x, d_tb, d_cig, d_sg, d_sgtb, d_bnd, d_wts, d_cats, d_spill, d_flow;
+  DevBuf d_x, d_tb, d_cig, d_sg, d_sgtb, d_bnd, d_wts, d_cats, d_flow;
   // the seed-scan filter's tables, marks and tile list (scanfilter.cu); `filt` describes the marks of the call's
   // sequences while `filt_on`.  Buffers that later work needs the room of are given back (drop_filter).
   DevBuf d_fpairs, d_fwords, d_ftiles;
@@ -128,19 +128,6 @@ struct Context {
   bool is_lane = false;
   double bin_ratio = 0.6;    // bin b holds a share of the work proportional to bin_ratio^b (later bins smaller)
   bool bins_by_size = false;  // bins are consecutive runs of pairs in increasing size (else a mix of sizes each)
-  int xdrop_warp_from = 20;  // x-drop bands wider than this run one warp per pass (DCNS_XDROP_WARP_FROM)
-  // x-drop bands wider than xdrop_warp_from and up to this run as one-warp wavefronts (DCNS_XDROP_WAVE; 0 = off)
-  int xdrop_wave_max_w = 256;
-  // register-band levels (w <= 20) as the row-interleaved kernel (DCNS_XDROP_FLAT=0: one pass per thread)
-  bool xdrop_flat = true;
-  // a pass of a row-interleaved level still running after this many rows moves to the wavefront form
-  // (DCNS_XDROP_HANDOFF; 0 = off)
-  int xdrop_handoff = 96;
-  // lanes that run each handed-off pass as a wavefront: 4, 8, 16 or 32 (DCNS_XDROP_RESUME_LANES)
-  int xdrop_resume_lanes = 8;
-  // register-band levels of this band and wider run every pass on lane groups from row 1 (DCNS_XDROP_GROUP_FROM;
-  // 0 = off)
-  int xdrop_group_from = 0;
   // warps per DP of the unweighted semi-global kernel: 2, 4 or 8 (DCNS_SG_WARPS; 0 = by the number of DPs)
   int sg_warps = 0;
   // unweighted semi-global DPs as a flow of stripe units over one persistent grid (DCNS_SG_FLOW=0: one CTA per DP)
@@ -151,16 +138,11 @@ struct Context {
   // resident thread (DCNS_SCAN_TILES)
   int scan_tiles_per_thread = 8;
   bool scan_filter = true;  // DCNS_SCAN_FILTER=0: every window against its whole reference, as without the filter
-  // per-bin x-drop pass forms and seed-scan tiling target chosen by the autotuner (empty: the values above for every
-  // bin)
+  // per-bin seed-scan tiling target chosen by the autotuner (empty: the value above for every bin)
   struct BinTune {
-    int xdrop_warp_from, xdrop_wave_max_w;
-    bool xdrop_flat;
-    int xdrop_handoff, xdrop_resume_lanes, xdrop_group_from;
     int scan_tiles;
   };
   std::vector<BinTune> bin_tune;
-  std::vector<double> last_bin_xdrop_ms;  // x-drop kernel time of each bin of the last binned call
   std::vector<double> last_bin_scan_ms;   // seed-scan kernel time of each bin of the last binned call
   // Level-0 turnstile of one binned call: the bins enqueue their level-0 scans on the parent's bulk stream in bin
   // order, so the scans run one after another and the first bins' host work overlaps the later bins' scans.

@@ -176,17 +176,15 @@ int dcns_measure_scan_roofline(dcns_ctx *ctx, double *gcups);
 int dcns_ctx_set_lanes(dcns_ctx *ctx, int lanes, int bins);
 
 /* Autotuner (no counterpart in the reference): aligns the resident batch once per candidate pipeline shape (lanes,
- * bins, and the geometric ratio of bin sizes), times each call, and keeps the fastest on the context; then, per bin,
- * the x-drop pass forms by that bin's x-drop kernel time, and by whole-call time the seed scan's tiling target and
- * (2-gap mode) the 2-piece kernel's warps per DP (dcns_get_tuning reports them).  The pipeline shape is returned (any
- * pointer may be NULL).  Results do not depend on any of these; this only tunes throughput for batches like this. */
+ * bins, and the geometric ratio of bin sizes), times each call, and keeps the fastest on the context; then, by
+ * whole-call time, the seed scan's tiling target (and per bin, by that bin's scan time) and (2-gap mode) the 2-piece
+ * kernel's form (dcns_get_tuning reports them).  The pipeline shape is returned (any pointer may be NULL).  Results do
+ * not depend on any of these; this only tunes throughput for batches like this. */
 int dcns_autotune(dcns_ctx *ctx, dcns_batch *batch, const dcns_params *params, int mode, int *lanes, int *bins,
                   double *bin_ratio);
 
 /* The context's kernel shapes (no counterpart in the reference): what dcns_autotune chose, or the defaults and the
- * DCNS_* environment settings.  Per bin (at most 16 reported): the x-drop band from which passes run one warp each,
- * the widest band of the one-warp wavefront form, whether the register-band levels run row-interleaved, the rows
- * after which a register-band pass moves to the wavefront form (0: never), and the lanes per such pass (8, 16, 32). */
+ * DCNS_* environment settings. */
 typedef struct {
   int32_t lanes, bins;
   double bin_ratio;
@@ -196,9 +194,10 @@ typedef struct {
   int32_t sg_flow;                /* 1: 2-piece DPs run as a flow of 128-row stripe units over one persistent grid */
   int32_t sg_flow_blocks;         /* resident blocks per SM of that grid: 4, 5 or 6 */
   int32_t bins_by_size;           /* 1: bins are runs of pairs in increasing size (the largest last); 0: mixed */
-  int32_t n_bins_tuned;           /* bins with their own x-drop forms below (0: every bin uses bin 0's values) */
+  int32_t n_bins_tuned;           /* bins with their own tiling target below (0: every bin uses bin 0's value) */
+  /* no longer set (an x-drop pass has one form per band width): zero */
   int32_t xdrop_warp_from[16], xdrop_wave_max_w[16], xdrop_flat[16], xdrop_handoff[16], xdrop_resume_lanes[16];
-  int32_t xdrop_group_from[16]; /* register-band levels of this band and wider: every pass on lane groups (0: off) */
+  int32_t xdrop_group_from[16];
   int32_t scan_tiles[16];       /* each bin's seed-scan tiling target */
 } dcns_tuning;
 int dcns_get_tuning(const dcns_ctx *ctx, dcns_tuning *out);
