@@ -220,8 +220,9 @@ void launch_scan_generic(const ScanTask *tasks, const int *idx, int n, const int
 void launch_scan_generic_wave(const ScanTask *tasks, const int *idx, int n, const int64_t *seq_base, Arena ar,
                               Params p, unsigned long long *keys, int32_t *scratch, int64_t per_task,
                               cudaStream_t st);
+// window: every task is at most kScanW columns wide.
 void launch_reverse(ScanTask *tasks, int first, int n, const unsigned long long *keys, const int64_t *pair_base,
-                    const int32_t *pair_len, Arena ar, Params p, cudaStream_t st);
+                    const int32_t *pair_len, Arena ar, Params p, bool window, cudaStream_t st);
 // Chained x-drop levels (one launch per band width, work lists and counts in device memory): a level runs the passes
 // of list_in, appends those that must restart to list_out (band doubled) and those whose traceback slot did not fit to
 // retry.  fetch: passes handed out, zero before the launch.  A host-driven round has no list_out (the host reads the

@@ -579,7 +579,7 @@ bool run_filtered_round(Context &C, ScanState &S, const Params &P, int64_t first
   launch_scan_tiles_rec(D, T, C.arena, P, C.d_keys.as<unsigned long long>(), cnt, C.nsm * C.scan_blocks_per_sm, C.st);
   DCNS_CK(cudaEventRecord(C.ev1, C.st));
   launch_reverse(C.d_tasks.as<ScanTask>(), (int)d0, (int)n, C.d_keys.as<unsigned long long>(), C.seqbase_dev,
-                 nullptr, C.arena, P, C.st);
+                 nullptr, C.arena, P, true, C.st);
   C.stats.scan_launches += 1;
   C.stats.kernel_launches += 3;
   int tiles = 0;
@@ -647,7 +647,7 @@ void run_scan_round(Context &C, ScanState &S, const Params &P, int64_t first, in
     C.stats.kernel_launches += (nthread > 0) + (nwave > 0);
   }
   launch_reverse(C.d_tasks.as<ScanTask>(), (int)d0, (int)n, C.d_keys.as<unsigned long long>(), C.seqbase_dev,
-                 nullptr, C.arena, P, C.st);
+                 nullptr, C.arena, P, generic.empty(), C.st);
   C.stats.kernel_launches += 1;
   d2h(C, S.tasks.data() + first, C.d_tasks, (size_t)n, (size_t)d0);
   sync(C);

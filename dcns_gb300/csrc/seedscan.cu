@@ -632,7 +632,53 @@ void launch_scan_generic(const ScanTask *tasks, const int *idx, int n, const int
 // (getSeeds :150-166); start = end - (reverse end).
 constexpr int kRevMax = 128;
 
-__global__ void reverse_kernel(ScanTask *__restrict__ tasks, int first, int n,
+// The reverse scan of a window of at most kScanW columns (striped semantics, which the reference's dispatch always
+// picks at these sizes: at most 2 x 38 rows of int8 scores) with the DP's row in one thread's registers: the maximum's
+// first place in row-major order.  Scores by byte permutation; columns past the read (cols < kScanW) score -128, which
+// keeps them below the maximum of the row above; the row's first maximum as one key (value, then column).  Bound:
+// integer issue (about 350 instructions a row).  Against the general form below, whose rows lay in local memory: one
+// 1 kb pair's windows 209 -> 30 us, those of the largest bin of the 10,000-pair batch (some 100,000) 1.03 -> 0.17 ms.
+__device__ void sw_reverse_window(const Arena &ar, const Params &P, const SeqView &s1, int rows, const SeqView &s2,
+                                  int cols, int &bi, int &bj) {
+  const int open = P.open1, ext = P.ext1, g = max(P.ext1, P.open1);
+  uint32_t sel[(kScanW + 1) / 2];  // two 16-bit selectors a word
+  Syms16 q{0, 0};
+#pragma unroll
+  for (int p = 0; p < kScanW; ++p) {
+    if (p % 16 == 0) q = load16(ar, s2, cols, p);
+    const uint32_t sl = p < cols ? sym_selector(q) & 0xFFFFu : 0xDDD5u;  // byte 5: -128
+    sel[p / 2] = p % 2 ? sel[p / 2] | sl << 16 : sl;
+    next_sym(q);
+  }
+  int H[kScanW], E[kScanW];
+#pragma unroll
+  for (int p = 0; p < kScanW; ++p) H[p] = 0, E[p] = 0;
+  int best = 0;
+  bi = bj = -1;
+  Syms16 r{0, 0};
+  for (int i = 0; i < rows; ++i) {
+    if (i % 16 == 0) r = load16(ar, s1, rows, i);
+    const uint32_t prof = sym_profile(r, P.match, P.mismatch);
+    next_sym(r);
+    int diag = 0, F = g, key = 0;
+#pragma unroll
+    for (int p = 0; p < kScanW; ++p) {
+      const int sc = perm_score(prof, 0x00008000u, p % 2 ? sel[p / 2] >> 16 : sel[p / 2]);
+      const int pre = __viaddmax_s32_relu(diag, sc, E[p]);
+      diag = H[p];
+      const int t = pre + open;
+      E[p] = __viaddmax_s32(E[p], ext, t);
+      H[p] = max(pre, F);
+      F = __viaddmax_s32(F, g, t);
+      key = max(key, H[p] * 64 + (63 - p));
+    }
+    if ((key >> 6) > best) best = key >> 6, bi = i, bj = 63 - (key & 63);
+  }
+}
+
+// WINDOW: every task is a window of at most kScanW columns.
+template <bool WINDOW>
+__global__ void __launch_bounds__(128) reverse_kernel(ScanTask *__restrict__ tasks, int first, int n,
                                const unsigned long long *__restrict__ keys, const int64_t *__restrict__ seq_base,
                                Arena ar, Params P) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -651,12 +697,16 @@ __global__ void reverse_kernel(ScanTask *__restrict__ tasks, int first, int n,
   const int e1 = min(row - T.lo + 1, lim), e2 = min(col + 1, lim);
   const int64_t b1 = seq_base[2 * T.pair], b2 = seq_base[2 * T.pair + 1];
   const int end1 = row, end2 = T.s2 + col;
-  int32_t H[kRevMax + 1], Hp[kRevMax + 1], E[kRevMax + 1];
   int best, bi, bj;
-  if (e2 > kRevMax) return;  // windows wider than kRevMax are rejected by the host before launch
-  sw_one([&](int i) { return 4 - base_code(ar, b1 + end1 - i); }, e1,
-         [&](int p) { return 4 - base_code(ar, b2 + end2 - p); }, e2, P.open1, P.ext1, P.match, P.mismatch,
-         striped_for(e1, e2, P.open1, P.ext1, P.match), H, Hp, E, best, bi, bj);
+  if constexpr (WINDOW) {
+    sw_reverse_window(ar, P, SeqView{b1, end1, 1}, e1, SeqView{b2, end2, 1}, e2, bi, bj);
+  } else {
+    int32_t H[kRevMax + 1], Hp[kRevMax + 1], E[kRevMax + 1];
+    if (e2 > kRevMax) return;  // windows wider than kRevMax are rejected by the host before launch
+    sw_one([&](int i) { return 4 - base_code(ar, b1 + end1 - i); }, e1,
+           [&](int p) { return 4 - base_code(ar, b2 + end2 - p); }, e2, P.open1, P.ext1, P.match, P.mismatch,
+           striped_for(e1, e2, P.open1, P.ext1, P.match), H, Hp, E, best, bi, bj);
+  }
   T.start1 = end1 - bi;
   T.start2 = end2 - bj;
 }
@@ -731,7 +781,8 @@ __global__ void l0_emit_kernel(const unsigned long long *__restrict__ keys, int6
 
 // The reverse re-scan of every compacted level-0 window (one thread each, all busy): the window's start is the
 // argmax of Smith-Waterman on the reverse complements ending at the forward maximum, over at most tw + window
-// cells each way (findSimilarFragmentsForPairedSequence4.cpp:131-201).
+// cells each way (findSimilarFragmentsForPairedSequence4.cpp:131-201).  Level 0 on the device has windows of at most
+// kScanW columns.
 __global__ void __launch_bounds__(128) l0_reverse_kernel(L0Rec *__restrict__ recs, const int *__restrict__ count,
                                                          const int64_t *__restrict__ wstart,
                                                          const int2 *__restrict__ plen, int np,
@@ -756,11 +807,8 @@ __global__ void __launch_bounds__(128) l0_reverse_kernel(L0Rec *__restrict__ rec
     const int e1 = min(row + 1, lim), e2 = min(col + 1, lim);
     const int64_t b1 = seq_base[2 * p], b2 = seq_base[2 * p + 1];
     const int end1 = row, end2 = s2 + col;
-    int32_t H[kRevMax + 1], Hp[kRevMax + 1], E[kRevMax + 1];
-    int best, bi, bj;
-    sw_one([&](int i) { return 4 - base_code(ar, b1 + end1 - i); }, e1,
-           [&](int k) { return 4 - base_code(ar, b2 + end2 - k); }, e2, P.open1, P.ext1, P.match, P.mismatch,
-           striped_for(e1, e2, P.open1, P.ext1, P.match), H, Hp, E, best, bi, bj);
+    int bi, bj;
+    sw_reverse_window(ar, P, SeqView{b1, end1, 1}, e1, SeqView{b2, end2, 1}, e2, bi, bj);
     r.end2 = end2;
     r.start1 = end1 - bi;
     r.start2 = end2 - bj;
@@ -781,10 +829,13 @@ void launch_l0_select(const unsigned long long *keys, int64_t n0, const int64_t 
 }
 
 void launch_reverse(ScanTask *tasks, int first, int n, const unsigned long long *keys, const int64_t *pair_base,
-                    const int32_t *pair_len, Arena ar, Params p, cudaStream_t st) {
+                    const int32_t *pair_len, Arena ar, Params p, bool window, cudaStream_t st) {
   (void)pair_len;
   if (n <= 0) return;
-  reverse_kernel<<<(n + 127) / 128, 128, 0, st>>>(tasks, first, n, keys, pair_base, ar, p);
+  if (p.window <= kScanW && window)
+    reverse_kernel<true><<<(n + 127) / 128, 128, 0, st>>>(tasks, first, n, keys, pair_base, ar, p);
+  else
+    reverse_kernel<false><<<(n + 127) / 128, 128, 0, st>>>(tasks, first, n, keys, pair_base, ar, p);
 }
 
 }  // namespace dcns

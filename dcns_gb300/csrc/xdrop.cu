@@ -80,32 +80,6 @@ __device__ __forceinline__ void xd_route(XTask &T, int id, const XLevelArgs &A) 
 }
 
 // ------------------------------------------------------------------ a group of lanes per pass
-// Sixteen symbols of a DP sequence from offset o on (forward, or the reverse complement read backwards): 2-bit codes
-// and N bits, in reading order.  Offsets outside [0, n) give any symbols.
-struct XSyms {
-  uint32_t w, n;
-};
-__device__ __forceinline__ XSyms xd_load16(const Arena &ar, const SeqView &s, int n, int o) {
-  XSyms r{0u, 0u};
-  if (o <= -16 || o >= n) return r;
-  const int64_t lo = s.base + s.a + (s.dir == 0 ? (int64_t)o : -(int64_t)o - 15);
-  if (lo < 0) {
-    const int sh = (int)-lo;  // at most 15
-    r.w = __ldg(ar.pk) << (2 * sh);
-    r.n = (__ldg(ar.nm) << sh) & 0xFFFFu;
-  } else {
-    r.w = __funnelshift_r(__ldg(ar.pk + (lo >> 4)), __ldg(ar.pk + (lo >> 4) + 1), 2u * (uint32_t)(lo & 15));
-    r.n = __funnelshift_r(__ldg(ar.nm + (lo >> 5)), __ldg(ar.nm + (lo >> 5) + 1), (uint32_t)(lo & 31)) & 0xFFFFu;
-  }
-  if (s.dir != 0) {
-    const uint32_t b = __brev(r.w);
-    r.w = ~(((b >> 1) & 0x55555555u) | ((b << 1) & 0xAAAAAAAAu));
-    r.n = __brev(r.n) >> 16;
-  }
-  for (uint32_t m = r.n; m; m &= m - 1) r.w &= ~(3u << (2 * (__ffs(m) - 1)));  // an N carries code 0
-  return r;
-}
-
 // One pass per group of L lanes (32 / L groups per warp), lane m owning K neighbouring diagonals.  In one step every
 // lane of a group computes its K cells of one row, lane m one row behind lane m - 1: the horizontal gap state and the
 // row's running maximum come from lane m - 1 as it left them a step ago, and the vertical gap state of the cell
@@ -145,14 +119,12 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
   const int m0 = pads / K, p0 = pads - m0 * K;  // the band's first cell
   const int n = *A.L.count_in;
   const int open = P.open1, ext = P.ext1, gext = max(P.ext1, P.open1);
-  const uint32_t mmrep = (uint32_t)(uint8_t)P.mismatch * 0x01010101u;
-  const uint32_t mx = (uint32_t)(uint8_t)(P.match ^ P.mismatch);
   const int q0 = m * K - pads - w;  // query offset of the lane's cell p in row i: q0 + i - 1 + p
 
   int32_t M[K], F[K];
   uint32_t sel[K];
   int32_t e_out = NEG, best_out = 0, bk_out = 0;  // what the lane leaves to the next: gap state, row maximum (packed)
-  XSyms rs{0, 0}, qs{0, 0};
+  Syms16 rs{0, 0}, qs{0, 0};
   SeqView s1{0, 0, 0}, s2{0, 0, 0};
   int id = -1, i = 0, n1 = 0, n2 = 0, last_step = 0;
   int score = 0, e1 = 0, e2 = 0, rows = 0, st = -1;  // the last lane's; st: the pass's status once it ended
@@ -160,9 +132,6 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
   bool more = in_group;
 #pragma unroll
   for (int p = 0; p < K; ++p) M[p] = NEG, F[p] = NEG, sel[p] = 0x4444u;
-
-  auto selector = [](const XSyms &s) { return ((s.w & 3u) | ((s.n & 1u) << 2)) * 0x1111u + 0x8880u; };
-  auto advance = [](XSyms &s) { s.w >>= 2, s.n >>= 1; };
 
   // Sixteen rows at a time: a pass that ends inside a block idles to its end (a few rows of some hundred), which
   // leaves the rows themselves free of votes.
@@ -218,9 +187,9 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
         sel[0] = 0x4444u;
 #pragma unroll
         for (int p = 0; p < K - 1; ++p) {
-          if (p % 16 == 0) qs = xd_load16(ar, s2, n2, q0 + p);
-          sel[p + 1] = selector(qs);
-          advance(qs);
+          if (p % 16 == 0) qs = load16(ar, s2, n2, q0 + p);
+          sel[p + 1] = sym_selector(qs);
+          next_sym(qs);
         }
       }
     }
@@ -228,8 +197,8 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
     const bool have = id >= 0;
     if (have) {  // the next sixteen rows' symbols, from where the lane's pass is
       const int r = max(i, 1) - 1;
-      qs = xd_load16(ar, s2, n2, q0 + K - 1 + r);
-      rs = xd_load16(ar, s1, n1, r);
+      qs = load16(ar, s2, n2, q0 + K - 1 + r);
+      rs = load16(ar, s1, n1, r);
     }
 
     // ---- one row per lane.  `edges`: some lane has not begun its pass, or may reach the last column
@@ -246,20 +215,19 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
       if (on) {
 #pragma unroll
         for (int p = 0; p + 1 < K; ++p) sel[p] = sel[p + 1];
-        sel[K - 1] = selector(qs);
-        prof = (rs.n & 1u) ? 0u : mmrep ^ (mx << (8u * (rs.w & 3u)));
-        advance(qs);
-        advance(rs);
+        sel[K - 1] = sym_selector(qs);
+        prof = sym_profile(rs, P.match, P.mismatch);
+        next_sym(qs);
+        next_sym(rs);
       }
       auto cell = [&](int p, int32_t fin) {
         if (WIDE ? (p == p0 && m == m0) : (p == P0 && m == 0)) e = NEG, b = 0, bk = 0;
-        uint32_t sc;
-        asm("prmt.b32 %0, %1, %2, %3;" : "=r"(sc) : "r"(prof), "r"(0u), "r"(sel[p]));
+        const int sc = perm_score(prof, 0u, sel[p]);
         if (EDGES) fin = p >= lim ? NEG : fin;
         int32_t v;
         if constexpr (CODES) {
           bool pv, ph, p1, p2;
-          v = __vibmax_s32(fin, M[p] + (int)sc, &pv);  // pv: the vertical gap wins ties with the diagonal
+          v = __vibmax_s32(fin, M[p] + sc, &pv);  // pv: the vertical gap wins ties with the diagonal
           v = __vibmax_s32(e, v, &ph);                 // ph: the horizontal gap wins ties
           if (EDGES) v = p > lim ? NEG : v;
           const int32_t h = v + open;
@@ -269,7 +237,7 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
           cw[p / 8] |= d << (4 * (p % 8));
         } else {
           // the gap's chain is one add-max a cell: max(e, A) + open and e + ext give max(e + max(ext, open), A + open)
-          const int32_t A_ = __viaddmax_s32(M[p], (int)sc, fin), ao = A_ + open;
+          const int32_t A_ = __viaddmax_s32(M[p], sc, fin), ao = A_ + open;
           v = max(A_, e);
           if (EDGES) v = p > lim ? NEG : v;
           F[p] = EDGES ? __viaddmax_s32(fin, ext, v + open) : __viaddmax_s32(fin, ext, __viaddmax_s32(e, open, ao));
