@@ -478,6 +478,15 @@ int warmup_rows(const Params &P, int tw) {
   return tw + (P.match * tw + g - 1) / g + 4;
 }
 
+// Warm-up rows of an exact scan whose maxima count from min_score on: a path that reaches it within the window has at
+// most match * tw - min_score to spend on vertical gaps, the first of whose rows costs the opening.
+int warmup_rows_above(const Params &P, int tw) {
+  const int K = warmup_rows(P, tw), spare = P.match * tw - P.min_score;
+  if (K == INT_MAX) return K;
+  const int g = std::min(-P.open1, -P.ext1);
+  return std::min(K, tw + std::max(0, spare) / g + 4);
+}
+
 // The lowest value the filter's bound still has at the checked row at or after a cell of min_score.
 int filter_threshold(const Params &P) { return P.min_score + P.open1 + 2 * P.ext1; }
 
@@ -486,7 +495,7 @@ int filter_threshold(const Params &P) { return P.min_score + P.open1 + 2 * P.ext
 // scoring, a threshold of 24 marks one 16 x 16 block in 5,000 by chance, the actual 32 one in 100,000), 16-bit room
 // for a row chunk's highest score, and a warm-up for the exact scan's tiles.
 bool filter_ok(const Params &P) {
-  const int K = warmup_rows(P, kScanW);
+  const int K = warmup_rows_above(P, kScanW);
   return fast_scan_ok(P) && P.step <= kScanW && P.mismatch <= -P.match && P.open1 <= -P.match &&
          2 * P.ext1 <= -P.match && filter_threshold(P) >= 12 * P.match && P.min_score <= 16000 && K != INT_MAX &&
          30000 / P.match >= 4 * K + 512;
@@ -497,7 +506,7 @@ bool filter_ok(const Params &P) {
 bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vector<int64_t> &order,
                   const std::vector<int32_t> &nfast, const Params &P) {
   const int64_t np = (int64_t)pairs.size();
-  const int K = warmup_rows(P, kScanW), fnew = 32 - kFiltOverlap;
+  const int K = warmup_rows_above(P, kScanW), fnew = 32 - kFiltOverlap;
   auto ntile = [&](int64_t p) -> int64_t {
     if (nfast[p] <= 0) return 0;
     const int strips = (pairs[p].n2 + kFiltCols - 1) / kFiltCols;
@@ -514,7 +523,7 @@ bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vecto
   // row chunks: none longer than 16-bit scores allow; shorter ones where there are too few tasks for the GPU
   const int64_t limit = 30000 / P.match - K - 256, want = (int64_t)C.nsm * 20 * 8;
   int64_t chunk = limit;
-  if (tasks < want) chunk = std::min(limit, std::max<int64_t>(2 * K, (rows + want - 1) / want));
+  if (tasks < want) chunk = std::min(limit, std::max<int64_t>(K, (rows + want - 1) / want));
   std::vector<FiltPair> tab(np);
   std::vector<int32_t> slot(np);
   int64_t words = 0, duos = 0, task = 0;
@@ -557,11 +566,12 @@ bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vecto
   return true;
 }
 
-// The tile list for `items` duos or tasks; short tiles where there are few, so that they spread over the GPU.
+// The tile list for `items` duos or tasks; short tiles where there are few, so that they spread over the GPU: a row
+// takes a lone warp some 0.5 us, and a tile its warm-up rows besides.
 FiltTiles filter_tiles(Context &C, int64_t items, int *count) {
   const int64_t cap = std::min<int64_t>(INT32_MAX, (int64_t)(C.d_ftiles.cap / sizeof(FiltTile)));
   return FiltTiles{C.d_ftiles.as<FiltTile>(), count, (int32_t)cap,
-                   items >= (int64_t)C.nsm * C.scan_blocks_per_sm * kScanThreads ? 256 : 64};
+                   items >= (int64_t)C.nsm * C.scan_blocks_per_sm * kScanThreads ? 256 : items >= 8192 ? 64 : 24};
 }
 
 // A round's scan through the filter's marks (tasks [first, first + n) are on the device), then the reverse scans and
@@ -681,7 +691,7 @@ void compute_scan_tasks(Context &C, ScanState &S, const Params &P) {
     if (fast && C.filt_on) {  // still: the buffers above may have needed its room
       C.stats.ms_scan_prep += ms_since(t0);
       h2d(C, C.d_tasks, S.tasks.data() + first, (size_t)n, (size_t)(first - S.ns));
-      const bool done = run_filtered_round(C, S, P, first, n, warmup_rows(P, kScanW));
+      const bool done = run_filtered_round(C, S, P, first, n, C.filt.warm);
       tp = phase(C, "sc_filtered", tp);
       if (done) {
         C.stats.ms_scan += ms_since(t0);
@@ -918,7 +928,9 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   if (filtered) {
     launch_filter(C.filt, C.arena, P, filter_threshold(P), bulk);
     launch_filter_plan_l0(C.filt, D, nduo, ft, bulk);
-    launch_scan_tiles_l0(D, ft, C.arena, P, C.d_keys.as<unsigned long long>(), C.d_counter.as<int>(),
+    L0Desc F = D;
+    F.warm = C.filt.warm;
+    launch_scan_tiles_l0(F, ft, C.arena, P, C.d_keys.as<unsigned long long>(), C.d_counter.as<int>(),
                          C.nsm * C.scan_blocks_per_sm, bulk);
     C.stats.kernel_launches += 2;
   } else {

@@ -23,10 +23,13 @@
 // the two shuffles of a step cost 2 of its 70 instructions.
 //
 // Measured on the 10,000-pair batch (534 G cells over all windows, 112 G over the pairs; serialised launch times):
-// level 0 87 ms before, now 17.3 ms in the filter, 0.5 ms in its lists and 4.8 ms in the exact scan of the marked
-// rows; the recursion rounds, which reuse the marks, 12 ms before and 3.4 ms now.  The whole call: 143 to 71 ms; two
-// 200 kb pairs: 166 to 83 ms.  Bound: integer issue, as the exact scan.  References that are marked nearly everywhere
-// (tandem repeats against themselves) overflow the tile list and pay for the filter on top of the whole scan.
+// level 0 87 ms before, now 17.6 ms in the filter, 0.5 ms in its lists and 3.1 ms in the exact scan of the marked
+// rows; the recursion rounds, which reuse the marks, 12 ms before and 2.5 ms now.  Bound: integer issue (ALU pipe at
+// 80 %), as the exact scan.  The bound kept at match * window every 16 rows costs the filter 2 % and saves the exact
+// scans 28 % (10.1 to 7.3 ms before the floor above min_score in those).  Widths of 8 to 24 columns a lane, chosen per
+// pair to fit the query, would save 14 % of the columns but ran 1.5x slower mixed in one launch (instruction cache)
+// and no faster sorted by width.  References that are marked nearly everywhere (tandem repeats against themselves)
+// overflow the tile list and pay for the filter on top of the whole scan.
 #include <type_traits>
 
 #include "device_common.cuh"
@@ -73,7 +76,7 @@ struct Stream {  // a lane's reference symbols, sixteen at a time
 };
 
 __global__ void __launch_bounds__(32 * kFWarps, 5)
-    filter_kernel(FiltDesc D, Arena ar, int open, int ext, int match, int mismatch, int thr) {
+    filter_kernel(FiltDesc D, Arena ar, int open, int ext, int match, int mismatch, int thr, int top) {
   __shared__ uint4 prof_all[kFWarps][4 * (kFC / 4) * 32];
   const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
   const int t = blockIdx.x * kFWarps + wb;
@@ -112,7 +115,7 @@ __global__ void __launch_bounds__(32 * kFWarps, 5)
   for (int p = 0; p < kFC; ++p) Ga[p] = open2, R[p] = open2;
   uint32_t lastT = open2, dg = open2, mrun;
   uint32_t acc0 = 0, acc1 = 0;
-  const uint32_t thr2 = fpack2(thr + open - 1);
+  const uint32_t thr2 = fpack2(thr + open - 1), top2 = fpack2(top + open);
 
   // One step: Gi holds the lane's previous row, Go receives this one.
   auto row = [&](uint32_t(&Gi)[kFC], uint32_t(&Go)[kFC], auto check, auto with_n) {
@@ -163,6 +166,10 @@ __global__ void __launch_bounds__(32 * kFWarps, 5)
         row(Gb, Ga, Yes{}, Yes{});
       }
     }
+    // No window's own DP exceeds match * window, so the bound need not either: kept down every 16 rows, a long
+    // alignment marks some 40 rows and columns around its path instead of half its score's worth.
+#pragma unroll
+    for (int p = 0; p < kFC; ++p) Ga[p] = __vmins2(Ga[p], top2), R[p] = __vmins2(R[p], top2);
     wcur = wnext, ncur = nnext;
     const uint32_t gt = __vcmpgts2(mrun, thr2);
     const uint32_t bit = 1u << (blk & 31);
@@ -258,7 +265,7 @@ __global__ void __launch_bounds__(256) filter_plan_rec_kernel(FiltDesc D, const 
 void launch_filter(const FiltDesc &D, Arena ar, Params p, int thr, cudaStream_t st) {
   if (D.ntasks <= 0) return;
   filter_kernel<<<(D.ntasks + kFWarps - 1) / kFWarps, 32 * kFWarps, 0, st>>>(D, ar, p.open1, p.ext1, p.match,
-                                                                            p.mismatch, thr);
+                                                                            p.mismatch, thr, p.match * p.window);
 }
 
 void launch_filter_plan_l0(const FiltDesc &D, L0Desc L, int64_t nduo, FiltTiles T, cudaStream_t st) {

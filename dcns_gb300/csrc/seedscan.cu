@@ -208,7 +208,7 @@ constexpr int kProfSyms = 4;                   // reference symbols A, C, G, T (
 constexpr size_t kProfBytes = sizeof(uint4) * kProfSyms * kProfGroups * kScanThreads;
 
 template <int W, int MODE>
-__global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc l0, FiltTiles ft, int64_t ntiles,
+__global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc l0, FiltTiles ft, int floor, int64_t ntiles,
                                                    Arena ar, int open, int ext, int match, int mismatch,
                                                    unsigned long long *__restrict__ keys, int *__restrict__ counter) {
   // Score table per reference symbol (index = 2-bit code | N << 2): bytes 0..4 = s(ref, read code 0..4) - open,
@@ -291,7 +291,9 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc 
     if (tl.task[1] < 0 || cs1 >= ce1) cs1 = ce1 = INT_MAX;
     // per-half threshold in G units: best + open while counting, unreachable (0x7FFF) otherwise
     uint32_t cmpb = 0x7FFF7FFFu;
-    int best0 = 0, best1 = 0, brow0 = -1, brow1 = -1, bcol0 = -1, bcol1 = -1;
+    // (floor: maxima up to it do not count; a filtered scan starts below min_score, which spares a rising alignment the
+    // search for its column in every row)
+    int best0 = MODE >= 3 ? floor : 0, best1 = best0, brow0 = -1, brow1 = -1, bcol0 = -1, bcol1 = -1;
 
     int r = tl.row_begin;
     int nev = min_above(r - 1, zr0, zr1, cs0, ce0, cs1, ce1);
@@ -396,34 +398,34 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc 
       if (r >= tl.row_end) break;
       row(Gb, Ga);
     }
-    if (tl.task[0] >= 0 && best0 > 0) atomicMax(keys + tl.task[0], scan_key(best0, brow0, bcol0));
-    if (tl.task[1] >= 0 && best1 > 0) atomicMax(keys + tl.task[1], scan_key(best1, brow1, bcol1));
+    if (tl.task[0] >= 0 && brow0 >= 0) atomicMax(keys + tl.task[0], scan_key(best0, brow0, bcol0));
+    if (tl.task[1] >= 0 && brow1 >= 0) atomicMax(keys + tl.task[1], scan_key(best1, brow1, bcol1));
   }
 }
 
 void launch_scan(RecDesc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter, int grid,
                  cudaStream_t st) {
   if (ntiles <= 0) return;
-  scan_kernel<kScanW, 2><<<grid, kScanThreads, kProfBytes, st>>>(d, L0Desc{}, FiltTiles{}, ntiles, ar, p.open1, p.ext1, p.match,
+  scan_kernel<kScanW, 2><<<grid, kScanThreads, kProfBytes, st>>>(d, L0Desc{}, FiltTiles{}, 0, ntiles, ar, p.open1, p.ext1, p.match,
                                                                  p.mismatch, keys, work_counter);
 }
 
 void launch_scan_l0(L0Desc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter,
                     int64_t grid, cudaStream_t st) {
   if (ntiles <= 0) return;
-  scan_kernel<kScanW, 1><<<(unsigned)grid, kScanThreads, kProfBytes, st>>>(RecDesc{}, d, FiltTiles{}, ntiles, ar, p.open1, p.ext1, p.match,
+  scan_kernel<kScanW, 1><<<(unsigned)grid, kScanThreads, kProfBytes, st>>>(RecDesc{}, d, FiltTiles{}, 0, ntiles, ar, p.open1, p.ext1, p.match,
                                                                  p.mismatch, keys, work_counter);
 }
 
 void launch_scan_tiles_l0(L0Desc d, FiltTiles T, Arena ar, Params p, unsigned long long *keys, int *work_counter,
                           int grid, cudaStream_t st) {
-  scan_kernel<kScanW, 3><<<grid, kScanThreads, kProfBytes, st>>>(RecDesc{}, d, T, 0, ar, p.open1, p.ext1, p.match,
+  scan_kernel<kScanW, 3><<<grid, kScanThreads, kProfBytes, st>>>(RecDesc{}, d, T, p.min_score - 1, 0, ar, p.open1, p.ext1, p.match,
                                                                  p.mismatch, keys, work_counter);
 }
 
 void launch_scan_tiles_rec(RecDesc d, FiltTiles T, Arena ar, Params p, unsigned long long *keys, int *work_counter,
                            int grid, cudaStream_t st) {
-  scan_kernel<kScanW, 4><<<grid, kScanThreads, kProfBytes, st>>>(d, L0Desc{}, T, 0, ar, p.open1, p.ext1, p.match,
+  scan_kernel<kScanW, 4><<<grid, kScanThreads, kProfBytes, st>>>(d, L0Desc{}, T, p.min_score - 1, 0, ar, p.open1, p.ext1, p.match,
                                                                  p.mismatch, keys, work_counter);
 }
 

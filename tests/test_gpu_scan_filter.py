@@ -46,9 +46,9 @@ def test_column_edges(engines, oracle, n2):
     assert found > 0 or n2 < 100
 
 
-@pytest.mark.parametrize("n1", [1, 19, 20, 38, 159, 160, 161, 319, 320, 321, 495, 512, 1000])
+@pytest.mark.parametrize("n1", [1, 19, 20, 38, 59, 60, 61, 119, 120, 121, 159, 160, 161, 319, 320, 321, 495, 512, 1000])
 def test_row_edges(engines, oracle, n1):
-    """Row chunks of few pairs are 160 rows (twice the warm-up); one pair alone, and among others."""
+    """Row chunks of few pairs are as short as the warm-up; one pair alone, and among others."""
     rng = np.random.default_rng(200 + n1)
     pairs = [planted(rng, n1, int(n2), 1) for n2 in (600, 333)]
     same(engines, oracle, pairs[:1])
