@@ -199,6 +199,9 @@ void launch_pack(const int8_t *codes, const int64_t *src_off, const int64_t *dst
                  uint32_t *pk, uint32_t *nm, cudaStream_t st);
 void launch_scan(RecDesc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter, int grid,
                  cudaStream_t st);
+// launch_scan leaves the column of each maximum open: this finds it for the tasks of at least min_score.
+void launch_scan_columns(const ScanTask *tasks, int first, int n, const int64_t *seq_base, Arena ar, Params p,
+                         int min_score, int warm, unsigned long long *keys, cudaStream_t st);
 void launch_scan_l0(L0Desc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter,
                     int64_t grid, cudaStream_t st);
 // The filter, its tile lists, and the exact scan over a tile list (level 0; a round's tasks).

@@ -202,7 +202,9 @@ __device__ __forceinline__ ScanTile rec_tile(const RecDesc &D, int64_t t) {
 }
 
 // MODE 1: level-0 tiles from the per-pair table; MODE 2: round tiles from the duo table; MODE 3, 4: level-0 and round
-// tiles from the filter's list.
+// tiles from the filter's list.  MODE 2 leaves the maximum's column open (0 in the key): every tile starts from no
+// maximum at all, and the search for the column of each new one, in whichever lane, took a third of the launch; the
+// tasks whose column is asked for find it afterwards, each in one row (scan_column_kernel).
 constexpr int kProfGroups = (kScanW + 3) / 4;  // query columns in groups of four (one 128-bit shared load)
 constexpr int kProfSyms = 4;                   // reference symbols A, C, G, T (2-bit codes 0..3); N rows below
 constexpr size_t kProfBytes = sizeof(uint4) * kProfSyms * kProfGroups * kScanThreads;
@@ -370,10 +372,13 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc 
       if (gt) {
         if (gt & 0xFFFFu) {
           const int v = half_s16(rmax, 0);
-          int col = W - 1;
+          int col = 0;
+          if constexpr (MODE != 2) {
+            col = W - 1;
 #pragma unroll
-          for (int p = W - 1; p >= 0; --p)
-            if (half_s16(Go[p], 0) == v) col = p;
+            for (int p = W - 1; p >= 0; --p)
+              if (half_s16(Go[p], 0) == v) col = p;
+          }
           best0 = v - open;
           brow0 = r;
           bcol0 = col;
@@ -381,10 +386,13 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc 
         }
         if (gt & 0xFFFF0000u) {
           const int v = half_s16(rmax, 1);
-          int col = W - 1;
+          int col = 0;
+          if constexpr (MODE != 2) {
+            col = W - 1;
 #pragma unroll
-          for (int p = W - 1; p >= 0; --p)
-            if (half_s16(Go[p], 1) == v) col = p;
+            for (int p = W - 1; p >= 0; --p)
+              if (half_s16(Go[p], 1) == v) col = p;
+          }
           best1 = v - open;
           brow1 = r;
           bcol1 = col;
@@ -401,6 +409,62 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc 
     if (tl.task[0] >= 0 && brow0 >= 0) atomicMax(keys + tl.task[0], scan_key(best0, brow0, bcol0));
     if (tl.task[1] >= 0 && brow1 >= 0) atomicMax(keys + tl.task[1], scan_key(best1, brow1, bcol1));
   }
+}
+
+// The first column of every task's maximum, in the row that launch_scan found: the DP again over the warm-up rows
+// before it, one thread per task.
+__global__ void __launch_bounds__(128) scan_column_kernel(const ScanTask *__restrict__ tasks, int first, int n,
+                                                          const int64_t *__restrict__ seq_base, Arena ar, Params P,
+                                                          int min_score, int warm,
+                                                          unsigned long long *__restrict__ keys) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const unsigned long long key = keys[first + k];
+  if (!key) return;
+  int best, row, col;
+  scan_unkey(key, best, row, col);
+  const ScanTask T = tasks[first + k];
+  if (best < min_score || !T.striped || T.tw > kScanW) return;  // (the generic kernels report the column themselves)
+  const SeqView s1{seq_base[2 * T.pair], 0, 0}, s2{seq_base[2 * T.pair + 1], T.s2, 0};
+  const int open = P.open1, ext = P.ext1, g = max(P.ext1, P.open1);
+  uint32_t sel[kScanW];
+  int H[kScanW], E[kScanW];
+  Syms16 q{0, 0};
+#pragma unroll
+  for (int p = 0; p < kScanW; ++p) {
+    if (p % 16 == 0) q = load16(ar, s2, T.tw, p);
+    sel[p] = p < T.tw ? sym_selector(q) : 0xDDD5u;  // past the window: -128
+    next_sym(q);
+    H[p] = 0, E[p] = 0;
+  }
+  Syms16 r{0, 0};
+  const int from = max(T.lo, row - warm);
+  for (int i = from; i <= row; ++i) {
+    if ((i - from) % 16 == 0) r = load16(ar, s1, T.hi, i);
+    const uint32_t prof = sym_profile(r, P.match, P.mismatch);
+    next_sym(r);
+    int diag = 0, F = g;
+#pragma unroll
+    for (int p = 0; p < kScanW; ++p) {
+      const int pre = __viaddmax_s32_relu(diag, perm_score(prof, 0x00008000u, sel[p]), E[p]);
+      diag = H[p];
+      const int t = pre + open;
+      E[p] = __viaddmax_s32(E[p], ext, t);
+      H[p] = max(pre, F);
+      F = __viaddmax_s32(F, g, t);
+    }
+  }
+  col = 0;
+#pragma unroll
+  for (int p = kScanW - 1; p >= 0; --p)
+    if (H[p] == best) col = p;
+  keys[first + k] = scan_key(best, row, col);
+}
+
+void launch_scan_columns(const ScanTask *tasks, int first, int n, const int64_t *seq_base, Arena ar, Params p,
+                         int min_score, int warm, unsigned long long *keys, cudaStream_t st) {
+  if (n <= 0) return;
+  scan_column_kernel<<<(n + 127) / 128, 128, 0, st>>>(tasks, first, n, seq_base, ar, p, min_score, warm, keys);
 }
 
 void launch_scan(RecDesc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter, int grid,
