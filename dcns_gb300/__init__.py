@@ -339,7 +339,7 @@ def _pairs(pairs):
     seqs = [_codes(x).reshape(-1) for ab in pairs for x in ab]
     if len(seqs) != 2 * n:
         raise ValueError("every pair must hold exactly two sequences")
-    ptr = np.fromiter((x.ctypes.data for x in seqs), np.uint64, 2 * n)
+    ptr = np.fromiter((x.__array_interface__["data"][0] for x in seqs), np.uint64, 2 * n)
     lens = np.fromiter((x.shape[0] for x in seqs), np.int64, 2 * n)
     sa = np.zeros(n, _PAIR_DT)
     sa["seq1"], sa["seq2"] = ptr[0::2], ptr[1::2]
@@ -621,7 +621,8 @@ class Engine:
         off = np.zeros(n + 1, np.int64)
         self._check(fn(self.h, arr, n, C.byref(params(**kw)), int(want_cigar), out.ctypes.data_as(_I32P),
                        cig.ctypes.data_as(_U32P), cap, off.ctypes.data_as(_I64P)))
-        cigars = [[int(c) for c in cig[off[k]:off[k + 1]]] for k in range(n)]
+        words, at = cig[:off[n]].tolist(), off.tolist()
+        cigars = [words[at[k]:at[k + 1]] for k in range(n)]
         return out[:n], cigars
 
     def SemiGlobal_xextend(self, tasks, cigar=False, **kw):

@@ -20,7 +20,8 @@ struct ResultsImpl {
   std::vector<int64_t> off, frag;
   std::vector<double> pv, ev;
   std::vector<uint32_t> cig;
-  void finish(const std::vector<std::vector<FragOut>> &fr, const dcns_stats &st) {
+  // Lays the fragments out flat (and frees them).
+  void finish(std::vector<std::vector<FragOut>> &fr, const dcns_stats &st) {
     off.assign(fr.size() + 1, 0);
     int64_t nf = 0, nc = 0;
     for (size_t k = 0; k < fr.size(); ++k) {
@@ -32,17 +33,31 @@ struct ResultsImpl {
     pv.resize(nf);
     ev.resize(nf);
     cig.resize(nc);
-    int64_t i = 0, c = 0;
-    for (auto &v : fr)
-      for (auto &f : v) {
-        int64_t *r = frag.data() + i * 7;
-        r[0] = f.s1, r[1] = f.e1, r[2] = f.s2, r[3] = f.e2, r[4] = f.score, r[5] = c, r[6] = (int64_t)f.cigar.size();
-        pv[i] = f.p;
-        ev[i] = f.e;
-        std::memcpy(cig.data() + c, f.cigar.data(), f.cigar.size() * sizeof(uint32_t));
-        c += (int64_t)f.cigar.size();
-        ++i;
+    // blocks of pairs, each with its first CIGAR word
+    const int64_t n = (int64_t)fr.size(), per = 256;
+    std::vector<int64_t> cfirst((n + per - 1) / per + 1, 0);
+    for (int64_t k = 0; k < n; ++k) {
+      int64_t words = 0;
+      for (auto &f : fr[k]) words += (int64_t)f.cigar.size();
+      cfirst[k / per + 1] += words;
+    }
+    for (size_t b = 1; b < cfirst.size(); ++b) cfirst[b] += cfirst[b - 1];
+    host_parallel((n + per - 1) / per, [&](int64_t b) {
+      int64_t c = cfirst[b];
+      for (int64_t k = b * per, e = std::min(n, k + per); k < e; ++k) {
+        int64_t i = off[k];
+        for (auto &f : fr[k]) {
+          int64_t *r = frag.data() + i * 7;
+          r[0] = f.s1, r[1] = f.e1, r[2] = f.s2, r[3] = f.e2, r[4] = f.score, r[5] = c, r[6] = (int64_t)f.cigar.size();
+          pv[i] = f.p;
+          ev[i] = f.e;
+          std::memcpy(cig.data() + c, f.cigar.data(), f.cigar.size() * sizeof(uint32_t));
+          c += (int64_t)f.cigar.size();
+          ++i;
+        }
+        std::vector<FragOut>().swap(fr[k]);  // its fragments are no longer needed
       }
+    });
     pub.n_pairs = (int64_t)fr.size();
     pub.n_fragments = nf;
     pub.n_cigar = nc;

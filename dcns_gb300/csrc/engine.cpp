@@ -119,6 +119,7 @@ Context::~Context() {
   h_out.release();
   h_tasks.release();
   h_tiles.release();
+  h_x.release();
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   if (ev2) cudaEventDestroy(ev2);
@@ -333,6 +334,34 @@ void parallel_for(int64_t n, const std::function<void(int64_t)> &f, int64_t min_
     return;
   }
   HostPool::get().run(n, f);
+}
+
+// Sum of f(0) .. f(n - 1), in parallel.
+template <class F>
+int64_t parallel_sum(int64_t n, F f) {
+  constexpr int64_t kBlock = 2048;
+  std::atomic<int64_t> total(0);
+  parallel_for(
+      (n + kBlock - 1) / kBlock,
+      [&](int64_t b) {
+        int64_t s = 0;
+        for (int64_t i = b * kBlock, e = std::min(n, i + kBlock); i < e; ++i) s += f(i);
+        total += s;
+      },
+      4);
+  return total;
+}
+
+// A large copy between pageable memory and a pinned buffer, in parallel.
+void copy_blocks(void *dst, const void *src, size_t bytes) {
+  constexpr size_t kBlock = 256 << 10;
+  parallel_for(
+      (int64_t)((bytes + kBlock - 1) / kBlock),
+      [&](int64_t b) {
+        const size_t at = (size_t)b * kBlock;
+        std::memcpy(static_cast<char *>(dst) + at, static_cast<const char *>(src) + at, std::min(kBlock, bytes - at));
+      },
+      4);
 }
 
 template <class T>
@@ -593,9 +622,10 @@ bool run_filtered_round(Context &C, ScanState &S, const Params &P, int64_t first
   C.stats.scan_launches += 1;
   C.stats.kernel_launches += 3;
   int tiles = 0;
+  d2h(C, C.h_tiles.as<ScanTask>(), C.d_tasks, (size_t)n, (size_t)d0);
   DCNS_CK(cudaMemcpyAsync(&tiles, cnt + 1, sizeof(int), cudaMemcpyDeviceToHost, C.st));
-  d2h(C, S.tasks.data() + first, C.d_tasks, (size_t)n, (size_t)d0);
   sync(C);
+  copy_blocks(S.tasks.data() + first, C.h_tiles.p, sizeof(ScanTask) * n);
   C.stats.scan_rounds += 1;
   C.stats.ms_scan_xfer += ms_since(tx);
   float ms = 0;
@@ -722,16 +752,18 @@ void compute_scan_tasks(Context &C, ScanState &S, const Params &P, int columns_f
   const bool fast_ok = fast_scan_ok(P);
   if (C.filt_on) {  // a round of windows under the filter (all of them short reads: the fast kernel's)
     bool fast = true;
-    for (int64_t k = first; k < first + n; ++k) {
-      ScanTask &T = S.task(k);
-      T.striped = striped_for_host(T.hi - T.lo, T.tw, P.open1, P.ext1, P.match) ? 1 : 0;
-      fast &= T.striped && T.tw <= kScanW;
-    }
+    fast = parallel_sum(n, [&](int64_t k) -> int64_t {
+             ScanTask &T = S.task(first + k);
+             T.striped = striped_for_host(T.hi - T.lo, T.tw, P.open1, P.ext1, P.match) ? 1 : 0;
+             return !(T.striped && T.tw <= kScanW);
+           }) == 0;
     C.d_keys.ensure(C, sizeof(unsigned long long) * (S.size() - S.ns));
     C.d_tasks.ensure(C, sizeof(ScanTask) * (S.size() - S.ns));
     if (fast && C.filt_on) {  // still: the buffers above may have needed its room
+      C.h_tiles.ensure(sizeof(ScanTask) * n);
+      copy_blocks(C.h_tiles.p, S.tasks.data() + first, sizeof(ScanTask) * n);
       C.stats.ms_scan_prep += ms_since(t0);
-      h2d(C, C.d_tasks, S.tasks.data() + first, (size_t)n, (size_t)(first - S.ns));
+      h2d(C, C.d_tasks, C.h_tiles.as<ScanTask>(), (size_t)n, (size_t)(first - S.ns));
       const bool done = run_filtered_round(C, S, P, first, n, C.filt.warm);
       tp = phase(C, "sc_filtered", tp);
       if (done) {
@@ -760,12 +792,14 @@ void compute_scan_tasks(Context &C, ScanState &S, const Params &P, int columns_f
   for (size_t i = 1; i <= fast.size(); ++i)
     if (i == fast.size() || tk(fast[i]).pair != tk(fast[i - 1]).pair) gb.push_back(i);
   parallel_for((int64_t)gb.size() - 1, [&](int64_t g) {
-    std::sort(fast.begin() + gb[g], fast.begin() + gb[g + 1], [&](int32_t a, int32_t b) {
+    const auto before = [&](int32_t a, int32_t b) {
       const ScanTask &x = tk(a), &y = tk(b);
       if (x.lo != y.lo) return x.lo < y.lo;
       if (x.hi != y.hi) return x.hi < y.hi;
       return x.s2 < y.s2;
-    });
+    };
+    if (!std::is_sorted(fast.begin() + gb[g], fast.begin() + gb[g + 1], before))
+      std::sort(fast.begin() + gb[g], fast.begin() + gb[g + 1], before);
   });
   tp = phase(C, "sc_sort", tp);
   std::vector<RecDuo> duo;
@@ -1172,59 +1206,85 @@ void scan_and_link(Context &C, const std::vector<PairIn> &pairs, const Params &P
   int64_t level0_tasks = 0;
   for (int64_t p = 0; p < np; ++p) level0_tasks += window_count(pairs[p].n2, P, one_gap);
   const int mini = P.min_score / P.match;
-  std::vector<SeedSet> sets(np);
+  linked.assign(np, {});
   std::vector<uint8_t> done(np, 0);
+  std::atomic<int64_t> link_ns(0);
   int64_t cells_rev = 0, visited_final = 0;
+  std::vector<int64_t> todo(np);
+  for (int64_t p = 0; p < np; ++p) todo[p] = p;
   for (int round = 0;; ++round) {
     if (round > 0) compute_scan_tasks(C, S, P, P.min_score);
     auto t0 = Clock::now();
-    std::vector<std::vector<std::pair<int32_t, int32_t>>> reqs(np);
-    std::vector<int64_t> pc(np, 0), pr(np, 0), pv(np, 0);
-    std::vector<int64_t> todo;
-    for (int64_t p = 0; p < np; ++p)
-      if (!done[p]) todo.push_back(p);
-    parallel_for((int64_t)todo.size(), [&](int64_t q) {
-      const int64_t p = todo[q];
-      ReplayCtx R{S, P, mini, {}, 0, 0, 0};
-      SeedSet g;
-      const bool ok = replay_pair(R, p, g);
-      if (ok) {
-        sets[p].swap(g);
-        done[p] = 1;
-        pc[p] = R.cells;
-        pr[p] = R.cells_rev;
-        pv[p] = R.visited;
-      } else {
-        reqs[p].swap(R.req);
-      }
-    });
-    int64_t nreq = 0;
-    for (int64_t p = 0; p < np; ++p) {
-      cells += pc[p];
-      cells_rev += pr[p];
-      visited_final += pv[p];
-      for (auto &rq : reqs[p]) {
-        const int32_t t = rq.first;
-        if ((rq.second == 0 ? S.left[t] : S.right[t]) >= 0) continue;
-        const ScanTask P0 = S.task(t);
-        ScanTask ch{};
-        ch.pair = P0.pair;
-        ch.s2 = P0.s2;
-        ch.tw = P0.tw;
-        if (rq.second == 0) {
-          ch.lo = P0.lo;
-          ch.hi = P0.start1;
-        } else {
-          ch.lo = P0.end1 + 1;
-          ch.hi = P0.hi;
-        }
-        (rq.second == 0 ? S.left[t] : S.right[t]) = (int32_t)S.size();
-        S.tasks.push_back(ch);
-        ++nreq;
-      }
-      S.left.resize(S.size(), -1);
-      S.right.resize(S.size(), -1);
+    const int64_t m = (int64_t)todo.size();
+    std::vector<std::vector<std::pair<int32_t, int32_t>>> reqs(m);
+    std::vector<int64_t> pc(m, 0), pr(m, 0), pv(m, 0), nq(m + 1, 0);
+    // a pair whose replay completes is linked at once, on the same thread; pairs of long sequences hold thousands of
+    // seeds, so even a few are spread over the pool
+    parallel_for(
+        m,
+        [&](int64_t q) {
+          const int64_t p = todo[q];
+          SeedArena::mine().reset();
+          ReplayCtx R{S, P, mini, {}, 0, 0, 0};
+          SeedSet g;
+          if (replay_pair(R, p, g)) {
+            const auto tl = Clock::now();
+            link_seeds(g);
+            linked[p].assign(g.begin(), g.end());
+            link_ns += std::chrono::duration_cast<std::chrono::nanoseconds>(Clock::now() - tl).count();
+            done[p] = 1;
+            pc[q] = R.cells;
+            pr[q] = R.cells_rev;
+            pv[q] = R.visited;
+          } else {
+            // its new tasks: each requested child once (-2 until it has its id)
+            reqs[q].reserve(R.req.size());
+            for (const auto &rq : R.req) {
+              int32_t &child = rq.second == 0 ? S.left[rq.first] : S.right[rq.first];
+              if (child != -1) continue;
+              child = -2;
+              reqs[q].push_back(rq);
+            }
+            nq[q + 1] = (int64_t)reqs[q].size();
+          }
+        },
+        S.size() >= 1024 ? 2 : 64);
+    for (int64_t q = 0; q < m; ++q) {
+      cells += pc[q];
+      cells_rev += pr[q];
+      visited_final += pv[q];
+      nq[q + 1] += nq[q];
     }
+    const int64_t base = S.size(), nreq = nq[m];
+    if (base + nreq >= INT32_MAX) throw Error(DCNS_ERR_NOMEM, "too many recursion tasks");
+    S.tasks.resize(base + nreq);
+    S.left.resize(base + nreq, -1);
+    S.right.resize(base + nreq, -1);
+    if (nreq > 0)
+      parallel_for(m, [&](int64_t q) {
+        int64_t id = base + nq[q];
+        for (const auto &rq : reqs[q]) {
+          const int32_t t = rq.first;
+          const ScanTask &P0 = S.task(t);
+          ScanTask ch{};
+          ch.pair = P0.pair;
+          ch.s2 = P0.s2;
+          ch.tw = P0.tw;
+          if (rq.second == 0) {
+            ch.lo = P0.lo;
+            ch.hi = P0.start1;
+          } else {
+            ch.lo = P0.end1 + 1;
+            ch.hi = P0.hi;
+          }
+          (rq.second == 0 ? S.left[t] : S.right[t]) = (int32_t)id;
+          S.tasks[id++] = ch;
+        }
+      });
+    int64_t left = 0;
+    for (int64_t q = 0; q < m; ++q)
+      if (!done[todo[q]]) todo[left++] = todo[q];
+    todo.resize(left);
     C.stats.ms_replay += ms_since(t0);
     phase(C, "replay", t0);
     if (nreq == 0) break;
@@ -1235,16 +1295,7 @@ void scan_and_link(Context &C, const std::vector<PairIn> &pairs, const Params &P
   C.stats.cells_scan_reverse += cells_rev;
   C.stats.tasks_scan += level0_tasks + visited_final;
   C.stats.tasks_scan_speculative += (S.size() - S.ns) - visited_final;
-  auto t0 = Clock::now();
-  linked.assign(np, {});
-  parallel_for(
-      np,
-      [&](int64_t p) {
-        link_seeds(sets[p]);
-        linked[p].assign(sets[p].begin(), sets[p].end());
-      },
-      2);  // a pair of long sequences holds thousands of seeds: spread even a few pairs over the pool
-  C.stats.ms_link += ms_since(t0);
+  C.stats.ms_link += (double)link_ns / 1e6 / HostPool::get().size();  // spread over the pool
 }
 
 // ------------------------------------------------------------------ 5. x-drop passes
@@ -1459,16 +1510,31 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
   const int w0 = X[0].w;
   int64_t maxdim = 1, max_n1 = 1, tb_words = 1 << 20, cig_words = 1;
   bool uniform = w0 >= 1;
-  for (int64_t k = 0; k < n; ++k) {
-    XTask &T = X[k];
-    uniform &= T.w == w0;
-    T.want_codes = want_codes ? 1 : 0;
-    T.status = 0;
-    T.score = T.end1 = T.end2 = T.rows = 0;
-    T.iii = T.jjj = T.ncig = 0;
-    maxdim = std::max<int64_t>(maxdim, std::max(T.n1, T.n2));
-    if (T.tb_rows <= 0) max_n1 = std::max<int64_t>(max_n1, T.n1);
-    if (want_codes) cig_words += (int64_t)std::max(T.n1, 0) + std::max(T.n2, 0) + 2;
+  {
+    std::mutex mu;
+    parallel_for(
+        (n + 4095) / 4096,
+        [&](int64_t b) {
+          int64_t dim = 1, n1 = 1, cig = 0;
+          bool uni = true;
+          for (int64_t k = b * 4096, e = std::min(n, k + 4096); k < e; ++k) {
+            XTask &T = X[k];
+            uni &= T.w == w0;
+            T.want_codes = want_codes ? 1 : 0;
+            T.status = 0;
+            T.score = T.end1 = T.end2 = T.rows = 0;
+            T.iii = T.jjj = T.ncig = 0;
+            dim = std::max<int64_t>(dim, std::max(T.n1, T.n2));
+            if (T.tb_rows <= 0) n1 = std::max<int64_t>(n1, T.n1);
+            if (want_codes) cig += (int64_t)std::max(T.n1, 0) + std::max(T.n2, 0) + 2;
+          }
+          std::lock_guard<std::mutex> lk(mu);
+          uniform &= uni;
+          maxdim = std::max(maxdim, dim);
+          max_n1 = std::max(max_n1, n1);
+          cig_words += cig;
+        },
+        4);
   }
   // Traceback slots: as many rows as the pass expects, or min(n1, slot_rows), the arena sized for eight or four slots
   // at the first width (a band restart takes a new slot of twice the width).  Where nothing is known a slot is reserved for
@@ -1477,11 +1543,10 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
   // with whole-pass slots).
   if (want_codes) {
     auto words_for = [&](int64_t rows) {
-      int64_t wsum = 1 << 20;
-      for (int64_t k = 0; k < n; ++k)
-        wsum += X[k].tb_rows > 0 ? 8 * xd_slot_words(w0, std::min<int64_t>(X[k].n1, X[k].tb_rows))
-                                 : 4 * xd_slot_words(w0, std::min<int64_t>(X[k].n1, rows));
-      return wsum;
+      return (1 << 20) + parallel_sum(n, [&](int64_t k) {
+               return X[k].tb_rows > 0 ? 8 * xd_slot_words(w0, std::min<int64_t>(X[k].n1, X[k].tb_rows))
+                                       : 4 * xd_slot_words(w0, std::min<int64_t>(X[k].n1, rows));
+             });
     };
     const int64_t room = (int64_t)((C.budget > C.used ? C.budget - C.used : 0) / 4);
     const int64_t want = std::min<int64_t>(max_n1, 2048);
@@ -1521,7 +1586,9 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
     int *lists = C.d_idx.as<int>();
     int *cnt = lists + 3 * n;  // [0], [1]: the two work-list counts, [2]: retry count, [4 + L]: level L's fetch
     unsigned long long *cur = C.d_counter.as<unsigned long long>();  // [0]: traceback arena, [1]: CIGAR arena
-    h2d(C, C.d_x, X.data(), (size_t)n);
+    C.h_x.ensure(sizeof(XTask) * n);
+    copy_blocks(C.h_x.p, X.data(), sizeof(XTask) * n);
+    h2d(C, C.d_x, C.h_x.as<XTask>(), (size_t)n);
     DCNS_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * (4 + nlev), C.st));
     DCNS_CK(cudaMemsetAsync(cur, 0, sizeof(unsigned long long) * 2, C.st));
     launch_xdrop_iota(lists, (int)n, cnt, C.st);
@@ -1549,13 +1616,14 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
     C.h_misc.ensure(sizeof(int32_t) * (n + 8) + 64);
     int32_t *hret = C.h_misc.as<int32_t>();  // [0]: leftover count, [1]: retry count, [8..]: retry list
     unsigned long long hcur[2] = {0, 0};
-    d2h(C, X.data(), C.d_x, (size_t)n);
+    d2h(C, C.h_x.as<XTask>(), C.d_x, (size_t)n);
     DCNS_CK(cudaMemcpyAsync(hret, cnt + in, sizeof(int), cudaMemcpyDeviceToHost, C.st));
     DCNS_CK(cudaMemcpyAsync(hret + 1, cnt + 2, sizeof(int), cudaMemcpyDeviceToHost, C.st));
     DCNS_CK(cudaMemcpyAsync(hret + 8, lists + 2 * n, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, C.st));
     DCNS_CK(cudaMemcpyAsync(hcur, cur, sizeof(hcur), cudaMemcpyDeviceToHost, C.st));
     tp = phase(C, "xc_enqueue", tp);
     sync(C);
+    copy_blocks(X.data(), C.h_x.p, sizeof(XTask) * n);
     tp = phase(C, "xc_sync", tp);
     {
       float ms = 0;
@@ -1582,21 +1650,24 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
         if (X[k].status == 0) (*hoff)[k] = X[k].cig_dense;
       }
     }
-    for (int64_t k = 0; k < n; ++k) {
+    C.stats.xdrop_passes += parallel_sum(n, [&](int64_t k) {
       int lev = 0;
       while ((w0 << lev) < X[k].w) ++lev;
-      C.stats.xdrop_passes += lev + 1;
-    }
+      return lev + 1;
+    });
     tp = phase(C, "xc_cigars", tp);
     if (C.trace) std::fprintf(stderr, "[dcns trace] x-drop chain: %lld passes, %d levels, %zu retries\n", (long long)n, nlev, retry.size());
     run_xdrop_rounds(C, X, P, want_codes, flat, hoff, retry, true);
     tp = phase(C, "xc_retry", tp);
   }
-  for (int64_t k = 0; k < n; ++k) {
-    const int64_t cells = band_cells(X[k].rows, X[k].w, X[k].n2);
-    C.stats.cells_xdrop += cells;
-    if (want_codes) C.stats.bytes_codes_xdrop += (cells + 1) / 2;
-  }
+  std::atomic<int64_t> odd(0);  // half bytes of the codes, rounded up per pass
+  const int64_t cells = parallel_sum(n, [&](int64_t k) {
+    const int64_t c = band_cells(X[k].rows, X[k].w, X[k].n2);
+    if (c & 1) odd.fetch_add(1, std::memory_order_relaxed);
+    return c;
+  });
+  C.stats.cells_xdrop += cells;
+  if (want_codes) C.stats.bytes_codes_xdrop += (cells + odd) / 2;
   C.stats.ms_xdrop += ms_since(t0);
 }
 
@@ -1619,8 +1690,11 @@ void extend_seeds(Context &C, const std::vector<PairIn> &pairs, const Params &P,
                   std::vector<std::vector<XSeedOut>> &res, std::vector<uint32_t> &cig_flat) {
   const int64_t np = (int64_t)pairs.size();
   res.assign(np, {});
-  std::vector<XTask> F;
-  for (int64_t p = 0; p < np; ++p) {
+  auto tp = Clock::now();
+  std::vector<int64_t> fbeg(np + 1, 0);
+  for (int64_t p = 0; p < np; ++p) fbeg[p + 1] = fbeg[p] + (int64_t)linked[p].size();
+  std::vector<XTask> F((size_t)fbeg[np]);
+  parallel_for(np, [&](int64_t p) {
     res[p].resize(linked[p].size());
     for (size_t s = 0; s < linked[p].size(); ++s) {
       const Seed4 &sd = linked[p][s];
@@ -1633,19 +1707,18 @@ void extend_seeds(Context &C, const std::vector<PairIn> &pairs, const Params &P,
       x.n2 = pairs[p].n2 - x.a2;
       x.dir = 0;
       x.w = P.w;
-      F.push_back(x);
+      F[fbeg[p] + (int64_t)s] = x;
     }
-  }
+  });
   C.stats.seeds += (int64_t)F.size();
-  auto tp = phase(C, "xs_build_fwd", Clock::now());
+  tp = phase(C, "xs_build_fwd", tp);
   run_xdrop(C, F, P, false, nullptr, nullptr);
   tp = phase(C, "xs_run_fwd", tp);
   const int64_t nf = (int64_t)F.size();
   // The reverse pass depends on the forward end alone, and the seeds of one alignment mostly extend to the same end:
   // one reverse pass per distinct end of a pair serves them all.  rev[k]: forward pass k's reverse pass within its
   // pair (-1: no forward end); rfirst[p]: the pair's first reverse pass.
-  std::vector<int64_t> fbeg(np + 1, 0), rfirst(np + 1, 0);
-  for (int64_t p = 0; p < np; ++p) fbeg[p + 1] = fbeg[p] + (int64_t)linked[p].size();
+  std::vector<int64_t> rfirst(np + 1, 0);
   std::vector<int32_t> rev(nf);
   std::vector<int32_t> rlead(nf);  // at fbeg[p] + q: the forward pass that reverse pass q of pair p was made from
   parallel_for(np, [&](int64_t p) {
@@ -1701,16 +1774,18 @@ void extend_seeds(Context &C, const std::vector<PairIn> &pairs, const Params &P,
   // the algorithm's cells and passes: one reverse pass per seed
   C.stats.cells_xdrop = cells0, C.stats.bytes_codes_xdrop = codes0, C.stats.xdrop_passes = passes0;
   tp = phase(C, "xs_run_rev", tp);
-  for (int64_t p = 0; p < np; ++p)
+  std::atomic<int64_t> cells(0), codes(0), passes(0);
+  parallel_for(np, [&](int64_t p) {
+    int64_t pc = 0, pb = 0, pp = 0;
     for (int64_t k = fbeg[p]; k < fbeg[p + 1]; ++k) {
       if (rev[k] < 0) continue;
       const int64_t q = rfirst[p] + rev[k];
       const XTask &r = R[q], &f = F[k];
       XSeedOut &o = res[p][k - fbeg[p]];
-      const int64_t cells = band_cells(r.rows, r.w, r.n2);
-      C.stats.cells_xdrop += cells;
-      if (want_cigar) C.stats.bytes_codes_xdrop += (cells + 1) / 2;
-      for (int w = P.w; w <= r.w; w *= 2) C.stats.xdrop_passes += 1;
+      const int64_t c = band_cells(r.rows, r.w, r.n2);
+      pc += c;
+      if (want_cigar) pb += (c + 1) / 2;
+      for (int w = P.w; w <= r.w; w *= 2) ++pp;
       o.score = r.score;
       if (want_cigar) o.cig_off = hoff[q], o.cig_len = r.ncig;
       if (r.end1 - 1 < 0 || r.end2 - 1 < 0) continue;
@@ -1725,6 +1800,11 @@ void extend_seeds(Context &C, const std::vector<PairIn> &pairs, const Params &P,
         o.end2 -= r.jjj;
       }
     }
+    cells += pc, codes += pb, passes += pp;
+  });
+  C.stats.cells_xdrop += cells;
+  C.stats.bytes_codes_xdrop += codes;
+  C.stats.xdrop_passes += passes;
 }
 
 // ------------------------------------------------------------------ 2-gap stage (:532-616)
@@ -2310,6 +2390,8 @@ void align_weighted(Context &C, const std::vector<PairIn> &pairs, const std::vec
   C.stats.bytes_device = device_bytes(C);
 }
 
+void host_parallel(int64_t n, const std::function<void(int64_t)> &f) { parallel_for(n, f, 4); }
+
 // ------------------------------------------------------------------ entry points
 void align_core(Context &C, const std::vector<PairIn> &pairs, const Params &P, int mode,
                 std::vector<std::vector<FragOut>> &out);
@@ -2549,7 +2631,7 @@ void align_core(Context &C, const std::vector<PairIn> &pairs, const Params &P, i
     target[bb] -= wk;
   }
   for (auto &b : bins) std::sort(b.begin(), b.end());  // each bin keeps the caller's pair order
-  std::atomic<int> next(0);
+  std::atomic<int> next(nl);  // lane l begins with bin l, so that its buffers fit that bin from call to call
   Context::Turnstile turn;
   auto pass_turn = [&](int b, bool failed) {
     std::lock_guard<std::mutex> lk(turn.mu);
@@ -2565,7 +2647,7 @@ void align_core(Context &C, const std::vector<PairIn> &pairs, const Params &P, i
     Context &L = *C.lanes[l];
     try {
       DCNS_CK(cudaSetDevice(C.device));
-      for (int b; (b = next.fetch_add(1)) < kBins;) {
+      for (int b = l; b < kBins; b = next.fetch_add(1)) {
         struct Pass {  // every bin passes the turnstile, whether or not it reached its level-0 scan
           decltype(pass_turn) &fn;
           int b;

@@ -2,7 +2,9 @@
 // C ABI (capi.cpp) exposes.
 #pragma once
 
+#include <algorithm>
 #include <chrono>
+#include <functional>
 #include <cstdint>
 #include <condition_variable>
 #include <mutex>
@@ -83,7 +85,61 @@ struct SeedLess {
     return false;
   }
 };
-using SeedSet = std::set<Seed4, SeedLess>;
+
+// Nodes of the seed sets of the pair at hand, from blocks of the thread that replays it: a replay builds and drops a
+// set per recursion level, and the heap (and its locks, as sets moved between threads) took most of its time.  A
+// thread keeps 256 KB.
+class SeedArena {
+ public:
+  static SeedArena &mine() {
+    static thread_local SeedArena a;
+    return a;
+  }
+  void *take(size_t bytes) {
+    bytes = (bytes + 15) & ~size_t(15);
+    if (at_ + bytes > size_) grow(bytes);
+    void *p = blocks_.back().get() + at_;
+    at_ += bytes;
+    return p;
+  }
+  // Drops everything taken (no set of an earlier pair may be alive).
+  void reset() {
+    if (blocks_.size() > 1) {
+      blocks_.clear();
+      size_ = 0;
+    }
+    at_ = 0;
+  }
+
+ private:
+  static constexpr size_t kKept = 256 << 10;
+  void grow(size_t bytes) {
+    const size_t want = std::max(bytes, blocks_.empty() ? kKept : std::max(kKept, 2 * size_));
+    blocks_.emplace_back(new char[want]);
+    size_ = want;
+    at_ = 0;
+  }
+  std::vector<std::unique_ptr<char[]>> blocks_;
+  size_t at_ = 0, size_ = 0;
+};
+template <class T>
+struct SeedAlloc {
+  using value_type = T;
+  SeedAlloc() = default;
+  template <class U>
+  SeedAlloc(const SeedAlloc<U> &) {}
+  T *allocate(size_t n) { return static_cast<T *>(SeedArena::mine().take(n * sizeof(T))); }
+  void deallocate(T *, size_t) {}
+  template <class U>
+  bool operator==(const SeedAlloc<U> &) const {
+    return true;
+  }
+  template <class U>
+  bool operator!=(const SeedAlloc<U> &) const {
+    return false;
+  }
+};
+using SeedSet = std::set<Seed4, SeedLess, SeedAlloc<Seed4>>;
 
 // Weighted variants: device category ids of every pair's seq1 (pair p at wbase[p]) and the category table.
 struct WeightSet {
@@ -113,7 +169,7 @@ struct Context {
   bool filt_on = false;
   const WeightSet *weights = nullptr;  // set during a weighted call
   // pinned staging
-  HostBuf h_codes, h_misc, h_out, h_tasks, h_tiles;
+  HostBuf h_codes, h_misc, h_out, h_tasks, h_tiles, h_x;
 
   // arena layout of the batch being aligned (the context's own upload buffers, or a resident batch)
   std::vector<int64_t> seq_base;  // 2 per pair
@@ -164,6 +220,9 @@ struct Context {
 
   ~Context();
 };
+
+// f(0) .. f(n - 1) on the host worker pool (and the calling thread).
+void host_parallel(int64_t n, const std::function<void(int64_t)> &f);
 
 void init_context(Context &C, int device, size_t budget);
 // Frees the context's grow-only device buffers (after its stream is idle), so the next call sizes them afresh.
