@@ -1346,7 +1346,7 @@ XScratch xdrop_scratch(const Context &C, int64_t w, int64_t n) {
 bool xdrop_packed(const std::vector<XTask> &X, const Params &P) {
   int64_t d = 0;
   for (const XTask &T : X) d = std::max<int64_t>(d, std::min(T.n1, T.n2));
-  return d * P.match < (1 << 20);
+  return d * std::max(P.match, P.mismatch) < (1 << 20);
 }
 
 // Runs the passes `subset` of X to completion in host-driven rounds (band restarts, traceback-slot growth), then

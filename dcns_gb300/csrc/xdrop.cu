@@ -93,9 +93,9 @@ __device__ __forceinline__ void xd_route(XTask &T, int id, const XLevelArgs &A) 
 // discarded.  Groups take their next pass from the level's list as they finish.
 //
 // The row's first maximum travels as one word, value * 1024 + 1023 - cell, and cells outside the DP hold -2^20: both
-// hold while match * the shorter sequence stays under 2^20 and the band at K L - P0 cells.  P0 >= 0: the band leaves
-// exactly P0 cells of the first lane unused (the doubled bands of w = 10).  P0 = -1: any band, maximum and cell in
-// two words.
+// hold while the higher score * the shorter sequence stays under 2^20 and the band at K L - P0 cells.  P0 >= 0: the
+// band leaves exactly P0 cells of the first lane unused (the doubled bands of w = 10).  P0 = -1: any band, maximum and
+// cell in two words.
 //
 // Measured on one GB300 against the forms this one replaces (one thread per pass, then 8-lane stripe wavefronts from
 // row 96 or from band 40 on one warp; serialised level times per call): 10,000 pairs 41 -> 8.9 ms, of which 3x fewer

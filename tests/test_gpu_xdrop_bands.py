@@ -63,6 +63,13 @@ def test_scores_past_the_packed_word(lib, oracle):
     check(lib, oracle, tasks, match=127, mismatch=-127, open1=-120, ext1=-60, xdrop=2000)
 
 
+def test_mismatches_past_the_packed_word(lib, oracle):
+    """A mismatch that scores more than a match: the mismatches, not the matches, reach 2^20."""
+    rng = np.random.default_rng(12)
+    check(lib, oracle, [similar(rng, 12000, 11990, 0.3, 0.0), similar(rng, 200, 180, 0.3, 0.0)],
+          match=1, mismatch=127, open1=-10, ext1=-5)
+
+
 def test_long_passes_and_empty_ones(lib, oracle):
     """Passes of 5,000 rows outgrow slots of 2,048; empty and one-base sequences among them."""
     rng = np.random.default_rng(9)
