@@ -61,6 +61,10 @@ __device__ __forceinline__ void next_sym(Syms16 &s) { s.w >>= 2, s.n >>= 1; }
 __device__ __forceinline__ uint32_t sym_selector(const Syms16 &s) {
   return ((s.w & 3u) | ((s.n & 1u) << 2)) * 0x1111u + 0x8880u;
 }
+// As sym_selector, for 256 times the score (byte 0 picks a zero behind the profile).
+__device__ __forceinline__ uint32_t sym_selector256(const Syms16 &s) {
+  return ((s.w & 3u) | ((s.n & 1u) << 2)) * 0x1110u + 0x8804u;
+}
 __device__ __forceinline__ uint32_t sym_profile(const Syms16 &s, int match, int mismatch) {
   const uint32_t rep = (uint32_t)(uint8_t)mismatch * 0x01010101u, x = (uint32_t)(uint8_t)(match ^ mismatch);
   return (s.n & 1u) ? 0u : rep ^ (x << (8u * (s.w & 3u)));

@@ -92,16 +92,28 @@ __device__ __forceinline__ void xd_route(XTask &T, int id, const XLevelArgs &A) 
 // capacity, band-edge restart, score, x-drop, non-positive maximum); the steps the other lanes are ahead are
 // discarded.  Groups take their next pass from the level's list as they finish.
 //
-// The row's first maximum travels as one word, value * 1024 + 1023 - cell, and cells outside the DP hold -2^20: both
-// hold while the higher score * the shorter sequence stays under 2^20 and the band at K L - P0 cells.  P0 >= 0: the
-// band leaves exactly P0 cells of the first lane unused (the doubled bands of w = 10).  P0 = -1: any band, maximum and
-// cell in two words.
+// The row's first maximum travels as one word, value * 1024 + the cell counted from the band's end (1023 for its
+// first cell, so that one test finds a maximum on either edge), and cells outside the DP hold -2^20: both hold while
+// the higher score * the shorter sequence stays under 2^20 and the band at K L - P0 cells.  P0 >= 0: the band leaves
+// exactly P0 cells of the first lane unused (the doubled bands of w = 10).  P0 = -1: any band, maximum and cell in two
+// words.
+//
+// Passes with codes (P0 >= 0) hold 256 times the values and the codes below them: a vertical gap state ends in 1, a
+// horizontal one in 2, a diagonal in 0, so the maxima settle ties as the reference's comparisons do (horizontal before
+// vertical before diagonal) and leave the winner's code behind; 4 and 8 mark an extended gap, in copies that go to
+// the codes only.  The gap's chain is one add-max a cell, as without codes.
+//
+// A row costs its instructions, 2-3 cycles each: 73 and 106 of them (119 and 192 with codes) at 3 and 6 cells a lane,
+// where 95 and 130 (153 and 226) went with the profile's N test, the slot's and the last row's test and a branch to
+// the decisions in every row.  Blocks that hold an N, begin a pass or may reach an end or the slot's run the full row
+// (EDGES).  Level times per call, before -> after: two 200 kb pairs 8.01 -> 5.71 ms; 50,000 extension tasks
+// 6.37 -> 5.11 ms; one 1 kb pair 190 -> 142 us.
 //
 // Measured on one GB300 against the forms this one replaces (one thread per pass, then 8-lane stripe wavefronts from
-// row 96 or from band 40 on one warp; serialised level times per call): 10,000 pairs 41 -> 8.9 ms, of which 3x fewer
-// reverse passes account for 9 ms; 50,000 extension tasks 28.8 -> 7.6 ms; 10,000-row passes of two 200 kb pairs
-// 12.0 and 9.7 ms -> 1.4 and 1.5 ms at bands 10 and 20.  Bound: the latency of a row (0.15 us: the shuffles, then
-// the gap's chain through the lane's cells) where passes are long or few, integer issue on short ones.
+// row 96 or from band 40 on one warp; serialised level times per call): 10,000 pairs 41 -> 6.0 ms, of which 3x fewer
+// reverse passes account for 9 ms; 50,000 extension tasks 28.8 -> 5.1 ms; 10,000-row passes of two 200 kb pairs
+// 12.0 and 9.7 ms -> 1.2 and 1.05 ms at bands 10 and 20.  Bound: the latency of a row (0.12 us without codes, 0.15
+// and 0.22 us with them: the shuffles, then the lane's cells) where passes are long or few, integer issue on short ones.
 //
 // Cells left of column 1 start from the same low value and never reach a cell inside (nothing is added to them but a
 // few matches); cells right of column n2 feed only cells right of it, but the last column takes no vertical gap and
@@ -111,27 +123,39 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
   constexpr bool WIDE = P0 < 0;
   constexpr int NG = 32 / L, KL = K * L, WN = (K + 7) / 8;
   constexpr int BYTES = K <= 4 ? 2 : 4 * WN;
-  constexpr int32_t NEG = WIDE ? kOut : -(1 << 20);
+  constexpr bool TAGS = CODES && !WIDE;  // codes below the values
+  constexpr int S = TAGS ? 256 : 1;  // the scale of the cells' values
+  constexpr int32_t NEG = WIDE ? kOut : -(1 << 20) * S, NEG_E = NEG | (TAGS ? 2 : 0), NEG_F = NEG | (TAGS ? 1 : 0);
   const int lane = threadIdx.x & 31, g = lane / L, m = lane - g * L;
   const bool in_group = g < NG, lead = m == 0, tail_lane = m == L - 1;
   const int first = in_group ? g * L : lane;
   const int w = A.w, nk = 2 * w + 1, pads = WIDE ? KL - nk : P0;
   const int m0 = pads / K, p0 = pads - m0 * K;  // the band's first cell
   const int n = *A.L.count_in;
-  const int open = P.open1, ext = P.ext1, gext = max(P.ext1, P.open1);
+  const int open = P.open1 * S, ext = P.ext1 * S, gext = max(P.ext1, P.open1) * S;
+  // a horizontal gap extended: never where opening is dearer by the row (then e + ext < max(A, e) + open)
+  const int ext_code = ext + (P.ext1 >= P.open1 ? 8 : 0);
+  const uint32_t prof_rep = (uint32_t)(uint8_t)P.mismatch * 0x01010101u;
+  const uint32_t prof_x = (uint32_t)(uint8_t)(P.match ^ P.mismatch);
   const int q0 = m * K - pads - w;  // query offset of the lane's cell p in row i: q0 + i - 1 + p
 
   int32_t M[K], F[K];
   uint32_t sel[K];
-  int32_t e_out = NEG, best_out = 0, bk_out = 0;  // what the lane leaves to the next: gap state, row maximum (packed)
+  int32_t e_out = NEG_E, best_out = 0, bk_out = 0;  // what the lane leaves to the next: gap state, row maximum (packed)
   Syms16 rs{0, 0}, qs{0, 0};
   SeqView s1{0, 0, 0}, s2{0, 0, 0};
   int id = -1, i = 0, n1 = 0, n2 = 0, last_step = 0;
   int score = 0, e1 = 0, e2 = 0, rows = 0, st = -1;  // the last lane's; st: the pass's status once it ended
+  int row1 = 0;
+  bool live = false;  // not WIDE: the last lane of a pass that goes on
+  int32_t best = 0;  // not WIDE: the best row's packed maximum so far (of row e1)
+  const int32_t xd = min(max(P.xdrop, -1), 1 << 20) * 1024;
+  // the packed word's cell: KL - 1 - cell, and 1023 for the band's first
+  const int32_t bc0 = m == 0 ? 1023 + P0 : KL - 1 - m * K;
   uint8_t *out = nullptr;
   bool more = in_group;
 #pragma unroll
-  for (int p = 0; p < K; ++p) M[p] = NEG, F[p] = NEG, sel[p] = 0x4444u;
+  for (int p = 0; p < K; ++p) M[p] = NEG, F[p] = NEG_F, sel[p] = 0x4444u;
 
   // Sixteen rows at a time: a pass that ends inside a block idles to its end (a few rows of some hundred), which
   // leaves the rows themselves free of votes.
@@ -174,21 +198,21 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
         // steps whose bytes fit the slot (rows past it are never kept), at most 2^31 - 1 of them
         last_step = (int)min((int64_t)INT32_MAX, 4 * (int64_t)cap / (L * BYTES));
         i = 1 - m;
-        score = e1 = e2 = rows = 0;
+        score = e1 = e2 = rows = best = 0;
         st = -1;
-        e_out = NEG, best_out = 0, bk_out = 0;
+        e_out = NEG_E, best_out = 0, bk_out = 0;
         // row 0: cell (0, 0) = 0, which is the diagonal of (1, 1), at band cell w; the rest is outside
 #pragma unroll
         for (int p = 0; p < K; ++p) {
           M[p] = m * K + p - pads == w ? 0 : NEG;
-          F[p] = NEG;
+          F[p] = NEG_F;
         }
         // selectors of row 1's first K - 1 cells, one place on (the row moves them back)
         sel[0] = 0x4444u;
 #pragma unroll
         for (int p = 0; p < K - 1; ++p) {
           if (p % 16 == 0) qs = load16(ar, s2, n2, q0 + p);
-          sel[p + 1] = sym_selector(qs);
+          sel[p + 1] = TAGS ? sym_selector256(qs) : sym_selector(qs);
           next_sym(qs);
         }
       }
@@ -201,7 +225,11 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
       rs = load16(ar, s1, n1, r);
     }
 
-    // ---- one row per lane.  `edges`: some lane has not begun its pass, or may reach the last column
+    uint8_t *at = nullptr;
+    if (CODES && have) at = out + (int64_t)(i + m - 1) * (L * BYTES);
+    // ---- one row per lane.  `edges`: some lane has not begun its pass, may reach the last column or row or its slot's
+    // end, or holds an N
+    live = have && tail_lane;
     auto row = [&](auto edges) {
       constexpr bool EDGES = decltype(edges)::value;
       const bool on = !EDGES || (have && i >= 1);
@@ -215,17 +243,36 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
       if (on) {
 #pragma unroll
         for (int p = 0; p + 1 < K; ++p) sel[p] = sel[p + 1];
-        sel[K - 1] = sym_selector(qs);
-        prof = sym_profile(rs, P.match, P.mismatch);
-        next_sym(qs);
-        next_sym(rs);
+        if (EDGES) {
+          sel[K - 1] = (TAGS ? sym_selector256(qs) : sym_selector(qs));
+          prof = sym_profile(rs, P.match, P.mismatch);
+          next_sym(qs);
+          next_sym(rs);
+        } else {  // no N
+          sel[K - 1] = (qs.w & 3u) * (TAGS ? 0x1110u : 0x1111u) + (TAGS ? 0x8804u : 0x8880u);
+          prof = prof_rep ^ __funnelshift_l(0u, prof_x, rs.w << 3);
+          qs.w >>= 2, rs.w >>= 2;
+        }
       }
       auto cell = [&](int p, int32_t fin) {
-        if (WIDE ? (p == p0 && m == m0) : (p == P0 && m == 0)) e = NEG, b = 0, bk = 0;
+        if (WIDE ? (p == p0 && m == m0) : (p == P0 && m == 0)) e = NEG_E, b = 0, bk = 0;
         const int sc = perm_score(prof, 0u, sel[p]);
-        if (EDGES) fin = p >= lim ? NEG : fin;
+        if (EDGES) fin = p >= lim ? NEG_F : fin;
         int32_t v;
-        if constexpr (CODES) {
+        if constexpr (TAGS) {
+          const int32_t A_ = __viaddmax_s32(M[p], sc, fin);
+          v = max(A_, e);
+          const int32_t he = (A_ & ~255) + (open + 2);
+          const int32_t he_code = __viaddmax_s32(e, ext_code, he);
+          e = __viaddmax_s32(e, gext, he);
+          if (EDGES) v = p > lim ? NEG : v;
+          const int32_t c = v & ~255, h = c + (open + 1);
+          const int32_t f_code = __viaddmax_s32(fin, ext + 4, h);
+          F[p] = __viaddmax_s32(fin, ext, h);
+          const uint32_t d = ((uint32_t)v & 3u) | ((uint32_t)f_code & ~3u);
+          cw[p / 8] += (((d & 7u) | ((uint32_t)he_code & ~7u)) & 15u) * (1u << (4 * (p % 8)));
+          v = c;
+        } else if constexpr (CODES) {
           bool pv, ph, p1, p2;
           v = __vibmax_s32(fin, M[p] + sc, &pv);  // pv: the vertical gap wins ties with the diagonal
           v = __vibmax_s32(e, v, &ph);                 // ph: the horizontal gap wins ties
@@ -247,20 +294,19 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
         if constexpr (WIDE) {
           if (v > b) b = v, bk = m * K + p;
         } else {
-          b = max(b, v * 1024 + (KL - 1 - p) - m * K);
+          b = __viaddmax_s32(v * (1024 / S) + (p == P0 ? bc0 : KL - 1 - m * K), -p, b);
         }
       };
       if (on) cell(0, F[1]);
       int32_t fr = __shfl_down_sync(0xFFFFFFFFu, F[0], 1);
-      if (tail_lane) fr = NEG;
+      if (tail_lane) fr = NEG_F;
       if (on) {
 #pragma unroll
         for (int p = 1; p < K; ++p) cell(p, p + 1 < K ? F[p + 1] : fr);
         e_out = e, best_out = b, bk_out = bk;
       }
       if constexpr (CODES) {  // the step's bytes of a group lie next to each other
-        if (on && have && i + m <= last_step) {
-          uint8_t *const at = out + (int64_t)(i + m - 1) * (L * BYTES);
+        if (on && have && (!EDGES || i + m <= last_step)) {
           if constexpr (BYTES == 2) {
             *reinterpret_cast<uint16_t *>(at) = (uint16_t)cw[0];
           } else {
@@ -268,27 +314,53 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
             for (int c = 0; c < WN; ++c) reinterpret_cast<uint32_t *>(at)[c] = cw[c];
           }
         }
+        at += L * BYTES;
       }
       // the last lane's row is complete: take its decisions
-      if (on && have && tail_lane && st < 0) {
-        if (CODES && i > last_step - (L - 1)) {
-          st = 2;
-        } else {
-          rows = i;
-          const int rb = WIDE ? b : b >> 10;
-          const int k = (WIDE ? bk : KL - 1 - (b & 1023)) - pads;
-          const int j = rb > 0 ? i - w + k : -1;
-          if (rb > 0 && j != n2 && j != 1 && (k == 0 || k == 2 * w)) {
-            st = 1;
+      if constexpr (!WIDE) {
+        if (!EDGES || on) {
+          if (b > (best | 1023)) best = b, e1 = i;
+          const int32_t low = __viaddmax_s32(best & ~1023, -xd, 1024);
+          const bool last = EDGES && (i >= n1 || i + m > last_step);
+          if (live && (b < low || ((uint32_t)(b + 1) & 1023u) <= 1u || last)) {
+            const int c = b & 1023, k = c == 1023 ? 0 : KL - 1 - c - pads, j = i - w + k;
+            if (CODES && EDGES && i + m > last_step)
+              st = 2, rows = i - 1;
+            else if (b >= 1024 && (k == 0 || k == 2 * w) && j != n2 && j != 1)
+              st = 1, rows = i;
+            else if (b < low || (EDGES && i >= n1))
+              st = 0, rows = i;
+            if (st >= 0) {
+              live = false;
+              score = best >> 10;
+              row1 = e1;
+              const int cb = best & 1023;
+              e2 = score > 0 ? e1 - w + (cb == 1023 ? 0 : KL - 1 - cb - pads) : 0;
+            }
+          }
+        }
+      } else {
+        if (on && have && tail_lane && st < 0) {
+          if (CODES && i > last_step - (L - 1)) {
+            st = 2;
           } else {
-            if (rb > score) score = rb, e1 = i, e2 = j;
-            if (score - rb > P.xdrop || rb <= 0 || i >= n1) st = 0;
+            rows = i;
+            const int rb = WIDE ? b : b >> 10;
+            const int k = (WIDE ? bk : KL - 1 - (b & 1023)) - pads;
+            const int j = rb > 0 ? i - w + k : -1;
+            if (rb > 0 && j != n2 && j != 1 && (k == 0 || k == 2 * w)) {
+              st = 1;
+            } else {
+              if (rb > score) score = rb, e1 = i, e2 = j;
+              if (score - rb > P.xdrop || rb <= 0 || i >= n1) st = 0;
+            }
           }
         }
       }
       ++i;
     };
-    if (__any_sync(0xFFFFFFFFu, have && (i < 1 || i + 15 + w >= n2))) {
+    const bool ends = q0 + K - 1 + i + 15 >= n2 || (tail_lane && i + 15 >= n1) || (CODES && i + m + 15 > last_step);
+    if (__any_sync(0xFFFFFFFFu, have && (i < 1 || ends || (qs.n | rs.n) != 0))) {
       for (int r = 0; r < 16; ++r) row(std::true_type{});
     } else {
       for (int r = 0; r < 16; ++r) row(std::false_type{});
@@ -298,7 +370,7 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
       XTask &T = A.tasks[id];
       T.status = st;
       T.rows = rows;
-      if (st == 0) T.score = score, T.end1 = e1, T.end2 = e2;
+      if (st == 0) T.score = score, T.end1 = WIDE ? e1 : row1, T.end2 = e2;
       xd_route(T, id, A);
     }
     const unsigned done = __ballot_sync(0xFFFFFFFFu, fin);
