@@ -238,7 +238,10 @@ struct XLevel {
 };
 constexpr int kXdropBandMaxW = 325;  // wider bands run one warp per pass with the band in scratch
 int64_t xd_slot_words(int w, int64_t rows);  // 32-bit words of a traceback slot (a multiple of 4)
-void launch_xdrop_iota(int *list, int n, int *count, cudaStream_t st);
+constexpr int kXdropOrderBins = 64;
+// The first level's work list; `bins`: 2 kXdropOrderBins zeroed ints of scratch.
+void launch_xdrop_list(const XTask *tasks, int *list, int n, int *count, int max_rows, int *bins, int nsm,
+                       cudaStream_t st);
 // packed: the higher score * min(n1, n2) < 2^20 for every pass.  scratch, per_warp, warps: bands above kXdropBandMaxW.
 void launch_xdrop_level(XTask *tasks, const XLevel &lv, Arena ar, Params p, uint32_t *tb, int w, int n_bound, int nsm,
                         int32_t *scratch, int64_t per_warp, int warps, bool codes, bool packed, cudaStream_t st);

@@ -1576,7 +1576,7 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
       scratch_ints = std::max(scratch_ints, scr[L].warps * scr[L].per_warp);
     }
     C.d_x.ensure(C, sizeof(XTask) * n);
-    C.d_idx.ensure(C, sizeof(int32_t) * (3 * n + 4 + nlev + 64));
+    C.d_idx.ensure(C, sizeof(int32_t) * (3 * n + 4 + nlev + 2 * kXdropOrderBins));
     C.d_counter.ensure(C, 64);
     if (want_codes) {
       C.d_tb.ensure(C, sizeof(uint32_t) * tb_words);
@@ -1589,9 +1589,10 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
     C.h_x.ensure(sizeof(XTask) * n);
     copy_blocks(C.h_x.p, X.data(), sizeof(XTask) * n);
     h2d(C, C.d_x, C.h_x.as<XTask>(), (size_t)n);
-    DCNS_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * (4 + nlev), C.st));
+    DCNS_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * (4 + nlev + 2 * kXdropOrderBins), C.st));
     DCNS_CK(cudaMemsetAsync(cur, 0, sizeof(unsigned long long) * 2, C.st));
-    launch_xdrop_iota(lists, (int)n, cnt, C.st);
+    launch_xdrop_list(C.d_x.as<XTask>(), lists, (int)n, cnt, (int)std::min<int64_t>(maxdim, INT32_MAX), cnt + 4 + nlev,
+                      C.nsm, C.st);
     DCNS_CK(cudaEventRecord(C.ev0, C.st));
     int in = 0;
     for (int L = 0; L < nlev; ++L) {

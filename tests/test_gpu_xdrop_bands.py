@@ -93,3 +93,20 @@ def test_seeds_of_one_alignment_share_its_reverse_pass(lib, oracle):
         for k, (a, b) in enumerate(pairs):
             exp, _ = oracle.find(a, b, two_gap=two_gap)
             assert [f.key() for f in got[k]] == [f.key() for f in exp], (k, two_gap)
+
+
+def test_lists_by_length_and_in_order_agree(lib, oracle):
+    """A call past 16 passes per multiprocessor hands its passes out longest first, the same tasks in smaller calls go
+    in order: the same results.  Lengths from 0 to the longest, which stands alone in its class."""
+    rng = np.random.default_rng(13)
+    n = 16 * 152 + 70
+    tasks = [similar(rng, int(rng.integers(0, 130)), int(rng.integers(0, 130)), 0.9, 0.02) for _ in range(n)]
+    tasks[5] = similar(rng, 640, 640, 0.97, 0.01)
+    for cig in (False, True):
+        out, cigars = lib.SemiGlobal_xextend(tasks, cigar=cig, w=3)
+        for k in range(0, n, 1000):
+            part, pc = lib.SemiGlobal_xextend(tasks[k:k + 1000], cigar=cig, w=3)
+            assert np.array_equal(out[k:k + 1000], part)
+            if cig:
+                assert all(np.array_equal(a, b) for a, b in zip(cigars[k:k + 1000], pc))
+    check(lib, oracle, tasks[:120], w=3)
