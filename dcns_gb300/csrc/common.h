@@ -259,9 +259,9 @@ int sg_ctas_per_sm(int nw);
 // before the launch, and column checkpoints, at 16-byte offsets; every DP of a launch alike).  minb: 4, 5 or 6
 // resident blocks per SM (the register budget of the unweighted kernel's instantiation).
 void launch_semiglobal_flow(const SgFlow &f, Arena ar, Params p, const SgWeights *wt, uint8_t *tb, bool path, int nsm,
-                            int minb, cudaStream_t st);
+                            int blocks_per_sm, cudaStream_t st);
 int64_t sg_flow_units(int n1, int n2, int w);  // stripe units of one DP in the flow form (at least 1)
-int64_t sg_flow_grid_warps(int nsm, int minb);  // warps of the flow kernel's persistent grid
+int64_t sg_flow_grid_warps(int nsm, int blocks);  // warps of the flow kernel's persistent grid
 int64_t sg_ck_row_bytes(int n1, int n2, int w);  // checkpoints of one DP (multiples of 16): the rows between stripes,
 int64_t sg_ck_col_bytes(int n1, int n2, int w);  // and the columns between tiles
 void launch_sg_retrace(SgTask *tasks, const int *idx, int n, Arena ar, Params p, const SgWeights *wt, uint8_t *tb,

@@ -171,8 +171,7 @@ void init_context(Context &C, int device, size_t budget) {
     C.sg_flow = std::atoi(e) != 0;
   }
   if (const char *e = std::getenv("DCNS_SG_FLOW_BLOCKS")) {
-    const int v = std::atoi(e);
-    C.sg_flow_blocks = (v == 5 || v == 6) ? v : 4;
+    C.sg_flow_blocks = std::atoi(e) == 1 ? 1 : 2;
   }
   if (const char *e = std::getenv("DCNS_BIN_RATIO")) C.bin_ratio = std::max(0.1, std::min(4.0, std::atof(e)));
   if (const char *e = std::getenv("DCNS_BINS_BY_SIZE")) C.bins_by_size = std::atoi(e) != 0;
@@ -1874,6 +1873,7 @@ void run_semiglobal(Context &C, std::vector<SgTask> &G, const Params &P, bool wa
     h2d(C, C.d_idx, idx.data(), (size_t)m);
     h2d(C, C.d_sg, G.data(), (size_t)n);
     SgFlow F{};
+    int64_t busy = 0;  // stripes that can be under way at a time
     if (flow) {
       // units (stripes) and boundary rows in queue order; flow state in one buffer:
       // dps | order | counters
@@ -1884,12 +1884,15 @@ void run_semiglobal(Context &C, std::vector<SgTask> &G, const Params &P, bool wa
         const SgTask &g = G[idx[q]];
         nst[q] = (int32_t)sg_flow_units(g.n1, g.n2, P.bandwidth);
         units += nst[q];
+        const int64_t steps = std::min<int64_t>(g.n2, 2 * (int64_t)P.bandwidth + 128) + 31;
+        busy += std::min<int64_t>(nst[q], steps / (g.n1 > P.bandwidth ? 175 : 63) + 1);
         dps[q] = SgFlowDP{brows, 0, 0, 0, -1, -1, 0, kOut, kOut};
         if (!want_codes) brows += std::max(g.n2, 0) + 2;
       }
-      // hand-out order: stripe-major within groups of consecutive DPs holding at least eight grid-fulls of units;
+      // hand-out order: stripe-major within groups of consecutive DPs holding at least sixteen grid-fulls of units
+      // (with eight the DPs of a 200 kb pair fall into two groups, whose long ones run one after the other: 116 ms, 78);
       // inside a group the DPs go by stripe count, most first, so the DPs that have a stripe s form a prefix
-      const int64_t group_units = 8 * sg_flow_grid_warps(C.nsm, C.sg_flow_blocks);
+      const int64_t group_units = 16 * sg_flow_grid_warps(C.nsm, 2);
       std::vector<int2> order((size_t)units);
       {
         int64_t u = 0;
@@ -1934,11 +1937,17 @@ void run_semiglobal(Context &C, std::vector<SgTask> &G, const Params &P, bool wa
       C.d_bnd.ensure(C, (size_t)sg_bnd_bytes(grid, maxn2, nw));
     }
     DCNS_CK(cudaEventRecord(C.ev0, C.st));
-    if (flow)
-      launch_semiglobal_flow(F, C.arena, P, W, C.d_sgtb.as<uint8_t>(), want_codes, C.nsm, C.sg_flow_blocks, C.st);
-    else
+    if (flow) {
+      // A warp alone on its scheduler goes at the speed of a step's latency, and a chain of stripes at that of its
+      // slowest: one block per SM where that holds most of the stripes that can run.  Three DPs of 80,000 rows (690
+      // stripes at a time, 608 warps) 12.1 ms with one, 15.7 with two; six 20.1 and 16.7.
+      const int64_t one = sg_flow_grid_warps(C.nsm, 1);
+      launch_semiglobal_flow(F, C.arena, P, W, C.d_sgtb.as<uint8_t>(), want_codes, C.nsm,
+                             4 * busy <= 5 * one ? 1 : C.sg_flow_blocks, C.st);
+    } else {
       launch_semiglobal(C.d_sg.as<SgTask>(), C.d_idx.as<int>(), (int)m, C.arena, P, C.d_sgtb.as<uint8_t>(),
                         C.d_bnd.p, maxn2, C.d_counter.as<int>(), grid, nw, C.st);
+    }
     DCNS_CK(cudaEventRecord(C.ev1, C.st));
     int flow_err = 0;
     if (flow) DCNS_CK(cudaMemcpyAsync(&flow_err, F.err, sizeof(int), cudaMemcpyDeviceToHost, C.st));
@@ -2541,19 +2550,19 @@ void autotune(Context &C, Batch &B, const Params &P, int mode) {
     for (int b = 0; b < nb; ++b) C.bin_tune[b].scan_tiles = bin_t[b];
   }
   if (mode == DCNS_MODE_TWO_GAP) {
-    // the stripe flow with 4, 5 or 6 blocks per SM (-4, -5, -6 below), or one CTA per DP with 2, 4 or 8 warps (0: by
-    // the number of DPs)
-    int best_w = -4;
+    // the stripe flow with 2 blocks per SM or 1 (-2, -1 below), or one CTA per DP with 2, 4 or 8 warps (0: by the
+    // number of DPs)
+    int best_w = -2;
     double best_w_ms = 1e300;
-    for (int nw : {-4, -5, -6, 0, 2, 4, kSgNW}) {
+    for (int nw : {-2, -1, 0, 2, 4, kSgNW}) {
       C.sg_flow = nw < 0;
-      C.sg_flow_blocks = nw < 0 ? -nw : 4;
+      C.sg_flow_blocks = nw < 0 ? -nw : 2;
       C.sg_warps = std::max(nw, 0);
       const double ms = std::min(run(best), run(best));
       if (best_w_ms == 1e300 || better(ms, best_w_ms)) best_w_ms = ms, best_w = nw;
     }
     C.sg_flow = best_w < 0;
-    C.sg_flow_blocks = best_w < 0 ? -best_w : 4;
+    C.sg_flow_blocks = best_w < 0 ? -best_w : 2;
     C.sg_warps = std::max(best_w, 0);
   }
 }

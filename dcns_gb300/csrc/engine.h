@@ -188,8 +188,8 @@ struct Context {
   int sg_warps = 0;
   // unweighted semi-global DPs as a flow of stripe units over one persistent grid (DCNS_SG_FLOW=0: one CTA per DP)
   bool sg_flow = true;
-  // resident blocks per SM of the stripe-flow kernel: 4 (128 registers), 5 (96) or 6 (80) (DCNS_SG_FLOW_BLOCKS)
-  int sg_flow_blocks = 4;
+  // blocks per SM of the stripe-flow kernel, 1 or 2, at most (DCNS_SG_FLOW_BLOCKS)
+  int sg_flow_blocks = 2;
   // seed-scan tiling target: reference rows are split into chunks while a launch has fewer tiles than this many per
   // resident thread (DCNS_SCAN_TILES)
   int scan_tiles_per_thread = 8;

@@ -395,8 +395,10 @@ __device__ __forceinline__ int sg_wait_at_least(const int *flag, int need, const
   return -1;
 }
 
-constexpr int kSgFlowWarps = 4;  // warps per block of the flow kernel
+constexpr int kSgFlowWarps = 4;   // warps per block of the flow kernel
+constexpr int kSgFlowBlocks = 2;  // blocks per SM that its registers must allow
 constexpr int kSgChunk = 16;      // steps between two looks at the stripe above
+constexpr int kSgUnroll = 8;      // of them unrolled
 
 // ---- traceback checkpoints
 // A DP whose path is wanted keeps no direction code per cell.  It keeps what is needed to compute any 128 x 128 tile
@@ -562,23 +564,37 @@ struct __align__(16) SgFeed {
   uint32_t sel;
 };
 
-// CK: the DPs keep traceback checkpoints.  MINB: resident blocks per SM the register allocation must allow.
+// CK: the DPs keep traceback checkpoints.
 //
-// Steps run in chunks of 16.  A chunk whose columns lie inside the band of every row of the stripe, off the band's
-// last column and the stale column, takes the cell without any band test (9 of 22 operations): under the default band
-// of 20,000 all but the first two and the last of a stripe.
+// Steps run in chunks of 16 of one of four kinds.  Inside: the columns of all lanes lie in the band of every row of the
+// stripe, off the band's last column and the stale column: no band test (9 of 22 operations a cell).  Left: some rows
+// have not reached their band's first column.  What lies left of a row's band feeds only cells left of the next rows'
+// bands, but for its horizontal states and the row's maximum: those alone are masked.  Right: some rows are past
+// their band's last column.  What lies right of it feeds only cells right of the next rows' bands, but for the
+// vertical states that reach the next row's last column, which takes none: those and the maximum are masked.  Any:
+// both ends in one chunk, and the stripes that hold a stale column.
 //
-// Bound: integer issue (ALU pipe at 59 %, issue slots at 55 %) where there are many DPs, and the chain of stripes (a
-// stripe starts 31 + 3 chunks + the band's 128 columns of steps after the one above) where there are few long ones.
-// Measured on one GB300, against direction codes for every cell, band tests in every cell, progress counters with
-// release and acquire, and 5 blocks per SM: 2,715 DPs of the 500-pair batch 39.9 -> 16.8 ms, 400 DPs of 3 kb with a
-// path 14.3 -> 4.85 ms, 30 DPs of a 200 kb pair 497 -> 159 ms.  Chunks of 8, 16 and 32 steps: 162, 159 and 170 ms on
-// the long DPs, 18.3, 16.8 and 16.7 ms on the batch; 3, 4, 5 and 6 blocks per SM (before the tagged cells): 173, 183,
-// 215 and 250 ms and 19.5, 19.1, 20.5 and 22.8 ms.  The weighted DPs ran one warp each before, 32 rows at a time:
-// 1,072 DPs 128.5 -> 4.8 ms.
-template <bool CK, int KIND, int MINB>
-__global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow F, Arena ar, Params P, SgWeights W,
-                                                                         uint8_t *__restrict__ tb) {
+// Bound: the latency of a step (185-215 cycles for 81 instructions without checkpoints, 230 with them) times the chain
+// of stripes.  A stripe starts 31 + 2 chunks of steps behind the one above, and under a sliding band 128 columns more
+// at its left end, and again ends so much later at its right end: with the full band tests there, 2.3 times the
+// instructions, a chunk's wait was passed back along the band and all stripes went at half speed.  Two blocks per SM:
+// a stripe slowed by its neighbours on the scheduler slows the chain behind it, so more warps than the DPs can use at
+// a time cost more than they give.
+//
+// Measured on one GB300: one DP of 20,000 more rows under bands of 2,000 and 20,000: 6.2 -> 3.0 ms, 35 -> 19 us a
+// stripe.  Of it the chunk looked ahead one instead of two chunks 0.5 ms, the left kind 0.3, the right kind 2.0.
+// 30 DPs of a 200 kb pair 497 (direction codes for every cell, band tests in every cell, progress counters with
+// release and acquire, 5 blocks per SM) -> 159 (codes computed again from checkpoints, tests only at the ends,
+// tagged cells) -> 78 ms; 2,715 DPs of the 500-pair batch 39.9 -> 16.8 -> 13.6 ms; 400 DPs of 3 kb with a path
+// 14.3 -> 4.85 -> 3.65 ms; the weighted drivers' 1,072 DPs 128.5 (one warp each, 32 rows at a time) -> 4.2 -> 3.0 ms.
+// Blocks per SM, 2 / 3 / 4 (the last before the right kind): 78 / 102 / 142 ms on the long DPs, 13.6 / 13.8 / 15.9 on
+// the batch.  Steps unrolled 1 / 4 / 8 / 16: 15.4 / 14.2 / 13.8 / 14.3 ms on the batch.  The checkpoints' address
+// computed once per stripe and their test left out of chunks without such a column: 101 -> 83 instructions a step.
+enum SgEdge { kSgInside, kSgLeft, kSgRight, kSgAny };
+template <bool CK, int KIND>
+__global__ void __launch_bounds__(32 * kSgFlowWarps, kSgFlowBlocks) sg_flow_kernel(SgFlow F, Arena ar, Params P,
+                                                                                      SgWeights W,
+                                                                                      uint8_t *__restrict__ tb) {
   __shared__ SgFeed stage[kSgFlowWarps][2][kSgChunk];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w = P.bandwidth;
@@ -631,25 +647,45 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow
     // all rows, off the last and the stale column (rows past the DP compute what nobody reads)
     const int in_lo = max(r0 + kSgRows - 1 - w, 1) - jstart + 31;
     const int in_hi = min(r0 + w, n2 - 1) - jstart;
+    const bool plain_right = KIND != 0 || rl < r_last - 1;  // no row of the stripe passes its stale column on
     int abandon = 0;  // 0 computing, 1 the DP stopped, -1 a wait ran out
     // column jstart + kSgChunk * chunk + lane of the row above, as it is now, and whether stripe s - 1 has written it
     // (tag s; the columns past row 128s's band hold kOut)
-    auto look = [&](int chunk, SgCell &v) {
-      const int j = jstart + kSgChunk * chunk + lane;
-      v = SgCell{kOut, kOut, kOut, s};
-      if (s > 0 && lane < kSgChunk && j <= upB) v = sg_ld_cell(bin + j);
+    auto look = [&](int chunk, SgCell &v) {  // the load alone, so that nothing waits for it: see `there`
+      v = sg_ld_cell(bin + min(jstart + kSgChunk * chunk + (lane & (kSgChunk - 1)), upB));
     };
-    auto stage_cells = [&](int chunk, const SgCell &v) {
+    auto there = [&](int chunk, SgCell &v) {
+      const bool need = s > 0 && lane < kSgChunk && jstart + kSgChunk * chunk + lane <= upB;
+      const bool ok = !need || v.tag == s;
+      if (!need) v = SgCell{kOut, kOut, kOut, s};
+      return __all_sync(0xFFFFFFFFu, ok) != 0;
+    };
+    // the words that hold those columns' symbols (loaded a chunk before they are staged)
+    auto look_syms = [&](int chunk) {
       const int j = jstart + kSgChunk * chunk + lane;
-      if (lane < kSgChunk)
-        stage[warp][chunk & 1][lane] = SgFeed{v.m, v.f1, v.f2, j <= n2 ? sg_selector(s2.at(ar, j - 1)) : 0x4444u};
+      uint2 r{0u, 0u};
+      if (lane < kSgChunk && j <= n2) {
+        const int64_t k = s2.base + s2.a + (s2.dir == 0 ? j - 1 : 1 - j);
+        r = uint2{__ldg(ar.pk + (k >> 4)), __ldg(ar.nm + (k >> 5))};
+      }
+      return r;
+    };
+    auto stage_cells = [&](int chunk, const SgCell &v, const uint2 &sy) {
+      const int j = jstart + kSgChunk * chunk + lane;
+      if (lane < kSgChunk) {
+        const uint32_t k = (uint32_t)(s2.base + s2.a + (s2.dir == 0 ? j - 1 : 1 - j));
+        const uint32_t two = (sy.x >> (2u * (k & 15u))) & 3u, n = (sy.y >> (k & 31u)) & 1u;
+        const uint32_t code = s2.dir == 0 ? two : 3u - two;
+        stage[warp][chunk & 1][lane] =
+            SgFeed{v.m, v.f1, v.f2, j <= n2 && n == 0u ? code | (code | 8u) * 0x1110u : 0x4444u};
+      }
     };
     // Looks until stripe s - 1 has written the chunk's columns (every wait ends or runs out of iterations, as
     // sg_wait_at_least).
     auto wait_cells = [&](int chunk, SgCell &v) {
       for (int it = 0;; ++it) {
         look(chunk, v);
-        if (__all_sync(0xFFFFFFFFu, v.tag == s)) return;
+        if (there(chunk, v)) return;
         if (__any_sync(0xFFFFFFFFu, sg_ld_relaxed(&D.stop) != 0)) {
           abandon = 1;
           return;
@@ -662,8 +698,9 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow
       }
     };
     SgCell ahead;
+    uint2 syms = look_syms(0);
     wait_cells(0, ahead);
-    stage_cells(0, ahead);
+    stage_cells(0, ahead, syms);
     // the diagonal of the stripe's first row at column jstart: cell (0, 0) = 0 for the DP's first row, else the
     // row above at jstart - 1 (kOut at column 0), written before column jstart
     int diag = kOut;
@@ -674,15 +711,20 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow
       if (lane == 0) diag = d.m;
       if (__any_sync(0xFFFFFFFFu, d.tag != s)) abandon = -1;
     }
-    if (abandon == 0) wait_cells(1, ahead);
-    stage_cells(1, ahead);
     __syncwarp();
     int outM = kOut, outF1 = kOut, outF2 = kOut;
     uint32_t outS = 0x4444u;
+    const int cl = i0 - w;  // the lane's first row's first column, or less than 1
     const bool lane0 = lane == 0, write_bnd = lane == 31 && produce;
+    // the lane's part of column checkpoint j: 3 kSgRows ints each, kSgTile columns apart
+    static_assert(kSgTile == kSgRows, "");
+    int *const ckp = CK ? sg_ck_col(tb, T, w, s, jstart / kSgTile * kSgTile) - (int64_t)3 * (jstart / kSgTile * kSgTile) +
+                              kSgR * lane
+                        : nullptr;
 
-    auto step = [&](int t, const SgFeed *srow, auto inside) {
-      constexpr bool IN = decltype(inside)::value;
+    auto step = [&](int t, const SgFeed *srow, auto edge, auto cks) {
+      constexpr bool CKS = decltype(cks)::value;
+      constexpr SgEdge EDGE = decltype(edge)::value;
       int upM = __shfl_up_sync(0xFFFFFFFFu, outM, 1);
       int aF1 = __shfl_up_sync(0xFFFFFFFFu, outF1, 1);
       int aF2 = KIND == 1 ? kOut : __shfl_up_sync(0xFFFFFFFFu, outF2, 1);
@@ -694,20 +736,35 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow
       sel = lane0 ? rec.sel : sel;
       const int j = jstart + t - lane;
       int dg = diag;
-      const bool stale_col = !IN && KIND == 0 && stale_rows != 0 && j == n2 - 1;
+      const bool stale_col = EDGE == kSgAny && KIND == 0 && stale_rows != 0 && j == n2 - 1;
 #pragma unroll
       for (int k = 0; k < kSgR; ++k) {
-        bool valid = true, last = false;
-        if constexpr (!IN) {
+        bool valid = true, last = false, end = false;
+        if constexpr (EDGE == kSgLeft) valid = j >= max(cl + k, 1);
+        if constexpr (EDGE == kSgRight) {
+          const int c1 = min(cl + k + 2 * w, n2);
+          valid = j <= c1;
+          if (KIND != 0 && j == c1) aF1 = kOut, aF2 = kOut;
+          end = j >= c1;
+        }
+        if constexpr (EDGE == kSgAny) {
           const int i = i0 + k, c0 = max(i - w, 1), c1 = min(i + w, n2);
           valid = i <= n1_eff && j >= c0 && j <= c1;
           last = j == c1;
         }
         int cF1, cF2;
-        const int cM = sg_cell<false, KIND, IN>(sg_row_score<KIND>(prof[k], rp[k], sel), dg, aF1, aF2, e1[k], e2[k],
+        const int cM = sg_cell<false, KIND, EDGE != kSgAny>(sg_row_score<KIND>(prof[k], rp[k], sel), dg, aF1, aF2, e1[k], e2[k],
                                                 valid, last, rp[k], P, cF1, cF2, nullptr);
+        if constexpr (EDGE == kSgRight && KIND == 0) {
+          cF1 = end ? kOut : cF1;
+          cF2 = end ? kOut : cF2;
+        }
+        if constexpr (EDGE == kSgLeft) {
+          e1[k] = valid ? e1[k] : kOut;
+          if (KIND != 1) e2[k] = valid ? e2[k] : kOut;
+        }
         bool keep;
-        best[k] = __vibmax_s32(best[k], cM, &keep);  // keep: !(cM > best), the first maximum of the row stays
+        best[k] = __vibmax_s32(best[k], (EDGE == kSgLeft || EDGE == kSgRight) && !valid ? kOut : cM, &keep);  // keep: !(cM > best), the first maximum of the row stays
         bestj[k] = keep ? bestj[k] : j;
         if (stale_col && valid) {
           if ((stale_rows >> k) & 1) D.stale_last = cM;
@@ -719,9 +776,9 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow
         aF1 = cF1, aF2 = cF2;
         if (k == kSgR - 1) outM = cM;
       }
-      if constexpr (CK) {
-        if ((j & (kSgTile - 1)) == 0 && (IN || (j >= jstart && j <= jend))) {
-          int *const c = sg_ck_col(tb, T, w, s, j) + kSgR * lane;
+      if constexpr (CKS) {
+        if ((j & (kSgTile - 1)) == 0 && (EDGE == kSgInside || (j >= jstart && j <= jend))) {
+          int *const c = ckp + (int64_t)3 * j;
           *reinterpret_cast<int4 *>(c) = make_int4(prevM[0], prevM[1], prevM[2], prevM[3]);
           *reinterpret_cast<int4 *>(c + kSgRows) = make_int4(e1[0], e1[1], e1[2], e1[3]);
           if (KIND != 1) *reinterpret_cast<int4 *>(c + 2 * kSgRows) = make_int4(e2[0], e2[1], e2[2], e2[3]);
@@ -731,24 +788,46 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, MINB) sg_flow_kernel(SgFlow
       outF1 = aF1, outF2 = aF2, outS = sel;
     };
 
-    // Chunks of kSgChunk steps.  At a chunk's start the warp looks at the columns of the chunk two ahead (and at the
-    // DP's stop flag); at its end they are staged if they were all there, so the steps hide the round trip to L2, and
-    // a warp that runs too close behind its producer waits there.
+    // Chunks of kSgChunk steps.  At a chunk's start the warp looks at the columns of the next one (and at the DP's
+    // stop flag); at its end they are staged if they were all there, so the steps hide the round trip to L2, and a
+    // warp that runs too close behind its producer waits there.
     for (int tc = 0; tc < nsteps && abandon == 0; tc += kSgChunk) {
       const int chunk = tc / kSgChunk;
       const SgFeed *const srow = stage[warp][chunk & 1];
       const int stopped = sg_ld_relaxed(&D.stop);
-      look(chunk + 2, ahead);
+      look(chunk + 1, ahead);
+      syms = look_syms(chunk + 1);
+      auto run = [&](auto edge, auto cks) {
+#pragma unroll kSgUnroll
+        for (int t = tc; t < tc + kSgChunk; ++t) step(t, srow, edge, cks);
+      };
+      const std::integral_constant<SgEdge, kSgInside> inside{};
+      const std::integral_constant<SgEdge, kSgLeft> left{};
+      const std::integral_constant<SgEdge, kSgRight> right{};
+      const std::integral_constant<SgEdge, kSgAny> any{};
+      const std::bool_constant<CK> ck{};
+      const int tend = min(tc + kSgChunk, nsteps);
       if (tc >= in_lo && tc + kSgChunk <= in_hi) {
-        for (int t = tc; t < tc + kSgChunk; ++t) step(t, srow, std::true_type{});
+        // the chunk's columns end at j1 and begin 31 + kSgChunk - 1 before it: a column checkpoint among them?
+        const int j1 = jstart + tc + kSgChunk - 1;
+        if (CK && (j1 & (kSgTile - 1)) <= 31 + kSgChunk - 1)
+          run(inside, ck);
+        else
+          run(inside, std::false_type{});
+      } else if (tc + kSgChunk <= in_hi) {
+        run(left, ck);
+      } else if (tc >= in_lo && plain_right) {
+        if (tend == tc + kSgChunk)
+          run(right, ck);
+        else
+          for (int t = tc; t < tend; ++t) step(t, srow, right, ck);
       } else {
-        const int tend = min(tc + kSgChunk, nsteps);
-        for (int t = tc; t < tend; ++t) step(t, srow, std::false_type{});
+        for (int t = tc; t < tend; ++t) step(t, srow, any, ck);
       }
       if (__any_sync(0xFFFFFFFFu, stopped != 0)) abandon = 1;  // the DP ended
-      if (abandon == 0 && !__all_sync(0xFFFFFFFFu, ahead.tag == s)) wait_cells(chunk + 2, ahead);
+      if (abandon == 0 && !there(chunk + 1, ahead)) wait_cells(chunk + 1, ahead);
       __syncwarp();
-      stage_cells(chunk + 2, ahead);
+      stage_cells(chunk + 1, ahead, syms);
       __syncwarp();
     }
     if (abandon < 0 && lane == 0) {
@@ -846,24 +925,20 @@ int64_t sg_flow_units(int n1, int n2, int w) {
   return std::max<int64_t>(1, (n1_eff + kSgRows - 1) / kSgRows);
 }
 
-int64_t sg_flow_grid_warps(int nsm, int minb) { return (int64_t)nsm * minb * kSgFlowWarps; }
+int64_t sg_flow_grid_warps(int nsm, int blocks) { return (int64_t)nsm * blocks * kSgFlowWarps; }
 
 void launch_semiglobal_flow(const SgFlow &f, Arena ar, Params p, const SgWeights *wt, uint8_t *tb, bool path, int nsm,
-                            int minb, cudaStream_t st) {
+                            int blocks_per_sm, cudaStream_t st) {
   if (f.total_units <= 0) return;
-  const int64_t warps = std::min<int64_t>(f.total_units, sg_flow_grid_warps(nsm, minb));
+  const int64_t warps = std::min<int64_t>(f.total_units, sg_flow_grid_warps(nsm, blocks_per_sm));
   const int blocks = (int)((warps + kSgFlowWarps - 1) / kSgFlowWarps), threads = 32 * kSgFlowWarps;
   auto run = [&](auto kernel) { kernel<<<blocks, threads, 0, st>>>(f, ar, p, wt ? *wt : SgWeights{}, tb); };
   if (wt && wt->pieces == 1)
-    path ? run(sg_flow_kernel<true, 1, 4>) : run(sg_flow_kernel<false, 1, 4>);
+    path ? run(sg_flow_kernel<true, 1>) : run(sg_flow_kernel<false, 1>);
   else if (wt)
-    path ? run(sg_flow_kernel<true, 2, 4>) : run(sg_flow_kernel<false, 2, 4>);
-  else if (minb == 6)
-    path ? run(sg_flow_kernel<true, 0, 6>) : run(sg_flow_kernel<false, 0, 6>);
-  else if (minb == 5)
-    path ? run(sg_flow_kernel<true, 0, 5>) : run(sg_flow_kernel<false, 0, 5>);
+    path ? run(sg_flow_kernel<true, 2>) : run(sg_flow_kernel<false, 2>);
   else
-    path ? run(sg_flow_kernel<true, 0, 4>) : run(sg_flow_kernel<false, 0, 4>);
+    path ? run(sg_flow_kernel<true, 0>) : run(sg_flow_kernel<false, 0>);
 }
 
 // ------------------------------------------------------------------ traceback of the flow's DPs: tiles computed again
@@ -910,8 +985,9 @@ __device__ __forceinline__ void sg_tile_codes(const SgTask &T, const Arena &ar, 
     prof[k] = KIND == 0 ? sg_profile(ci, P.match, P.mismatch) : sg_profile(ci, 1, 0);
     if constexpr (KIND != 0) rp[k].load(T, W, i, lv);
     prevM[k] = from ? col[k] : kOut;
-    e1[k] = from ? col[kSgRows + k] : kOut;
-    e2[k] = (from && KIND != 1) ? col[2 * kSgRows + k] : kOut;
+    const bool in = from && left >= i - w;  // left of its band a row has no horizontal gap
+    e1[k] = in ? col[kSgRows + k] : kOut;
+    e2[k] = (in && KIND != 1) ? col[2 * kSgRows + k] : kOut;
   }
   // the diagonal of the lane's first row at column ja: lanes above 0 take the lane above's checkpoint by shuffle
   int diag = kOut;

@@ -192,7 +192,7 @@ typedef struct {
   int32_t sg_warps;               /* warps per 2-piece DP when one CTA runs a DP (0: two for launches of many DPs,
                                      else eight) */
   int32_t sg_flow;                /* 1: 2-piece DPs run as a flow of 128-row stripe units over one persistent grid */
-  int32_t sg_flow_blocks;         /* resident blocks per SM of that grid: 4, 5 or 6 */
+  int32_t sg_flow_blocks;         /* blocks per SM of that grid: 1 or 2 */
   int32_t bins_by_size;           /* 1: bins are runs of pairs in increasing size (the largest last); 0: mixed */
   int32_t n_bins_tuned;           /* bins with their own tiling target below (0: every bin uses bin 0's value) */
   /* no longer set (an x-drop pass has one form per band width): zero */

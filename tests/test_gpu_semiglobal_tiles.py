@@ -77,3 +77,40 @@ def test_weighted_edges(lib, oracle):
                 assert [f.key() for f in got[k]] == [f.key() for f in exp], (k, pieces, bandwidth)
                 found += len(exp)
     assert found > 100
+
+
+def related(rng, n1, n2, shift):
+    """A pair that aligns from its first base on; after 150 bases one of the two holds `shift` bases more, so that the
+    path runs that far off the diagonal."""
+    a = W.random_seq(rng, max(n1, n2) + abs(shift) + 1)
+    b = bytes(a[:150]) + W.mutate(rng, bytes(a[150:]), 0.93, 0.004)
+    ins = bytes(W.random_seq(rng, abs(shift)))
+    a, b = (bytes(a), b[:150] + ins + b[150:]) if shift > 0 else (bytes(a[:150]) + ins + bytes(a[150:]), b)
+    return W.prepare(a[:n1].decode()), W.prepare(b[:n2].decode())
+
+
+@pytest.mark.parametrize("w", [20, 65, 79, 80, 96, 127, 143, 144, 160, 200, 333, 700])
+def test_sliding_bands(lib, oracle, w):
+    """Bands that slide over several stripes, with the path in their middle and along either edge: chunks that hold the
+    left end, the right end or both, stripes with the stale column, sequences that end inside the band."""
+    rng = np.random.default_rng(w)
+    tasks = [related(rng, n1, n2, s) for n1, n2 in ((900, 900), (1100, 700), (641, 1000), (1025, 1024), (897, 640 + w))
+             for s in (0, w - 3, 3 - w)]
+    for kw in (dict(), dict(ext2=-1, open2=-30)):
+        check(lib, oracle, tasks, bandwidth=w, zdrop=4000, **kw)
+
+
+@pytest.mark.parametrize("w", [65, 160, 333])
+def test_weighted_sliding_bands(lib, oracle, w):
+    rng = np.random.default_rng(w)
+    cats = [(2, -3, -4, -2, -45, 0, 4000), (3, -4, -6, -2, -60, -1, 4000), (1, -2, -3, -1, -30, 0, 4000)]
+    found = 0
+    for pieces in (1, 2):
+        cases = [related(rng, n1, n2, s) for n1, n2 in ((900, 900), (1100, 700), (641, 1000)) for s in (0, w - 3, 3 - w)]
+        cat = [rng.integers(0, 3, len(a)).astype(np.int16) for a, _ in cases]
+        got = lib.align_weighted(cases, cat, cats, pieces, bandwidth=w)
+        for k, ((a, b), c) in enumerate(zip(cases, cat)):
+            exp = oracle.find_weighted(a, b, c, cats, pieces, bandwidth=w)
+            assert [f.key() for f in got[k]] == [f.key() for f in exp], (k, pieces)
+            found += len(exp)
+    assert found >= 12
