@@ -950,9 +950,16 @@ void launch_semiglobal_flow(const SgFlow &f, Arena ar, Params p, const SgWeights
 // them until the path leaves them all.  The walk takes a run at a time: the lanes look at the next 32 cells in the
 // current direction, and a ballot says how far the state holds.  NT = 8 where the DPs leave SMs idle anyway (one
 // block per SM), else 4 (three blocks per SM).
+//
+// Bound: the steps of a tile (159 of them, two warps to a scheduler: five sixths of the time), then the walk's chain of
+// shared-memory reads and votes (520 cycles a run).  Half the tiles ahead are on the path; the others lie past a gap
+// that moved it across a tile's corner.  Steps that all lanes take without a test of it, the last operation of the
+// CIGAR in registers, tests of the band only in tiles that need them, and the reversal by all threads: 30 DPs of a
+// 200 kb pair 28.4 -> 24.8 ms, 2,715 DPs of the 500-pair batch 2.16 -> 1.90 ms, 400 DPs of 3 kb 0.84 -> 0.66 ms.
 
 struct SgTile {
   int s, ja, jb, tr;  // stripe, columns [ja, jb], rows up to tr
+  int inside;         // whether its cells lie in every row's band, off the last column
 };
 
 template <int KIND, bool INSIDE>
@@ -995,12 +1002,13 @@ __device__ __forceinline__ void sg_tile_codes(const SgTask &T, const Arena &ar, 
   int outM = prevM[kSgR - 1], outF1 = kOut, outF2 = kOut;
   __syncwarp();
   const int nsteps = jb - ja + 1 + (X.tr - 1 - kSgRows * ts) / kSgR;
-  for (int t = 0; t < nsteps; ++t) {
+  auto step = [&](int t, auto all) {  // all: every lane is in the tile
+    constexpr bool ALL = decltype(all)::value;
     int upM = __shfl_up_sync(0xFFFFFFFFu, outM, 1);
     int aF1 = __shfl_up_sync(0xFFFFFFFFu, outF1, 1);
     int aF2 = __shfl_up_sync(0xFFFFFFFFu, outF2, 1);
     const int c = t - lane, j = ja + c;
-    const bool on = c >= 0 && j <= jb;
+    const bool on = ALL || (c >= 0 && j <= jb);
     const SgFeed rec = feed[on ? c : 0];
     if (lane == 0) upM = rec.m, aF1 = rec.f1, aF2 = rec.f2;
     if (on) {
@@ -1028,7 +1036,13 @@ __device__ __forceinline__ void sg_tile_codes(const SgTask &T, const Arena &ar, 
       outF1 = aF1, outF2 = aF2;
     }
     diag = upM;
-  }
+  };
+  int t = 0;
+  const int full = min(nsteps, jb - ja + 1);
+  for (; t < min(nsteps, 31); ++t) step(t, std::false_type{});
+#pragma unroll 2
+  for (; t < full; ++t) step(t, std::true_type{});
+  for (; t < nsteps; ++t) step(t, std::false_type{});
   __syncwarp();
 }
 
@@ -1039,7 +1053,7 @@ __global__ void __launch_bounds__(32 * NT) sg_retrace_kernel(SgTask *__restrict_
                                                                    uint32_t *__restrict__ cig) {
   extern __shared__ uint4 rt_smem[];  // per warp: codes [column][lane] (a lane's four rows a word), then the feed
   __shared__ SgTile tile[NT];
-  __shared__ int more;
+  __shared__ int more, nops;
   const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
   auto codes_of = [&](int k) { return reinterpret_cast<uint32_t(*)[32]>(rt_smem) + k * kSgTile; };
   SgFeed *const feed = reinterpret_cast<SgFeed *>(reinterpret_cast<uint32_t(*)[32]>(rt_smem) + NT * kSgTile) +
@@ -1052,19 +1066,23 @@ __global__ void __launch_bounds__(32 * NT) sg_retrace_kernel(SgTask *__restrict_
   uint32_t *const out = cig + T.cig_off;
   const int cap = T.cig_cap;
   uint32_t last = 0xFFFFFFFFu;
+  int len = 0;
   bool full = false;
-  auto push = [&](uint32_t op, int n) {
-    if (nc > 0 && (last & 0xFu) == op) {
-      last += (uint32_t)n << 4;
-    } else {
+  auto push = [&](uint32_t op, int n) {  // the last operation stays in registers until another follows
+    if (op == last) {
+      len += n;
+      return;
+    }
+    if (len > 0) {
       if (nc >= cap) {
         full = true;
         return;
       }
-      last = ((uint32_t)n << 4) | op;
+      if (lane == 0) out[nc] = ((uint32_t)len << 4) | last;
       ++nc;
     }
-    if (lane == 0) out[nc - 1] = last;
+    last = op;
+    len = n;
   };
   auto in_band = [&](int i, int j) {
     return i > 0 && j > 0 && i <= rows && j >= max(i - w, 1) && (j < min(i + w, n2) || (KIND != 0 && j == min(i + w, n2)));
@@ -1102,25 +1120,26 @@ __global__ void __launch_bounds__(32 * NT) sg_retrace_kernel(SgTask *__restrict_
         }
         cur = (cur + k) % NT;
         const SgTile X = tile[cur];
-        uint32_t(*const code)[32] = codes_of(cur);
         const int rtop = kSgRows * s;  // rows above the tile end here
-        // the next 32 cells in the direction of the state
-        const int di = state == 2 || state >= 4 ? 0 : 1, dj = state == 1 || state == 3 ? 0 : 1;
-        const int ci = ii - di * lane, cj = jj - dj * lane;
-        const bool in = ci > rtop && cj >= X.ja && in_band(ci, cj);
-        int c = 255;
-        if (in) c = (int)((code[cj - X.ja][(ci - 1 - rtop) / kSgR] >> (8 * ((ci - 1 - rtop) % kSgR))) & 0xFFu);
-        const bool hold = in && (state == 0 ? (c & 7) == 0 : ((c >> (state + 2)) & 1) != 0);
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, hold);
-        const int run = m == 0xFFFFFFFFu ? 32 : __ffs(~m) - 1;
-        if (run > 0) {
-          push(state == 0 ? 0u : (state == 1 || state == 3) ? 2u : 1u, run);
-          ii -= di * run;
-          jj -= dj * run;
-        }
-        if (run < 32) {  // the cell the run ends at, if it lies in this tile, starts a new state
-          const int there = __shfl_sync(0xFFFFFFFFu, (int)in, run), fresh = __shfl_sync(0xFFFFFFFFu, c & 7, run);
-          if (there) {
+        // a tile's codes are bytes [column][row]
+        const uint8_t *const code = reinterpret_cast<const uint8_t *>(codes_of(cur));
+        auto in_tile = [&](int i, int j) { return i > rtop && j >= X.ja && (X.inside || in_band(i, j)); };
+        do {
+          // the next 32 cells in the direction of the state
+          const int di = state == 2 || state >= 4 ? 0 : 1, dj = state == 1 || state == 3 ? 0 : 1;
+          const int ci = ii - di * lane, cj = jj - dj * lane;
+          const bool in = in_tile(ci, cj);
+          const int c = in ? (int)code[(cj - X.ja) * kSgRows + (ci - 1 - rtop)] : 255;
+          const bool hold = in && (state == 0 ? (c & 7) == 0 : ((c >> (state + 2)) & 1) != 0);
+          const unsigned m = __ballot_sync(0xFFFFFFFFu, hold), mi = __ballot_sync(0xFFFFFFFFu, in);
+          const int run = m == 0xFFFFFFFFu ? 32 : __ffs(~m) - 1;
+          const int fresh = __shfl_sync(0xFFFFFFFFu, c & 7, run & 31);
+          if (run > 0) {
+            push(state == 0 ? 0u : (state == 1 || state == 3) ? 2u : 1u, run);
+            ii -= di * run;
+            jj -= dj * run;
+          }
+          if (run < 32 && ((mi >> run) & 1u)) {  // the cell the run ends at, if it lies in this tile, starts a new state
             state = fresh;
             if (state == 1 || state == 3) {
               push(2, 1);
@@ -1130,7 +1149,7 @@ __global__ void __launch_bounds__(32 * NT) sg_retrace_kernel(SgTask *__restrict_
               --jj;
             }
           }
-        }
+        } while (in_tile(ii, jj));
       }
       if (lane == 0) {
         more = need;
@@ -1138,7 +1157,7 @@ __global__ void __launch_bounds__(32 * NT) sg_retrace_kernel(SgTask *__restrict_
           int i = ii, j = jj;
           const bool go_up = state != 2 && state != 4, go_left = state != 1 && state != 3;
           for (int k = 0; k < NT; ++k) {
-            SgTile X{-1, 0, -1, 0};
+            SgTile X{-1, 0, -1, 0, 0};
             if (i > 0 && j > 0) {
               X.s = (i - 1) / kSgRows;
               const int r0 = kSgRows * X.s + 1, jstart = max(r0 - w, 1);
@@ -1147,6 +1166,8 @@ __global__ void __launch_bounds__(32 * NT) sg_retrace_kernel(SgTask *__restrict_
               X.jb = k == 0 ? j : min((j - 1) / kSgTile * kSgTile + kSgTile, min(min(r0 + kSgRows - 1, n1_eff) + w, n2));
               X.tr = k == 0 ? i : min(r0 + kSgRows - 1, rows);
               if (X.jb < X.ja) X.s = -1;
+              const int r1 = r0 + kSgRows - 1;
+              X.inside = r1 <= n1_eff && X.ja >= max(r1 - w, 1) && X.jb < min(r0 + w, n2);
               const int up = i - r0 + 1, lf = j - c0 + 1;  // moves until the diagonal leaves at the top, at the left
               const int d = !go_up ? lf : !go_left ? up : min(up, lf);
               if (go_up) i -= d;
@@ -1161,23 +1182,28 @@ __global__ void __launch_bounds__(32 * NT) sg_retrace_kernel(SgTask *__restrict_
     if (!more) break;
     const SgTile X = tile[wb];
     if (X.s >= 0) {
-      const int r0 = kSgRows * X.s + 1, r1 = r0 + kSgRows - 1;
-      if (r1 <= n1_eff && X.ja >= max(r1 - w, 1) && X.jb < min(r0 + w, n2))
+      if (X.inside)
         sg_tile_codes<KIND, true>(T, ar, P, W, tb, X, codes_of(wb), feed, lane);
       else
         sg_tile_codes<KIND, false>(T, ar, P, W, tb, X, codes_of(wb), feed, lane);
     }
   }
-  if (threadIdx.x == 0) {
+  if (wb == 0) {
     if (ii > 0) push(2, ii);
     if (jj > 0) push(1, jj);
-    for (int a = 0, b = nc - 1; a < b; ++a, --b) {  // the reference reverses the walk (:915)
-      const uint32_t tmp = out[a];
-      out[a] = out[b];
-      out[b] = tmp;
+    push(0xFFFFFFFFu, 0);  // the last operation out
+    if (lane == 0) {
+      nops = nc;
+      T.ncig = nc;
+      if (full) T.status = 3;
     }
-    T.ncig = nc;
-    if (full) T.status = 3;
+  }
+  __syncthreads();
+  nc = nops;
+  for (int a = threadIdx.x; a < nc / 2; a += 32 * NT) {  // the reference reverses the walk (:915)
+    const uint32_t tmp = out[a];
+    out[a] = out[nc - 1 - a];
+    out[nc - 1 - a] = tmp;
   }
 }
 
