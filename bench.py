@@ -9,7 +9,7 @@ Reported (one JSON line, rank 0):
   value   algorithmic GCUPS of the whole pipeline with the sequences resident in HBM (dcns_align_batch)
   e2e     the same through the public call with host buffers (dcns_align_pairs): H2D of the codes, the pipeline,
           and the D2H of the fragments inside the timed region
-  roofline  the seed-scan kernel (dominant) against the live-measured integer-issue ceiling of its instruction mix
+  roofline  the seed-scan stage (dominant) against the live-measured integer-issue ceiling of the exact scan
   cpu_baseline  the oracle restatement of the reference over all host cores on a fixed sample of the workload (every
           k-th pair, 64 per thread)
   per_pair_launch, serving  the one-pair-per-call form and the continuous-batching loop (p50/p99) for comparison
@@ -130,9 +130,10 @@ def workload(n_pairs, rank=0):
     return W.batched_pairs(n_pairs=n_pairs, seed=shard_seed(rank))
 
 
-# DRAM bytes per algorithmic cell of the level-0 scan launch: ncu, 3,000 pairs of this workload, 18.51 MB read and 0
-# written for 161.25 G cells (profiles/scan_kernel_batched_3000pairs.md); traffic grows with the cells.
-SCAN_DRAM_BYTES_PER_CELL = 18.51392e6 / 161254407231
+# DRAM bytes per algorithmic cell of the level-0 launches (filter, then the rows it leaves): ncu, 3,000 pairs of this
+# workload, 7.93 + 9.87 MB read and 0 written for 161.25 G cells (profiles/filter_and_scan_3000pairs.md); traffic grows
+# with the cells.
+SCAN_DRAM_BYTES_PER_CELL = 17.79686e6 / 161254407231
 
 
 def level0_cells(pairs, window=38, step=8):
@@ -271,7 +272,7 @@ def line_long_pairs(eng, timed, threads, gpu, scan_peak, n=8, steps=2, cpu_query
             "value": round(cells / (tot_ms * 1e-3) / 1e9, 3), "unit": "GCUPS", "steps": steps,
             "ms_per_step": round(tot_ms / steps, 2), "pairs_per_s": round(n * steps / (tot_ms * 1e-3), 2),
             "fragments": nfrag,
-            "scan_roofline": {"kernel": "scan_kernel<38> (row-chunked)", "achieved": round(achieved, 1),
+            "scan_roofline": {"kernel": "filter_kernel, then scan_kernel<38> on the rows it leaves", "achieved": round(achieved, 1),
                               "peak": round(scan_peak, 1), "unit": "GCUPS", "frac": round(achieved / scan_peak, 4),
                               "share_of_step": round(scan_ms / tot_ms, 4)},
             "cpu_baseline": {"value": cpu_cells / dt / 1e9, "unit": "GCUPS", "cores": threads, "kind": "port",
@@ -331,8 +332,8 @@ def line_seeded_chromosome(eng, timed, threads, gpu, steps=3, n_seeds=16, cpu_se
             "sg_kernel": {"ms_per_step": round(sg_ms / steps, 2), "gcups": round(cells / (sg_ms * 1e-3) / 1e9, 2),
                           "traceback_ms_per_step": round(tb_ms / steps, 2)},
             "device_bytes": int(dev),
-            "device_memory_note": "device buffers the call holds (sequences, DP codes of one DP per seed at 1 byte "
-                                  "per band cell, boundary rows); the reference's dense traceback matrix for this "
+            "device_memory_note": "device buffers the call holds (sequences, DP checkpoints of one DP per seed at "
+                                  "28 bytes per 128 band cells, boundary rows); the reference's dense traceback matrix for this "
                                   f"pair would be {(len(a) + 1) * (len(b) + 1) / 1e9:.0f} GB",
             "cpu_baseline": {"value": cpu_cells / dt / 1e9, "unit": "GCUPS", "cores": len(sample), "kind": "port",
                              "seconds": dt,
@@ -520,11 +521,13 @@ def main():
     # ---- roofline of the dominant kernel (seed scan)
     peak = eng.measure_scan_roofline()
     achieved = scan_cells / (scan_ms * 1e-3) / 1e9 if scan_ms > 0 else None
-    roofline = {"bound": "int-issue", "kernel": "scan_kernel<38>", "achieved": round(achieved, 2) if achieved else None,
+    roofline = {"bound": "int-issue", "kernel": "filter_kernel, then scan_kernel<38> on the rows it leaves",
+                "achieved": round(achieved, 2) if achieved else None,
                 "peak": round(peak, 2), "unit": "GCUPS", "frac": round(achieved / peak, 4) if achieved else None,
-                "peak_kind": "measured live: the scan's per-cell int16x2 instruction mix at full occupancy",
+                "peak_kind": "measured live: the exact scan's per-cell int16x2 instruction mix at full occupancy; achieved "
+                             "counts the cells that the reference evaluates, most of which the filter proves away",
                 "traffic": round(SCAN_DRAM_BYTES_PER_CELL * level0_cells(pairs) / 1e9, 4) if args.mode == 1 else None,
-                "traffic_unit": "GB per level-0 launch (ncu bytes per cell x this batch's level-0 cells)",
+                "traffic_unit": "GB per level-0 scan (ncu bytes per cell x this batch's level-0 cells)",
                 "scan_share_of_single_lane_step": round(scan_ms / single_ms, 4),
                 "single_lane_ms_per_step": round(single_ms / 2, 2),
                 "timing": "CUDA events around each scan launch, two single-lane steps after the timed region"}
