@@ -206,8 +206,9 @@ void launch_scan_l0(L0Desc d, int64_t ntiles, Arena ar, Params p, unsigned long 
                     int64_t grid, cudaStream_t st);
 // The filter, its tile lists, and the exact scan over a tile list (level 0; a round's tasks).
 void launch_filter(const FiltDesc &D, Arena ar, Params p, int thr, cudaStream_t st);
-void launch_filter_plan_l0(const FiltDesc &D, L0Desc L, int64_t nduo, FiltTiles T, cudaStream_t st);
-void launch_filter_plan_rec(const FiltDesc &D, const ScanTask *tasks, int first, int n, FiltTiles T, cudaStream_t st);
+void launch_filter_plan_l0(const FiltDesc &D, L0Desc L, int64_t nduo, FiltTiles T, int nsm, cudaStream_t st);
+void launch_filter_plan_rec(const FiltDesc &D, const ScanTask *tasks, int first, int n, FiltTiles T, int nsm,
+                            cudaStream_t st);
 void launch_scan_tiles_l0(L0Desc d, FiltTiles T, Arena ar, Params p, unsigned long long *keys, int *work_counter,
                           int grid, cudaStream_t st);
 void launch_scan_tiles_rec(RecDesc d, FiltTiles T, Arena ar, Params p, unsigned long long *keys, int *work_counter,

@@ -613,7 +613,7 @@ bool run_filtered_round(Context &C, ScanState &S, const Params &P, int64_t first
   DCNS_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * 2, C.st));
   const RecDesc D{nullptr, C.d_tasks.as<ScanTask>(), C.seqbase_dev, 0, INT32_MAX, warm, 0};
   DCNS_CK(cudaEventRecord(C.ev0, C.st));
-  launch_filter_plan_rec(C.filt, C.d_tasks.as<ScanTask>(), (int)d0, (int)n, T, C.st);
+  launch_filter_plan_rec(C.filt, C.d_tasks.as<ScanTask>(), (int)d0, (int)n, T, C.nsm, C.st);
   launch_scan_tiles_rec(D, T, C.arena, P, C.d_keys.as<unsigned long long>(), cnt, C.nsm * C.scan_blocks_per_sm, C.st);
   DCNS_CK(cudaEventRecord(C.ev1, C.st));
   launch_reverse(C.d_tasks.as<ScanTask>(), (int)d0, (int)n, C.d_keys.as<unsigned long long>(), C.seqbase_dev,
@@ -996,7 +996,7 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   };
   if (filtered) {
     launch_filter(C.filt, C.arena, P, filter_threshold(P), bulk);
-    launch_filter_plan_l0(C.filt, D, nduo, ft, bulk);
+    launch_filter_plan_l0(C.filt, D, nduo, ft, C.nsm, bulk);
     L0Desc F = D;
     F.warm = C.filt.warm;
     launch_scan_tiles_l0(F, ft, C.arena, P, C.d_keys.as<unsigned long long>(), C.d_counter.as<int>(),

@@ -112,3 +112,23 @@ def test_batch_in_bins(engines):
     rng = np.random.default_rng(9)
     pairs = [planted(rng, int(rng.integers(60, 400)), int(rng.integers(60, 400))) for _ in range(4200)]
     assert same(engines, None, pairs) > 1000
+
+
+def test_plans_by_warps_and_by_threads_agree(lib):
+    """A call of more than 256 window pairs per multiprocessor plans its exact tiles a thread to each, the same pairs
+    one by one a warp to each: the same fragments.  References from one word of marks to many chunks."""
+    rng = np.random.default_rng(31)
+    pairs = []
+    for k in range(140):
+        n1 = int(rng.integers(60, 12000)) if k % 3 else int(rng.integers(490, 540))
+        a, b = W.planted_pair(rng, n1, int(rng.integers(4400, 5200)), int(rng.integers(0, 8)), 40, 200, 0.8, 0.97, 0.01, 0.0)
+        pairs.append((W.prepare(a), W.prepare(b)))
+    assert sum(len(b) // 16 for _, b in pairs) > 256 * 152
+    found = 0
+    for mode in (1, 2):
+        whole = lib.align_pairs(pairs, mode)
+        found += sum(len(w) for w in whole)
+        for k, p in enumerate(pairs):
+            alone = lib.align_pairs([p], mode)[0]
+            assert [f.key() for f in whole[k]] == [f.key() for f in alone], (k, mode)
+    assert found > 200
