@@ -1575,7 +1575,7 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
       scratch_ints = std::max(scratch_ints, scr[L].warps * scr[L].per_warp);
     }
     C.d_x.ensure(C, sizeof(XTask) * n);
-    C.d_idx.ensure(C, sizeof(int32_t) * (3 * n + 4 + nlev + 2 * kXdropOrderBins));
+    C.d_idx.ensure(C, sizeof(int32_t) * (3 * n + 2 + 2 * nlev + 2 * kXdropOrderBins));
     C.d_counter.ensure(C, 64);
     if (want_codes) {
       C.d_tb.ensure(C, sizeof(uint32_t) * tb_words);
@@ -1583,21 +1583,22 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
     }
     if (scratch_ints > 1) C.d_scratch.ensure(C, sizeof(int32_t) * scratch_ints);
     int *lists = C.d_idx.as<int>();
-    int *cnt = lists + 3 * n;  // [0], [1]: the two work-list counts, [2]: retry count, [4 + L]: level L's fetch
+    // counts, zeroed at once: of the retry list, of each level's work list (and what the last one leaves), the levels'
+    // fetches, the order's classes
+    int *retry_cnt = lists + 3 * n, *cnt = retry_cnt + 1, *fetch = cnt + nlev + 1, *bins = fetch + nlev;
     unsigned long long *cur = C.d_counter.as<unsigned long long>();  // [0]: traceback arena, [1]: CIGAR arena
     C.h_x.ensure(sizeof(XTask) * n);
     copy_blocks(C.h_x.p, X.data(), sizeof(XTask) * n);
     h2d(C, C.d_x, C.h_x.as<XTask>(), (size_t)n);
-    DCNS_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * (4 + nlev + 2 * kXdropOrderBins), C.st));
+    DCNS_CK(cudaMemsetAsync(retry_cnt, 0, sizeof(int) * (2 + 2 * nlev + 2 * kXdropOrderBins), C.st));
     DCNS_CK(cudaMemsetAsync(cur, 0, sizeof(unsigned long long) * 2, C.st));
-    launch_xdrop_list(C.d_x.as<XTask>(), lists, (int)n, cnt, (int)std::min<int64_t>(maxdim, INT32_MAX), cnt + 4 + nlev,
+    launch_xdrop_list(C.d_x.as<XTask>(), lists, (int)n, cnt, (int)std::min<int64_t>(maxdim, INT32_MAX), bins,
                       C.nsm, C.st);
     DCNS_CK(cudaEventRecord(C.ev0, C.st));
     int in = 0;
     for (int L = 0; L < nlev; ++L) {
       const int out = 1 - in;
-      DCNS_CK(cudaMemsetAsync(cnt + out, 0, sizeof(int), C.st));
-      const XLevel lv{lists + in * n, cnt + in, lists + out * n, cnt + out, lists + 2 * n, cnt + 2, cnt + 4 + L, cur,
+      const XLevel lv{lists + in * n, cnt + L, lists + out * n, cnt + L + 1, lists + 2 * n, retry_cnt, fetch + L, cur,
                       want_codes ? tb_words : 0};
       launch_xdrop_level(C.d_x.as<XTask>(), lv, C.arena, P, C.d_tb.as<uint32_t>(), w0 << L, (int)n, C.nsm,
                          C.d_scratch.as<int32_t>(), scr[L].per_warp, scr[L].warps, want_codes, packed, C.st);
@@ -1613,14 +1614,14 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
     }
     C.stats.kernel_launches += nlev + 1 + (want_codes ? 3 : 0);
     C.stats.xdrop_rounds += 1;
-    C.h_misc.ensure(sizeof(int32_t) * (n + 8) + 64);
-    int32_t *hret = C.h_misc.as<int32_t>();  // [0]: leftover count, [1]: retry count, [8..]: retry list
-    unsigned long long hcur[2] = {0, 0};
+    // pinned: the two arena cursors, the retry count and the levels' counts (at most 1 + 33), the retry list
+    C.h_misc.ensure(sizeof(int32_t) * (40 + n));
+    const unsigned long long *hcur = C.h_misc.as<unsigned long long>();
+    int32_t *hcnt = C.h_misc.as<int32_t>() + 4, *hlist = hcnt + 36;
     d2h(C, C.h_x.as<XTask>(), C.d_x, (size_t)n);
-    DCNS_CK(cudaMemcpyAsync(hret, cnt + in, sizeof(int), cudaMemcpyDeviceToHost, C.st));
-    DCNS_CK(cudaMemcpyAsync(hret + 1, cnt + 2, sizeof(int), cudaMemcpyDeviceToHost, C.st));
-    DCNS_CK(cudaMemcpyAsync(hret + 8, lists + 2 * n, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, C.st));
-    DCNS_CK(cudaMemcpyAsync(hcur, cur, sizeof(hcur), cudaMemcpyDeviceToHost, C.st));
+    DCNS_CK(cudaMemcpyAsync(C.h_misc.p, cur, sizeof(unsigned long long) * 2, cudaMemcpyDeviceToHost, C.st));
+    DCNS_CK(cudaMemcpyAsync(hcnt, retry_cnt, sizeof(int) * (2 + nlev), cudaMemcpyDeviceToHost, C.st));
+    DCNS_CK(cudaMemcpyAsync(hlist, lists + 2 * n, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, C.st));
     tp = phase(C, "xc_enqueue", tp);
     sync(C);
     copy_blocks(X.data(), C.h_x.p, sizeof(XTask) * n);
@@ -1634,8 +1635,8 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
         C.stats.ms_xdrop_tb_kernel += ms;
       }
     }
-    if (hret[0] != 0) throw Error(DCNS_ERR_DEVICE, "x-drop band restarts did not converge");
-    std::vector<int32_t> retry(hret + 8, hret + 8 + hret[1]);
+    if (hcnt[1 + nlev] != 0) throw Error(DCNS_ERR_DEVICE, "x-drop band restarts did not converge");
+    std::vector<int32_t> retry(hlist, hlist + hcnt[0]);
     std::sort(retry.begin(), retry.end());
     if (want_codes) {
       const int64_t cw = (int64_t)hcur[1];  // words of the packed CIGARs
