@@ -176,7 +176,16 @@ void worker_loop(std::shared_ptr<Server> Sp, Context *C) {
     std::vector<Server::Req> batch;
     {
       std::unique_lock<std::mutex> lk(S->mu);
+      const bool idle = S->running && S->queue.empty();
       S->cv_work.wait(lk, [&] { return !S->running || !S->queue.empty(); });
+      if (idle && S->running) {
+        // A worker that was idle gives the requests that come with the one that woke it a moment to arrive: a batch of
+        // a few small requests takes little longer than one (0.6 ms), and they would wait for it.
+        lk.unlock();
+        std::this_thread::sleep_for(std::chrono::microseconds(100));
+        lk.lock();
+        if (S->running && S->queue.empty()) continue;  // another worker took them
+      }
       if (!S->running && S->queue.empty()) return;
       // admission: arrival order, up to the in-flight limit, the worker's memory budget and the batch's scan cap
       int64_t bytes = 0, cells = 0;
