@@ -498,18 +498,21 @@ struct ScanState {
 // The fast kernel's table stores s - open in int8 and pads short windows with -16384 in int16 lanes.
 bool fast_scan_ok(const Params &P) { return P.window <= kScanW && P.match - P.open1 <= 127; }
 
+// The most a column of the read can add to a path's score (a mismatch may score above a match).
+int column_gain(const Params &P) { return std::max(P.match, P.mismatch); }
+
 int warmup_rows(const Params &P, int tw) {
   // A positive-scoring local path over tw read columns spans at most tw diagonal rows plus fewer than
-  // match*tw/g vertical-gap rows (g = cheapest gap row), so a scan restarted K rows early is exact from row K on.
+  // gain*tw/g vertical-gap rows (g = cheapest gap row), so a scan restarted K rows early is exact from row K on.
   const int g = std::min(-P.open1, -P.ext1);
   if (g <= 0) return INT_MAX;
-  return tw + (P.match * tw + g - 1) / g + 4;
+  return tw + (column_gain(P) * tw + g - 1) / g + 4;
 }
 
 // Warm-up rows of an exact scan whose maxima count from min_score on: a path that reaches it within the window has at
-// most match * tw - min_score to spend on vertical gaps, the first of whose rows costs the opening.
+// most gain * tw - min_score to spend on vertical gaps, the first of whose rows costs the opening.
 int warmup_rows_above(const Params &P, int tw) {
-  const int K = warmup_rows(P, tw), spare = P.match * tw - P.min_score;
+  const int K = warmup_rows(P, tw), spare = column_gain(P) * tw - P.min_score;
   if (K == INT_MAX) return K;
   const int g = std::min(-P.open1, -P.ext1);
   return std::min(K, tw + std::max(0, spare) / g + 4);
