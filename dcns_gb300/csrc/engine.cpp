@@ -495,11 +495,11 @@ struct ScanState {
   int64_t size() const { return (int64_t)tasks.size(); }
 };
 
-// The fast kernel's table stores s - open in int8 and pads short windows with -16384 in int16 lanes.
-bool fast_scan_ok(const Params &P) { return P.window <= kScanW && P.match - P.open1 <= 127; }
-
 // The most a column of the read can add to a path's score (a mismatch may score above a match).
 int column_gain(const Params &P) { return std::max(P.match, P.mismatch); }
+
+// The fast kernel's table stores s - open in int8 and pads short windows with -16384 in int16 lanes.
+bool fast_scan_ok(const Params &P) { return P.window <= kScanW && column_gain(P) - P.open1 <= 127; }
 
 int warmup_rows(const Params &P, int tw) {
   // A positive-scoring local path over tw read columns spans at most tw diagonal rows plus fewer than

@@ -37,6 +37,15 @@ def test_long_gaps_inside_a_window(lib, oracle, mismatch, gap):
     check(lib, oracle, tasks, match=1, mismatch=mismatch, open1=-gap, ext1=-gap)
 
 
+@pytest.mark.parametrize("mismatch,open1", [(100, -27), (100, -28), (100, -100), (127, -1), (64, -64)])
+def test_scores_beyond_the_table(lib, oracle, mismatch, open1):
+    """The fast scan holds a score less the opening in eight bits: up to 127 of it, and beyond."""
+    read = runs((A, 38))
+    tasks = [(runs((C, 300)), read), (runs((A, 40), (C, 3), (A, 40)), read),
+             (runs((C, 19), (A, 50), (C, 19)), read[:21])]
+    check(lib, oracle, tasks, match=1, mismatch=mismatch, open1=open1, ext1=-1)
+
+
 @pytest.mark.parametrize("mode", [1, 2])
 @pytest.mark.parametrize("kw", [dict(open1=-9, min_score=60), dict(open1=-3, min_score=80)], ids=["9", "3"])
 def test_whole_alignments(lib, oracle, mode, kw):
