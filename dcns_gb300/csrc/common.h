@@ -87,8 +87,22 @@ struct FiltTile {
 };
 struct FiltTiles {
   FiltTile *list;
-  int *count;  // tiles wanted (more than cap: the list is incomplete)
-  int32_t cap, rows;  // rows: the most a tile counts
+  unsigned long long *count;  // tiles wanted (two long repeats want more than 2^31: a place past cap is not written)
+  int32_t cap, rows;          // rows: the most a tile counts
+};
+// The place in the list of the k-th of the tiles taken from `at` on (-1: past the list's end).
+__host__ __device__ inline int32_t filt_place(unsigned long long at, int32_t k, int32_t cap) {
+  const unsigned long long p = at + (unsigned long long)k;
+  return p < (unsigned long long)cap ? (int32_t)p : -1;
+}
+// Whether every wanted tile is in the list.
+__host__ __device__ inline bool filt_listed(unsigned long long wanted, int32_t cap) {
+  return wanted <= (unsigned long long)cap;
+}
+// The scan's counters: its work queue, level 0's selected windows, the filter's wanted tiles.
+struct ScanCounts {
+  int32_t queue, selected;
+  unsigned long long tiles;
 };
 
 // A level-0 window whose maximum reached min_score, compacted in task order.

@@ -599,9 +599,9 @@ bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vecto
 
 // The tile list for `items` duos or tasks; short tiles where there are few, so that they spread over the GPU: a row
 // takes a lone warp some 0.5 us, and a tile its warm-up rows besides.
-FiltTiles filter_tiles(Context &C, int64_t items, int *count) {
+FiltTiles filter_tiles(Context &C, int64_t items) {
   const int64_t cap = std::min<int64_t>(INT32_MAX, (int64_t)(C.d_ftiles.cap / sizeof(FiltTile)));
-  return FiltTiles{C.d_ftiles.as<FiltTile>(), count, (int32_t)cap,
+  return FiltTiles{C.d_ftiles.as<FiltTile>(), &C.d_counter.as<ScanCounts>()->tiles, (int32_t)cap,
                    items >= (int64_t)C.nsm * C.scan_blocks_per_sm * kScanThreads ? 256 : items >= 8192 ? 64 : 24};
 }
 
@@ -610,22 +610,22 @@ FiltTiles filter_tiles(Context &C, int64_t items, int *count) {
 bool run_filtered_round(Context &C, ScanState &S, const Params &P, int64_t first, int64_t n, int warm) {
   auto tx = Clock::now();
   const int64_t d0 = first - S.ns;
-  int *cnt = C.d_counter.as<int>();  // [0]: the scan's queue, [1]: tiles
-  const FiltTiles T = filter_tiles(C, n, cnt + 1);
+  const FiltTiles T = filter_tiles(C, n);
   DCNS_CK(cudaMemsetAsync(C.d_keys.as<unsigned long long>() + d0, 0, sizeof(unsigned long long) * n, C.st));
-  DCNS_CK(cudaMemsetAsync(cnt, 0, sizeof(int) * 2, C.st));
+  DCNS_CK(cudaMemsetAsync(C.d_counter.p, 0, sizeof(ScanCounts), C.st));
   const RecDesc D{nullptr, C.d_tasks.as<ScanTask>(), C.seqbase_dev, 0, INT32_MAX, warm, 0};
   DCNS_CK(cudaEventRecord(C.ev0, C.st));
   launch_filter_plan_rec(C.filt, C.d_tasks.as<ScanTask>(), (int)d0, (int)n, T, C.nsm, C.st);
-  launch_scan_tiles_rec(D, T, C.arena, P, C.d_keys.as<unsigned long long>(), cnt, C.nsm * C.scan_blocks_per_sm, C.st);
+  launch_scan_tiles_rec(D, T, C.arena, P, C.d_keys.as<unsigned long long>(), &C.d_counter.as<ScanCounts>()->queue,
+                        C.nsm * C.scan_blocks_per_sm, C.st);
   DCNS_CK(cudaEventRecord(C.ev1, C.st));
   launch_reverse(C.d_tasks.as<ScanTask>(), (int)d0, (int)n, C.d_keys.as<unsigned long long>(), C.seqbase_dev,
                  nullptr, C.arena, P, true, C.st);
   C.stats.scan_launches += 1;
   C.stats.kernel_launches += 3;
-  int tiles = 0;
+  unsigned long long tiles = 0;
   d2h(C, C.h_tiles.as<ScanTask>(), C.d_tasks, (size_t)n, (size_t)d0);
-  DCNS_CK(cudaMemcpyAsync(&tiles, cnt + 1, sizeof(int), cudaMemcpyDeviceToHost, C.st));
+  DCNS_CK(cudaMemcpyAsync(&tiles, T.count, sizeof(tiles), cudaMemcpyDeviceToHost, C.st));
   sync(C);
   copy_blocks(S.tasks.data() + first, C.h_tiles.p, sizeof(ScanTask) * n);
   C.stats.scan_rounds += 1;
@@ -633,7 +633,7 @@ bool run_filtered_round(Context &C, ScanState &S, const Params &P, int64_t first
   float ms = 0;
   DCNS_CK(cudaEventElapsedTime(&ms, C.ev0, C.ev1));
   C.stats.ms_scan_kernel += ms;
-  return tiles <= T.cap;
+  return filt_listed(tiles, T.cap);
 }
 
 // Launches the scan over `tiles` plus the generic kernel over `generic` (device slots), then the reverse scans for
@@ -972,14 +972,14 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   int64_t *d_wst = C.d_scratch.as<int64_t>();
   int2 *d_plen = reinterpret_cast<int2 *>(d_wst + np + 1);
   int *d_blk = reinterpret_cast<int *>(d_plen + np);
-  int *d_count = C.d_counter.as<int>() + 1;
+  ScanCounts *const d_counts = C.d_counter.as<ScanCounts>();
   const bool filtered = C.scan_filter && filter_ok(P) && filter_setup(C, pairs, order, nfast, P);
-  const FiltTiles ft = filtered ? filter_tiles(C, nduo, C.d_counter.as<int>() + 2) : FiltTiles{};
+  const FiltTiles ft = filtered ? filter_tiles(C, nduo) : FiltTiles{};
   h2d(C, C.d_tiles, tab, (size_t)np);
   DCNS_CK(cudaMemcpyAsync(d_wst, wst, sizeof(int64_t) * (np + 1), cudaMemcpyHostToDevice, C.st));
   DCNS_CK(cudaMemcpyAsync(d_plen, plen, sizeof(int2) * np, cudaMemcpyHostToDevice, C.st));
   DCNS_CK(cudaMemsetAsync(C.d_keys.p, 0, sizeof(unsigned long long) * n0, C.st));
-  DCNS_CK(cudaMemsetAsync(C.d_counter.p, 0, sizeof(int) * 3, C.st));
+  DCNS_CK(cudaMemsetAsync(d_counts, 0, sizeof(ScanCounts), C.st));
   L0Desc D{C.d_tiles.as<L0Pair>(), (int32_t)np, P.step, P.window, (int32_t)chunk, K, 0};
   // One thread per tile (not a persistent grid): blocks retire as they finish, so the short kernels of other lanes,
   // on higher-priority streams, are scheduled in between instead of waiting for the whole level-0 scan.
@@ -995,14 +995,14 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   DCNS_CK(cudaStreamWaitEvent(bulk, C.ev_bulk, 0));
   DCNS_CK(cudaEventRecord(C.ev0, bulk));
   auto scan_all = [&](cudaStream_t on) {
-    launch_scan_l0(D, ntiles, C.arena, P, C.d_keys.as<unsigned long long>(), C.d_counter.as<int>(), grid, on);
+    launch_scan_l0(D, ntiles, C.arena, P, C.d_keys.as<unsigned long long>(), &d_counts->queue, grid, on);
   };
   if (filtered) {
     launch_filter(C.filt, C.arena, P, filter_threshold(P), bulk);
     launch_filter_plan_l0(C.filt, D, nduo, ft, C.nsm, bulk);
     L0Desc F = D;
     F.warm = C.filt.warm;
-    launch_scan_tiles_l0(F, ft, C.arena, P, C.d_keys.as<unsigned long long>(), C.d_counter.as<int>(),
+    launch_scan_tiles_l0(F, ft, C.arena, P, C.d_keys.as<unsigned long long>(), &d_counts->queue,
                          C.nsm * C.scan_blocks_per_sm, bulk);
     C.stats.kernel_launches += 2;
   } else {
@@ -1020,25 +1020,25 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   C.stats.kernel_launches += 1;
   auto select = [&] {
     launch_l0_select(C.d_keys.as<unsigned long long>(), n0, d_wst, d_plen, (int)np, C.seqbase_dev, C.arena, P, d_blk,
-                     d_count, C.d_tasks.as<L0Rec>(), C.nsm, C.st);
+                     &d_counts->selected, C.d_tasks.as<L0Rec>(), C.nsm, C.st);
     C.stats.kernel_launches += 4;
   };
   select();
-  int got[2] = {0, 0};  // windows selected, tiles the filter wanted
-  DCNS_CK(cudaMemcpyAsync(got, d_count, sizeof(got), cudaMemcpyDeviceToHost, C.st));
+  ScanCounts got{};
+  DCNS_CK(cudaMemcpyAsync(&got, d_counts, sizeof(got), cudaMemcpyDeviceToHost, C.st));
   tp = phase(C, "l0_launch", tp);
   sync(C);
-  if (filtered && got[1] > ft.cap) {  // marked nearly everywhere: every window against its whole reference after all
+  if (filtered && !filt_listed(got.tiles, ft.cap)) {  // marked nearly everywhere: every window against its whole reference after all
     C.filt_on = false;
-    DCNS_CK(cudaMemsetAsync(C.d_counter.p, 0, sizeof(int) * 3, C.st));
+    DCNS_CK(cudaMemsetAsync(d_counts, 0, sizeof(ScanCounts), C.st));
     scan_all(C.st);
     select();
     C.stats.scan_launches += 1;
     C.stats.kernel_launches += 1;
-    DCNS_CK(cudaMemcpyAsync(got, d_count, sizeof(got), cudaMemcpyDeviceToHost, C.st));
+    DCNS_CK(cudaMemcpyAsync(&got, d_counts, sizeof(got), cudaMemcpyDeviceToHost, C.st));
     sync(C);
   }
-  const int nsel = got[0];
+  const int nsel = got.selected;
   tp = phase(C, "l0_sync", tp);
   C.h_tasks.ensure(sizeof(L0Rec) * std::max(nsel, 1));
   L0Rec *rec = C.h_tasks.as<L0Rec>();

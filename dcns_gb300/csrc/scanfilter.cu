@@ -281,9 +281,12 @@ __device__ __forceinline__ void filt_runs_warp(const FiltDesc &D, const FiltPair
 
 __device__ __forceinline__ void filt_emit(const FiltTiles &T, int a, int b, int rb, int re) {
   const int n = (re - rb + T.rows - 1) / T.rows, per = (re - rb + n - 1) / n;
-  const int at = atomicAdd(T.count, n);
-  for (int k = 0; k < n; ++k)
-    if (at + k < T.cap) T.list[at + k] = FiltTile{a, b, rb + k * per, min(re, rb + (k + 1) * per)};
+  const unsigned long long at = atomicAdd(T.count, (unsigned long long)n);
+  for (int k = 0; k < n; ++k) {
+    const int p = filt_place(at, k, T.cap);
+    if (p < 0) break;
+    T.list[p] = FiltTile{a, b, rb + k * per, min(re, rb + (k + 1) * per)};
+  }
 }
 
 // Plans: one thread, or WARP one warp, per item.  A thread waits for each word before it looks at the next, so a plan
