@@ -1226,7 +1226,9 @@ void scan_and_link(Context &C, const std::vector<PairIn> &pairs, const Params &P
         m,
         [&](int64_t q) {
           const int64_t p = todo[q];
-          SeedArena::mine().reset();
+          struct Arena {  // the sets of this pair go before the next begins
+            ~Arena() { SeedArena::mine().reset(); }
+          } arena;
           ReplayCtx R{S, P, mini, {}, 0, 0, 0};
           SeedSet g;
           if (replay_pair(R, p, g)) {

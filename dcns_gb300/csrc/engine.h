@@ -7,6 +7,7 @@
 #include <functional>
 #include <cstdint>
 #include <condition_variable>
+#include <cstring>
 #include <mutex>
 #include <memory>
 #include <set>
@@ -87,8 +88,9 @@ struct SeedLess {
 };
 
 // Nodes of the seed sets of the pair at hand, from blocks of the thread that replays it: a replay builds and drops a
-// set per recursion level, and the heap (and its locks, as sets moved between threads) took most of its time.  A
-// thread keeps 256 KB.
+// set per recursion level, and the heap (and its locks, as sets moved between threads) took most of its time.  Dropped
+// nodes are used again, so the blocks hold the nodes alive at a time (at most twice over): a chain of D seeds copies
+// D sets of up to D seeds, one after the other.  Between pairs a thread keeps 256 KB.
 class SeedArena {
  public:
   static SeedArena &mine() {
@@ -96,31 +98,43 @@ class SeedArena {
     return a;
   }
   void *take(size_t bytes) {
-    bytes = (bytes + 15) & ~size_t(15);
+    if (free_ && bytes <= kNode) {
+      void *p = free_;
+      std::memcpy(&free_, p, sizeof(free_));
+      return p;
+    }
+    bytes = std::max((bytes + 15) & ~size_t(15), kNode);
     if (at_ + bytes > size_) grow(bytes);
     void *p = blocks_.back().get() + at_;
     at_ += bytes;
     return p;
   }
+  void give(void *p, size_t bytes) {
+    if (bytes > kNode) return;  // not a node: dropped with the blocks
+    std::memcpy(p, &free_, sizeof(free_));
+    free_ = p;
+  }
   // Drops everything taken (no set of an earlier pair may be alive).
   void reset() {
     if (blocks_.size() > 1) {
-      blocks_.clear();
-      size_ = 0;
+      blocks_.resize(1);
+      size_ = kKept;
     }
     at_ = 0;
+    free_ = nullptr;
   }
 
  private:
-  static constexpr size_t kKept = 256 << 10;
+  static constexpr size_t kKept = 256 << 10, kNode = 48;  // kNode: a set's node, a seed and its links
   void grow(size_t bytes) {
-    const size_t want = std::max(bytes, blocks_.empty() ? kKept : std::max(kKept, 2 * size_));
+    const size_t want = std::max({kKept, bytes, 2 * size_});
     blocks_.emplace_back(new char[want]);
     size_ = want;
     at_ = 0;
   }
   std::vector<std::unique_ptr<char[]>> blocks_;
   size_t at_ = 0, size_ = 0;
+  void *free_ = nullptr;
 };
 template <class T>
 struct SeedAlloc {
@@ -129,7 +143,7 @@ struct SeedAlloc {
   template <class U>
   SeedAlloc(const SeedAlloc<U> &) {}
   T *allocate(size_t n) { return static_cast<T *>(SeedArena::mine().take(n * sizeof(T))); }
-  void deallocate(T *, size_t) {}
+  void deallocate(T *p, size_t n) { SeedArena::mine().give(p, n * sizeof(T)); }
   template <class U>
   bool operator==(const SeedAlloc<U> &) const {
     return true;
