@@ -28,6 +28,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <deque>
 #include <condition_variable>
@@ -260,6 +261,8 @@ class HostPool {
     const std::function<void(int64_t)> *f;
     int64_t n;
     std::atomic<int64_t> next{0}, done{0};
+    std::atomic<bool> failed{false};
+    std::exception_ptr error;  // the first that an item threw
     std::mutex m;
     std::condition_variable cv;
   };
@@ -268,6 +271,7 @@ class HostPool {
     return *pool;
   }
   int size() const { return (int)th_.size() + 1; }
+  // An item that throws (an allocation that fails) ends the job: run() throws it in the calling thread.
   void run(int64_t n, const std::function<void(int64_t)> &f) {
     auto J = std::make_shared<Job>();
     J->f = &f;
@@ -282,12 +286,15 @@ class HostPool {
       std::unique_lock<std::mutex> lk(J->m);
       J->cv.wait(lk, [&] { return J->done.load() >= n; });
     }
-    std::lock_guard<std::mutex> lk(mu_);
-    for (auto it = q_.begin(); it != q_.end(); ++it)
-      if (it->get() == J.get()) {
-        q_.erase(it);
-        break;
-      }
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      for (auto it = q_.begin(); it != q_.end(); ++it)
+        if (it->get() == J.get()) {
+          q_.erase(it);
+          break;
+        }
+    }
+    if (J->failed) std::rethrow_exception(J->error);
   }
   static thread_local bool in_worker;
 
@@ -299,7 +306,13 @@ class HostPool {
   }
   static void work(Job &J) {
     for (int64_t i; (i = J.next.fetch_add(1)) < J.n;) {
-      (*J.f)(i);
+      try {
+        if (!J.failed) (*J.f)(i);
+      } catch (...) {
+        std::lock_guard<std::mutex> lk(J.m);
+        if (!J.error) J.error = std::current_exception();
+        J.failed = true;
+      }
       if (J.done.fetch_add(1) + 1 == J.n) {
         std::lock_guard<std::mutex> lk(J.m);
         J.cv.notify_all();
