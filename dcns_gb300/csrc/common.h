@@ -79,7 +79,9 @@ struct FiltDesc {
   const FiltPair *pairs;
   const int32_t *slot;  // pair -> place in `pairs`
   uint32_t *words;
+  unsigned long long *seen;  // per pair: words looked at (upper half) and how many of them were mostly marks
   int32_t npairs, ntasks, chunk, warm;  // chunk: rows per row chunk; warm: the exact scan's warm-up rows
+  int32_t max_words, pad;  // the most words of marks that a strip of a pair has
 };
 // Rows [rb, re) of level-0 duo b of pair slot a, or of task a: what the exact scan runs after the filter.
 struct FiltTile {
@@ -87,8 +89,10 @@ struct FiltTile {
 };
 struct FiltTiles {
   FiltTile *list;
-  unsigned long long *count;  // tiles wanted (two long repeats want more than 2^31: a place past cap is not written)
+  unsigned long long *count;  // [0]: tiles wanted (two long repeats want more than 2^31: a place past cap is not
+                              // written), [1]: the rows that those tiles compute, warm-up included
   int32_t cap, rows;          // rows: the most a tile counts
+  unsigned long long most;    // rows from which on the whole scan is the shorter one
 };
 // The place in the list of the k-th of the tiles taken from `at` on (-1: past the list's end).
 __host__ __device__ inline int32_t filt_place(unsigned long long at, int32_t k, int32_t cap) {
@@ -102,7 +106,7 @@ __host__ __device__ inline bool filt_listed(unsigned long long wanted, int32_t c
 // The scan's counters: its work queue, level 0's selected windows, the filter's wanted tiles.
 struct ScanCounts {
   int32_t queue, selected;
-  unsigned long long tiles;
+  unsigned long long tiles, rows;
 };
 
 // A level-0 window whose maximum reached min_score, compacted in task order.

@@ -570,7 +570,7 @@ bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vecto
   if (tasks < want) chunk = std::min(limit, std::max<int64_t>(K, (rows + want - 1) / want));
   std::vector<FiltPair> tab(np);
   std::vector<int32_t> slot(np);
-  int64_t words = 0, duos = 0, task = 0;
+  int64_t words = 0, duos = 0, task = 0, max_words = 1;
   for (int64_t q = 0; q < np; ++q) {
     const int64_t p = order[q];
     FiltPair &e = tab[q];
@@ -588,12 +588,13 @@ bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vecto
     e.pad = 0;
     slot[p] = (int32_t)q;
     words += t * e.nch * e.wpc * 64;
+    max_words = std::max<int64_t>(max_words, (int64_t)e.nch * e.wpc);
     duos += (nfast[p] + 1) / 2;
     task += t * e.nch;
   }
   if (task >= INT32_MAX / 2) return false;
   const int64_t cap = std::min<int64_t>(1 << 26, std::max<int64_t>(1 << 16, 4 * duos));
-  const size_t tb = sizeof(FiltPair) * np + sizeof(int32_t) * np + 256;
+  const size_t tb = (sizeof(FiltPair) + sizeof(unsigned long long) + sizeof(int32_t)) * np + 256;
   const size_t need = tb + sizeof(uint32_t) * words + sizeof(FiltTile) * cap;
   const size_t have = C.d_fpairs.cap + C.d_fwords.cap + C.d_ftiles.cap;
   if (need > have && C.used - have + 2 * need > C.budget) return false;
@@ -601,52 +602,75 @@ bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vecto
   C.d_fwords.ensure(C, sizeof(uint32_t) * words);
   C.d_ftiles.ensure(C, sizeof(FiltTile) * cap);
   if (!C.d_fpairs.cap || !C.d_fwords.cap || !C.d_ftiles.cap) return false;  // one made room for another
-  int32_t *d_slot = reinterpret_cast<int32_t *>(C.d_fpairs.as<FiltPair>() + np);
+  unsigned long long *const d_seen = reinterpret_cast<unsigned long long *>(C.d_fpairs.as<FiltPair>() + np);
+  int32_t *const d_slot = reinterpret_cast<int32_t *>(d_seen + np);
   h2d(C, C.d_fpairs, tab.data(), (size_t)np);
   DCNS_CK(cudaMemcpyAsync(d_slot, slot.data(), sizeof(int32_t) * np, cudaMemcpyHostToDevice, C.st));
-  C.filt = FiltDesc{C.d_fpairs.as<FiltPair>(), d_slot, C.d_fwords.as<uint32_t>(), (int32_t)np, (int32_t)task,
-                    (int32_t)chunk, K};
+  DCNS_CK(cudaMemsetAsync(d_seen, 0, sizeof(unsigned long long) * np, C.st));
+  C.filt = FiltDesc{C.d_fpairs.as<FiltPair>(), d_slot, C.d_fwords.as<uint32_t>(), d_seen, (int32_t)np, (int32_t)task,
+                    (int32_t)chunk, K, (int32_t)max_words, 0};
   C.filt_on = true;
   return true;
 }
 
 // The tile list for `items` duos or tasks; short tiles where there are few, so that they spread over the GPU: a row
-// takes a lone warp some 0.5 us, and a tile its warm-up rows besides.
-FiltTiles filter_tiles(Context &C, int64_t items) {
+// takes a lone warp some 0.5 us, and a tile its warm-up rows besides.  whole_rows: what the scan without the filter
+// computes, warm-up included.  A list that computes more is not scanned, unless it is one wave of short tiles at most
+// (the whole scan's wave has some 600 rows): references marked nearly everywhere want tiles over all of their rows.
+FiltTiles filter_tiles(Context &C, int64_t items, int64_t whole_rows) {
   const int64_t cap = std::min<int64_t>(INT32_MAX, (int64_t)(C.d_ftiles.cap / sizeof(FiltTile)));
-  return FiltTiles{C.d_ftiles.as<FiltTile>(), &C.d_counter.as<ScanCounts>()->tiles, (int32_t)cap,
-                   items >= (int64_t)C.nsm * C.scan_blocks_per_sm * kScanThreads ? 256 : items >= 8192 ? 64 : 24};
+  const int64_t resident = (int64_t)C.nsm * C.scan_blocks_per_sm * kScanThreads;
+  const int32_t rows = items >= resident ? 256 : items >= 8192 ? 64 : 24;
+  return FiltTiles{C.d_ftiles.as<FiltTile>(), &C.d_counter.as<ScanCounts>()->tiles, (int32_t)cap, rows,
+                   (unsigned long long)std::max<int64_t>(whole_rows, resident * (rows + C.filt.warm))};
+}
+bool filter_listed(const FiltTiles &T, const ScanCounts &n) { return filt_listed(n.tiles, T.cap) && n.rows <= T.most; }
+
+// After a list that was too short for tiles worth scanning: room for all of them (and more where a later round of the
+// call wants it).  False: they are not worth it, or the budget has no such room.
+bool filter_grow(Context &C, const FiltTiles &T, const ScanCounts &n) {
+  const unsigned long long rows = n.rows ? n.rows : n.tiles * (T.rows + C.filt.warm);  // (not counted: whole tiles)
+  if (rows > T.most || n.tiles > INT32_MAX / 2) return false;
+  const size_t bytes = sizeof(FiltTile) * (size_t)n.tiles;
+  if (C.used - C.d_ftiles.cap + 2 * bytes > C.budget) return false;
+  C.d_ftiles.ensure(C, bytes);
+  return C.filt_on && C.d_ftiles.cap >= bytes;
 }
 
 // A round's scan through the filter's marks (tasks [first, first + n) are on the device), then the reverse scans and
-// the download.  False: the tile list was too short, and the keys hold only part of the maxima.
-bool run_filtered_round(Context &C, ScanState &S, const Params &P, int64_t first, int64_t n, int warm) {
+// the download.  False: the tile list was too short or would take longer than the whole scan, and nothing was scanned.
+bool run_filtered_round(Context &C, ScanState &S, const Params &P, int64_t first, int64_t n, int64_t whole_rows,
+                        int warm) {
   auto tx = Clock::now();
   const int64_t d0 = first - S.ns;
-  const FiltTiles T = filter_tiles(C, n);
-  DCNS_CK(cudaMemsetAsync(C.d_keys.as<unsigned long long>() + d0, 0, sizeof(unsigned long long) * n, C.st));
-  DCNS_CK(cudaMemsetAsync(C.d_counter.p, 0, sizeof(ScanCounts), C.st));
   const RecDesc D{nullptr, C.d_tasks.as<ScanTask>(), C.seqbase_dev, 0, INT32_MAX, warm, 0};
-  DCNS_CK(cudaEventRecord(C.ev0, C.st));
-  launch_filter_plan_rec(C.filt, C.d_tasks.as<ScanTask>(), (int)d0, (int)n, T, C.nsm, C.st);
-  launch_scan_tiles_rec(D, T, C.arena, P, C.d_keys.as<unsigned long long>(), &C.d_counter.as<ScanCounts>()->queue,
-                        C.nsm * C.scan_blocks_per_sm, C.st);
-  DCNS_CK(cudaEventRecord(C.ev1, C.st));
-  launch_reverse(C.d_tasks.as<ScanTask>(), (int)d0, (int)n, C.d_keys.as<unsigned long long>(), C.seqbase_dev,
-                 nullptr, C.arena, P, true, C.st);
-  C.stats.scan_launches += 1;
-  C.stats.kernel_launches += 3;
-  unsigned long long tiles = 0;
-  d2h(C, C.h_tiles.as<ScanTask>(), C.d_tasks, (size_t)n, (size_t)d0);
-  DCNS_CK(cudaMemcpyAsync(&tiles, T.count, sizeof(tiles), cudaMemcpyDeviceToHost, C.st));
-  sync(C);
+  ScanCounts counts{};
+  FiltTiles T{};
+  for (int attempt = 0;; ++attempt) {
+    T = filter_tiles(C, n, whole_rows);
+    DCNS_CK(cudaMemsetAsync(C.d_keys.as<unsigned long long>() + d0, 0, sizeof(unsigned long long) * n, C.st));
+    DCNS_CK(cudaMemsetAsync(C.d_counter.p, 0, sizeof(ScanCounts), C.st));
+    DCNS_CK(cudaEventRecord(C.ev0, C.st));
+    launch_filter_plan_rec(C.filt, C.d_tasks.as<ScanTask>(), (int)d0, (int)n, T, C.nsm, C.st);
+    launch_scan_tiles_rec(D, T, C.arena, P, C.d_keys.as<unsigned long long>(), &C.d_counter.as<ScanCounts>()->queue,
+                          C.nsm * C.scan_blocks_per_sm, C.st);
+    DCNS_CK(cudaEventRecord(C.ev1, C.st));
+    launch_reverse(C.d_tasks.as<ScanTask>(), (int)d0, (int)n, C.d_keys.as<unsigned long long>(), C.seqbase_dev,
+                   nullptr, C.arena, P, true, C.st);
+    C.stats.scan_launches += 1;
+    C.stats.kernel_launches += 3;
+    d2h(C, C.h_tiles.as<ScanTask>(), C.d_tasks, (size_t)n, (size_t)d0);
+    DCNS_CK(cudaMemcpyAsync(&counts, C.d_counter.p, sizeof(counts), cudaMemcpyDeviceToHost, C.st));
+    sync(C);
+    if (attempt > 0 || filter_listed(T, counts) || !filter_grow(C, T, counts)) break;
+  }
   copy_blocks(S.tasks.data() + first, C.h_tiles.p, sizeof(ScanTask) * n);
   C.stats.scan_rounds += 1;
   C.stats.ms_scan_xfer += ms_since(tx);
   float ms = 0;
   DCNS_CK(cudaEventElapsedTime(&ms, C.ev0, C.ev1));
   C.stats.ms_scan_kernel += ms;
-  return filt_listed(tiles, T.cap);
+  return filter_listed(T, counts);
 }
 
 // Launches the scan over `tiles` plus the generic kernel over `generic` (device slots), then the reverse scans for
@@ -766,12 +790,13 @@ void compute_scan_tasks(Context &C, ScanState &S, const Params &P, int columns_f
   auto tp = t0;
   const bool fast_ok = fast_scan_ok(P);
   if (C.filt_on) {  // a round of windows under the filter (all of them short reads: the fast kernel's)
-    bool fast = true;
-    fast = parallel_sum(n, [&](int64_t k) -> int64_t {
-             ScanTask &T = S.task(first + k);
-             T.striped = striped_for_host(T.hi - T.lo, T.tw, P.open1, P.ext1, P.match) ? 1 : 0;
-             return !(T.striped && T.tw <= kScanW);
-           }) == 0;
+    std::atomic<bool> fast(true);
+    const int64_t rows = parallel_sum(n, [&](int64_t k) -> int64_t {
+      ScanTask &T = S.task(first + k);
+      T.striped = striped_for_host(T.hi - T.lo, T.tw, P.open1, P.ext1, P.match) ? 1 : 0;
+      if (!(T.striped && T.tw <= kScanW)) fast = false;
+      return std::max(T.hi - T.lo, 0);
+    });
     C.d_keys.ensure(C, sizeof(unsigned long long) * (S.size() - S.ns));
     C.d_tasks.ensure(C, sizeof(ScanTask) * (S.size() - S.ns));
     if (fast && C.filt_on) {  // still: the buffers above may have needed its room
@@ -779,7 +804,8 @@ void compute_scan_tasks(Context &C, ScanState &S, const Params &P, int columns_f
       copy_blocks(C.h_tiles.p, S.tasks.data() + first, sizeof(ScanTask) * n);
       C.stats.ms_scan_prep += ms_since(t0);
       h2d(C, C.d_tasks, C.h_tiles.as<ScanTask>(), (size_t)n, (size_t)(first - S.ns));
-      const bool done = run_filtered_round(C, S, P, first, n, C.filt.warm);
+      // the whole scan has two tasks to a tile
+      const bool done = run_filtered_round(C, S, P, first, n, rows / 2, C.filt.warm);
       tp = phase(C, "sc_filtered", tp);
       if (done) {
         C.stats.ms_scan += ms_since(t0);
@@ -987,7 +1013,8 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   int *d_blk = reinterpret_cast<int *>(d_plen + np);
   ScanCounts *const d_counts = C.d_counter.as<ScanCounts>();
   const bool filtered = C.scan_filter && filter_ok(P) && filter_setup(C, pairs, order, nfast, P);
-  const FiltTiles ft = filtered ? filter_tiles(C, nduo) : FiltTiles{};
+  const int64_t whole_rows = total_rows + (chunk < INT32_MAX ? total_rows / chunk * K : 0);
+  const FiltTiles ft = filtered ? filter_tiles(C, nduo, whole_rows) : FiltTiles{};
   h2d(C, C.d_tiles, tab, (size_t)np);
   DCNS_CK(cudaMemcpyAsync(d_wst, wst, sizeof(int64_t) * (np + 1), cudaMemcpyHostToDevice, C.st));
   DCNS_CK(cudaMemcpyAsync(d_plen, plen, sizeof(int2) * np, cudaMemcpyHostToDevice, C.st));
@@ -1010,13 +1037,16 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   auto scan_all = [&](cudaStream_t on) {
     launch_scan_l0(D, ntiles, C.arena, P, C.d_keys.as<unsigned long long>(), &d_counts->queue, grid, on);
   };
-  if (filtered) {
-    launch_filter(C.filt, C.arena, P, filter_threshold(P), bulk);
-    launch_filter_plan_l0(C.filt, D, nduo, ft, C.nsm, bulk);
+  auto scan_marked = [&](const FiltTiles &T, cudaStream_t on) {
+    launch_filter_plan_l0(C.filt, D, nduo, T, C.nsm, on);
     L0Desc F = D;
     F.warm = C.filt.warm;
-    launch_scan_tiles_l0(F, ft, C.arena, P, C.d_keys.as<unsigned long long>(), &d_counts->queue,
-                         C.nsm * C.scan_blocks_per_sm, bulk);
+    launch_scan_tiles_l0(F, T, C.arena, P, C.d_keys.as<unsigned long long>(), &d_counts->queue,
+                         C.nsm * C.scan_blocks_per_sm, on);
+  };
+  if (filtered) {
+    launch_filter(C.filt, C.arena, P, filter_threshold(P), bulk);
+    scan_marked(ft, bulk);
     C.stats.kernel_launches += 2;
   } else {
     scan_all(bulk);
@@ -1041,10 +1071,15 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   DCNS_CK(cudaMemcpyAsync(&got, d_counts, sizeof(got), cudaMemcpyDeviceToHost, C.st));
   tp = phase(C, "l0_launch", tp);
   sync(C);
-  if (filtered && !filt_listed(got.tiles, ft.cap)) {  // marked nearly everywhere: every window against its whole reference after all
-    C.filt_on = false;
+  if (filtered && !filter_listed(ft, got)) {  // a longer list, or every window against its whole reference after all
     DCNS_CK(cudaMemsetAsync(d_counts, 0, sizeof(ScanCounts), C.st));
-    scan_all(C.st);
+    if (filter_grow(C, ft, got)) {
+      scan_marked(filter_tiles(C, nduo, whole_rows), C.st);
+      C.stats.kernel_launches += 1;
+    } else {
+      C.filt_on = false;
+      scan_all(C.st);
+    }
     select();
     C.stats.scan_launches += 1;
     C.stats.kernel_launches += 1;

@@ -28,8 +28,13 @@
 // 80 %), as the exact scan.  The bound kept at match * window every 16 rows costs the filter 2 % and saves the exact
 // scans 28 % (10.1 to 7.3 ms before the floor above min_score in those).  Widths of 8 to 24 columns a lane, chosen per
 // pair to fit the query, would save 14 % of the columns but ran 1.5x slower mixed in one launch (instruction cache)
-// and no faster sorted by width.  References that are marked nearly everywhere (tandem repeats against themselves)
-// overflow the tile list and pay for the filter on top of the whole scan.
+// and no faster sorted by width.
+//
+// References that are marked nearly everywhere: the filter stops where a pair's marks so far say that the exact scan
+// would compute most rows anyway, a list of more rows than the whole scan's is not scanned, and one that is only too
+// short is made again.  A pair of 200 kb that holds a 17-base word every 27, 60, 120 bases and no seed: 31.5, 32.5,
+// 31.7 ms without the filter, 37.9, 38.0, 39.8 with the list's capacity as the only test, 32.1, 32.0, 11.9 now; of
+// 40 and 2 kb 0.31 -> 0.71 -> 0.47, 0.47, 0.33.  The watch over the marks costs the filter 1.4 %.
 #include <type_traits>
 
 #include "device_common.cuh"
@@ -57,6 +62,24 @@ __device__ __forceinline__ int filt_pair_of(const FiltDesc &D, int t) {
   return lo;
 }
 
+// Blocks that the exact scan of a window pair around the lane's strip computes for a word of marks: those marked in
+// this strip or the next three, and the warm-up before each run (some four blocks; runs closer than that are one).
+__device__ __forceinline__ int filt_cost(uint32_t marks) {
+  marks |= __shfl_down_sync(0xFFFFFFFFu, marks, 1);
+  marks |= __shfl_down_sync(0xFFFFFFFFu, marks, 2);
+  marks |= marks << 1;
+  marks |= marks << 2;
+  return __popc(marks | marks << 1);
+}
+// Whether a pair is marked nearly everywhere: most of its words of marks so far cost the exact scan five eighths of
+// their rows or more (the filter is a fifth of the whole scan; words of few blocks count too little, since a run's
+// warm-up may lie before them).  The rest of them are then set without the DP (marks only say where the exact scan
+// looks), so that such a pair costs little more than the scan of every window that follows.
+__device__ __forceinline__ bool filt_dense(unsigned long long seen) {
+  const uint32_t words = (uint32_t)(seen >> 32), dense = (uint32_t)seen;
+  return words >= 16 && dense > words / 2;
+}
+
 struct Stream {  // a lane's reference symbols, sixteen at a time
   const uint32_t *pk, *nm;
   int64_t k;  // arena index of the next sixteen
@@ -81,7 +104,9 @@ __global__ void __launch_bounds__(32 * kFWarps, 5)
   const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
   const int t = blockIdx.x * kFWarps + wb;
   if (t >= D.ntasks) return;  // whole warp
-  const FiltPair P = D.pairs[filt_pair_of(D, t)];
+  const int slot = filt_pair_of(D, t);
+  const FiltPair P = D.pairs[slot];
+  unsigned long long seen = __ldcg(D.seen + slot);
   const int rel = t - P.task_begin, ct = rel / P.nch, ch = rel % P.nch;
   uint4 *const prof = prof_all[wb];
   const uint32_t open2 = fpack2(open), ext2 = fpack2(ext), nopen2 = fpack2(-open);
@@ -106,6 +131,13 @@ __global__ void __launch_bounds__(32 * kFWarps, 5)
   const int rbeg = ch == 0 ? 0 : rows0 - D.warm;  // lane 0's row at step 0
   const int nblk = (rows1 - rbeg + 31 + 3 + 15) / 16;
   uint32_t *out = D.words + P.word_begin + (int64_t)rel * P.wpc * 64 + lane;
+  const int strip = 2 * ct * kFNew + lane, strips = (P.n2 + kFC - 1) / kFC;  // strips of the query among the warp's
+  const int used = __popc(__ballot_sync(0xFFFFFFFFu, strip < strips)) +
+                   __popc(__ballot_sync(0xFFFFFFFFu, strip + kFNew < strips));
+  if (filt_dense(seen)) {
+    for (int k = 0; k < P.wpc; ++k, out += 64) out[0] = out[32] = ~0u;
+    return;
+  }
   Stream str{ar.pk, ar.nm, P.ref_base + rbeg - lane};
   uint32_t wcur, ncur, wnext, nnext;
   str.load(wcur, ncur);
@@ -179,7 +211,17 @@ __global__ void __launch_bounds__(32 * kFWarps, 5)
       out[0] = acc0;
       out[32] = acc1;
       out += 64;
+      bool dense = false;
+      if (__any_sync(0xFFFFFFFFu, (acc0 | acc1) != 0))
+        dense = 8 * (int)__reduce_add_sync(0xFFFFFFFFu, (unsigned)(filt_cost(acc0) + filt_cost(acc1))) >
+                5 * used * ((blk & 31) + 1);
       acc0 = acc1 = 0;
+      if (lane == 0) atomicAdd(D.seen + slot, (1ull << 32) | (dense ? 1u : 0u));
+      if (filt_dense(seen)) {  // as it was a word ago: nothing waits for it
+        for (int k = (blk >> 5) + 1; k < P.wpc; ++k, out += 64) out[0] = out[32] = ~0u;
+        return;
+      }
+      seen = __ldcg(D.seen + slot);
     }
   }
 }
@@ -188,7 +230,7 @@ __global__ void __launch_bounds__(32 * kFWarps, 5)
 // order; runs closer than the exact scan's warm-up are one (the rows between them would be computed twice).
 template <class Emit>
 __device__ __forceinline__ void filt_runs(const FiltDesc &D, const FiltPair &P, int c_lo, int c_hi, int lo, int hi,
-                                          Emit emit) {
+                                          Emit &emit) {
   const int k0 = c_lo / kFC, k1 = (c_hi - 1) / kFC;
   int cs = -1, ce = -1;
   for (int ch = lo / D.chunk; ch <= (hi - 1) / D.chunk; ++ch) {
@@ -224,11 +266,84 @@ __device__ __forceinline__ void filt_runs(const FiltDesc &D, const FiltPair &P, 
   if (cs >= 0) emit(cs, ce);
 }
 
-// The same by a whole warp: the lanes load 32 words at a time, and the runs of the words that hold marks are followed
-// in order by all lanes together; lane 0 emits.
-template <class Emit>
+// A list's tiles from one thread's runs.  (Their rows are not counted: the plans of many items have longer tiles, whose
+// warm-up matters little, and an addition per thread took a quarter of the plan.)
+struct FiltEmit {
+  const FiltTiles &T;
+  int a, b;
+  __device__ __forceinline__ void operator()(int rb, int re) {
+    const int n = (re - rb + T.rows - 1) / T.rows, per = (re - rb + n - 1) / n;
+    // one addition for the threads that are here together, whose tiles then lie next to each other: 4,000 pairs' plans
+    // 161 and 159 us (an addition each, 32 bits; 172 and 198 in 64 bits) -> 65 and 58, their scans 1.04 -> 0.90 ms
+    const unsigned here = __activemask();
+    const int lead = __ffs(here) - 1;
+    int before = 0, all = 0;
+    for (unsigned m = here; m; m &= m - 1) {
+      const int l = __ffs(m) - 1, v = __shfl_sync(here, n, l);
+      before += l < (int)(threadIdx.x & 31) ? v : 0;
+      all += v;
+    }
+    unsigned long long at = 0;
+    if ((int)(threadIdx.x & 31) == lead) at = atomicAdd(T.count, (unsigned long long)all);
+    at = __shfl_sync(here, at, lead) + (unsigned)before;
+    for (int k = 0; k < n; ++k) {
+      const int p = filt_place(at, k, T.cap);
+      if (p < 0) break;
+      T.list[p] = FiltTile{a, b, rb + k * per, min(re, rb + (k + 1) * per)};
+    }
+  }
+};
+
+// The same from a warp's runs: every lane holds one, and 32 of them go out at a time, with one addition to the counters
+// and each run's tiles written by all lanes.
+struct FiltEmitWarp {
+  const FiltTiles &T;
+  int a, b, warm, held = 0;
+  int rb = 0, re = 0;  // the lane's run
+  unsigned long long rows = 0;
+  __device__ __forceinline__ void operator()(int from, int to) {
+    if ((int)(threadIdx.x & 31) == held) rb = from, re = to;
+    if (++held == 32) flush();
+  }
+  __device__ __forceinline__ void flush() {
+    const int lane = threadIdx.x & 31;
+    const int n = lane < held ? (re - rb + T.rows - 1) / T.rows : 0, per = n > 0 ? (re - rb + n - 1) / n : 0;
+    if (n > 0) rows += (unsigned long long)(re - rb) + (unsigned long long)n * warm;
+    int end = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xFFFFFFFFu, end, d);
+      if (lane >= d) end += v;
+    }
+    unsigned long long at = 0;
+    if (lane == 31) at = atomicAdd(T.count, (unsigned long long)end);
+    at = __shfl_sync(0xFFFFFFFFu, at, 31);
+    for (int r = 0; r < held; ++r) {
+      const int rn = __shfl_sync(0xFFFFFFFFu, n, r), rper = __shfl_sync(0xFFFFFFFFu, per, r);
+      const int from = __shfl_sync(0xFFFFFFFFu, rb, r), to = __shfl_sync(0xFFFFFFFFu, re, r);
+      const int first = __shfl_sync(0xFFFFFFFFu, end, r) - rn;
+      for (int k = lane; k < rn; k += 32) {
+        const int p = filt_place(at, first + k, T.cap);
+        if (p < 0) break;
+        T.list[p] = FiltTile{a, b, from + k * rper, min(to, from + (k + 1) * rper)};
+      }
+    }
+    held = 0;
+  }
+  __device__ __forceinline__ void finish() {
+    if (held > 0) flush();
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) rows += __shfl_down_sync(0xFFFFFFFFu, rows, d);
+    if ((threadIdx.x & 31) == 0 && rows) atomicAdd(T.count + 1, rows);
+  }
+};
+
+// The runs of words [kPlanWords seg, kPlanWords (seg + 1)) of the rows' words by a whole warp: the lanes load 32 words
+// at a time, and the runs of the words that hold marks are followed in order by all lanes together.  A run that goes on
+// in the next segment is two.
+constexpr int kPlanWords = 128;
 __device__ __forceinline__ void filt_runs_warp(const FiltDesc &D, const FiltPair &P, int c_lo, int c_hi, int lo, int hi,
-                                               Emit emit) {
+                                               int seg, FiltEmitWarp &emit) {
   const int lane = threadIdx.x & 31;
   const int k0 = c_lo / kFC, k1 = (c_hi - 1) / kFC;
   int lmin = 31, lmax = 0;
@@ -237,12 +352,13 @@ __device__ __forceinline__ void filt_runs_warp(const FiltDesc &D, const FiltPair
     lmin = min(lmin, l), lmax = max(lmax, l);
   }
   const int ch0 = lo / D.chunk, items = ((hi - 1) / D.chunk - ch0 + 1) * P.wpc;
+  const int end = (int)min((int64_t)items, (int64_t)(seg + 1) * kPlanWords);
   int cs = -1, ce = -1;
-  for (int base = 0; base < items; base += 32) {
+  for (int base = seg * kPlanWords; base < end; base += 32) {
     const int it = base + lane;
     uint32_t v = 0;
     int row = 0, rlo = 0, rhi = 0;
-    if (it < items) {
+    if (it < end) {
       const int ch = ch0 + it / P.wpc, wi = it % P.wpc;
       const int rbeg = ch == 0 ? 0 : ch * D.chunk - D.warm;
       rlo = max(lo, ch * D.chunk), rhi = (int)min((int64_t)hi, (int64_t)(ch + 1) * D.chunk);
@@ -270,30 +386,20 @@ __device__ __forceinline__ void filt_runs_warp(const FiltDesc &D, const FiltPair
         if (cs >= 0 && a - D.warm <= ce) {
           ce = max(ce, e);
         } else {
-          if (cs >= 0 && lane == 0) emit(cs, ce);
+          if (cs >= 0) emit(cs, ce);
           cs = a, ce = e;
         }
       }
     }
   }
-  if (cs >= 0 && lane == 0) emit(cs, ce);
-}
-
-__device__ __forceinline__ void filt_emit(const FiltTiles &T, int a, int b, int rb, int re) {
-  const int n = (re - rb + T.rows - 1) / T.rows, per = (re - rb + n - 1) / n;
-  const unsigned long long at = atomicAdd(T.count, (unsigned long long)n);
-  for (int k = 0; k < n; ++k) {
-    const int p = filt_place(at, k, T.cap);
-    if (p < 0) break;
-    T.list[p] = FiltTile{a, b, rb + k * per, min(re, rb + (k + 1) * per)};
-  }
+  if (cs >= 0) emit(cs, ce);
 }
 
 // Plans: one thread, or WARP one warp, per item.  A thread waits for each word before it looks at the next, so a plan
-// of few items is as long as its longest reference has words; with a warp to each item the words come 32 at a time.
-// Up to 256 items per multiprocessor: one pair of 5 kb (312 and 350 items) 66 -> 7 and 60 -> 7 us, two pairs of
-// 200 kb 385 -> 140 and 472 -> 94 us.  The plans of 10,000 pairs have some 100,000 items each, of a few words, and keep
-// their threads.
+// of few items is as long as its longest reference has words; with a warp to each item and segment of it
+// (blockIdx.y) the words come 32 at a time.  Up to 256 items per multiprocessor: one pair of 5 kb (312 and 350 items)
+// 66 -> 7 and 60 -> 7 us, two pairs of 200 kb 385 -> 140 and 472 -> 94 us.  The plans of 10,000 pairs have some 100,000
+// items each, of a few words, and keep their threads.
 constexpr int kPlanWarpItems = 256;
 
 // Level-0 tiles: an item per two windows of a pair (slot of the level-0 table, duo).
@@ -312,11 +418,14 @@ __global__ void __launch_bounds__(256) filter_plan_l0_kernel(FiltDesc D, L0Desc 
   const FiltPair P = D.pairs[lo];
   const int duo = (int)(t - P.duo_begin), last = min(2 * duo + 1, L.pairs[lo].nfast - 1);
   const int c_lo = 2 * duo * L.step, c_hi = min(P.n2, last * L.step + L.window);
-  auto emit = [&](int a, int b) { filt_emit(T, lo, duo, a, b); };
-  if constexpr (WARP)
-    filt_runs_warp(D, P, c_lo, c_hi, 0, P.n1, emit);
-  else
+  if constexpr (WARP) {
+    FiltEmitWarp emit{T, lo, duo, D.warm};
+    filt_runs_warp(D, P, c_lo, c_hi, 0, P.n1, (int)blockIdx.y, emit);
+    emit.finish();
+  } else {
+    FiltEmit emit{T, lo, duo};
     filt_runs(D, P, c_lo, c_hi, 0, P.n1, emit);
+  }
 }
 
 // Tiles of a round's tasks: an item per task.
@@ -329,11 +438,14 @@ __global__ void __launch_bounds__(256) filter_plan_rec_kernel(FiltDesc D, const 
   const ScanTask x = tasks[first + k];
   if (x.tw <= 0 || x.hi <= x.lo) return;
   const FiltPair P = D.pairs[D.slot[x.pair]];
-  auto emit = [&](int a, int b) { filt_emit(T, first + k, 0, a, b); };
-  if constexpr (WARP)
-    filt_runs_warp(D, P, x.s2, x.s2 + x.tw, x.lo, x.hi, emit);
-  else
+  if constexpr (WARP) {
+    FiltEmitWarp emit{T, first + k, 0, D.warm};
+    filt_runs_warp(D, P, x.s2, x.s2 + x.tw, x.lo, x.hi, (int)blockIdx.y, emit);
+    emit.finish();
+  } else {
+    FiltEmit emit{T, first + k, 0};
     filt_runs(D, P, x.s2, x.s2 + x.tw, x.lo, x.hi, emit);
+  }
 }
 
 }  // namespace
@@ -346,8 +458,9 @@ void launch_filter(const FiltDesc &D, Arena ar, Params p, int thr, cudaStream_t 
 
 void launch_filter_plan_l0(const FiltDesc &D, L0Desc L, int64_t nduo, FiltTiles T, int nsm, cudaStream_t st) {
   if (nduo <= 0) return;
+  const unsigned segs = (unsigned)((D.max_words + kPlanWords - 1) / kPlanWords);
   if (nduo <= (int64_t)kPlanWarpItems * nsm)
-    filter_plan_l0_kernel<true><<<(unsigned)((nduo + 7) / 8), 256, 0, st>>>(D, L, nduo, T);
+    filter_plan_l0_kernel<true><<<dim3((unsigned)((nduo + 7) / 8), segs), 256, 0, st>>>(D, L, nduo, T);
   else
     filter_plan_l0_kernel<false><<<(unsigned)((nduo + 255) / 256), 256, 0, st>>>(D, L, nduo, T);
 }
@@ -355,8 +468,9 @@ void launch_filter_plan_l0(const FiltDesc &D, L0Desc L, int64_t nduo, FiltTiles 
 void launch_filter_plan_rec(const FiltDesc &D, const ScanTask *tasks, int first, int n, FiltTiles T, int nsm,
                             cudaStream_t st) {
   if (n <= 0) return;
+  const unsigned segs = (unsigned)((D.max_words + kPlanWords - 1) / kPlanWords);
   if (n <= kPlanWarpItems * nsm)
-    filter_plan_rec_kernel<true><<<(n + 7) / 8, 256, 0, st>>>(D, tasks, first, n, T);
+    filter_plan_rec_kernel<true><<<dim3((unsigned)((n + 7) / 8), segs), 256, 0, st>>>(D, tasks, first, n, T);
   else
     filter_plan_rec_kernel<false><<<(n + 255) / 256, 256, 0, st>>>(D, tasks, first, n, T);
 }

@@ -241,7 +241,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc 
   const uint32_t open2 = pack2(open), ext2 = pack2(ext), fext2 = pack2(max(ext, open));
   const uint32_t open_lo = open2 & 0xFFFFu, open_hi = open2 & 0xFFFF0000u;
 
-  if (MODE >= 3) ntiles = filt_listed(*ft.count, ft.cap) ? (int64_t)*ft.count : 0;  // else the host scans everything
+  if (MODE >= 3)  // else the host scans everything
+    ntiles = filt_listed(ft.count[0], ft.cap) && ft.count[1] <= ft.most ? (int64_t)ft.count[0] : 0;
   for (;;) {
     const int t = atomicAdd(counter, 1);
     if (t >= ntiles) break;
