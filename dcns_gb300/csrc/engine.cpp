@@ -307,7 +307,7 @@ class HostPool {
   static void work(Job &J) {
     for (int64_t i; (i = J.next.fetch_add(1)) < J.n;) {
       try {
-        if (!J.failed) (*J.f)(i);
+        if (!J.failed.load(std::memory_order_relaxed)) (*J.f)(i);
       } catch (...) {
         std::lock_guard<std::mutex> lk(J.m);
         if (!J.error) J.error = std::current_exception();

@@ -139,18 +139,19 @@ class SeedArena {
 template <class T>
 struct SeedAlloc {
   using value_type = T;
+  SeedArena *arena = &SeedArena::mine();  // looked up once per set
   SeedAlloc() = default;
   template <class U>
-  SeedAlloc(const SeedAlloc<U> &) {}
-  T *allocate(size_t n) { return static_cast<T *>(SeedArena::mine().take(n * sizeof(T))); }
-  void deallocate(T *p, size_t n) { SeedArena::mine().give(p, n * sizeof(T)); }
+  SeedAlloc(const SeedAlloc<U> &o) : arena(o.arena) {}
+  T *allocate(size_t n) { return static_cast<T *>(arena->take(n * sizeof(T))); }
+  void deallocate(T *p, size_t n) { arena->give(p, n * sizeof(T)); }
   template <class U>
-  bool operator==(const SeedAlloc<U> &) const {
-    return true;
+  bool operator==(const SeedAlloc<U> &o) const {
+    return arena == o.arena;
   }
   template <class U>
-  bool operator!=(const SeedAlloc<U> &) const {
-    return false;
+  bool operator!=(const SeedAlloc<U> &o) const {
+    return arena != o.arena;
   }
 };
 using SeedSet = std::set<Seed4, SeedLess, SeedAlloc<Seed4>>;
