@@ -215,9 +215,10 @@ struct SgFlow {
 // ---- kernel launchers (defined in the .cu files)
 void launch_pack(const int8_t *codes, const int64_t *src_off, const int64_t *dst_base, const int32_t *len, int nseq,
                  uint32_t *pk, uint32_t *nm, cudaStream_t st);
-void launch_scan(RecDesc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter, int grid,
-                 cudaStream_t st);
-// launch_scan leaves the column of each maximum open: this finds it for the tasks of at least min_score.
+// columns: the column of each maximum is found on the way.
+void launch_scan(RecDesc d, int64_t ntiles, bool columns, Arena ar, Params p, unsigned long long *keys,
+                 int *work_counter, int grid, cudaStream_t st);
+// launch_scan without columns leaves them open: this finds them for the tasks of at least min_score.
 void launch_scan_columns(const ScanTask *tasks, int first, int n, const int64_t *seq_base, Arena ar, Params p,
                          int min_score, int warm, unsigned long long *keys, cudaStream_t st);
 void launch_scan_l0(L0Desc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter,

@@ -261,7 +261,6 @@ class HostPool {
     const std::function<void(int64_t)> *f;
     int64_t n;
     std::atomic<int64_t> next{0}, done{0};
-    std::atomic<bool> failed{false};
     std::exception_ptr error;  // the first that an item threw
     std::mutex m;
     std::condition_variable cv;
@@ -294,7 +293,7 @@ class HostPool {
           break;
         }
     }
-    if (J->failed) std::rethrow_exception(J->error);
+    if (J->error) std::rethrow_exception(J->error);
   }
   static thread_local bool in_worker;
 
@@ -306,14 +305,15 @@ class HostPool {
   }
   static void work(Job &J) {
     for (int64_t i; (i = J.next.fetch_add(1)) < J.n;) {
+      int64_t ended = 1;
       try {
-        if (!J.failed.load(std::memory_order_relaxed)) (*J.f)(i);
+        (*J.f)(i);
       } catch (...) {
+        ended += std::max<int64_t>(0, J.n - J.next.exchange(J.n));  // the items not begun are not
         std::lock_guard<std::mutex> lk(J.m);
         if (!J.error) J.error = std::current_exception();
-        J.failed = true;
       }
-      if (J.done.fetch_add(1) + 1 == J.n) {
+      if (J.done.fetch_add(ended) + ended == J.n) {
         std::lock_guard<std::mutex> lk(J.m);
         J.cv.notify_all();
       }
@@ -676,7 +676,7 @@ bool run_filtered_round(Context &C, ScanState &S, const Params &P, int64_t first
 // Launches the scan over `tiles` plus the generic kernel over `generic` (device slots), then the reverse scans for
 // recursion tasks [first, first+n) (device slots first - ns ...); downloads those tasks.
 void run_scan_round(Context &C, ScanState &S, const Params &P, int64_t first, int64_t n, const RecDuo *duos,
-                    int64_t nduo, int64_t ntiles, int32_t chunk, int warm, int columns_from,
+                    int64_t nduo, int64_t ntiles, int32_t chunk, int warm, int columns_from, bool columns_inside,
                     const std::vector<int32_t> &generic) {
   auto tx = Clock::now();
   const int64_t d0 = first - S.ns;  // device slot of the first task
@@ -691,9 +691,9 @@ void run_scan_round(Context &C, ScanState &S, const Params &P, int64_t first, in
                                             (ntiles + kScanThreads - 1) / kScanThreads);
     const RecDesc D{C.d_tiles.as<RecDuo>(), C.d_tasks.as<ScanTask>(), C.seqbase_dev, (int32_t)nduo, chunk, warm, 0};
     DCNS_CK(cudaEventRecord(C.ev0, C.st));
-    launch_scan(D, ntiles, C.arena, P, C.d_keys.as<unsigned long long>(), C.d_counter.as<int>(), std::max(grid, 1),
-                C.st);
-    if (columns_from != INT_MAX) {
+    launch_scan(D, ntiles, columns_inside, C.arena, P, C.d_keys.as<unsigned long long>(), C.d_counter.as<int>(),
+                std::max(grid, 1), C.st);
+    if (columns_from != INT_MAX && !columns_inside) {
       launch_scan_columns(C.d_tasks.as<ScanTask>(), (int)d0, (int)n, C.seqbase_dev, C.arena, P, columns_from, warm,
                           C.d_keys.as<unsigned long long>(), C.st);
       C.stats.kernel_launches += 1;
@@ -745,38 +745,51 @@ void run_scan_round(Context &C, ScanState &S, const Params &P, int64_t first, in
   }
 }
 
-// Rows per tile of duos with these row counts on `resident` persistent threads (INT32_MAX: whole duos).  The threads
-// take their tiles in waves, and a wave lasts a tile's rows and its K warm-up rows, so a target of `most` tiles per
-// thread, each a fraction of a wave short of filling the GPU, pays for the last wave and for every warm-up: of the
-// smallest chunks that leave 1, 2, ... `most` full waves, the one whose waves take the fewest rows.  8,750 windows
-// against 7.5 kb (4,375 duos): three waves of 320 + 80 rows before, one of 699 + 80 now; the scan 0.67 -> 0.65 ms, and
-// 0.55 ms without the search for columns (launch_scan).
-int64_t scan_chunk(const std::vector<int32_t> &drows, int64_t resident, int most, int K) {
-  if (drows.empty() || (int64_t)drows.size() >= most * resident) return INT32_MAX;
+// Rows per tile of duos with these row counts (INT32_MAX: whole duos).  A tile takes its rows and K warm-up rows; a
+// whole duo has no warm-up.  With one warp to a scheduler a row takes its latency (0.50 us), with two and three 1.75 and
+// 2.5 times that (9,000 windows against 5 to 10 kb), and the persistent threads take what does not fit in waves.  Of the
+// smallest chunks that fill the multiprocessors with 1, 2, ... blocks each (or, of more duos than threads, leave 2, 3,
+// ... `most` full waves), the one of the least time by that count.  10,000 windows against 160 rows: 113 us whole, 186
+// in four chunks; 10 against 300: 161 whole, 82 in eight; 8,757 windows against 5 to 10 kb in chunks for 1, 2, 3, 4, 5
+// blocks: 2.1, 1.02, 1.22, 0.92, 1.04 ms.
+int64_t scan_chunk(const std::vector<int32_t> &drows, int nsm, int blocks_per_sm, int most, int K) {
+  const int64_t n = (int64_t)drows.size(), resident = (int64_t)nsm * blocks_per_sm * kScanThreads;
+  if (n == 0 || n >= most * resident) return INT32_MAX;
   const int32_t longest = *std::max_element(drows.begin(), drows.end());
-  if (longest <= 0) return INT32_MAX;
-  const int32_t step = std::max(1, longest / 512);
-  std::map<int32_t, int64_t> count;  // duos by rows (rounded up to some 512 values)
-  for (int32_t r : drows) ++count[(r + step - 1) / step * step];
+  if (longest <= K) return INT32_MAX;
+  const int32_t step = (longest + 63) / 64;
+  std::array<int64_t, 65> count{};  // duos by rows, rounded up to 64 values
+  for (int32_t r : drows) ++count[(std::max(r, 0) + step - 1) / step];
+  std::vector<std::pair<int64_t, int64_t>> rows_of;  // (rows, duos)
+  for (int64_t k = 1; k <= 64; ++k)
+    if (count[k]) rows_of.push_back({k * step, count[k]});
   auto tiles = [&](int64_t chunk) {
-    int64_t n = 0;
-    for (const auto &e : count) n += e.second * std::max<int64_t>(1, (e.first + chunk - 1) / chunk);
-    return n;
+    int64_t t = count[0];
+    for (const auto &e : rows_of) t += e.second * ((e.first + chunk - 1) / chunk);
+    return t;
   };
-  int64_t best = INT32_MAX, best_rows = INT64_MAX;
-  for (int w = 1; w <= most; ++w) {
-    if (tiles(longest) > w * resident) continue;  // more duos than that many waves
-    int64_t lo = std::max<int64_t>(K / 2, 1), hi = std::max<int64_t>(longest, lo);
-    while (lo < hi) {  // the smallest chunk with at most w waves of tiles
+  auto time = [&](int64_t t, int64_t rows) {  // in quarters of a row's latency
+    const int64_t blocks = std::min<int64_t>(blocks_per_sm, ((t + kScanThreads - 1) / kScanThreads + nsm - 1) / nsm);
+    const int64_t warps = (blocks * (kScanThreads / 32) + 3) / 4;  // on the fullest scheduler
+    return (t + resident - 1) / resident * rows * (3 * warps + 1);
+  };
+  int64_t best = INT32_MAX, best_time = time(n, longest);
+  auto fill = [&](int64_t target) {
+    if (n > target) return;
+    int64_t lo = std::max<int64_t>(K / 2, 1), hi = 64 * (int64_t)step;
+    while (lo < hi) {  // the smallest chunk with at most that many tiles
       const int64_t mid = (lo + hi) / 2;
-      if (tiles(mid) <= w * resident)
+      if (tiles(mid) <= target)
         hi = mid;
       else
         lo = mid + 1;
     }
-    const int64_t rows = (tiles(lo) + resident - 1) / resident * (lo + K);
-    if (rows < best_rows) best_rows = rows, best = lo;
-  }
+    const int64_t t = time(tiles(lo), lo + K);
+    if (t < best_time) best_time = t, best = lo;
+  };
+  for (int k = 1; k <= blocks_per_sm; ++k) fill((int64_t)nsm * kScanThreads * k);
+  if (n > resident)
+    for (int w = 2; w <= most; ++w) fill(w * resident);
   return best >= longest ? INT32_MAX : best;
 }
 
@@ -832,16 +845,18 @@ void compute_scan_tasks(Context &C, ScanState &S, const Params &P, int columns_f
   std::vector<size_t> gb{0};
   for (size_t i = 1; i <= fast.size(); ++i)
     if (i == fast.size() || tk(fast[i]).pair != tk(fast[i - 1]).pair) gb.push_back(i);
-  parallel_for((int64_t)gb.size() - 1, [&](int64_t g) {
+  const int64_t groups = (int64_t)gb.size() - 1;
+  parallel_for((groups + 63) / 64, [&](int64_t b) {
     const auto before = [&](int32_t a, int32_t b) {
       const ScanTask &x = tk(a), &y = tk(b);
       if (x.lo != y.lo) return x.lo < y.lo;
       if (x.hi != y.hi) return x.hi < y.hi;
       return x.s2 < y.s2;
     };
-    if (!std::is_sorted(fast.begin() + gb[g], fast.begin() + gb[g + 1], before))
-      std::sort(fast.begin() + gb[g], fast.begin() + gb[g + 1], before);
-  });
+    for (int64_t g = 64 * b; g < std::min(groups, 64 * b + 64); ++g)
+      if (!std::is_sorted(fast.begin() + gb[g], fast.begin() + gb[g + 1], before))
+        std::sort(fast.begin() + gb[g], fast.begin() + gb[g + 1], before);
+  }, 4);
   tp = phase(C, "sc_sort", tp);
   std::vector<RecDuo> duo;
   for (size_t g = 0; g + 1 < gb.size(); ++g)
@@ -855,9 +870,9 @@ void compute_scan_tasks(Context &C, ScanState &S, const Params &P, int columns_f
     if (duo[d].b >= 0) lo = std::min(lo, tk(duo[d].b).lo), hi = std::max(hi, tk(duo[d].b).hi);
     drows[d] = hi - lo;
   }
-  const int64_t resident = (int64_t)C.nsm * C.scan_blocks_per_sm * kScanThreads;
   const int K = warmup_rows(P, kScanW);
-  const int64_t chunk = K == INT_MAX ? INT32_MAX : scan_chunk(drows, resident, C.scan_tiles_per_thread, K);
+  const int64_t chunk =
+      K == INT_MAX ? INT32_MAX : scan_chunk(drows, C.nsm, C.scan_blocks_per_sm, C.scan_tiles_per_thread, K);
   // longest duos first for the work queue: a counting sort by log-length (linear time); tile_begin follows that order
   std::vector<RecDuo> ord(nd);
   {
@@ -889,7 +904,13 @@ void compute_scan_tasks(Context &C, ScanState &S, const Params &P, int columns_f
   C.stats.ms_scan_prep += ms_since(t0);
   C.d_tasks.ensure(C, sizeof(ScanTask) * (S.size() - S.ns));
   h2d(C, C.d_tasks, S.tasks.data() + first, (size_t)n, (size_t)(first - S.ns));
-  run_scan_round(C, S, P, first, n, duo.data(), nd, ntiles, (int32_t)chunk, K, columns_from, generic);
+  // The columns of the maxima on the way, or in a second DP over up to K rows before each maximum: on the way where the
+  // references are so short that the second is a large part of the call.  One, ten, 300 and 5,000 windows of 38 against
+  // 120 rows: 96, 131, 202, 720 us on the way, 108, 147, 222, 820 after; from 400 rows on 5,000 windows take the same,
+  // 8,750 windows against 7.5 kb 0.65 ms of scan on the way, 0.55 after.
+  const bool inside = columns_from != INT_MAX && nd > 0 &&
+                      *std::max_element(drows.begin(), drows.end()) <= (K == INT_MAX ? INT_MAX : 4 * K);
+  run_scan_round(C, S, P, first, n, duo.data(), nd, ntiles, (int32_t)chunk, K, columns_from, inside, generic);
   tp = phase(C, "sc_round", tp);
   C.stats.ms_scan += ms_since(t0);
   S.left.resize(S.size(), -1);

@@ -201,10 +201,11 @@ __device__ __forceinline__ ScanTile rec_tile(const RecDesc &D, int64_t t) {
   return tl;
 }
 
-// MODE 1: level-0 tiles from the per-pair table; MODE 2: round tiles from the duo table; MODE 3, 4: level-0 and round
+// MODE 1: level-0 tiles from the per-pair table; MODE 2, 5: round tiles from the duo table; MODE 3, 4: level-0 and round
 // tiles from the filter's list.  MODE 2 leaves the maximum's column open (0 in the key): every tile starts from no
 // maximum at all, and the search for the column of each new one, in whichever lane, took a third of the launch; the
-// tasks whose column is asked for find it afterwards, each in one row (scan_column_kernel).
+// tasks whose column is asked for find it afterwards, each in one row (scan_column_kernel).  MODE 5 finds it on the way:
+// for references so short that the second DP, over up to a warm-up of rows, would be as long as the first.
 constexpr int kProfGroups = (kScanW + 3) / 4;  // query columns in groups of four (one 128-bit shared load)
 constexpr int kProfSyms = 4;                   // reference symbols A, C, G, T (2-bit codes 0..3); N rows below
 constexpr size_t kProfBytes = sizeof(uint4) * kProfSyms * kProfGroups * kScanThreads;
@@ -241,13 +242,14 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc 
   const uint32_t open2 = pack2(open), ext2 = pack2(ext), fext2 = pack2(max(ext, open));
   const uint32_t open_lo = open2 & 0xFFFFu, open_hi = open2 & 0xFFFF0000u;
 
-  if (MODE >= 3)  // else the host scans everything
+  constexpr bool kListed = MODE == 3 || MODE == 4;
+  if (kListed)  // else the host scans everything
     ntiles = filt_listed(ft.count[0], ft.cap) && ft.count[1] <= ft.most ? (int64_t)ft.count[0] : 0;
   for (;;) {
     const int t = atomicAdd(counter, 1);
     if (t >= ntiles) break;
     const ScanTile tl = MODE == 1   ? l0_tile(l0, t)
-                        : MODE == 2 ? rec_tile(rec, t)
+                        : MODE == 2 || MODE == 5 ? rec_tile(rec, t)
                         : MODE == 3 ? l0_filtered_tile(l0, ft.list[t])
                                     : rec_filtered_tile(rec, ft.list[t]);
 
@@ -296,7 +298,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc 
     uint32_t cmpb = 0x7FFF7FFFu;
     // (floor: maxima up to it do not count; a filtered scan starts below min_score, which spares a rising alignment the
     // search for its column in every row)
-    int best0 = MODE >= 3 ? floor : 0, best1 = best0, brow0 = -1, brow1 = -1, bcol0 = -1, bcol1 = -1;
+    int best0 = kListed ? floor : 0, best1 = best0, brow0 = -1, brow1 = -1, bcol0 = -1, bcol1 = -1;
 
     int r = tl.row_begin;
     int nev = min_above(r - 1, zr0, zr1, cs0, ce0, cs1, ce1);
@@ -468,11 +470,12 @@ void launch_scan_columns(const ScanTask *tasks, int first, int n, const int64_t 
   scan_column_kernel<<<(n + 127) / 128, 128, 0, st>>>(tasks, first, n, seq_base, ar, p, min_score, warm, keys);
 }
 
-void launch_scan(RecDesc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter, int grid,
-                 cudaStream_t st) {
+void launch_scan(RecDesc d, int64_t ntiles, bool columns, Arena ar, Params p, unsigned long long *keys,
+                 int *work_counter, int grid, cudaStream_t st) {
   if (ntiles <= 0) return;
-  scan_kernel<kScanW, 2><<<grid, kScanThreads, kProfBytes, st>>>(d, L0Desc{}, FiltTiles{}, 0, ntiles, ar, p.open1, p.ext1, p.match,
-                                                                 p.mismatch, keys, work_counter);
+  const auto kernel = columns ? scan_kernel<kScanW, 5> : scan_kernel<kScanW, 2>;
+  kernel<<<grid, kScanThreads, kProfBytes, st>>>(d, L0Desc{}, FiltTiles{}, 0, ntiles, ar, p.open1, p.ext1, p.match,
+                                                 p.mismatch, keys, work_counter);
 }
 
 void launch_scan_l0(L0Desc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter,
@@ -917,7 +920,7 @@ int scan_occupancy_impl() {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProfBytes) == cudaSuccess;
   };
   if (!opt_in(scan_kernel<kScanW, 1>) || !opt_in(scan_kernel<kScanW, 2>) || !opt_in(scan_kernel<kScanW, 3>) ||
-      !opt_in(scan_kernel<kScanW, 4>)) {
+      !opt_in(scan_kernel<kScanW, 4>) || !opt_in(scan_kernel<kScanW, 5>)) {
     (void)cudaGetLastError();
     return 0;
   }
