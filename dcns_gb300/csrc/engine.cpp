@@ -1439,18 +1439,33 @@ void run_xdrop_rounds(Context &C, std::vector<XTask> &X, const Params &P, bool w
     X[k].iii = X[k].jjj = X[k].ncig = 0;
     rows_cap[k] = full_slots ? (int64_t)X[k].n1 : std::min<int64_t>(X[k].n1, 1024);
   }
-  std::vector<int32_t> pend(subset);
+  std::vector<int32_t> pend(subset), later;
   C.d_x.ensure(C, sizeof(XTask) * n);
   while (!pend.empty()) {
+    int64_t words = 0;
+    if (want_codes) {
+      // as many of the pending passes as the budget has room for: their slots, CIGARs, lists and wide bands' rows
+      const int64_t others = (int64_t)(C.used - C.d_tb.cap - C.d_cig.cap) + 16 * (int64_t)pend.size() + 4096;
+      const int64_t room = (int64_t)C.budget - others;
+      int64_t cig = 0, scratch = 0;
+      size_t m = 0;
+      for (; m < pend.size(); ++m) {
+        XTask &T = X[pend[m]];
+        const int64_t slot = std::min<int64_t>(INT32_MAX / 4 * 4, xd_slot_words(T.w, rows_cap[pend[m]]));
+        const int64_t c = (int64_t)std::max(T.n1, 0) + std::max(T.n2, 0) + 2;
+        const XScratch sc = xdrop_scratch(C, T.w, (int64_t)pend.size());
+        scratch = std::max(scratch, (int64_t)sizeof(int32_t) * sc.warps * sc.per_warp - (int64_t)C.d_scratch.cap);
+        if (m > 0 && 4 * (words + slot) + std::max<int64_t>(C.d_cig.cap, 4 * (cig + c)) + scratch > room) break;
+        T.tb_off = words;
+        T.tb_cap = (int32_t)slot;
+        words += slot;
+        cig += c;
+      }
+      later.assign(pend.begin() + m, pend.end());
+      pend.resize(m);
+    }
     // Only the pending passes travel: gathered into a compact pinned array, indexed 0..m-1 on the device.
     const int64_t m = (int64_t)pend.size();
-    int64_t words = 0;
-    if (want_codes)
-      for (int32_t k : pend) {
-        X[k].tb_off = words;
-        X[k].tb_cap = (int32_t)std::min<int64_t>(INT32_MAX / 4 * 4, xd_slot_words(X[k].w, rows_cap[k]));
-        words += X[k].tb_cap;
-      }
     if (want_codes) C.d_tb.ensure(C, sizeof(uint32_t) * std::max<int64_t>(words, 1));
     auto tp = phase(C, "xd_prep0", Clock::now());
     C.h_misc.ensure(sizeof(XTask) * m);
@@ -1564,6 +1579,8 @@ void run_xdrop_rounds(Context &C, std::vector<XTask> &X, const Params &P, bool w
       tp = phase(C, "xd_tb_host", tp);
     }
     pend.swap(next);
+    pend.insert(pend.end(), later.begin(), later.end());
+    later.clear();
   }
 }
 
@@ -1651,11 +1668,15 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
     C.d_x.ensure(C, sizeof(XTask) * n);
     C.d_idx.ensure(C, sizeof(int32_t) * (3 * n + 2 + 2 * nlev + 2 * kXdropOrderBins));
     C.d_counter.ensure(C, 64);
-    if (want_codes) {
-      C.d_tb.ensure(C, sizeof(uint32_t) * tb_words);
-      C.d_cig.ensure(C, sizeof(uint32_t) * 2 * cig_words);  // slots, then the packed CIGARs
-    }
     if (scratch_ints > 1) C.d_scratch.ensure(C, sizeof(int32_t) * scratch_ints);
+    if (want_codes) {
+      C.d_cig.ensure(C, sizeof(uint32_t) * 2 * cig_words);  // slots, then the packed CIGARs
+      // the arena as far as the budget goes: passes that find it full are retried in rounds of what fits
+      const size_t others = C.used - C.d_tb.cap;
+      const int64_t left = C.budget > others ? (int64_t)((C.budget - others) / sizeof(uint32_t)) : 0;
+      tb_words = std::min(tb_words, std::max<int64_t>(left / 4 * 4, 1 << 10));
+      C.d_tb.ensure(C, sizeof(uint32_t) * tb_words);
+    }
     int *lists = C.d_idx.as<int>();
     // counts, zeroed at once: of the retry list, of each level's work list (and what the last one leaves), the levels'
     // fetches, the order's classes
@@ -1895,7 +1916,8 @@ void run_semiglobal(Context &C, std::vector<SgTask> &G, const Params &P, bool wa
   if (cigars) cigars->assign(n, {});
   // device work split into batches whose direction-code stores fit a fraction of the budget
   const size_t free_budget = C.budget > C.used ? C.budget - C.used : 0;
-  const int64_t cap_bytes = std::max<int64_t>((int64_t)(free_budget / 2), (int64_t)64 << 20);
+  const int64_t cap_bytes =
+      std::max<int64_t>((int64_t)(free_budget / 2), std::min<int64_t>((int64_t)64 << 20, (int64_t)(free_budget / 4 * 3)));
   int64_t k0 = 0;
   C.d_sg.ensure(C, sizeof(SgTask) * n);
   // the stripe-flow form: per DP also its boundary row (DPs without a path) and flow state
