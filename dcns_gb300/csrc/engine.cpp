@@ -568,8 +568,12 @@ bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vecto
   const int64_t limit = 30000 / P.match - K - 256, want = (int64_t)C.nsm * 20 * 8;
   int64_t chunk = limit;
   if (tasks < want) chunk = std::min(limit, std::max<int64_t>(K, (rows + want - 1) / want));
-  std::vector<FiltPair> tab(np);
-  std::vector<int32_t> slot(np);
+  // the pairs' table, their counters (zero) and their places in the table, in one buffer and one copy
+  const size_t o_seen = sizeof(FiltPair) * np, o_slot = o_seen + sizeof(unsigned long long) * np;
+  const size_t tb = o_slot + sizeof(int32_t) * np;
+  std::vector<char> host(tb, 0);
+  FiltPair *const tab = reinterpret_cast<FiltPair *>(host.data());
+  int32_t *const slot = reinterpret_cast<int32_t *>(host.data() + o_slot);
   int64_t words = 0, duos = 0, task = 0, max_words = 1;
   for (int64_t q = 0; q < np; ++q) {
     const int64_t p = order[q];
@@ -594,7 +598,6 @@ bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vecto
   }
   if (task >= INT32_MAX / 2) return false;
   const int64_t cap = std::min<int64_t>(1 << 26, std::max<int64_t>(1 << 16, 4 * duos));
-  const size_t tb = (sizeof(FiltPair) + sizeof(unsigned long long) + sizeof(int32_t)) * np + 256;
   const size_t need = tb + sizeof(uint32_t) * words + sizeof(FiltTile) * cap;
   const size_t have = C.d_fpairs.cap + C.d_fwords.cap + C.d_ftiles.cap;
   if (need > have && C.used - have + 2 * need > C.budget) return false;
@@ -602,13 +605,11 @@ bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vecto
   C.d_fwords.ensure(C, sizeof(uint32_t) * words);
   C.d_ftiles.ensure(C, sizeof(FiltTile) * cap);
   if (!C.d_fpairs.cap || !C.d_fwords.cap || !C.d_ftiles.cap) return false;  // one made room for another
-  unsigned long long *const d_seen = reinterpret_cast<unsigned long long *>(C.d_fpairs.as<FiltPair>() + np);
-  int32_t *const d_slot = reinterpret_cast<int32_t *>(d_seen + np);
-  h2d(C, C.d_fpairs, tab.data(), (size_t)np);
-  DCNS_CK(cudaMemcpyAsync(d_slot, slot.data(), sizeof(int32_t) * np, cudaMemcpyHostToDevice, C.st));
-  DCNS_CK(cudaMemsetAsync(d_seen, 0, sizeof(unsigned long long) * np, C.st));
-  C.filt = FiltDesc{C.d_fpairs.as<FiltPair>(), d_slot, C.d_fwords.as<uint32_t>(), d_seen, (int32_t)np, (int32_t)task,
-                    (int32_t)chunk, K, (int32_t)max_words, 0};
+  char *const dev = C.d_fpairs.as<char>();
+  DCNS_CK(cudaMemcpyAsync(dev, host.data(), tb, cudaMemcpyHostToDevice, C.st));
+  C.filt = FiltDesc{reinterpret_cast<FiltPair *>(dev), reinterpret_cast<int32_t *>(dev + o_slot),
+                    C.d_fwords.as<uint32_t>(), reinterpret_cast<unsigned long long *>(dev + o_seen), (int32_t)np,
+                    (int32_t)task, (int32_t)chunk, K, (int32_t)max_words, 0};
   C.filt_on = true;
   return true;
 }

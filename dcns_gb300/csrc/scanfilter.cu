@@ -217,6 +217,7 @@ __global__ void __launch_bounds__(32 * kFWarps, 5)
                 5 * used * ((blk & 31) + 1);
       acc0 = acc1 = 0;
       if (lane == 0) atomicAdd(D.seen + slot, (1ull << 32) | (dense ? 1u : 0u));
+      if (blk == nblk - 1) break;
       if (filt_dense(seen)) {  // as it was a word ago: nothing waits for it
         for (int k = (blk >> 5) + 1; k < P.wpc; ++k, out += 64) out[0] = out[32] = ~0u;
         return;
