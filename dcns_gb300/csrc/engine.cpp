@@ -545,6 +545,19 @@ bool filter_ok(const Params &P) {
          30000 / P.match >= 4 * K + 512;
 }
 
+// Room for one of the filter's buffers; false, and none of them, where the device has no memory left (other contexts and
+// libraries may hold it): the call scans every window instead.
+bool filter_room(Context &C, DevBuf &b, size_t bytes) {
+  try {
+    b.ensure(C, bytes);
+  } catch (const Error &e) {
+    if (e.code != DCNS_ERR_NOMEM) throw;
+    drop_filter(C);
+    return false;
+  }
+  return true;
+}
+
 // Filter tasks of pairs in level-0 order (order, nduo per pair): the table, the marks' words, and the buffers.
 // False: not now (the buffers do not fit the budget), scan every window instead.
 bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vector<int64_t> &order,
@@ -601,9 +614,9 @@ bool filter_setup(Context &C, const std::vector<PairIn> &pairs, const std::vecto
   const size_t need = tb + sizeof(uint32_t) * words + sizeof(FiltTile) * cap;
   const size_t have = C.d_fpairs.cap + C.d_fwords.cap + C.d_ftiles.cap;
   if (need > have && C.used - have + 2 * need > C.budget) return false;
-  C.d_fpairs.ensure(C, tb);
-  C.d_fwords.ensure(C, sizeof(uint32_t) * words);
-  C.d_ftiles.ensure(C, sizeof(FiltTile) * cap);
+  if (!filter_room(C, C.d_fpairs, tb) || !filter_room(C, C.d_fwords, sizeof(uint32_t) * words) ||
+      !filter_room(C, C.d_ftiles, sizeof(FiltTile) * cap))
+    return false;
   if (!C.d_fpairs.cap || !C.d_fwords.cap || !C.d_ftiles.cap) return false;  // one made room for another
   char *const dev = C.d_fpairs.as<char>();
   DCNS_CK(cudaMemcpyAsync(dev, host.data(), tb, cudaMemcpyHostToDevice, C.st));
@@ -634,8 +647,7 @@ bool filter_grow(Context &C, const FiltTiles &T, const ScanCounts &n) {
   if (rows > T.most || n.tiles > INT32_MAX / 2) return false;
   const size_t bytes = sizeof(FiltTile) * (size_t)n.tiles;
   if (C.used - C.d_ftiles.cap + 2 * bytes > C.budget) return false;
-  C.d_ftiles.ensure(C, bytes);
-  return C.filt_on && C.d_ftiles.cap >= bytes;
+  return filter_room(C, C.d_ftiles, bytes) && C.filt_on && C.d_ftiles.cap >= bytes;
 }
 
 // A round's scan through the filter's marks (tasks [first, first + n) are on the device), then the reverse scans and
