@@ -169,6 +169,8 @@ int64_t predict_cells(int64_t n1, int64_t n2, const Params &P) {
   return n1 * (n2 / std::max(P.step, 1) + 1) * P.window;
 }
 
+constexpr int64_t kJoinCells = 100000000000;  // predicted cells from which on a lone request waits for others
+
 void worker_loop(std::shared_ptr<Server> Sp, Context *C) {
   Server *S = Sp.get();
   DCNS_CK(cudaSetDevice(C->device));
@@ -176,17 +178,15 @@ void worker_loop(std::shared_ptr<Server> Sp, Context *C) {
     std::vector<Server::Req> batch;
     {
       std::unique_lock<std::mutex> lk(S->mu);
-      const bool idle = S->running && S->queue.empty();
       S->cv_work.wait(lk, [&] { return !S->running || !S->queue.empty(); });
-      if (idle && S->running) {
-        // A worker that was idle gives the requests that come with the one that woke it a moment to arrive: a batch of
-        // a few small requests takes little longer than one (0.6 ms), and they would wait for it.
-        lk.unlock();
-        std::this_thread::sleep_for(std::chrono::microseconds(100));
-        lk.lock();
-        if (S->running && S->queue.empty()) continue;  // another worker took them
+      // A lone request starts at once.  One that will keep the worker for many times the wait (a seed scan of some 7 ms)
+      // gives those that come with it a moment to join: they would wait for all of it.
+      if (S->running && S->max_inflight > 1 && S->queue.size() == 1 && S->queue.front().cells >= kJoinCells)
+        S->cv_work.wait_for(lk, std::chrono::microseconds(100), [&] { return !S->running || S->queue.size() != 1; });
+      if (S->queue.empty()) {
+        if (!S->running) return;
+        continue;  // another worker took it
       }
-      if (!S->running && S->queue.empty()) return;
       // admission: arrival order, up to the in-flight limit, the worker's memory budget and the batch's scan cap
       int64_t bytes = 0, cells = 0;
       while (!S->queue.empty() && (int)batch.size() < S->max_inflight) {
