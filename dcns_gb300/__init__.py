@@ -151,11 +151,9 @@ class Tuning(C.Structure):
                 "scan_tiles_per_thread": self.scan_tiles_per_thread, "sg_warps": self.sg_warps,
                 "sg_flow": bool(self.sg_flow), "sg_flow_blocks": self.sg_flow_blocks,
                 "bins_by_size": bool(self.bins_by_size),
-                "xdrop_per_bin": [{"warp_from": self.xdrop_warp_from[b], "wave_max_w": self.xdrop_wave_max_w[b],
-                                   "row_interleaved": bool(self.xdrop_flat[b]),
-                                   "handoff_rows": self.xdrop_handoff[b],
-                                   "handoff_lanes": self.xdrop_resume_lanes[b],
-                                   "groups_from_band": self.xdrop_group_from[b],
+                # an x-drop pass has one form per band width: its former settings have no value (None)
+                "xdrop_per_bin": [{**dict.fromkeys(("warp_from", "wave_max_w", "row_interleaved", "handoff_rows",
+                                                    "handoff_lanes", "groups_from_band")),
                                    "scan_tiles": self.scan_tiles[b]} for b in range(n)]}
 
 
@@ -484,7 +482,7 @@ class Engine:
         return self.tuning()
 
     def tuning(self) -> dict:
-        """The context's kernel shapes: pipeline shape, scan tiling, 2-piece warps and the per-bin x-drop forms."""
+        """The context's kernel shapes: pipeline shape, scan tiling (per bin too) and the 2-piece kernel's form."""
         t = Tuning()
         self._check(self.lib.dcns_get_tuning(self.h, C.byref(t)))
         return t.as_dict()
