@@ -841,6 +841,7 @@ void compute_scan_tasks(Context &C, ScanState &S, const Params &P, int columns_f
       }
     }
   }
+  C.scanned_whole = true;
   std::vector<int32_t> fast, generic;  // device slots
   for (int64_t k = first; k < first + n; ++k) {
     ScanTask &T = S.task(k);
@@ -1069,6 +1070,7 @@ int64_t scan_level0(Context &C, ScanState &S, const std::vector<PairIn> &pairs, 
   DCNS_CK(cudaStreamWaitEvent(bulk, C.ev_bulk, 0));
   DCNS_CK(cudaEventRecord(C.ev0, bulk));
   auto scan_all = [&](cudaStream_t on) {
+    C.scanned_whole = true;
     launch_scan_l0(D, ntiles, C.arena, P, C.d_keys.as<unsigned long long>(), &d_counts->queue, grid, on);
   };
   auto scan_marked = [&](const FiltTiles &T, cudaStream_t on) {
@@ -2557,6 +2559,7 @@ void align_batch(Context &C, Batch &B, const Params &P, int mode, std::vector<st
   C.stats = dcns_stats{};
   out.assign(B.lens.size(), {});
   if (B.lens.empty()) return;
+  C.scanned_whole = false;
   C.arena = B.arena;
   C.seq_base = B.seq_base;
   C.seqbase_dev = B.sb.as<int64_t>();
@@ -2628,8 +2631,9 @@ void autotune(Context &C, Batch &B, const Params &P, int mode) {
     C.bin_tune.assign(std::max(C.bins, C.max_lanes), Context::BinTune{C.scan_tiles_per_thread});
   // the scan's tiling target (tiles per resident thread before reference rows are split into chunks; it matters
   // for batches of few long pairs) and, on the 2-gap path, the 2-piece kernel's warps per DP: by whole-call time
-  // (for the whole call, and per bin by that bin's seed-scan kernel time over the same runs)
-  {
+  // (for the whole call, and per bin by that bin's seed-scan kernel time over the same runs).  Where the filter cut
+  // every scan of the last trial there is no such tiling, and nothing to choose.
+  if (C.scanned_whole) {
     const int t0 = C.scan_tiles_per_thread;
     const int nb = (int)C.bin_tune.size();
     std::vector<double> bin_best(nb, 1e300);
@@ -2796,6 +2800,7 @@ void align_core(Context &C, const std::vector<PairIn> &pairs, const Params &P, i
         L.sg_flow_blocks = C.sg_flow_blocks;
         L.scan_tiles_per_thread = bt.scan_tiles;
         L.scan_filter = C.scan_filter;
+        if (b == l) L.scanned_whole = false;  // the lane's first bin
         L.call_t0 = C.call_t0;
         L.lane_id = l;
         L.trace = C.trace;
@@ -2825,7 +2830,10 @@ void align_core(Context &C, const std::vector<PairIn> &pairs, const Params &P, i
   for (int l = 0; l < nl; ++l) C.lanes[l]->l0_turn = nullptr;
   for (int l = 0; l < nl; ++l)
     if (codes[l]) throw Error(codes[l], errs[l]);
-  for (int l = 0; l < nl; ++l) add_stats(C.stats, st[l]);
+  for (int l = 0; l < nl; ++l) {
+    add_stats(C.stats, st[l]);
+    C.scanned_whole |= C.lanes[l]->scanned_whole;
+  }
   C.last_bin_scan_ms = std::move(bin_scan_ms);
 }
 

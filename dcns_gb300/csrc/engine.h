@@ -182,6 +182,7 @@ struct Context {
   DevBuf d_fpairs, d_fwords, d_ftiles;
   FiltDesc filt{};
   bool filt_on = false;
+  bool scanned_whole = false;  // some windows of the call went without the filter (where the tiling target matters)
   const WeightSet *weights = nullptr;  // set during a weighted call
   // pinned staging
   HostBuf h_codes, h_misc, h_out, h_tasks, h_tiles, h_x;

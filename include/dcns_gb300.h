@@ -177,8 +177,8 @@ int dcns_ctx_set_lanes(dcns_ctx *ctx, int lanes, int bins);
 
 /* Autotuner (no counterpart in the reference): aligns the resident batch once per candidate pipeline shape (lanes,
  * bins, and the geometric ratio of bin sizes), times each call, and keeps the fastest on the context; then, by
- * whole-call time, the seed scan's tiling target (and per bin, by that bin's scan time) and (2-gap mode) the 2-piece
- * kernel's form (dcns_get_tuning reports them).  The pipeline shape is returned (any pointer may be NULL).  Results do
+ * whole-call time, the seed scan's tiling target (and per bin, by that bin's scan time; only where some scan runs
+ * without the filter) and (2-gap mode) the 2-piece kernel's form (dcns_get_tuning reports them).  The pipeline shape is returned (any pointer may be NULL).  Results do
  * not depend on any of these; this only tunes throughput for batches like this. */
 int dcns_autotune(dcns_ctx *ctx, dcns_batch *batch, const dcns_params *params, int mode, int *lanes, int *bins,
                   double *bin_ratio);
