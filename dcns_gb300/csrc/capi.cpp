@@ -152,15 +152,19 @@ std::vector<PairIn> to_pairs(const dcns_pair *pairs, int64_t n) {
 }
 
 // Predicted device memory of one request: sequence arena and upload staging, level-0 scan keys and window records,
-// recursion tasks, and x-drop passes (one per eighth of the windows) with their traceback slots (3 x min(n1, 1024)
-// rows of 4-bit band codes) and CIGAR slots (n1 + n2 + 2 words, twice); in 2-gap mode one forward 2-piece DP's
-// direction codes (n1 rows of the band, bytes).  A heuristic for admission only: the engine checks the real sizes.
+// recursion tasks, the seed-scan filter's marks (a word of 32 blocks of 16 rows for each of the 64 strips of a warp,
+// 58 of them new) and tiles (four to two windows), and x-drop passes (one per eighth of the windows) with their
+// traceback slots (four of min(n1, 1024) rows) and CIGAR slots (n1 + n2 + 2 words, twice); in 2-gap mode one 2-piece DP's
+// checkpoints and boundary row.  A heuristic for admission only: the engine checks the real sizes.
 int64_t predict_bytes(int64_t n1, int64_t n2, const Params &P, int mode) {
   const int64_t windows = n2 / std::max(P.step, 1) + 2;
   const int64_t passes = windows / 8 + 1;
-  const int64_t wpr = (2 * (int64_t)P.w + 1 + 7) / 8;
-  int64_t b = 2 * (n1 + n2) + 96 * windows + passes * (3 * std::min<int64_t>(n1, 1024) * wpr * 4 + 8 * (n1 + n2 + 2));
-  if (mode == DCNS_MODE_TWO_GAP) b += n1 * std::min<int64_t>(n2, 2 * (int64_t)P.bandwidth + 160);
+  const int64_t marks = (n2 / (kFiltCols * 2 * (32 - kFiltOverlap)) + 1) * (n1 / 512 + 2) * 64 * 4;
+  int64_t b = 2 * (n1 + n2) + 96 * windows + marks + 32 * windows +
+              passes * (4 * 4 * xd_slot_words(P.w, std::min<int64_t>(n1, 1024)) + 8 * (n1 + n2 + 2));
+  if (mode == DCNS_MODE_TWO_GAP)
+    b += sg_ck_row_bytes((int)n1, (int)n2, P.bandwidth) + sg_ck_col_bytes((int)n1, (int)n2, P.bandwidth) +
+         (int64_t)sizeof(SgCell) * (n2 + 2);
   return b + 4096;
 }
 

@@ -54,3 +54,26 @@ def test_long_request_and_company(lib):
     assert alone == want[0] and len(alone) > 0
     for k, m in enumerate(mixed):
         assert m == want[k], k
+
+
+def test_two_gap_requests_share_a_batch(lib):
+    """Admission by predicted bytes: a 2-piece DP keeps checkpoints of 28 bytes per 128 cells, not a byte a cell, so
+    requests of 4 kb (16 MB of cells, 11 MB predicted in all, 21 with a byte a cell) share a batch of 100 MB by more than five."""
+    rng = np.random.default_rng(4)
+    x, y = W.planted_pair(rng, 60000, 60000, 60, 60, 300, 0.8, 0.95, 0.01, 0.0)
+    first = (W.prepare(x), W.prepare(y))
+    reqs = []
+    for _ in range(24):
+        a, b = W.planted_pair(rng, 4000, 4000, 3, 40, 120, 0.85, 0.97, 0.01, 0.0)
+        reqs.append((W.prepare(a), W.prepare(b)))
+    lib.serve_start(2, max_inflight=64, workers=1, batch_cells=10 ** 15, admit_bytes=100 << 20)
+    try:
+        tickets = [lib.submit(a, b) for a, b in [first] + reqs]  # the first keeps the worker while the others queue
+        got = [lib.wait(t) for t in tickets]
+        st = lib.serve_stats()
+    finally:
+        lib.serve_stop()
+    assert st["max_batch"] > 5, st
+    want = lib.align_pairs([first] + reqs, 2)
+    for k, g in enumerate(got):
+        assert g == want[k], k
