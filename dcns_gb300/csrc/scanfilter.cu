@@ -35,6 +35,7 @@
 // short is made again.  A pair of 200 kb that holds a 17-base word every 27, 60, 120 bases and no seed: 31.5, 32.5,
 // 31.7 ms without the filter, 37.9, 38.0, 39.8 with the list's capacity as the only test, 32.1, 32.0, 11.9 now; of
 // 40 and 2 kb 0.31 -> 0.71 -> 0.47, 0.47, 0.33.  The watch over the marks costs the filter 1.4 %.
+#include <algorithm>
 #include <type_traits>
 
 #include "device_common.cuh"
@@ -295,56 +296,78 @@ struct FiltEmit {
   }
 };
 
-// The same from a warp's runs: every lane holds one, and 32 of them go out at a time, with one addition to the counters
-// and each run's tiles written by all lanes.
+// The same from a warp's runs: every lane holds one, and 32 of them go out at a time, each run's tiles written by all
+// lanes.  What a warp holds at its end goes out with the other warps' of the block, by one addition to each counter:
+// additions to one place are served one after the other, and two for each of some 25,000 warps took 50 us where the
+// block's take 12.
+constexpr int kPlanThreads = 256;
 struct FiltEmitWarp {
   const FiltTiles &T;
   int a, b, warm, held = 0;
   int rb = 0, re = 0;  // the lane's run
-  unsigned long long rows = 0;
   __device__ __forceinline__ void operator()(int from, int to) {
     if ((int)(threadIdx.x & 31) == held) rb = from, re = to;
-    if (++held == 32) flush();
+    if (++held < 32) return;
+    int n, per, end;
+    const unsigned rows = tally(n, per, end);
+    unsigned long long at = 0;
+    if ((threadIdx.x & 31) == 31)
+      at = atomicAdd(T.count, (unsigned long long)end), atomicAdd(T.count + 1, (unsigned long long)rows);
+    write(__shfl_sync(0xFFFFFFFFu, at, 31), n, per, end);
+    held = 0;
   }
-  __device__ __forceinline__ void flush() {
+  // Of the lane's run: its tiles and their rows; of the runs up to the lane's: their tiles.  The warp's rows.
+  __device__ __forceinline__ unsigned tally(int &n, int &per, int &end) const {
     const int lane = threadIdx.x & 31;
-    const int n = lane < held ? (re - rb + T.rows - 1) / T.rows : 0, per = n > 0 ? (re - rb + n - 1) / n : 0;
-    if (n > 0) rows += (unsigned long long)(re - rb) + (unsigned long long)n * warm;
-    int end = n;
+    n = lane < held ? (re - rb + T.rows - 1) / T.rows : 0;
+    per = n > 0 ? (re - rb + n - 1) / n : 0;
+    end = n;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const int v = __shfl_up_sync(0xFFFFFFFFu, end, d);
       if (lane >= d) end += v;
     }
-    unsigned long long at = 0;
-    if (lane == 31) at = atomicAdd(T.count, (unsigned long long)end);
-    at = __shfl_sync(0xFFFFFFFFu, at, 31);
+    return __reduce_add_sync(0xFFFFFFFFu, n > 0 ? (unsigned)(re - rb + n * warm) : 0u);
+  }
+  __device__ __forceinline__ void write(unsigned long long at, int n, int per, int end) const {
     for (int r = 0; r < held; ++r) {
       const int rn = __shfl_sync(0xFFFFFFFFu, n, r), rper = __shfl_sync(0xFFFFFFFFu, per, r);
       const int from = __shfl_sync(0xFFFFFFFFu, rb, r), to = __shfl_sync(0xFFFFFFFFu, re, r);
       const int first = __shfl_sync(0xFFFFFFFFu, end, r) - rn;
-      for (int k = lane; k < rn; k += 32) {
+      for (int k = threadIdx.x & 31; k < rn; k += 32) {
         const int p = filt_place(at, first + k, T.cap);
         if (p < 0) break;
         T.list[p] = FiltTile{a, b, from + k * rper, min(to, from + (k + 1) * rper)};
       }
     }
-    held = 0;
   }
-  __device__ __forceinline__ void finish() {
-    if (held > 0) flush();
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) rows += __shfl_down_sync(0xFFFFFFFFu, rows, d);
-    if ((threadIdx.x & 31) == 0 && rows) atomicAdd(T.count + 1, rows);
+  __device__ __forceinline__ void finish() const {  // every warp of the block
+    constexpr int W = kPlanThreads / 32;
+    __shared__ int tiles[W];
+    __shared__ unsigned rows[W];
+    __shared__ unsigned long long base;
+    const int w = threadIdx.x >> 5;
+    int n, per, end;
+    const unsigned r = tally(n, per, end);
+    if ((threadIdx.x & 31) == 31) tiles[w] = end, rows[w] = r;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned long long t = 0, s = 0;
+      for (int k = 0; k < W; ++k) t += (unsigned)tiles[k], s += rows[k];
+      if (t) base = atomicAdd(T.count, t), atomicAdd(T.count + 1, s);
+    }
+    __syncthreads();
+    if (held == 0) return;
+    unsigned long long at = base;
+    for (int k = 0; k < w; ++k) at += (unsigned)tiles[k];
+    write(at, n, per, end);
   }
 };
 
-// The runs of words [kPlanWords seg, kPlanWords (seg + 1)) of the rows' words by a whole warp: the lanes load 32 words
-// at a time, and the runs of the words that hold marks are followed in order by all lanes together.  A run that goes on
-// in the next segment is two.
-constexpr int kPlanWords = 128;
+// The runs of part `part` of `parts` of the rows' words by a whole warp: the lanes load 32 words at a time, and the runs
+// of the words that hold marks are followed in order by all lanes together.  A run that goes on in the next part is two.
 __device__ __forceinline__ void filt_runs_warp(const FiltDesc &D, const FiltPair &P, int c_lo, int c_hi, int lo, int hi,
-                                               int seg, FiltEmitWarp &emit) {
+                                               int part, int parts, FiltEmitWarp &emit) {
   const int lane = threadIdx.x & 31;
   const int k0 = c_lo / kFC, k1 = (c_hi - 1) / kFC;
   int lmin = 31, lmax = 0;
@@ -353,10 +376,11 @@ __device__ __forceinline__ void filt_runs_warp(const FiltDesc &D, const FiltPair
     lmin = min(lmin, l), lmax = max(lmax, l);
   }
   const int ch0 = lo / D.chunk, items = ((hi - 1) / D.chunk - ch0 + 1) * P.wpc;
-  const int end = (int)min((int64_t)items, (int64_t)(seg + 1) * kPlanWords);
+  const int per = ((items + parts - 1) / parts + 31) / 32 * 32;  // words of a part
+  const int end = (int)min((int64_t)items, (int64_t)(part + 1) * per);
   int cs = -1, ce = -1;
-  for (int base = seg * kPlanWords; base < end; base += 32) {
-    const int it = base + lane;
+  for (int64_t base = (int64_t)part * per; base < end; base += 32) {
+    const int it = (int)base + lane;
     uint32_t v = 0;
     int row = 0, rlo = 0, rhi = 0;
     if (it < end) {
@@ -397,55 +421,61 @@ __device__ __forceinline__ void filt_runs_warp(const FiltDesc &D, const FiltPair
 }
 
 // Plans: one thread, or WARP one warp, per item.  A thread waits for each word before it looks at the next, so a plan
-// of few items is as long as its longest reference has words; with a warp to each item and segment of it
-// (blockIdx.y) the words come 32 at a time.  Up to 256 items per multiprocessor: one pair of 5 kb (312 and 350 items)
+// of few items is as long as its longest reference has words; with a warp to each item, or to each part of it
+// (blockIdx.y) where the items are so few that they leave multiprocessors idle, the words come 32 at a time.  Up to 256 items per multiprocessor: one pair of 5 kb (312 and 350 items)
 // 66 -> 7 and 60 -> 7 us, two pairs of 200 kb 385 -> 140 and 472 -> 94 us.  The plans of 10,000 pairs have some 100,000
 // items each, of a few words, and keep their threads.
 constexpr int kPlanWarpItems = 256;
 
 // Level-0 tiles: an item per two windows of a pair (slot of the level-0 table, duo).
 template <bool WARP>
-__global__ void __launch_bounds__(256) filter_plan_l0_kernel(FiltDesc D, L0Desc L, int64_t nduo, FiltTiles T) {
+__global__ void __launch_bounds__(kPlanThreads, WARP ? 5 : 6)
+    filter_plan_l0_kernel(FiltDesc D, L0Desc L, int64_t nduo, FiltTiles T) {
   const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / (WARP ? 32 : 1);
-  if (t >= nduo) return;
-  int lo = 0, hi = D.npairs - 1;
-  while (lo < hi) {  // the pair whose duos hold t
-    const int mid = (lo + hi + 1) >> 1;
-    if (D.pairs[mid].duo_begin <= t)
-      lo = mid;
-    else
-      hi = mid - 1;
+  int slot = 0, duo = 0, c_lo = 0, c_hi = 0;
+  if (t < nduo) {
+    int hi = D.npairs - 1;
+    while (slot < hi) {  // the pair whose duos hold t
+      const int mid = (slot + hi + 1) >> 1;
+      if (D.pairs[mid].duo_begin <= t)
+        slot = mid;
+      else
+        hi = mid - 1;
+    }
+    duo = (int)(t - D.pairs[slot].duo_begin);
+    c_lo = 2 * duo * L.step;
+    c_hi = min(D.pairs[slot].n2, min(2 * duo + 1, L.pairs[slot].nfast - 1) * L.step + L.window);
   }
-  const FiltPair P = D.pairs[lo];
-  const int duo = (int)(t - P.duo_begin), last = min(2 * duo + 1, L.pairs[lo].nfast - 1);
-  const int c_lo = 2 * duo * L.step, c_hi = min(P.n2, last * L.step + L.window);
   if constexpr (WARP) {
-    FiltEmitWarp emit{T, lo, duo, D.warm};
-    filt_runs_warp(D, P, c_lo, c_hi, 0, P.n1, (int)blockIdx.y, emit);
+    FiltEmitWarp emit{T, slot, duo, D.warm};
+    if (t < nduo) {
+      const FiltPair P = D.pairs[slot];
+      filt_runs_warp(D, P, c_lo, c_hi, 0, P.n1, (int)blockIdx.y, (int)gridDim.y, emit);
+    }
     emit.finish();
-  } else {
-    FiltEmit emit{T, lo, duo};
+  } else if (t < nduo) {
+    FiltEmit emit{T, slot, duo};
+    const FiltPair P = D.pairs[slot];
     filt_runs(D, P, c_lo, c_hi, 0, P.n1, emit);
   }
 }
 
 // Tiles of a round's tasks: an item per task.
 template <bool WARP>
-__global__ void __launch_bounds__(256) filter_plan_rec_kernel(FiltDesc D, const ScanTask *__restrict__ tasks,
-                                                              int first, int n, FiltTiles T) {
+__global__ void __launch_bounds__(kPlanThreads, WARP ? 5 : 6)
+    filter_plan_rec_kernel(FiltDesc D, const ScanTask *__restrict__ tasks, int first, int n, FiltTiles T) {
   const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / (WARP ? 32 : 1);
-  if (t >= n) return;
-  const int k = (int)t;
-  const ScanTask x = tasks[first + k];
-  if (x.tw <= 0 || x.hi <= x.lo) return;
-  const FiltPair P = D.pairs[D.slot[x.pair]];
+  ScanTask x{};
+  if (t < n) x = tasks[first + (int)t];
+  const bool on = x.tw > 0 && x.hi > x.lo;
   if constexpr (WARP) {
-    FiltEmitWarp emit{T, first + k, 0, D.warm};
-    filt_runs_warp(D, P, x.s2, x.s2 + x.tw, x.lo, x.hi, (int)blockIdx.y, emit);
+    FiltEmitWarp emit{T, first + (int)t, 0, D.warm};
+    if (on)
+      filt_runs_warp(D, D.pairs[D.slot[x.pair]], x.s2, x.s2 + x.tw, x.lo, x.hi, (int)blockIdx.y, (int)gridDim.y, emit);
     emit.finish();
-  } else {
-    FiltEmit emit{T, first + k, 0};
-    filt_runs(D, P, x.s2, x.s2 + x.tw, x.lo, x.hi, emit);
+  } else if (on) {
+    FiltEmit emit{T, first + (int)t, 0};
+    filt_runs(D, D.pairs[D.slot[x.pair]], x.s2, x.s2 + x.tw, x.lo, x.hi, emit);
   }
 }
 
@@ -457,11 +487,16 @@ void launch_filter(const FiltDesc &D, Arena ar, Params p, int thr, cudaStream_t 
                                                                             p.mismatch, thr, p.match * p.window);
 }
 
+// Parts of an item: of 128 words and more, while their warps all fit (32 to a multiprocessor).
+unsigned plan_parts(const FiltDesc &D, int64_t items, int nsm) {
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>((D.max_words + 127) / 128, 32 * nsm / items));
+}
+
 void launch_filter_plan_l0(const FiltDesc &D, L0Desc L, int64_t nduo, FiltTiles T, int nsm, cudaStream_t st) {
   if (nduo <= 0) return;
-  const unsigned segs = (unsigned)((D.max_words + kPlanWords - 1) / kPlanWords);
   if (nduo <= (int64_t)kPlanWarpItems * nsm)
-    filter_plan_l0_kernel<true><<<dim3((unsigned)((nduo + 7) / 8), segs), 256, 0, st>>>(D, L, nduo, T);
+    filter_plan_l0_kernel<true>
+        <<<dim3((unsigned)((nduo + 7) / 8), plan_parts(D, nduo, nsm)), kPlanThreads, 0, st>>>(D, L, nduo, T);
   else
     filter_plan_l0_kernel<false><<<(unsigned)((nduo + 255) / 256), 256, 0, st>>>(D, L, nduo, T);
 }
@@ -469,9 +504,9 @@ void launch_filter_plan_l0(const FiltDesc &D, L0Desc L, int64_t nduo, FiltTiles 
 void launch_filter_plan_rec(const FiltDesc &D, const ScanTask *tasks, int first, int n, FiltTiles T, int nsm,
                             cudaStream_t st) {
   if (n <= 0) return;
-  const unsigned segs = (unsigned)((D.max_words + kPlanWords - 1) / kPlanWords);
   if (n <= kPlanWarpItems * nsm)
-    filter_plan_rec_kernel<true><<<dim3((unsigned)((n + 7) / 8), segs), 256, 0, st>>>(D, tasks, first, n, T);
+    filter_plan_rec_kernel<true>
+        <<<dim3((unsigned)((n + 7) / 8), plan_parts(D, n, nsm)), kPlanThreads, 0, st>>>(D, tasks, first, n, T);
   else
     filter_plan_rec_kernel<false><<<(n + 255) / 256, 256, 0, st>>>(D, tasks, first, n, T);
 }
