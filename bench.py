@@ -531,6 +531,14 @@ def main():
                 "scan_share_of_single_lane_step": round(scan_ms / single_ms, 4),
                 "single_lane_ms_per_step": round(single_ms / 2, 2),
                 "timing": "CUDA events around each scan launch, two single-lane steps after the timed region"}
+    sm_mhz = clk.summary().get("sm_mhz")
+    if sm_mhz and scan_ms > 0:
+        # what the stage cannot do without (the filter's three ALU operations per two cells of every pair, once) at the
+        # ALU pipes' rate: how busy the machine is with needed work, which `frac` above does not say
+        alu = torch.cuda.get_device_properties(local).multi_processor_count * 64 * sm_mhz * 1e6
+        floor_ms = 1.5 * sum(len(a) * len(b) for a, b in pairs) / alu * 1e3
+        roofline["alu_floor_ms_per_step"] = round(floor_ms, 3)
+        roofline["alu_floor_frac"] = round(floor_ms / (scan_ms / 2), 4)
 
     extras = {}
     if not args.no_extras:

@@ -276,8 +276,8 @@ void launch_semiglobal(SgTask *tasks, const int *idx, int n, Arena ar, Params p,
                        int max_n2, int *work_counter, int grid, int nw, cudaStream_t st);
 int sg_ctas_per_sm(int nw);
 // wt: the weighted DPs (null: the unweighted).  path: the DPs keep traceback checkpoints in tb (row checkpoints, zero
-// before the launch, and column checkpoints, at 16-byte offsets; every DP of a launch alike).  minb: 4, 5 or 6
-// resident blocks per SM (the register budget of the unweighted kernel's instantiation).
+// before the launch, and column checkpoints, at 16-byte offsets; every DP of a launch alike).  blocks_per_sm: 1 or 2
+// blocks of the persistent grid.
 void launch_semiglobal_flow(const SgFlow &f, Arena ar, Params p, const SgWeights *wt, uint8_t *tb, bool path, int nsm,
                             int blocks_per_sm, cudaStream_t st);
 int64_t sg_flow_units(int n1, int n2, int w);  // stripe units of one DP in the flow form (at least 1)

@@ -1767,7 +1767,9 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
       return lev + 1;
     });
     tp = phase(C, "xc_cigars", tp);
-    if (C.trace) std::fprintf(stderr, "[dcns trace] x-drop chain: %lld passes, %d levels, %zu retries\n", (long long)n, nlev, retry.size());
+    if (C.trace)
+      std::fprintf(stderr, "[dcns trace] x-drop chain: %lld passes, %d levels, %zu retries\n", (long long)n, nlev,
+                   retry.size());
     run_xdrop_rounds(C, X, P, want_codes, flat, hoff, retry, true);
     tp = phase(C, "xc_retry", tp);
   }
@@ -1941,8 +1943,9 @@ void run_semiglobal(Context &C, std::vector<SgTask> &G, const Params &P, bool wa
     return sg_ck_row_bytes(g.n1, g.n2, P.bandwidth) + sg_ck_col_bytes(g.n1, g.n2, P.bandwidth);
   };
   auto flow_bytes = [&](const SgTask &g) -> int64_t {
-    return flow ? (want_codes ? 0 : (int64_t)sizeof(SgCell) * (std::max(g.n2, 0) + 2)) + (int64_t)sizeof(SgFlowDP) + 8 * sg_flow_units(g.n1, g.n2, P.bandwidth)
-                : 0;
+    if (!flow) return 0;
+    const int64_t row = want_codes ? 0 : (int64_t)sizeof(SgCell) * (std::max(g.n2, 0) + 2);
+    return row + (int64_t)sizeof(SgFlowDP) + 8 * sg_flow_units(g.n1, g.n2, P.bandwidth);
   };
   while (k0 < n) {
     int64_t bytes = 0, rows = 0, extra = 0, k1 = k0;  // rows: of the bytes, the flow form's row checkpoints
@@ -1965,8 +1968,9 @@ void run_semiglobal(Context &C, std::vector<SgTask> &G, const Params &P, bool wa
       }
     const int64_t m = k1 - k0;
     if (want_codes) C.d_sgtb.ensure(C, (size_t)std::max<int64_t>(bytes, 1));
-    // the stripe flow (or, with sg_flow off, one CTA per unweighted DP).  CTA shape of the CTA kernel: many DPs run two warps each (short DPs stop within a few stripes, and
-    // more of them run at once); few DPs keep eight warps each for the stripes of long DPs
+    // the stripe flow (or, with sg_flow off, one CTA per unweighted DP).  CTA shape of the CTA kernel: many DPs run two
+    // warps each (short DPs stop within a few stripes, and more of them run at once); few DPs keep eight warps each for
+    // the stripes of long DPs
     const int nw = C.sg_warps > 0 ? C.sg_warps : (m >= (int64_t)C.nsm * 8 ? 2 : kSgNW);
     const int grid = (int)std::min<int64_t>(m, (int64_t)C.nsm * sg_ctas_per_sm(nw));
     int maxn2 = 1;
@@ -2731,7 +2735,8 @@ void align_core(Context &C, const std::vector<PairIn> &pairs, const Params &P, i
   //  * by size: consecutive runs of pairs in increasing work, so the last bin holds the largest pairs.  The host and
   //    x-drop work after a bin's scan grows with its number of pairs (seeds per pair do not grow with pair length),
   //    so the bin whose tail is on the critical path then has the fewest pairs; its shares grow bin to bin
-  //    (bin_ratio > 1: on the 10,000-pair workload 1.6 measured 146.6 ms per step against 184.5 at 0.6).
+  //    (bin_ratio > 1: on the 10,000-pair workload 37.1 ms per step at 1.6, 40.3 at 2.5, 43.6 at 1.0 and 53.8 at 0.6,
+  //    against 40.2 of the mixed bins).
   std::vector<double> target(kBins);
   {
     double tot = 0, wsum = 0, f = 1;

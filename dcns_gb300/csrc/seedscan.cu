@@ -211,9 +211,9 @@ constexpr int kProfSyms = 4;                   // reference symbols A, C, G, T (
 constexpr size_t kProfBytes = sizeof(uint4) * kProfSyms * kProfGroups * kScanThreads;
 
 template <int W, int MODE>
-__global__ void __launch_bounds__(kScanThreads) scan_kernel(RecDesc rec, L0Desc l0, FiltTiles ft, int floor, int64_t ntiles,
-                                                   Arena ar, int open, int ext, int match, int mismatch,
-                                                   unsigned long long *__restrict__ keys, int *__restrict__ counter) {
+__global__ void __launch_bounds__(kScanThreads)
+    scan_kernel(RecDesc rec, L0Desc l0, FiltTiles ft, int floor, int64_t ntiles, Arena ar, int open, int ext, int match,
+                int mismatch, unsigned long long *__restrict__ keys, int *__restrict__ counter) {
   // Score table per reference symbol (index = 2-bit code | N << 2): bytes 0..4 = s(ref, read code 0..4) - open,
   // byte 5 = 0xC0 and byte 6 = 0x00, which the padding selector (6, 5) turns into the lane value -16384.
   __shared__ uint32_t tab[16];
@@ -481,20 +481,20 @@ void launch_scan(RecDesc d, int64_t ntiles, bool columns, Arena ar, Params p, un
 void launch_scan_l0(L0Desc d, int64_t ntiles, Arena ar, Params p, unsigned long long *keys, int *work_counter,
                     int64_t grid, cudaStream_t st) {
   if (ntiles <= 0) return;
-  scan_kernel<kScanW, 1><<<(unsigned)grid, kScanThreads, kProfBytes, st>>>(RecDesc{}, d, FiltTiles{}, 0, ntiles, ar, p.open1, p.ext1, p.match,
-                                                                 p.mismatch, keys, work_counter);
+  scan_kernel<kScanW, 1><<<(unsigned)grid, kScanThreads, kProfBytes, st>>>(
+      RecDesc{}, d, FiltTiles{}, 0, ntiles, ar, p.open1, p.ext1, p.match, p.mismatch, keys, work_counter);
 }
 
 void launch_scan_tiles_l0(L0Desc d, FiltTiles T, Arena ar, Params p, unsigned long long *keys, int *work_counter,
                           int grid, cudaStream_t st) {
-  scan_kernel<kScanW, 3><<<grid, kScanThreads, kProfBytes, st>>>(RecDesc{}, d, T, p.min_score - 1, 0, ar, p.open1, p.ext1, p.match,
-                                                                 p.mismatch, keys, work_counter);
+  scan_kernel<kScanW, 3><<<grid, kScanThreads, kProfBytes, st>>>(
+      RecDesc{}, d, T, p.min_score - 1, 0, ar, p.open1, p.ext1, p.match, p.mismatch, keys, work_counter);
 }
 
 void launch_scan_tiles_rec(RecDesc d, FiltTiles T, Arena ar, Params p, unsigned long long *keys, int *work_counter,
                            int grid, cudaStream_t st) {
-  scan_kernel<kScanW, 4><<<grid, kScanThreads, kProfBytes, st>>>(d, L0Desc{}, T, p.min_score - 1, 0, ar, p.open1, p.ext1, p.match,
-                                                                 p.mismatch, keys, work_counter);
+  scan_kernel<kScanW, 4><<<grid, kScanThreads, kProfBytes, st>>>(
+      d, L0Desc{}, T, p.min_score - 1, 0, ar, p.open1, p.ext1, p.match, p.mismatch, keys, work_counter);
 }
 
 // ------------------------------------------------------------------ generic int32 Smith-Waterman (one thread)

@@ -753,8 +753,9 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, kSgFlowBlocks) sg_flow_kern
           last = j == c1;
         }
         int cF1, cF2;
-        const int cM = sg_cell<false, KIND, EDGE != kSgAny>(sg_row_score<KIND>(prof[k], rp[k], sel), dg, aF1, aF2, e1[k], e2[k],
-                                                valid, last, rp[k], P, cF1, cF2, nullptr);
+        const int cM =
+            sg_cell<false, KIND, EDGE != kSgAny>(sg_row_score<KIND>(prof[k], rp[k], sel), dg, aF1, aF2, e1[k], e2[k],
+                                                 valid, last, rp[k], P, cF1, cF2, nullptr);
         if constexpr (EDGE == kSgRight && KIND == 0) {
           cF1 = end ? kOut : cF1;
           cF2 = end ? kOut : cF2;
@@ -763,8 +764,8 @@ __global__ void __launch_bounds__(32 * kSgFlowWarps, kSgFlowBlocks) sg_flow_kern
           e1[k] = valid ? e1[k] : kOut;
           if (KIND != 1) e2[k] = valid ? e2[k] : kOut;
         }
-        bool keep;
-        best[k] = __vibmax_s32(best[k], (EDGE == kSgLeft || EDGE == kSgRight) && !valid ? kOut : cM, &keep);  // keep: !(cM > best), the first maximum of the row stays
+        bool keep;  // !(cM > best): the first maximum of the row stays
+        best[k] = __vibmax_s32(best[k], (EDGE == kSgLeft || EDGE == kSgRight) && !valid ? kOut : cM, &keep);
         bestj[k] = keep ? bestj[k] : j;
         if (stale_col && valid) {
           if ((stale_rows >> k) & 1) D.stale_last = cM;

@@ -354,9 +354,7 @@ __global__ void __launch_bounds__(128) xdrop_band_kernel(XLevelArgs A, Arena ar,
             st = 2;
           } else {
             rows = i;
-            const int rb = WIDE ? b : b >> 10;
-            const int k = (WIDE ? bk : KL - 1 - (b & 1023)) - pads;
-            const int j = rb > 0 ? i - w + k : -1;
+            const int rb = b, k = bk - pads, j = rb > 0 ? i - w + k : -1;
             if (rb > 0 && j != n2 && j != 1 && (k == 0 || k == 2 * w)) {
               st = 1;
             } else {
