@@ -1459,7 +1459,8 @@ void run_xdrop_rounds(Context &C, std::vector<XTask> &X, const Params &P, bool w
   while (!pend.empty()) {
     int64_t words = 0;
     if (want_codes) {
-      // as many of the pending passes as the budget has room for: their slots, CIGARs, lists and wide bands' rows
+      // as many of the pending passes as the budget has room for: their slots (half of it, the later stages need some
+      // too), CIGARs, lists and wide bands' rows
       const int64_t others = (int64_t)(C.used - C.d_tb.cap - C.d_cig.cap) + 16 * (int64_t)pend.size() + 4096;
       const int64_t room = (int64_t)C.budget - others;
       int64_t cig = 0, scratch = 0;
@@ -1470,7 +1471,10 @@ void run_xdrop_rounds(Context &C, std::vector<XTask> &X, const Params &P, bool w
         const int64_t c = (int64_t)std::max(T.n1, 0) + std::max(T.n2, 0) + 2;
         const XScratch sc = xdrop_scratch(C, T.w, (int64_t)pend.size());
         scratch = std::max(scratch, (int64_t)sizeof(int32_t) * sc.warps * sc.per_warp - (int64_t)C.d_scratch.cap);
-        if (m > 0 && 4 * (words + slot) + std::max<int64_t>(C.d_cig.cap, 4 * (cig + c)) + scratch > room) break;
+        const int64_t codes = 4 * (words + slot);
+        if (m > 0 && (codes > std::max<int64_t>(C.d_tb.cap, room / 2) ||
+                      codes + std::max<int64_t>(C.d_cig.cap, 4 * (cig + c)) + scratch > room))
+          break;
         T.tb_off = words;
         T.tb_cap = (int32_t)slot;
         words += slot;
@@ -1686,10 +1690,10 @@ void run_xdrop(Context &C, std::vector<XTask> &X, const Params &P, bool want_cod
     if (scratch_ints > 1) C.d_scratch.ensure(C, sizeof(int32_t) * scratch_ints);
     if (want_codes) {
       C.d_cig.ensure(C, sizeof(uint32_t) * 2 * cig_words);  // slots, then the packed CIGARs
-      // the arena as far as the budget goes: passes that find it full are retried in rounds of what fits
+      // the arena in half of what the budget leaves at most: passes that find it full are retried in rounds of what fits
       const size_t others = C.used - C.d_tb.cap;
       const int64_t left = C.budget > others ? (int64_t)((C.budget - others) / sizeof(uint32_t)) : 0;
-      tb_words = std::min(tb_words, std::max<int64_t>(left / 4 * 4, 1 << 10));
+      tb_words = std::min(tb_words, std::max<int64_t>(left / 8 * 4, 1 << 10));
       C.d_tb.ensure(C, sizeof(uint32_t) * tb_words);
     }
     int *lists = C.d_idx.as<int>();
