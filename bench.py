@@ -131,9 +131,9 @@ def workload(n_pairs, rank=0):
 
 
 # DRAM bytes per algorithmic cell of the level-0 launches (filter, then the rows it leaves): ncu, 3,000 pairs of this
-# workload, 7.93 + 9.87 MB read and 0 written for 161.25 G cells (profiles/filter_and_scan_3000pairs.md); traffic grows
+# workload, 7.97 + 9.79 MB read and 0 written for 161.25 G cells (profiles/filter_and_scan_3000pairs.md); traffic grows
 # with the cells.
-SCAN_DRAM_BYTES_PER_CELL = 17.79686e6 / 161254407231
+SCAN_DRAM_BYTES_PER_CELL = 17.757184e6 / 161254407231
 
 
 def level0_cells(pairs, window=38, step=8):

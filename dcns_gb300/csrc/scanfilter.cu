@@ -23,9 +23,9 @@
 // the two shuffles of a step cost 2 of its 70 instructions.
 //
 // Measured on the 10,000-pair batch (534 G cells over all windows, 112 G over the pairs; serialised launch times):
-// level 0 87 ms before, now 17.6 ms in the filter, 0.5 ms in its lists and 3.1 ms in the exact scan of the marked
-// rows; the recursion rounds, which reuse the marks, 12 ms before and 2.5 ms now.  Bound: integer issue (ALU pipe at
-// 80 %), as the exact scan.  The bound kept at match * window every 16 rows costs the filter 2 % and saves the exact
+// level 0 87 ms before, now 17.4 ms in the filter, 0.2 ms in its lists and 2.3 ms in the exact scan of the marked
+// rows; the recursion rounds, which reuse the marks, 12 ms before and 1.8 ms now.  Bound: integer issue (ALU pipe at
+// 78 %), as the exact scan.  The bound kept at match * window every 16 rows costs the filter 2 % and saves the exact
 // scans 28 % (10.1 to 7.3 ms before the floor above min_score in those).  Widths of 8 to 24 columns a lane, chosen per
 // pair to fit the query, would save 14 % of the columns but ran 1.5x slower mixed in one launch (instruction cache)
 // and no faster sorted by width.
